@@ -190,20 +190,31 @@ IEX_API int iex_spmm_f32_prefers_tc(int m, int k, int n, int nnz);
 IEX_API int iex_linear_f16(int tokens, int in_features, int out_features, const void* input,
                            const void* weight, void* out, void* stream);
 
-/* Backward pass of the dense branch on the same tensor-core kernel (operands read in their
- * other major-ness straight from the forward's tensors, no transposed copies).  Replace the two
- * cuBLAS calls of MyLinear.backward
- * (intrasm_engine/pytorch/cpp_extensions/layers_and_funcs/torch.py:20-31).
+/* The dense branch for any number of tokens, forward and backward, on the CTA-pair GEMM; operands
+ * are read in either major-ness straight from the forward's tensors (no transposed copies).
+ * Replace the cuBLAS calls of MyLinear
+ * (intrasm_engine/pytorch/cpp_extensions/layers_and_funcs/torch.py:17, :20-31).
+ *   any    out [tokens, out_features] = input [tokens, in_features] * weight^T; in_features a multiple of 8
  *   dgrad  dinput [tokens, in_features] = grad [tokens, out_features] * weight [out_features, in_features]
- *          tokens a multiple of 16 and <= 256; in_features, out_features multiples of 8.
  *   wgrad  dweight [out_features, in_features] = grad^T * input, input [tokens, in_features]
- *          any number of tokens that is a multiple of 8; in_features, out_features multiples of 8.
- * All row-major fp16, 16-byte aligned; fp32 accumulation. */
+ *          (dgrad, wgrad: in_features and out_features multiples of 8)
+ * All row-major fp16, operands 16-byte aligned; fp32 accumulation. */
+IEX_API int iex_linear_f16_any(int tokens, int in_features, int out_features, const void* input,
+                               const void* weight, void* out, void* stream);
 IEX_API int iex_linear_f16_dgrad(int tokens, int in_features, int out_features, const void* grad,
                                  const void* weight, void* dinput, void* stream);
 IEX_API int iex_linear_f16_wgrad(int tokens, int in_features, int out_features, const void* grad,
                                  const void* input, void* dweight, void* stream);
 
+/* Dense fp16 GEMM on CTA pairs: D[m, n] = sum_k A(m, k) * B(n, k), fp32 accumulation.
+ * a is stored [m, k] (a_mn = 0) or [k, m] (a_mn = 1), b [n, k] or [k, n], out [m, n] or, with
+ * out_transposed, [n, m]; lda, ldb, ldo are the elements between stored rows (multiples of 8 for the
+ * operands, whose bases are 16-byte aligned; a transposed output needs m and ldo multiples of 8).
+ * tile_n (0, or a multiple of 64 up to 256) and k_parts (0 to 4) override the choice of the tile
+ * width and of the number of CTA pairs that split k. */
+IEX_API int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long long lda, const void* b, int b_mn,
+                         long long ldb, void* out, int out_transposed, long long ldo, int tile_n, int k_parts,
+                         void* stream);
 /* CSR SpMM on tensor cores: out[r, :] = sum_p values[p] * dense[col[p], :].
  * Same contract as iex_spmm_f16_i16 / _i32 with batch = 1 and no bias (replaces
  * my_sputnik::CudaSpmm5, extensions.h:30), plus one precondition: column indices ascend

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 1) sddmm_tc_kernel(const Params prm)
     IEX_PROF_DUMP(threadIdx.x == 0, 0)
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // D fp32, A and B tf32, both K-major, N = 128, M = 128
       constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(TN >> 3) << 17) |
                                  (static_cast<uint32_t>(TM >> 4) << 24);

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const Params prm) 
     IEX_PROF_DUMP(threadIdx.x == 0, 0)
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // D fp32, A tf32 K-major, B tf32 MN-major, N = n, M = 128
       constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) |
                                  (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(TM >> 4) << 24);

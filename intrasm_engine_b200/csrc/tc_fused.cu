@@ -68,11 +68,6 @@ struct Params {
   __half* d_out_copies[kMaxPeers - 1];
   int d_num_copies;
   int d_b_mn;  // B operand of the dense branch is MN-major ([K, N]) instead of K-major ([N, K])
-  int d_a_mn;  // A operand of the dense branch is MN-major ([K, M]) instead of K-major ([M, K])
-  // Dense units over column blocks: with d_ncols > 0 the B operand is [K, d_ncols] (MN-major),
-  // a unit is (128-row tile, block of n columns), and d_parts = d_nblocks counts the blocks
-  // (no split-K).
-  int d_nblocks, d_ncols;
   // sparse branch: out[r * n + t]
   int s_tiles, s_m, s_nnz;
   int s_tile_rows;  // rows of a sparse tile (a multiple of 8, <= 128; rows above it stay zero)
@@ -115,7 +110,6 @@ __device__ int g_status = 0;  // last device-side failure (IEX_ERR_TIMEOUT) of t
 struct Unit {
   bool sparse;
   int tile, part, parts;
-  int nblock;  // column block of the B operand (dense units over column blocks), else 0
 };
 __device__ __forceinline__ Unit unit_of(int u, const Params& prm, int grid) {
   const int S = prm.s_tiles * prm.s_parts, D = prm.d_tiles * prm.d_parts;
@@ -129,12 +123,6 @@ __device__ __forceinline__ Unit unit_of(int u, const Params& prm, int grid) {
   un.parts = un.sparse ? prm.s_parts : prm.d_parts;
   un.tile = idx / un.parts;
   un.part = idx - un.tile * un.parts;
-  un.nblock = 0;
-  if (!un.sparse && prm.d_ncols > 0) {  // the "parts" of the list are column blocks
-    un.nblock = un.part;
-    un.part = 0;
-    un.parts = 1;
-  }
   return un;
 }
 
@@ -411,7 +399,7 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tma_a) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tma_b_dense) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tma_b_sparse) : "memory");
@@ -447,16 +435,11 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             const uint32_t a_dst = smem_base + s * stage_bytes;
             const uint32_t b_dst = a_dst + A_STAGE_BYTES;
             mbar_arrive_expect_tx(full_bar(s), b_stage_bytes + A_STAGE_BYTES);
-            if (prm.d_a_mn) {  // A [K, M]: two [128 k-rows x 64 cols] boxes
-              tma_load_2d(a_dst, &tma_a, full_bar(s), tile * BM, kb * BK);
-              tma_load_2d(a_dst + A_ATOM_BYTES, &tma_a, full_bar(s), tile * BM + 64, kb * BK);
-            } else {
-              tma_load_2d(a_dst, &tma_a, full_bar(s), kb * BK, tile * BM);
-              tma_load_2d(a_dst + A_ATOM_BYTES, &tma_a, full_bar(s), kb * BK + 64, tile * BM);
-            }
+            tma_load_2d(a_dst, &tma_a, full_bar(s), kb * BK, tile * BM);
+            tma_load_2d(a_dst + A_ATOM_BYTES, &tma_a, full_bar(s), kb * BK + 64, tile * BM);
             if (b_mn) {  // X [K, N]: one [128 k-rows x 64 cols] box per 64 columns
               for (int j = 0; j < n / 64; ++j)
-                tma_load_2d(b_dst + j * (BK * 128), &tma_b_dense, full_bar(s), un.nblock * n + j * 64, kb * BK);
+                tma_load_2d(b_dst + j * (BK * 128), &tma_b_dense, full_bar(s), j * 64, kb * BK);
             } else {  // X^T [N, K]: two [N rows x 64 k] boxes
               tma_load_2d(b_dst, &tma_b_dense, full_bar(s), kb * BK, 0);
               tma_load_2d(b_dst + n * 128, &tma_b_dense, full_bar(s), kb * BK + 64, 0);
@@ -471,7 +454,7 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_k = (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (8u << 24);
       const uint32_t idesc_mn = idesc_k | (1u << 16);
       uint32_t it = 0, unit_it = 0, a_full_ph = 0, b_full_ph = 0;
@@ -502,8 +485,8 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           }
         } else {
           const int kb0 = un.part * k_blocks / un.parts, kb1 = (un.part + 1) * k_blocks / un.parts;
-          const bool b_mn = prm.d_b_mn, a_mn = prm.d_a_mn;
-          const uint32_t idesc = (b_mn ? idesc_mn : idesc_k) | (a_mn ? (1u << 15) : 0u);
+          const bool b_mn = prm.d_b_mn;
+          const uint32_t idesc = b_mn ? idesc_mn : idesc_k;
           for (int kb = kb0; kb < kb1; ++kb, ++it) {
             const int s = it % S;
             const uint32_t ph = (it / S) & 1u;
@@ -512,12 +495,8 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             tcgen05_fence_after();
             const uint32_t a_base = smem_base + s * stage_bytes;
             const uint32_t b_base = a_base + A_STAGE_BYTES;
-            // K-major A: two 64-wide K atoms of 128 rows; MN-major A: two 64-wide M atoms of 128 k-rows
-            const uint64_t adesc0 = a_mn ? smem_desc(a_base, BK * 128, 1024) : smem_desc(a_base, 16, 1024);
-            auto a_step = [&](int ks) {
-              return a_mn ? desc_advance(adesc0, ks * (UMMA_K * 128))
-                          : desc_advance(adesc0, (ks >> 2) * A_ATOM_BYTES + (ks & 3) * 32);
-            };
+            const uint64_t adesc0 = smem_desc(a_base, 16, 1024);  // two 64-wide K atoms of 128 rows
+            auto a_step = [&](int ks) { return desc_advance(adesc0, (ks >> 2) * A_ATOM_BYTES + (ks & 3) * 32); };
             if (b_mn) {
               const uint64_t bdesc0 = smem_desc(b_base, BK * 128, 1024);
 #pragma unroll
@@ -622,14 +601,10 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(fmaxf(__uint_as_float(r[i]) + bias, 0.f));
           }
           const int copies = sparse ? 0 : prm.d_num_copies;
-          // dense units over column blocks: this unit's columns start at col0, the last block
-          // may be narrower (a multiple of 8 columns)
-          const int col0 = un.nblock * n;
-          const int n_valid = (!sparse && prm.d_ncols > 0) ? min(n, prm.d_ncols - col0) : n;
           for (int pe = 0; pe <= copies; ++pe) {
             __half* o = pe == 0 ? out : prm.d_out_copies[pe - 1];
             if (sn == 1) {
-              uint4* dst = reinterpret_cast<uint4*>(o + row * sm + col0 + c0);
+              uint4* dst = reinterpret_cast<uint4*>(o + row * sm + c0);
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
                 uint4 pk;
@@ -638,13 +613,13 @@ tc_units_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 for (int i = 0; i < 4; ++i)
                   h[i] = __floats2half2_rn(__uint_as_float(r[v * 8 + 2 * i]),
                                            __uint_as_float(r[v * 8 + 2 * i + 1]));
-                if (c0 + v * 8 < n_valid) dst[v] = pk;
+                if (c0 + v * 8 < n) dst[v] = pk;
               }
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i)
-                if (c0 + i < n_valid)  // n need not be a multiple of the 32 columns read at a time
-                  o[row * sm + (col0 + c0 + i) * sn] = __float2half_rn(__uint_as_float(r[i]));
+                if (c0 + i < n)  // n need not be a multiple of the 32 columns read at a time
+                  o[row * sm + (c0 + i) * sn] = __float2half_rn(__uint_as_float(r[i]));
             }
           }
         }
@@ -975,18 +950,34 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// Row-major fp16 matrix [rows, cols] (cols contiguous); box = [box_rows x 64 cols], 128B swizzle.
-int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows) {
+// Row-major fp16 matrix [rows, cols] (cols contiguous, rows `ld` elements apart, a multiple of 8);
+// box = [box_rows x box_cols].
+int make_map_f16(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows,
+                 int box_cols, bool swizzle) {
   EncodeFn fn = encode_fn();
   if (!fn) return IEX_ERR_DRIVER;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1u, 1u};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r != CUDA_SUCCESS) {
+    // A thread that has made no runtime call yet (an autograd worker) has no current context;
+    // selecting its device binds one.
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
   return r == CUDA_SUCCESS ? IEX_OK : IEX_ERR_DRIVER;
+}
+
+// Operand tile: box = [box_rows x 64 cols], 128-byte swizzle.
+int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows) {
+  return make_map_f16(map, base, rows, cols, cols, box_rows, 64, true);
 }
 
 // Per-device host state.  One process may drive several GPUs (the torch operators accept
@@ -1073,7 +1064,7 @@ int launch_units(const CUtensorMap& ta, const CUtensorMap& tbd, const CUtensorMa
   // 8 KB behind everything for the staged epilogue of dense tiles whose output is tokens-major
   // (contiguous along the tile's rows) and 16-byte friendly; otherwise two-byte stores
   prm.epi_offset = 0;
-  bool vec_ok = prm.d_tiles > 0 && prm.d_stride_m == 1 && prm.d_ncols == 0 && prm.d_stride_n % 8 == 0 &&
+  bool vec_ok = prm.d_tiles > 0 && prm.d_stride_m == 1 && prm.d_stride_n % 8 == 0 &&
                 prm.d_m % 8 == 0 && aligned16(prm.d_out);
   for (int i = 0; i < prm.d_num_copies; ++i) vec_ok = vec_ok && aligned16(prm.d_out_copies[i]);
   if (vec_ok && data + 8192 <= static_cast<size_t>(kDataBudget)) {
@@ -1099,7 +1090,7 @@ int launch_units(const CUtensorMap& ta, const CUtensorMap& tbd, const CUtensorMa
   const int units = prm.d_tiles * prm.d_parts + prm.s_tiles * prm.s_parts;
   const int grid = units < sm_count() * ctas_per_sm ? units : sm_count() * ctas_per_sm;
   int st = launch_overlapped(kern, dim3(grid), dim3((kFirstDecodeWarp + ND) * 32), smem, stream, ta, tbd, tbs, prm);
-  const int split_tiles = (prm.s_parts > 1 ? prm.s_tiles : 0) + (prm.d_parts > 1 && prm.d_ncols == 0 ? prm.d_tiles : 0);
+  const int split_tiles = (prm.s_parts > 1 ? prm.s_tiles : 0) + (prm.d_parts > 1 ? prm.d_tiles : 0);
   if (st == 0 && split_tiles > 0) {
     const int slices = (prm.n * (BM / 4) + kReduceThreads - 1) / kReduceThreads;
     st = launch_overlapped(tc_reduce_kernel, dim3(split_tiles, slices), dim3(kReduceThreads), 0, stream, prm);
@@ -1298,6 +1289,9 @@ extern "C" size_t iex_tc_workspace_bytes(int m_sparse, int sparse_parts, int m_d
 
 extern "C" int iex_linear_f16(int tokens, int in_features, int out_features, const void* input,
                               const void* weight, void* out, void* stream) {
+  // out_features a multiple of 8: the CTA-pair GEMM (same limits kept); otherwise the tile kernel
+  if (tokens > 0 && tokens % 16 == 0 && tokens <= 256 && out_features % 8 == 0 && aligned16(out))
+    return iex_linear_f16_any(tokens, in_features, out_features, input, weight, out, stream);
   return linear_impl(tokens, in_features, out_features, input, weight, out, 1, nullptr, 0, stream);
 }
 
@@ -1306,80 +1300,6 @@ extern "C" int iex_linear_f16_splitk(int tokens, int in_features, int out_featur
                                      size_t workspace_bytes, void* stream) {
   return linear_impl(tokens, in_features, out_features, input, weight, out, parts, workspace,
                      workspace_bytes, stream);
-}
-
-// The two products of the dense branch's backward pass on the same tensor-core kernel.
-//   dgrad:  dinput [tokens, in] = grad [tokens, out] * weight [out, in]
-//           D[f = in, t] = sum_c W[c, f] * grad[t, c]: A = weight read as [K = out, M = in]
-//           (MN-major), B = grad (K-major, like the forward's input).  tokens <= 256.
-//   wgrad:  dweight [out, in] = grad^T [out, tokens] * input [tokens, in]
-//           D[f = out, j = in] = sum_t grad[t, f] * input[t, j]: A = grad read as [K = tokens,
-//           M = out] (MN-major), B = input [K = tokens, N = in] (MN-major), units over blocks of
-//           256 columns of `in`.  Any number of tokens (K).
-extern "C" int iex_linear_f16_dgrad(int tokens, int in_features, int out_features, const void* grad,
-                                    const void* weight, void* dinput, void* stream) {
-  if (tokens < 0 || in_features < 0 || out_features < 0) return IEX_ERR_BAD_ARG;
-  if (tokens == 0 || in_features == 0) return IEX_OK;
-  if (!grad || !weight || !dinput) return IEX_ERR_BAD_ARG;
-  if (tokens % 16 != 0 || tokens > 256 || out_features % 8 != 0 || out_features == 0 || in_features % 8 != 0)
-    return IEX_ERR_UNSUPPORTED;
-  if (!aligned16(grad) || !aligned16(weight)) return IEX_ERR_UNSUPPORTED;
-  CUtensorMap ta, tb;
-  int st = make_map(&ta, weight, out_features, in_features, BK);  // [K rows, M cols], boxes of 128 k-rows
-  if (st) return st;
-  st = make_map(&tb, grad, tokens, out_features, tokens);
-  if (st) return st;
-  Params p{};
-  p.d_tiles = (in_features + BM - 1) / BM;
-  p.d_m = in_features;
-  p.d_out = static_cast<__half*>(dinput);
-  p.d_stride_m = 1;
-  p.d_stride_n = in_features;
-  p.d_a_mn = 1;
-  p.k = out_features;
-  p.n = tokens;
-  p.tmem_cols = tmem_cols_for(tokens);
-  p.status = status_word();
-  st = bind_workspace(p, 1, 1, nullptr, 0);
-  if (st) return st;
-  const int stages = dense_stages(tokens, kMaxStages);
-  if (stages < 2) return IEX_ERR_UNSUPPORTED;
-  return launch_units<0, uint16_t>(ta, tb, tb, p, stages, 1, static_cast<cudaStream_t>(stream));
-}
-
-extern "C" int iex_linear_f16_wgrad(int tokens, int in_features, int out_features, const void* grad,
-                                    const void* input, void* dweight, void* stream) {
-  if (tokens < 0 || in_features < 0 || out_features < 0) return IEX_ERR_BAD_ARG;
-  if (out_features == 0 || in_features == 0) return IEX_OK;
-  if (!grad || !input || !dweight) return IEX_ERR_BAD_ARG;
-  if (tokens % 8 != 0 || tokens == 0 || out_features % 8 != 0 || in_features % 8 != 0) return IEX_ERR_UNSUPPORTED;
-  if (!aligned16(grad) || !aligned16(input) || !aligned16(dweight)) return IEX_ERR_UNSUPPORTED;
-  const int nblk = in_features >= 256 ? 256 : ((in_features + 63) / 64) * 64;  // columns per unit
-  CUtensorMap ta, tb;
-  int st = make_map(&ta, grad, tokens, out_features, BK);  // [K = tokens rows, M = out cols]
-  if (st) return st;
-  st = make_map(&tb, input, tokens, in_features, BK);  // [K rows, N cols], boxes of 128 k-rows
-  if (st) return st;
-  Params p{};
-  p.d_tiles = (out_features + BM - 1) / BM;
-  p.d_m = out_features;
-  p.d_out = static_cast<__half*>(dweight);
-  p.d_stride_m = in_features;
-  p.d_stride_n = 1;
-  p.d_a_mn = 1;
-  p.d_b_mn = 1;
-  p.d_nblocks = (in_features + nblk - 1) / nblk;
-  p.d_ncols = in_features;
-  p.k = tokens;
-  p.n = nblk;
-  p.tmem_cols = tmem_cols_for(nblk);
-  p.status = status_word();
-  p.s_parts = 1;
-  p.d_parts = p.d_nblocks;  // the unit list counts column blocks where it would count K parts
-  p.partials = nullptr;
-  const int stages = dense_stages(nblk, kMaxStages);
-  if (stages < 2) return IEX_ERR_UNSUPPORTED;
-  return launch_units<0, uint16_t>(ta, tb, tb, p, stages, 1, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int iex_spmm_f16_tc(int m, int k, int n, int nnz, const int32_t* row_offsets,

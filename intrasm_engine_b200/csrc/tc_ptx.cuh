@@ -73,6 +73,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "l"(map), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
+// True in one lane of a converged warp.  A role that is one thread's work (issuing TMA copies or
+// tcgen05.mma) runs its whole loop under this and not under `lane == 0`: the compiler then knows that a
+// single thread is active and keeps descriptors and addresses in uniform registers.  Measured on
+// B200, four K16 instructions and a commit per step: 48 cycles per 128 x 64 instruction (what the
+// tensor pipe takes) against about 110 under `lane == 0` and 58 with an election per step.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(

@@ -16,36 +16,21 @@
 //   * linear_fp16, spmm_tc_half, fused_spmm_linear_half and csr_to_dense_half are new
 //     operators (dense branch, tensor-core SpMM, fused sparse||dense layer, CSR expansion);
 //     the reference has no kernel of its own for them.
-#include <ATen/ATen.h>
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGuard.h>
+#include "iex_torch_ops.h"
+
+#include <ATen/cuda/EmptyTensor.h>
 #include <torch/library.h>
 
 #include <algorithm>
 #include <cstdlib>
-#include <tuple>
 
-#include "iex_b200.h"
+namespace iex_torch {
 
-namespace {
-
-void* stream_of(const at::Tensor& t) {
-  return static_cast<void*>(at::cuda::getCurrentCUDAStream(t.get_device()).stream());
+at::Tensor empty(const at::Tensor& like, at::IntArrayRef sizes) {
+  return at::detail::empty_cuda(sizes, like.scalar_type(), like.device(), std::nullopt);
 }
-
-void check_status(int st, const char* what) {
-  TORCH_CHECK(st == 0, what, " failed with status ", st, ": ", iex_error_string(st));
-}
-
-void check_common(std::initializer_list<std::pair<const char*, const at::Tensor*>> named) {
-  const at::Tensor* first = nullptr;
-  for (const auto& [name, t] : named) {
-    TORCH_CHECK(t->is_cuda(), name, " must be a CUDA tensor");
-    TORCH_CHECK(t->is_contiguous(), name, " must be a contiguous tensor");
-    TORCH_CHECK(!t->is_sparse(), name, " must be a dense tensor");
-    if (first == nullptr) first = t;
-    TORCH_CHECK(t->device() == first->device(), name, " should be in the same device as the first argument");
-  }
+at::Tensor empty_bytes(const at::Tensor& like, int64_t bytes) {
+  return at::detail::empty_cuda({bytes}, at::kByte, like.device(), std::nullopt);
 }
 
 // CSR validation on the device (iex_csr_validate): returns 0 or the OR of IEX_CSR_* bits.
@@ -57,7 +42,7 @@ int64_t validate_csr_impl(const at::Tensor& row_offsets, const at::Tensor& colum
   TORCH_CHECK(i16 || column_indices.scalar_type() == at::kInt, "column_indices must be int16 or int32");
   TORCH_CHECK(row_offsets.scalar_type() == at::kInt && row_offsets.numel() == m + 1,
               "row_offsets must be int32 with m + 1 entries");
-  at::Tensor result = at::empty({1}, row_offsets.options());
+  at::Tensor result = empty(row_offsets, {1});
   check_status(iex_csr_validate(m, k, column_indices.numel(), row_offsets.data_ptr<int>(),
                                 column_indices.data_ptr(), i16 ? 16 : 32,
                                 row_indices != nullptr ? row_indices->data_ptr<int>() : nullptr,
@@ -121,7 +106,7 @@ at::Tensor spmm_f32(const at::Tensor& b, const at::Tensor& row_indices, const at
   c10::cuda::CUDAGuard guard(b.device());
   const int batch = b.size(0), k = b.size(1), n = b.size(2), nnz = column_indices.size(0);
   maybe_validate(row_offsets, column_indices, m, k, &row_indices, false);
-  at::Tensor out = per_batch_values ? at::zeros({batch, m, n}, b.options()) : at::empty({batch, m, n}, b.options());
+  at::Tensor out = per_batch_values ? at::zeros({batch, m, n}, b.options()) : empty(b, {batch, m, n});
   check_status(iex_spmm_f32(m, k, n, nnz, row_indices.data_ptr<int>(), values.data_ptr<float>(),
                             per_batch_values ? nnz : 0, row_offsets.data_ptr<int>(),
                             column_indices.data_ptr<int>(), b.data_ptr<float>(), nullptr,
@@ -156,7 +141,7 @@ at::Tensor spmm_sputnik_reuse_weight_half(const at::Tensor& b, const at::Tensor&
   c10::cuda::CUDAGuard guard(b.device());
   const int batch = b.size(0), k = b.size(1), n = b.size(2), nnz = column_indices.size(0);
   maybe_validate(row_offsets, column_indices, m, k, &row_indices, false);
-  at::Tensor out = at::empty({batch, m, n}, b.options());
+  at::Tensor out = empty(b, {batch, m, n});
   const int st = i16 ? iex_spmm_f16_i16(m, k, n, nnz, row_indices.data_ptr<int>(), values.data_ptr(),
                                         row_offsets.data_ptr<int>(),
                                         reinterpret_cast<const uint16_t*>(column_indices.data_ptr()),
@@ -189,7 +174,7 @@ at::Tensor sddmm_sputnik_atomic_upd_weight(const at::Tensor& a, const at::Tensor
   const int nnz = column_indices.size(0);
   c10::cuda::CUDAGuard guard(a.device());
   maybe_validate(row_offsets, column_indices, m, n, &row_indices, false);
-  at::Tensor out = at::empty({nnz}, a.options());
+  at::Tensor out = empty(a, {nnz});
   check_status(iex_sddmm_f32(m, k, n, nnz, row_indices.data_ptr<int>(), row_offsets.data_ptr<int>(),
                              column_indices.data_ptr<int>(), a.data_ptr<float>(), b.data_ptr<float>(),
                              out.data_ptr<float>(), batch, 0, stream_of(a)),
@@ -216,7 +201,7 @@ at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at
   const int nnz = column_indices.size(0);
   c10::cuda::CUDAGuard guard(a.device());
   maybe_validate(row_offsets, column_indices, m, n, &row_indices, false);
-  at::Tensor out = at::empty({nnz}, a.options());
+  at::Tensor out = empty(a, {nnz});
   check_status(iex_sddmm_f16(m, k, n, nnz, row_indices.data_ptr<int>(), row_offsets.data_ptr<int>(),
                              column_indices.data_ptr(), i16 ? 16 : 32, a.data_ptr(), b.data_ptr(),
                              out.data_ptr(), batch, stream_of(a)),
@@ -224,33 +209,7 @@ at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at
   return out;
 }
 
-// One block of at most 256 tokens (a multiple of 16) of the dense branch into `out` (a
-// contiguous [tokens, out_features] block).
-void linear_block(const at::Tensor& input, const at::Tensor& weight, at::Tensor out) {
-  const int64_t tokens = input.size(0), out_features = weight.size(0);
-  // A weight with few 128-row tiles would leave most SMs without work: split every tile's K
-  // range over about 128 / tiles CTAs (measured optimum on B200: 32 tiles -> 4 parts,
-  // 4 tiles -> 16).  The partial tiles live in a scratch tensor of the caching allocator.
-  const int64_t tiles = (out_features + 127) / 128;
-  const int parts = tiles > 0 ? static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(16, 128 / tiles))) : 1;
-  if (parts > 1 && tokens % 32 == 0 && input.size(1) >= 128 * parts) {
-    const size_t need = iex_tc_workspace_bytes(0, 1, static_cast<int>(out_features), parts,
-                                               static_cast<int>(tokens));
-    at::Tensor scratch = at::empty({static_cast<int64_t>(need)}, input.options().dtype(at::kByte));
-    check_status(iex_linear_f16_splitk(tokens, input.size(1), out_features, input.data_ptr(),
-                                       weight.data_ptr(), out.data_ptr(), parts, scratch.data_ptr(), need,
-                                       stream_of(input)),
-                 "iex_linear_f16_splitk");
-    return;
-  }
-  check_status(iex_linear_f16(tokens, input.size(1), out_features, input.data_ptr(), weight.data_ptr(),
-                              out.data_ptr(), stream_of(input)),
-               "iex_linear_f16");
-}
-
-// Dense branch on tensor cores: input @ weight^T (layers_and_funcs/torch.py:17).  Any number
-// of tokens: the kernel takes up to 256 at a time (a multiple of 16), so longer inputs run
-// block after block into the rows of one output, and a ragged tail is padded with zero rows.
+// Dense branch on tensor cores: input @ weight^T (layers_and_funcs/torch.py:17), any number of tokens.
 at::Tensor linear_fp16(const at::Tensor& input, const at::Tensor& weight) {
   TORCH_CHECK(input.dim() == 2 && weight.dim() == 2, "input and weight must be 2-D");
   TORCH_CHECK(input.size(1) == weight.size(1), "input and weight disagree on in_features");
@@ -258,75 +217,37 @@ at::Tensor linear_fp16(const at::Tensor& input, const at::Tensor& weight) {
   TORCH_CHECK(input.scalar_type() == at::kHalf && weight.scalar_type() == at::kHalf,
               "input and weight must be float16");
   c10::cuda::CUDAGuard guard(input.device());
-  const int64_t tokens = input.size(0), out_features = weight.size(0), in_features = input.size(1);
-  at::Tensor out = at::empty({tokens, out_features}, input.options());
-  if (tokens == 0 || out_features == 0) return out;
-  const int64_t whole = tokens / 16 * 16;
-  for (int64_t t0 = 0; t0 < whole; t0 += 256) {
-    const int64_t block = std::min<int64_t>(256, whole - t0);
-    linear_block(input.narrow(0, t0, block), weight, out.narrow(0, t0, block));
-  }
-  if (whole < tokens) {  // ragged tail: 16 rows, the missing ones zero
-    at::Tensor tail_in = at::zeros({16, in_features}, input.options());
-    tail_in.narrow(0, 0, tokens - whole).copy_(input.narrow(0, whole, tokens - whole));
-    at::Tensor tail_out = at::empty({16, out_features}, input.options());
-    linear_block(tail_in, weight, tail_out);
-    out.narrow(0, whole, tokens - whole).copy_(tail_out.narrow(0, 0, tokens - whole));
-  }
+  at::Tensor out = empty(input, {input.size(0), weight.size(0)});
+  check_status(iex_linear_f16_any(input.size(0), input.size(1), weight.size(0), input.data_ptr(), weight.data_ptr(),
+                                  out.data_ptr(), stream_of(input)),
+               "iex_linear_f16_any");
   return out;
 }
 
-// dinput = grad @ weight (blocks of up to 256 tokens, a ragged tail padded with zero rows)
+// dinput = grad @ weight
 at::Tensor linear_fp16_dgrad(const at::Tensor& grad, const at::Tensor& weight) {
   TORCH_CHECK(grad.dim() == 2 && weight.dim() == 2 && grad.size(1) == weight.size(0),
               "grad must be [tokens, out_features] and weight [out_features, in_features]");
   check_common({{"grad", &grad}, {"weight", &weight}});
   TORCH_CHECK(grad.scalar_type() == at::kHalf && weight.scalar_type() == at::kHalf, "grad and weight must be float16");
   c10::cuda::CUDAGuard guard(grad.device());
-  const int64_t tokens = grad.size(0), out_features = weight.size(0), in_features = weight.size(1);
-  at::Tensor dinput = at::empty({tokens, in_features}, grad.options());
-  if (tokens == 0 || in_features == 0) return dinput;
-  auto block = [&](const at::Tensor& g, at::Tensor d) {
-    check_status(iex_linear_f16_dgrad(g.size(0), in_features, out_features, g.data_ptr(), weight.data_ptr(),
-                                      d.data_ptr(), stream_of(grad)),
-                 "iex_linear_f16_dgrad");
-  };
-  const int64_t whole = tokens / 16 * 16;
-  for (int64_t t0 = 0; t0 < whole; t0 += 256) {
-    const int64_t rows = std::min<int64_t>(256, whole - t0);
-    block(grad.narrow(0, t0, rows), dinput.narrow(0, t0, rows));
-  }
-  if (whole < tokens) {
-    at::Tensor tail_in = at::zeros({16, out_features}, grad.options());
-    tail_in.narrow(0, 0, tokens - whole).copy_(grad.narrow(0, whole, tokens - whole));
-    at::Tensor tail_out = at::empty({16, in_features}, grad.options());
-    block(tail_in, tail_out);
-    dinput.narrow(0, whole, tokens - whole).copy_(tail_out.narrow(0, 0, tokens - whole));
-  }
+  at::Tensor dinput = empty(grad, {grad.size(0), weight.size(1)});
+  check_status(iex_linear_f16_dgrad(grad.size(0), weight.size(1), weight.size(0), grad.data_ptr(), weight.data_ptr(),
+                                    dinput.data_ptr(), stream_of(grad)),
+               "iex_linear_f16_dgrad");
   return dinput;
 }
 
-// dweight = grad^T @ input (the token dimension is the contraction; padded to a multiple of 8)
+// dweight = grad^T @ input (the token dimension is the contraction)
 at::Tensor linear_fp16_wgrad(const at::Tensor& grad, const at::Tensor& input) {
   TORCH_CHECK(grad.dim() == 2 && input.dim() == 2 && grad.size(0) == input.size(0),
               "grad must be [tokens, out_features] and input [tokens, in_features]");
   check_common({{"grad", &grad}, {"input", &input}});
   TORCH_CHECK(grad.scalar_type() == at::kHalf && input.scalar_type() == at::kHalf, "grad and input must be float16");
   c10::cuda::CUDAGuard guard(grad.device());
-  const int64_t tokens = grad.size(0), out_features = grad.size(1), in_features = input.size(1);
-  at::Tensor dweight = at::empty({out_features, in_features}, grad.options());
-  if (out_features == 0 || in_features == 0) return dweight;
-  at::Tensor g = grad, x = input;
-  if (tokens % 8 != 0 || tokens == 0) {
-    const int64_t padded = std::max<int64_t>(8, (tokens + 7) / 8 * 8);
-    g = at::zeros({padded, out_features}, grad.options());
-    x = at::zeros({padded, in_features}, input.options());
-    if (tokens > 0) {
-      g.narrow(0, 0, tokens).copy_(grad);
-      x.narrow(0, 0, tokens).copy_(input);
-    }
-  }
-  check_status(iex_linear_f16_wgrad(g.size(0), in_features, out_features, g.data_ptr(), x.data_ptr(),
+  if (grad.size(0) == 0) return at::zeros({grad.size(1), input.size(1)}, grad.options());
+  at::Tensor dweight = empty(grad, {grad.size(1), input.size(1)});
+  check_status(iex_linear_f16_wgrad(grad.size(0), input.size(1), grad.size(1), grad.data_ptr(), input.data_ptr(),
                                     dweight.data_ptr(), stream_of(grad)),
                "iex_linear_f16_wgrad");
   return dweight;
@@ -354,7 +275,7 @@ at::Tensor spmm_tc_half(const at::Tensor& x, const at::Tensor& row_offsets, cons
   const int bits = tc_sparse_checks(x, row_offsets, values, column_indices, m);
   c10::cuda::CUDAGuard guard(x.device());
   maybe_validate(row_offsets, column_indices, m, x.size(0), nullptr, true);
-  at::Tensor out = at::empty({m, x.size(1)}, x.options());
+  at::Tensor out = empty(x, {m, x.size(1)});
   check_status(iex_spmm_f16_tc(m, x.size(0), x.size(1), column_indices.size(0), row_offsets.data_ptr<int>(),
                                column_indices.data_ptr(), bits, values.data_ptr(), x.data_ptr(),
                                out.data_ptr(), stream_of(x)),
@@ -374,8 +295,8 @@ std::tuple<at::Tensor, at::Tensor> fused_spmm_linear_half(const at::Tensor& x, c
   c10::cuda::CUDAGuard guard(x.device());
   maybe_validate(row_offsets, column_indices, m, x.size(0), nullptr, true);
   const int64_t n = x.size(1), md = weight.size(0);
-  at::Tensor out_s = at::empty({m, n}, x.options());
-  at::Tensor out_d = at::empty({n, md}, x.options());
+  at::Tensor out_s = empty(x, {m, n});
+  at::Tensor out_d = empty(x, {n, md});
   check_status(iex_fused_spmm_linear_f16(m, md, x.size(0), n, column_indices.size(0),
                                          row_offsets.data_ptr<int>(), column_indices.data_ptr(), bits,
                                          values.data_ptr(), weight.data_ptr(), x.data_ptr(), out_s.data_ptr(),
@@ -393,7 +314,7 @@ at::Tensor csr_to_dense_half(const at::Tensor& row_offsets, const at::Tensor& va
   const bool i16 = column_indices.scalar_type() == at::kShort;
   TORCH_CHECK(i16 || column_indices.scalar_type() == at::kInt, "column_indices must be int16 or int32");
   c10::cuda::CUDAGuard guard(values.device());
-  at::Tensor out = at::empty({m, k}, values.options());
+  at::Tensor out = empty(values, {m, k});
   check_status(iex_csr_to_dense_f16(m, k, row_offsets.data_ptr<int>(), column_indices.data_ptr(),
                                     i16 ? 16 : 32, values.data_ptr(), out.data_ptr(), stream_of(values)),
                "iex_csr_to_dense_f16");
@@ -410,8 +331,7 @@ at::Tensor sddmm_plan(const at::Tensor& row_offsets, const at::Tensor& column_in
   c10::cuda::CUDAGuard guard(row_offsets.device());
   const int64_t nnz = column_indices.numel();
   const size_t bytes = iex_sddmm_plan_bytes(m, n, nnz);
-  at::Tensor plan = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))},
-                              row_offsets.options().dtype(at::kByte));
+  at::Tensor plan = empty_bytes(row_offsets, std::max<size_t>(bytes, 16));
   check_status(iex_sddmm_plan_build(m, n, nnz, row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
                                     plan.data_ptr(), bytes, stream_of(row_offsets)),
                "iex_sddmm_plan_build");
@@ -429,7 +349,7 @@ at::Tensor sddmm_tc_planned(const at::Tensor& a, const at::Tensor& b, const at::
   TORCH_CHECK(static_cast<size_t>(plan.numel()) >= iex_sddmm_plan_bytes(m, n, nnz),
               "plan was built for another pattern size");
   c10::cuda::CUDAGuard guard(a.device());
-  at::Tensor out = at::empty({nnz}, a.options());
+  at::Tensor out = empty(a, {nnz});
   check_status(iex_sddmm_f32_tc(m, k, n, nnz, plan.data_ptr(), a.data_ptr<float>(), b.data_ptr<float>(),
                                 out.data_ptr<float>(), 0, stream_of(a)),
                "iex_sddmm_f32_tc");
@@ -445,8 +365,7 @@ at::Tensor spmm_plan(const at::Tensor& row_offsets, const at::Tensor& column_ind
   c10::cuda::CUDAGuard guard(row_offsets.device());
   const int64_t nnz = column_indices.numel();
   const size_t bytes = iex_tile_plan_bytes(m, k, nnz, 64);
-  at::Tensor plan = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))},
-                              row_offsets.options().dtype(at::kByte));
+  at::Tensor plan = empty_bytes(row_offsets, std::max<size_t>(bytes, 16));
   check_status(iex_tile_plan_build(m, k, nnz, 64, row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
                                    plan.data_ptr(), bytes, stream_of(row_offsets)),
                "iex_tile_plan_build");
@@ -464,9 +383,9 @@ at::Tensor spmm_tc_planned(const at::Tensor& b, const at::Tensor& values, const 
   TORCH_CHECK(static_cast<size_t>(plan.numel()) >= iex_tile_plan_bytes(m, k, nnz, 64),
               "plan was built for another pattern size");
   c10::cuda::CUDAGuard guard(b.device());
-  at::Tensor out = at::empty({m, n}, b.options());
+  at::Tensor out = empty(b, {m, n});
   const size_t need = iex_spmm_f32_tc_workspace_bytes(m, k, n);
-  at::Tensor scratch = at::empty({static_cast<int64_t>(std::max<size_t>(need, 16))}, b.options().dtype(at::kByte));
+  at::Tensor scratch = empty_bytes(b, std::max<size_t>(need, 16));
   check_status(iex_spmm_f32_tc(m, k, n, nnz, plan.data_ptr(), values.data_ptr<float>(), b.data_ptr<float>(),
                                out.data_ptr<float>(), scratch.data_ptr(), need, stream_of(b)),
                "iex_spmm_f32_tc");
@@ -480,7 +399,7 @@ int64_t validate_csr(const at::Tensor& row_offsets, const at::Tensor& column_ind
   return validate_csr_impl(row_offsets, column_indices, m, k, nullptr, require_ascending);
 }
 
-}  // namespace
+}  // namespace iex_torch
 
 TORCH_LIBRARY(iex_ops, m) {
   m.def("spmm_sputnik_atomic(Tensor b, Tensor row_indices, Tensor values, Tensor row_offsets, Tensor column_indices, int m) -> Tensor");
@@ -503,6 +422,7 @@ TORCH_LIBRARY(iex_ops, m) {
 
 // CUDA dispatch key only: a CPU tensor reaches no implementation (there is no CPU path).
 TORCH_LIBRARY_IMPL(iex_ops, CUDA, m) {
+  using namespace iex_torch;
   m.impl("spmm_sputnik_atomic", &spmm_sputnik_atomic);
   m.impl("spmm_sputnik_reuse_weight", &spmm_sputnik_reuse_weight);
   m.impl("spmm_sputnik_reuse_weight_half", &spmm_sputnik_reuse_weight_half);
