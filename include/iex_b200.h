@@ -215,6 +215,18 @@ IEX_API int iex_linear_f16_wgrad(int tokens, int in_features, int out_features, 
 IEX_API int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long long lda, const void* b, int b_mn,
                          long long ldb, void* out, int out_transposed, long long ldo, int tile_n, int k_parts,
                          void* stream);
+/* Time this library expects iex_gemm_f16 to take on the current device, for choosing between ways. */
+IEX_API double iex_gemm_f16_estimate_us(int m, int n, int k, int b_mn, int out_transposed);
+
+/* CSR SpMM with 1 to 16 dense columns (decoding steps), fp16, fp32 accumulation, CUDA cores:
+ * out(r, t) = sum_p values[p] * x(col[p], t).  The strides are in elements, so x and out may be
+ * [k, n] / [m, n] or [n, k] / [n, m].  values 4-byte, column_indices 2 * sizeof(index) aligned. */
+IEX_API int iex_spmm_f16_skinny_supported(int k, int n);
+IEX_API int iex_spmm_f16_skinny(int m, int k, int n, int nnz, const int32_t* row_offsets,
+                                const void* column_indices, int index_bits, const void* values,
+                                const void* x, long long x_row_stride, long long x_col_stride, void* out,
+                                long long out_row_stride, long long out_col_stride, void* stream);
+
 /* CSR SpMM on tensor cores: out[r, :] = sum_p values[p] * dense[col[p], :].
  * Same contract as iex_spmm_f16_i16 / _i32 with batch = 1 and no bias (replaces
  * my_sputnik::CudaSpmm5, extensions.h:30), plus one precondition: column indices ascend
@@ -333,6 +345,16 @@ IEX_API int iex_peer_barrier_bounded(void* const* signals, int world, int rank, 
  * tensor-core linear as its dense tile operand.  index_bits is 16 or 32. */
 IEX_API int iex_csr_to_dense_f16(int m, int k, const int32_t* row_offsets, const void* column_indices,
                                  int index_bits, const void* values, void* out, void* stream);
+/* The same with `ld` >= k elements between the dense rows (the columns past k become zero). */
+IEX_API int iex_csr_to_dense_f16_ld(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices,
+                                    int index_bits, const void* values, void* out, void* stream);
+/* out[p] = dense[row(p) * ld + column_indices[p]] for every stored position p (fp16). */
+IEX_API int iex_csr_sample_f16(int m, int k, long long ld, const int32_t* row_offsets, const void* column_indices,
+                               int index_bits, const void* dense, void* out, void* stream);
+/* Copies rows of `cols` fp16 values into rows of `ld` values (a multiple of 8), zero-filled. */
+IEX_API int iex_pad_rows_f16(int rows, int cols, int ld, const void* in, void* out, void* stream);
+/* out = max(in, 0) over `count` fp16 values (a multiple of 8; NaN becomes 0). */
+IEX_API int iex_relu_f16(long long count, const void* in, void* out, void* stream);
 
 /* Dense matrix -> CSR on the device, in two calls, for the conversions the reference
  * delegates to xformers (_dense_to_sparse, intrasm_engine/pytorch/utils.py:143-153) and for

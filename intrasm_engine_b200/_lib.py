@@ -67,6 +67,18 @@ SIGNATURES = {
     # m n k a a_mn lda b b_mn ldb out out_transposed ldo tile_n k_parts stream
     "iex_gemm_f16": (c_int, [c_int, c_int, c_int, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll,
                              c_int, c_int, c_ptr]),
+    # m n k b_mn out_transposed
+    "iex_gemm_f16_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int, c_int]),
+    "iex_spmm_f16_skinny_supported": (c_int, [c_int, c_int]),
+    # m k n nnz row_offsets cols index_bits values x x_row x_col out out_row out_col stream
+    "iex_spmm_f16_skinny": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ll, c_ll,
+                                    c_ptr, c_ll, c_ll, c_ptr]),
+    # m k ld row_offsets cols index_bits values out stream
+    "iex_csr_to_dense_f16_ld": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
+    # m k ld row_offsets cols index_bits dense out stream
+    "iex_csr_sample_f16": (c_int, [c_int, c_int, c_ll, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
+    "iex_pad_rows_f16": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_ptr]),
+    "iex_relu_f16": (c_int, [c_ll, c_ptr, c_ptr, c_ptr]),
     # m k n nnz row_offsets cols index_bits values dense out stream
     "iex_spmm_f16_tc": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr,
                                 c_ptr, c_ptr]),

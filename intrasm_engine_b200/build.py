@@ -5,9 +5,9 @@ library exists) compiles every ``csrc/*.cu`` to an object file
 under ``build/`` (one nvcc process per file, in parallel) and links them into
 ``intrasm_engine_b200/libiex_b200.so``.  The CUDA runtime is linked statically, so the
 library has no load-time dependency besides libc/libstdc++ and the driver.
-It then compiles ``torch_ext/iex_torch_ext.cpp`` with g++ against the installed torch
-headers into ``intrasm_engine_b200/libiex_torch_ext.so``, the extension that registers
-``torch.ops.iex_ops`` and calls the C ABI (it finds ``libiex_b200.so`` beside itself through
+It then compiles ``torch_ext/*.cpp`` with g++ against the installed torch headers into
+``intrasm_engine_b200/libiex_torch_ext.so``, the extension that registers
+``torch.ops.iex_ops``, holds the native side of the operator classes and calls the C ABI (it finds ``libiex_b200.so`` beside itself through
 an ``$ORIGIN`` run path).  ``CMakeLists.txt`` beside this file describes the C-ABI build for
 CMake users.
 """
@@ -24,7 +24,8 @@ REPO_DIR = os.path.dirname(PKG_DIR)
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(REPO_DIR, "build", "iex_b200")
 LIB_PATH = os.path.join(PKG_DIR, "libiex_b200.so")
-EXT_SRC = os.path.join(PKG_DIR, "torch_ext", "iex_torch_ext.cpp")
+EXT_DIR = os.path.join(PKG_DIR, "torch_ext")
+EXT_SRCS = [os.path.join(EXT_DIR, f) for f in ("iex_torch_ext.cpp", "iex_autograd.cpp")]
 EXT_PATH = os.path.join(PKG_DIR, "libiex_torch_ext.so")
 
 NVCC_FLAGS = [
@@ -78,10 +79,13 @@ def _cuda_include() -> str:
 
 def build_torch_ext(force: bool = False) -> str:
     """Compile the torch extension that registers ``torch.ops.iex_ops``; returns its path."""
-    newest = max(os.path.getmtime(EXT_SRC), os.path.getmtime(LIB_PATH), os.path.getmtime(__file__),
-                 os.path.getmtime(os.path.join(REPO_DIR, "include", "iex_b200.h")))
+    deps = [*EXT_SRCS, os.path.join(EXT_DIR, "iex_torch_ops.h"), LIB_PATH, __file__,
+            os.path.join(REPO_DIR, "include", "iex_b200.h")]
+    newest = max(os.path.getmtime(d) for d in deps)
     if not force and os.path.exists(EXT_PATH) and os.path.getmtime(EXT_PATH) >= newest:
         return EXT_PATH
+    import sysconfig
+
     import torch
     torch_dir = os.path.dirname(torch.__file__)
     torch_lib = os.path.join(torch_dir, "lib")
@@ -91,18 +95,25 @@ def build_torch_ext(force: bool = False) -> str:
     # process two exception runtimes, and an error raised by TORCH_CHECK then crashes while
     # unwinding through the extension's frames.  IEX_CXX overrides.
     cxx = os.environ.get("IEX_CXX") or shutil.which("g++") or "g++"
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-           "-I", os.path.join(REPO_DIR, "include"),
-           "-I", torch_inc, "-I", os.path.join(torch_inc, "torch", "csrc", "api", "include"),
-           "-I", _cuda_include(),
-           EXT_SRC, "-o", EXT_PATH,
-           "-L", PKG_DIR, "-liex_b200",
-           "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
-           "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"torch extension build failed:\n{res.stdout}\n{res.stderr}")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility-inlines-hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+             "-I", os.path.join(REPO_DIR, "include"),
+             "-I", torch_inc, "-I", os.path.join(torch_inc, "torch", "csrc", "api", "include"),
+             "-I", _cuda_include(), "-I", sysconfig.get_paths()["include"]]
+
+    def run(cmd):
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"torch extension build failed:\n{res.stdout}\n{res.stderr}")
+
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    objs = [os.path.join(OBJ_DIR, os.path.basename(src)[:-4] + ".ext.o") for src in EXT_SRCS]
+    with ThreadPoolExecutor(max_workers=len(objs)) as pool:
+        list(pool.map(lambda so: run([cxx, *flags, "-c", so[0], "-o", so[1]]), zip(EXT_SRCS, objs)))
+    run([cxx, "-shared", *objs, "-o", EXT_PATH,
+         "-L", PKG_DIR, "-liex_b200",
+         "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+         "-Wl,-rpath,$ORIGIN"])
     return EXT_PATH
 
 

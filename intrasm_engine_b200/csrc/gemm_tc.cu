@@ -544,6 +544,11 @@ extern "C" int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long l
                            k_parts, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" double iex_gemm_f16_estimate_us(int m, int n, int k, int b_mn, int out_transposed) {
+  iex::tc::GemmPlan plan{};
+  return iex::tc::plan_gemm(m, n, k, b_mn != 0, out_transposed != 0, iex::tc::sm_count(), &plan);
+}
+
 // The dense branch, any number of tokens:
 //   forward  out [tokens, out]     = input [tokens, in] * weight [out, in]^T
 //   dgrad    dinput [tokens, in]   = grad [tokens, out] * weight [out, in]

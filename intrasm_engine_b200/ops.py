@@ -34,6 +34,7 @@ All are implemented for the CUDA dispatch key only: there is no CPU path.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 
 import torch
@@ -48,6 +49,18 @@ if not os.path.exists(EXT_PATH):
         "(there is no Python or CPU fallback for torch.ops.iex_ops)")
 
 torch.ops.load_library(EXT_PATH)
+
+
+def _load_native():
+    """The same shared object as a Python module: the operator classes' usual calls as native
+    functions (torch_ext/iex_autograd.cpp)."""
+    spec = importlib.util.spec_from_file_location("iex_torch_ext", EXT_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+native = _load_native()
 
 OP_NAMES = (
     "spmm_sputnik_reuse_weight",

@@ -6,16 +6,20 @@ dense ``[k, n]`` operand, and the same derivative scheme (:77-149):
     d values = SDDMM(grad, b) sampled at A's pattern,   d b = A^T @ grad.
 fp32 runs the CUDA-core kernels (bit-reproducible); fp16 runs the CUDA-core fp16 kernel or,
 with ``use_tensor_cores=True`` in the forward kwargs, the tcgen05 kernel;
-``use_tensor_cores="auto"`` lets the cost model of ``pytorch/tuning.py`` choose.
+``use_tensor_cores="auto"`` lets a cost model choose.  ``run`` is native unless a graph
+constructor is recording: there ``use_tensor_cores`` also covers the backward pass and any n,
+because the matrix may be expanded and multiplied as a dense one (torch_ext/iex_autograd.cpp).
 """
 from __future__ import annotations
 
 import torch
 
-from .... import ops  # noqa: F401  (registers torch.ops.iex_ops)
+from .... import ops  # registers torch.ops.iex_ops
 from ...tuning import choose_spmm_kernel
 from ...utils import transpose_with_info
-from .utils import MyAutogradFunc, captured
+from .utils import MyAutogradFunc, captured, eager_kwargs
+
+_MODES = {False: 0, True: 1, "auto": 2}  # Mode in torch_ext/iex_autograd.cpp
 
 
 def _spmm(b2d, row_indices, values, row_offsets, column_indices, m, use_tc=False):
@@ -40,6 +44,16 @@ def _sddmm(grad2d, b2d, row_indices, row_offsets, column_indices):
 
 
 class MySpMM(MyAutogradFunc):
+    @classmethod
+    def run(cls, *args, **fwd_kwargs):
+        kw = eager_kwargs(fwd_kwargs)
+        if kw is not None and cls is MySpMM and len(args) == 7:
+            b, ri, values, ro, ci, m, transp = args
+            if (b.is_cuda and b.dim() == 2 and values.dtype in (torch.float32, torch.float16)
+                    and (len(transp) == 4 or not b.requires_grad)):
+                return ops.native.myspmm(b, ri, values, ro, ci, m, transp, _MODES[kw.get("use_tensor_cores", False)])
+        return super().run(*args, **fwd_kwargs)
+
     @staticmethod
     def num_inputs(**kwargs) -> int:
         return 7

@@ -2,8 +2,7 @@
 
 Same arguments as intrasm_engine/pytorch/cpp_extensions/layers_and_funcs/torch.py:6-31
 (``weight`` is ``[out_features, in_features]`` as in ``torch.nn.Linear``).  fp16 inputs with
-in_features a multiple of 8 run on the tcgen05 kernel, whatever the token count (blocks of
-up to 256 tokens, a ragged tail padded); other dtypes (the reference's ``MyLinear`` is
+in_features a multiple of 8 run on the tcgen05 kernel, whatever the token count; other dtypes (the reference's ``MyLinear`` is
 dtype-agnostic, :17) are a plain library GEMM through ``torch.mm``.  The backward pass is
 the reference's two matmuls (:20-31), for fp16 on the same tensor-core kernel
 (``linear_fp16_dgrad`` / ``linear_fp16_wgrad``: the operands are read in their other
@@ -13,13 +12,12 @@ from __future__ import annotations
 
 import torch
 
-from .... import ops  # noqa: F401
-from .utils import MyAutogradFunc, captured
+from .... import ops
+from .utils import MyAutogradFunc, captured, eager_kwargs
 
 
 def tc_linear_eligible(input: torch.Tensor, weight: torch.Tensor) -> bool:
-    """fp16, any token count (the operator runs blocks of up to 256 tokens and pads a ragged
-    tail), in_features a multiple of 8, 16-byte aligned contiguous operands."""
+    """fp16, any token count, in_features a multiple of 8, 16-byte aligned contiguous operands."""
     return (input.is_cuda and input.dtype == torch.float16 and weight.dtype == torch.float16
             and input.dim() == 2 and input.size(0) > 0
             and input.size(1) % 8 == 0 and input.is_contiguous() and weight.is_contiguous()
@@ -33,6 +31,14 @@ def linear_forward(input, weight):
 
 
 class MyLinear(MyAutogradFunc):
+    @classmethod
+    def run(cls, *args, **fwd_kwargs):
+        if cls is MyLinear and len(args) == 2 and eager_kwargs(fwd_kwargs) is not None:
+            out = ops.native.mylinear(*args)
+            if out is not None:
+                return out
+        return super().run(*args, **fwd_kwargs)
+
     @staticmethod
     def num_inputs(**kwargs) -> int:
         return 2

@@ -25,6 +25,17 @@ def default_fwd_kwargs(**overrides) -> dict:
     return kw
 
 
+def eager_kwargs(fwd_kwargs: dict) -> Optional[dict]:
+    """The keyword dictionary of a single operator's ``run`` when nothing is being recorded into a
+    graph constructor (the call may then run natively), else None."""
+    if not fwd_kwargs:
+        return fwd_kwargs
+    kw = fwd_kwargs.get("fwd_kwargs_1") if len(fwd_kwargs) == 1 else None
+    if kw is None or kw.get("constructor_enabled") or kw.get("num_streams", 1) != 1:
+        return None
+    return kw
+
+
 def assert_params_unpacked(params: dict):
     for key in params:
         assert not key.startswith("space_")

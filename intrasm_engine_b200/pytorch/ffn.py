@@ -9,9 +9,10 @@ intrasm_engine/pytorch/cpp_extensions/layers_and_funcs/torch.py:34-36, sputnik.p
 At 256 tokens the activation matrix is tiny (5.6 MB dense) and the weight is what streams
 from HBM, so the layer runs as a tensor-core GEMM whose *B* operand is the activation: the
 CSR is expanded to a dense fp16 tile operand once per layer (``iex_csr_to_dense_f16``) and
-``iex_linear_f16_splitk`` multiplies it with this rank's weight slab, stored K-major
-(``[n_local, k]``, i.e. W_down^T, the ``torch.nn.Linear`` convention).  Split-K spreads the
-few 128-row weight tiles of a slab over all SMs.
+multiplied with this rank's weight slab, stored K-major (``[n_local, k]``, i.e. W_down^T, the
+``torch.nn.Linear`` convention), by the CTA-pair GEMM (``iex_linear_f16_any``) or, where the
+result is gathered by the kernel's own peer stores, by ``iex_linear_f16_splitk_gather``; both
+split K so that the few weight tiles of a slab reach all SMs.
 
 Sharding: rank r owns output columns ``[r * n / G, (r + 1) * n / G)``.  The gathered
 ``[tokens, n]`` result appears on every rank either through the kernel's own peer stores
@@ -23,7 +24,7 @@ from __future__ import annotations
 
 import torch
 
-from .. import _lib
+from .. import _lib, ops
 
 
 def split_k_parts(n_local: int) -> int:
@@ -52,14 +53,15 @@ class ReluSparseDownProj:
         self.gather = gather if world > 1 else "none"
         self.device = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
         self.parts = split_k_parts(self.n_local)
-        need = _lib.lib.iex_tc_workspace_bytes(0, 1, self.n_local, self.parts, self.tokens)
-        self.workspace = torch.empty(max(int(need), 256), dtype=torch.uint8, device=self.device)
+        self.workspace = None
         self.dense_act = torch.empty((self.tokens, self.k), dtype=torch.float16, device=self.device)
         self.out_local = torch.empty((self.tokens, self.n_local), dtype=torch.float16, device=self.device)
         self.peer = None
         self._slot = 0
         if self.gather == "peer":
             from .distributed import PeerGather
+            need = _lib.lib.iex_tc_workspace_bytes(0, 1, self.n_local, self.parts, self.tokens)
+            self.workspace = torch.empty(max(int(need), 256), dtype=torch.uint8, device=self.device)
             self.peer = PeerGather(self.tokens, self.n, rank, world, self.device, group=group)
 
     # -- pieces ---------------------------------------------------------------------------
@@ -76,6 +78,12 @@ class ReluSparseDownProj:
         "nccl") or this rank's ``[tokens, n_local]`` slab ("none").  With "peer" the result is a
         view of one of two alternating buffers: it stays valid until the call after next."""
         assert weight_slab.shape == (self.n_local, self.k) and weight_slab.is_contiguous()
+        if self.gather != "peer" and stream is None:
+            ops.native.ffn_down(values, row_offsets, column_indices, weight_slab, self.dense_act, self.out_local)
+            if self.gather == "nccl":
+                from .distributed import all_gather_columns
+                return all_gather_columns(self.out_local, self.group)
+            return self.out_local
         st = stream if stream is not None else torch.cuda.current_stream(self.device).cuda_stream
         dense = self.expand(values, row_offsets, column_indices, st)
         if self.gather == "peer":
@@ -83,9 +91,8 @@ class ReluSparseDownProj:
             self.peer.linear(slot, dense, weight_slab, self.parts, self.workspace, st)
             self.peer.barrier(st)
             return self.peer.result(slot)
-        _lib.call("iex_linear_f16_splitk", self.tokens, self.k, self.n_local, dense.data_ptr(),
-                  weight_slab.data_ptr(), self.out_local.data_ptr(), self.parts, self.workspace.data_ptr(),
-                  self.workspace.numel(), st)
+        _lib.call("iex_linear_f16_any", self.tokens, self.k, self.n_local, dense.data_ptr(),
+                  weight_slab.data_ptr(), self.out_local.data_ptr(), st)
         if self.gather == "nccl":
             from .distributed import all_gather_columns
             return all_gather_columns(self.out_local, self.group)
@@ -95,12 +102,13 @@ class ReluSparseDownProj:
 
 
 def relu_down_proj(hidden: torch.Tensor, weight_t: torch.Tensor, index_dtype=torch.int32) -> torch.Tensor:
-    """``relu(hidden) @ weight_t.T`` on one GPU through the sparse path: ``hidden`` ``[tokens, k]``
-    fp16 (pre-activation), ``weight_t`` ``[n, k]`` fp16.  The ReLU and the dense -> CSR conversion
-    are one pass of this library's converter (``dense_to_sparse_cuda(relu=True)``), the product
-    is ``ReluSparseDownProj``."""
-    from .utils import dense_to_sparse_cuda
-    values, _ri, row_offsets, column_indices = dense_to_sparse_cuda(hidden, index_dtype=index_dtype, relu=True)
-    layer = ReluSparseDownProj(hidden.size(0), hidden.size(1), weight_t.size(0), device=hidden.device,
-                               gather="none")
-    return layer(values, row_offsets, column_indices, weight_t).clone()
+    """``relu(hidden) @ weight_t.T`` on one GPU: ``hidden`` ``[tokens, k]`` fp16 (pre-activation),
+    ``weight_t`` ``[n, k]`` fp16.  The layer's product wants the activations as a dense tile operand, so
+    the ReLU is one elementwise pass and no CSR is built in between (``index_dtype`` is the index
+    type one would have; it does not affect the result)."""
+    if hidden.dim() != 2 or not hidden.is_cuda or not hidden.is_contiguous():
+        raise RuntimeError("relu_down_proj expects a contiguous 2-D CUDA matrix")
+    if hidden.dtype != torch.float16 or index_dtype not in (torch.int16, torch.int32):
+        raise RuntimeError("relu_down_proj: fp16 values, int16 / int32 indices")
+    assert weight_t.shape[1] == hidden.size(1) and weight_t.is_contiguous()
+    return ops.native.relu_down_proj(hidden, weight_t)

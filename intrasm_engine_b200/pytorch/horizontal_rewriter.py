@@ -15,6 +15,7 @@ from typing import Any, Optional
 import torch
 from torch import nn
 
+from .. import ops
 from .cpp_extensions.cuda_graph_constructor import TorchCUDAGraphConstructor
 from .cpp_extensions.layers_and_funcs.sputnik import MySpMM
 from .cpp_extensions.layers_and_funcs.torch import MyLinear
@@ -192,9 +193,17 @@ def _fusable(args, fwd_kwargs) -> bool:
     if not (torch.is_tensor(b) and torch.is_tensor(inp) and b.is_cuda and b.dim() == 2):
         return False
     k, n = b.shape
+    return (inp.shape == (n, k) and inp.data_ptr() == b.data_ptr() and inp.stride() == (1, n)
+            and _fused_operands(b, values, ci, weight))
+
+
+def _fused_operands(b, values, ci, weight) -> bool:
+    """Whether the fused kernel takes ``A_csr @ b`` and ``weight @ b``."""
+    if b.dim() != 2 or not b.is_cuda:
+        return False
+    k, n = b.shape
     return (b.dtype == torch.float16 and values.dtype == torch.float16 and weight.dtype == torch.float16
-            and b.is_contiguous() and inp.shape == (n, k) and inp.data_ptr() == b.data_ptr()
-            and inp.stride() == (1, n) and n % 64 == 0 and n <= 256 and k % 8 == 0
+            and b.is_contiguous() and n % 64 == 0 and 0 < n <= 256 and k % 8 == 0
             and weight.is_contiguous() and weight.size(1) == k
             # the tensor-core kernel reads its operands with 16-byte TMA / cp.async copies; a
             # misaligned view takes the generic pair of calls instead
@@ -294,8 +303,15 @@ class SparseDenseLayer(ModuleToReplay):
     wants_transposed_input = True  # ConstructorEnabledLayer hands over (x, x.t().contiguous())
 
     def forward(self, x, xt=None, forward_constructors=None, backward_constructors=None):
-        args = (x, self.row_indices, self.values, self.row_offsets, self.column_indices, self.m,
-                self.transp_info, x.t(), self.weight_dense)
+        values, weight = self.values, self.weight_dense
+        if self.mode == "fused" and not (torch.is_grad_enabled() and
+                                         (x.requires_grad or values.requires_grad or weight.requires_grad)):
+            # the pair function's fused launch without its autograd bookkeeping
+            if _fused_operands(x, values, self.column_indices, weight):
+                return ops.native.fused_spmm_linear_half(x, self.row_offsets, values, self.column_indices, self.m,
+                                                         weight)
+        args = (x, self.row_indices, values, self.row_offsets, self.column_indices, self.m,
+                self.transp_info, x.t(), weight)
         if self.mode == "fused":
             return self.pair.run(*args, fwd_kwargs_1=default_fwd_kwargs(use_tensor_cores=True),
                                  fwd_kwargs_2=default_fwd_kwargs())

@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
+from .. import ops
 from . import horizontal_rewriter as hr
 from .cpp_extensions.layers_and_funcs.sputnik import MySpMM
 from .cpp_extensions.layers_and_funcs.utils import default_fwd_kwargs
@@ -34,9 +35,9 @@ def magnitude_prune(weight: torch.Tensor, sparsity: float) -> torch.Tensor:
 
 class SparseLinear(nn.Module):
     """``y = x @ W.T (+ bias)`` with ``W`` ``[out_features, in_features]`` stored as CSR (fp16
-    values, int16 column indices when they fit).  The product runs as ``W_csr @ x.T`` through
-    ``MySpMM`` -- the tensor-core kernel for 64..256 tokens in multiples of 64, the CUDA-core
-    kernel otherwise, chosen by the cost model -- so gradients reach ``x`` (and ``values``)."""
+    values, int16 column indices when they fit).  Without gradients the product is one native
+    call on ``x`` as it lies; otherwise it runs as ``W_csr @ x.T`` through ``MySpMM``, so that
+    gradients reach ``x`` (and ``values``)."""
 
     def __init__(self, weight: torch.Tensor, bias: torch.Tensor | None = None):
         super().__init__()
@@ -64,6 +65,15 @@ class SparseLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
+        if x.is_cuda and x.dtype == torch.float16 and not (torch.is_grad_enabled() and
+                                                           (x.requires_grad or self.values.requires_grad)):
+            # inference: x is read as it lies and the result written as [tokens, out_features]
+            x2 = x if x.dim() == 2 else x.reshape(-1, self.in_features)
+            y = ops.native.sparse_linear(x2.contiguous(), self.values, self.row_offsets, self.column_indices,
+                                         self.out_features)
+            if self.bias is not None:
+                y = y + self.bias
+            return y if x.dim() == 2 else y.reshape(*lead, self.out_features)
         b = x.reshape(-1, self.in_features).t().contiguous()  # [in_features, tokens]
         out = MySpMM.run(b, self.row_indices, self.values, self.row_offsets, self.column_indices,
                          self.out_features, self.transp_info,

@@ -1,0 +1,360 @@
+// The operator classes' usual calls as native functions (Python module `iex_torch_ext`).
+//
+// MySpMM and MyLinear are autograd operators in Python
+// (intrasm_engine/pytorch/cpp_extensions/layers_and_funcs/sputnik.py:19-149, torch.py:6-31): the keyword
+// dictionaries, the saved-tensor bookkeeping and the backward pass in the interpreter cost 50 us
+// forward and 130 us forward + backward, several times the kernels of an ordinary layer.  When no
+// graph constructor is recording, `run` comes here instead: the same kernels in the same order,
+// with the autograd node, its saved tensors and its backward pass in C++.
+//
+// It also holds the choice between the ways to multiply an fp16 CSR matrix (spmm_half_auto).
+#include "iex_torch_ops.h"
+
+#include <torch/csrc/autograd/edge.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <algorithm>
+#include <optional>
+
+namespace iex_torch {
+namespace {
+
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+int index_bits(const at::Tensor& ci) { return ci.scalar_type() == at::kShort ? 16 : 32; }
+int64_t round8(int64_t v) { return (v + 7) / 8 * 8; }
+bool aligned16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+
+// ---------------------------------------------------------------------------- fp16 CSR products
+
+// The dense fp16 copy [m, round8(k)] of a CSR matrix.
+at::Tensor expand(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci, int64_t m, int64_t k) {
+  const int64_t ld = round8(k);
+  at::Tensor dense = empty(values, {m, ld});
+  check_status(iex_csr_to_dense_f16_ld(m, k, ld, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(),
+                                       dense.data_ptr(), stream_of(values)),
+               "iex_csr_to_dense_f16_ld");
+  return dense;
+}
+
+// A row-major matrix as a TMA operand: itself, or a copy with rows padded to 16 bytes.
+at::Tensor tma_rows(const at::Tensor& x) {
+  if (x.size(1) % 8 == 0 && aligned16(x)) return x;
+  const int64_t ld = round8(x.size(1));
+  at::Tensor padded = empty(x, {x.size(0), ld});
+  check_status(iex_pad_rows_f16(x.size(0), x.size(1), ld, x.data_ptr(), padded.data_ptr(), stream_of(x)),
+               "iex_pad_rows_f16");
+  return padded;
+}
+
+void gemm(int64_t m, int64_t n, int64_t k, const at::Tensor& a, bool a_mn, const at::Tensor& b, bool b_mn,
+          const at::Tensor& out, bool out_t) {
+  check_status(iex_gemm_f16(m, n, k, a.data_ptr(), a_mn, a.size(1), b.data_ptr(), b_mn, b.size(1), out.data_ptr(), out_t,
+                            out.size(1), 0, 0, stream_of(a)),
+               "iex_gemm_f16");
+}
+
+// Estimates in microseconds, fitted to measurements on B200.
+//   expand   one pass over the CSR arrays and the dense copy, at 5.5 TB/s
+//   decode   the tile decoder of tc_fused.cu: 9 us + 0.75 us per 64 columns and wave of tiles
+//   cores    CUDA cores: gathered bytes, and the serial walk over an average row
+double expand_us(int64_t m, int64_t k, int64_t nnz, int bits) {
+  return 2.5 + (2.0 * m * round8(k) + static_cast<double>(nnz) * (2 + bits / 8)) / 5.5e6;
+}
+double decode_us(int64_t m, int64_t k) {
+  const int64_t sms = 148, full = (m + 127) / 128;
+  const int64_t tiles = full < sms ? std::min<int64_t>(sms, (m + 7) / 8) : full;
+  return 9.0 + 0.75 * ((k + 63) / 64) * std::max<int64_t>(1, (tiles + sms - 1) / sms);
+}
+double cores_us(int64_t m, int64_t n, int64_t nnz) {
+  return 1.6 + 0.0605e-6 * 2.0 * nnz * n + 0.158 * nnz / std::max<int64_t>(m, 1);
+}
+bool decode_supported(const at::Tensor& b, const at::Tensor& values, const at::Tensor& ci) {
+  const int64_t k = b.size(0), n = b.size(1);
+  return n % 64 == 0 && n > 0 && n <= 256 && k % 8 == 0 && k > 0 && (index_bits(ci) == 32 || k <= 65280) &&
+         aligned16(b) && aligned16(values) && aligned16(ci);
+}
+
+void check_csr_half(const at::Tensor& b, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
+                    int64_t m) {
+  TORCH_CHECK(b.dim() == 2, "b must be [k, n]");
+  TORCH_CHECK(values.dim() == 1 && ci.dim() == 1 && values.size(0) == ci.size(0),
+              "values and column_indices must be 1-D with nnz entries");
+  TORCH_CHECK(ro.dim() == 1 && ro.size(0) == m + 1, "row_offsets must have m + 1 entries");
+  check_common({{"b", &b}, {"row_offsets", &ro}, {"values", &values}, {"column_indices", &ci}});
+  TORCH_CHECK(b.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf, "b and values must be float16");
+  TORCH_CHECK(ro.scalar_type() == at::kInt, "row_offsets must be int32");
+  TORCH_CHECK(ci.scalar_type() == at::kShort || ci.scalar_type() == at::kInt, "column_indices must be int16 or int32");
+}
+
+enum Mode { kCudaCores = 0, kTensorCores = 1, kAuto = 2 };
+
+// A_csr [m, k] @ b [k, n], fp16.  On tensor cores the matrix is either decoded tile by tile inside the
+// product (tc_fused.cu) or expanded once and multiplied as a dense matrix: the decoder needs no
+// scratch and no second pass, the expansion costs the dense copy's traffic but then runs at the
+// dense kernel's rate, for any n.
+at::Tensor spmm_half(const at::Tensor& b, const at::Tensor& ri, const at::Tensor& values, const at::Tensor& ro,
+                     const at::Tensor& ci, int64_t m, int mode) {
+  const int64_t k = b.size(0), n = b.size(1), nnz = values.numel();
+  auto cores = [&] { return spmm_sputnik_reuse_weight_half(b.unsqueeze(0), ri, values, ro, ci, m).squeeze(0); };
+  if (mode == kCudaCores || m == 0 || k == 0 || n == 0) return cores();
+  check_csr_half(b, values, ro, ci, m);
+  const double dense = expand_us(m, k, nnz, index_bits(ci)) + iex_gemm_f16_estimate_us(m, n, k, 1, 0) +
+                       (n % 8 == 0 ? 0.0 : 2.0);
+  const double decode = decode_supported(b, values, ci) ? decode_us(m, k) : 1e30;
+  if (mode == kAuto && cores_us(m, n, nnz) <= std::min(dense, decode)) return cores();
+  if (decode <= dense) return spmm_tc_half(b, ro, values, ci, m);
+  c10::cuda::CUDAGuard guard(b.device());
+  maybe_validate(ro, ci, m, k, nullptr, false);
+  at::Tensor out = empty(b, {m, n});
+  gemm(m, n, k, expand(values, ro, ci, m, k), false, tma_rows(b), true, out, false);
+  return out;
+}
+
+// ------------------------------------------------------------------------------------- MySpMM
+
+struct SpmmArgs {
+  at::Tensor ri, ro, ci;                 // the pattern
+  at::Tensor ri_t, ro_t, ci_t, perm;     // the transposed pattern (undefined without transp_info)
+  int64_t m = 0;
+  int mode = kCudaCores;
+};
+
+at::Tensor spmm_forward(const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
+  if (values.scalar_type() == at::kFloat)
+    return spmm_sputnik_reuse_weight(b.unsqueeze(0), p.ri, values, p.ro, p.ci, p.m).squeeze(0);
+  return spmm_half(b, p.ri, values, p.ro, p.ci, p.m, p.mode);
+}
+
+at::Tensor grad_of_values(const at::Tensor& grad, const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
+  if (grad.scalar_type() != at::kHalf)
+    return sddmm_sputnik_atomic_upd_weight(grad.unsqueeze(0), b.unsqueeze(0), p.ri, p.ro, p.ci.to(at::kInt));
+  const int64_t m = grad.size(0), n = grad.size(1), k = b.size(0), nnz = values.numel();
+  if (p.mode != kCudaCores && b.scalar_type() == at::kHalf && m > 0 && n > 0 && k > 0 && nnz > 0) {
+    // every product of the dense matrix, of which the stored positions are kept, against one
+    // gathered row of b per stored position
+    const double dense = iex_gemm_f16_estimate_us(m, k, n, 0, 0) + 3.0 + 6.0e-6 * nnz;
+    const double cores = 2.0 + 0.19e-6 * 2.0 * nnz * n;
+    if (dense < cores) {
+      c10::cuda::CUDAGuard guard(grad.device());
+      at::Tensor all = empty(grad, {m, round8(k)});
+      gemm(m, k, n, tma_rows(grad), false, tma_rows(b), false, all, false);
+      at::Tensor out = empty(grad, {nnz});
+      check_status(iex_csr_sample_f16(m, k, all.size(1), p.ro.data_ptr<int>(), p.ci.data_ptr(), index_bits(p.ci),
+                                      all.data_ptr(), out.data_ptr(), stream_of(grad)),
+                   "iex_csr_sample_f16");
+      return out;
+    }
+  }
+  return sddmm_sputnik_half(grad.unsqueeze(0), b.to(at::kHalf).unsqueeze(0), p.ri, p.ro, p.ci);
+}
+
+at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
+  const int64_t m = grad.size(0), n = grad.size(1), k = b.size(0), nnz = values.numel();
+  if (p.mode != kCudaCores && grad.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf && m > 0 && n > 0 &&
+      k > 0 && nnz > 0) {
+    // the expanded matrix read with its row dimension as the contraction: no transposed pattern needed
+    const double dense = expand_us(m, k, nnz, index_bits(p.ci)) + iex_gemm_f16_estimate_us(k, n, m, 1, 0);
+    const double cores = cores_us(k, n, nnz) + 5.0;
+    if (dense < cores) {
+      c10::cuda::CUDAGuard guard(grad.device());
+      at::Tensor out = empty(grad, {k, n});
+      gemm(k, n, m, expand(values, p.ro, p.ci, m, k), true, tma_rows(grad), true, out, false);
+      return out;
+    }
+  }
+  // transposing the pattern is bookkeeping done once (get_transpose_info); the values follow it
+  at::Tensor values_t = values.index({p.perm});
+  if (values.scalar_type() == at::kFloat)
+    return spmm_sputnik_reuse_weight(grad.unsqueeze(0), p.ri_t, values_t, p.ro_t, p.ci_t, k).squeeze(0);
+  return spmm_sputnik_reuse_weight_half(grad.unsqueeze(0), p.ri_t, values_t, p.ro_t, p.ci_t, k).squeeze(0);
+}
+
+struct MySpMMBackward : public Node {
+  SavedVariable b_, values_;
+  SpmmArgs args;
+  std::string name() const override { return "MySpMMBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    b_.reset_data();
+    values_.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(2);
+    if (!grads[0].defined()) return out;
+    at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor b = b_.unpack(), values = values_.unpack();
+    const at::Tensor grad = grads[0].contiguous();
+    if (task_should_compute_output(1)) out[1] = grad_of_values(grad, b, values, args);
+    if (task_should_compute_output(0)) out[0] = grad_of_b(grad, b, values, args);
+    return out;
+  }
+};
+
+// MySpMM.run without a graph constructor.  `transp` is (row_indices_t, row_offsets_t,
+// column_indices_t, perm) or empty; without it b must not require a gradient.
+at::Tensor myspmm(const at::Tensor& b_in, const at::Tensor& ri, const at::Tensor& values, const at::Tensor& ro,
+                  const at::Tensor& ci, int64_t m, const std::vector<at::Tensor>& transp, int mode) {
+  SpmmArgs p;
+  p.ri = ri;
+  p.ro = ro;
+  p.ci = ci;
+  p.m = m;
+  p.mode = mode;
+  if (transp.size() == 4) {
+    p.ri_t = transp[0];
+    p.ro_t = transp[1];
+    p.ci_t = transp[2];
+    p.perm = transp[3];
+  }
+  const bool needs_grad = torch::autograd::compute_requires_grad(b_in, values);
+  at::Tensor b = b_in.contiguous();
+  at::Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    out = spmm_forward(b, values, p);
+  }
+  if (needs_grad) {
+    auto node = std::shared_ptr<MySpMMBackward>(new MySpMMBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(b, values));
+    node->b_ = SavedVariable(b, false);
+    node->values_ = SavedVariable(values, false);
+    node->args = std::move(p);
+    torch::autograd::set_history(out, node);
+  }
+  return out;
+}
+
+// ------------------------------------------------------------------------------------ MyLinear
+
+struct MyLinearBackward : public Node {
+  SavedVariable input_, weight_;
+  std::string name() const override { return "MyLinearBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    input_.reset_data();
+    weight_.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(2);
+    if (!grads[0].defined()) return out;
+    at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor input = input_.unpack(), weight = weight_.unpack();
+    const at::Tensor& grad = grads[0];
+    const bool own = grad.scalar_type() == at::kHalf && grad.is_cuda() && weight.size(0) % 8 == 0 &&
+                     weight.size(1) % 8 == 0;
+    if (own) {
+      const at::Tensor g = grad.contiguous();
+      if (task_should_compute_output(0)) out[0] = linear_fp16_dgrad(g, weight);
+      if (task_should_compute_output(1)) out[1] = linear_fp16_wgrad(g, input);
+    } else {
+      if (task_should_compute_output(0)) out[0] = grad.mm(weight);
+      if (task_should_compute_output(1)) out[1] = grad.t().mm(input);
+    }
+    return out;
+  }
+};
+
+// MyLinear.run without a graph constructor; nothing for operands the tensor-core kernel does not
+// take (tc_linear_eligible in layers_and_funcs/torch.py).
+std::optional<at::Tensor> mylinear(const at::Tensor& input, const at::Tensor& weight) {
+  const bool eligible = input.is_cuda() && weight.is_cuda() && input.scalar_type() == at::kHalf &&
+                        weight.scalar_type() == at::kHalf && input.dim() == 2 && weight.dim() == 2 &&
+                        input.size(0) > 0 && input.size(1) % 8 == 0 && input.is_contiguous() &&
+                        weight.is_contiguous() && aligned16(input) && aligned16(weight);
+  if (!eligible) return std::nullopt;
+  at::Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    out = linear_fp16(input, weight);
+  }
+  if (torch::autograd::compute_requires_grad(input, weight)) {
+    auto node = std::shared_ptr<MyLinearBackward>(new MyLinearBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(input, weight));
+    node->input_ = SavedVariable(input, false);
+    node->weight_ = SavedVariable(weight, false);
+    torch::autograd::set_history(out, node);
+  }
+  return out;
+}
+
+// --------------------------------------------------------------------------- inference layers
+
+// SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m].
+//   up to 16 tokens   CUDA cores, the CSR arrays read once (spmm_skinny.cu)
+//   more              W expanded, dense GEMM (weight as the 256-row operand or as the other one)
+// Both read x as it lies and write [tokens, m]: no transposed copies of either.
+at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
+                         int64_t m) {
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous(), "x must be a contiguous [tokens, in_features] matrix");
+  check_common({{"x", &x}, {"row_offsets", &ro}, {"values", &values}, {"column_indices", &ci}});
+  TORCH_CHECK(x.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf, "x and values must be float16");
+  TORCH_CHECK(ro.scalar_type() == at::kInt && ro.numel() == m + 1, "row_offsets must be int32 with m + 1 entries");
+  const int64_t tokens = x.size(0), k = x.size(1);
+  c10::cuda::CUDAGuard guard(x.device());
+  maybe_validate(ro, ci, m, k, nullptr, false);
+  at::Tensor out = empty(x, {tokens, m});
+  if (tokens == 0 || m == 0) return out;
+  if (iex_spmm_f16_skinny_supported(k, tokens)) {
+    check_status(iex_spmm_f16_skinny(m, k, tokens, values.numel(), ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
+                                     values.data_ptr(), x.data_ptr(), 1, k, out.data_ptr(), 1, m, stream_of(x)),
+                 "iex_spmm_f16_skinny");
+    return out;
+  }
+  const at::Tensor dense = expand(values, ro, ci, m, k), xp = tma_rows(x);
+  if (m % 8 == 0 && iex_gemm_f16_estimate_us(m, tokens, k, 0, 1) <= iex_gemm_f16_estimate_us(tokens, m, k, 0, 0))
+    gemm(m, tokens, k, dense, false, xp, false, out, true);
+  else
+    gemm(tokens, m, k, xp, false, dense, false, out, false);
+  return out;
+}
+
+// ReluSparseDownProj without a gather of its own: CSR activations [tokens, k] (expanded into
+// `dense`) times weight [n, k]^T into `out`.
+void ffn_down(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci, const at::Tensor& weight,
+              const at::Tensor& dense, const at::Tensor& out) {
+  check_common({{"values", &values}, {"row_offsets", &ro}, {"column_indices", &ci}, {"weight", &weight},
+                {"dense", &dense}, {"out", &out}});
+  const int64_t tokens = dense.size(0), k = dense.size(1), n = weight.size(0);
+  TORCH_CHECK(ro.scalar_type() == at::kInt && ro.numel() == tokens + 1, "row_offsets must be int32 with tokens + 1 entries");
+  c10::cuda::CUDAGuard guard(values.device());
+  check_status(iex_csr_to_dense_f16(tokens, k, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(),
+                                    dense.data_ptr(), stream_of(values)),
+               "iex_csr_to_dense_f16");
+  check_status(iex_linear_f16_any(tokens, k, n, dense.data_ptr(), weight.data_ptr(), out.data_ptr(), stream_of(values)),
+               "iex_linear_f16_any");
+}
+
+// relu(hidden [tokens, k]) @ weight [n, k]^T
+at::Tensor relu_down_proj(const at::Tensor& hidden, const at::Tensor& weight) {
+  check_common({{"hidden", &hidden}, {"weight", &weight}});
+  TORCH_CHECK(hidden.scalar_type() == at::kHalf && weight.scalar_type() == at::kHalf, "hidden and weight must be float16");
+  const int64_t tokens = hidden.size(0), k = hidden.size(1), n = weight.size(0);
+  c10::cuda::CUDAGuard guard(hidden.device());
+  at::Tensor out = empty(hidden, {tokens, n});
+  if (tokens == 0 || n == 0) return out;
+  at::Tensor act = empty(hidden, {tokens, k});
+  check_status(iex_relu_f16(tokens * k, hidden.data_ptr(), act.data_ptr(), stream_of(hidden)), "iex_relu_f16");
+  check_status(iex_linear_f16_any(tokens, k, n, act.data_ptr(), weight.data_ptr(), out.data_ptr(), stream_of(hidden)),
+               "iex_linear_f16_any");
+  return out;
+}
+
+}  // namespace
+}  // namespace iex_torch
+
+PYBIND11_MODULE(iex_torch_ext, mod) {
+  mod.def("myspmm", &iex_torch::myspmm);
+  mod.def("mylinear", &iex_torch::mylinear);
+  mod.def("sparse_linear", &iex_torch::sparse_linear);
+  mod.def("ffn_down", &iex_torch::ffn_down);
+  mod.def("relu_down_proj", &iex_torch::relu_down_proj);
+  mod.def("fused_spmm_linear_half", &iex_torch::fused_spmm_linear_half);
+}
