@@ -218,6 +218,22 @@ IEX_API int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long long
 /* Time this library expects iex_gemm_f16 to take on the current device, for choosing between ways. */
 IEX_API double iex_gemm_f16_estimate_us(int m, int n, int k, int b_mn, int out_transposed);
 
+/* CSR SpMM and dense linear on the same activations in one launch, either of them alone with the
+ * other's row count 0.  x is [k, n] (n a multiple of 8) or, with x_tokens_major, [n, k] (k a multiple of
+ * 8); n <= 256.  Each output is [rows, n] or, with its tokens-major flag, [n, rows].  `bias`
+ * (nullable) makes the sparse output relu(sum + bias[row]).  Columns ascend within a row. */
+IEX_API int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n, int nnz, const int32_t* row_offsets,
+                                     const void* column_indices, int index_bits, const void* values,
+                                     const void* weight, const void* x, int x_tokens_major, const float* bias,
+                                     void* out_sparse, int sparse_tokens_major, void* out_dense,
+                                     int dense_tokens_major, void* stream);
+
+/* Two dense linears on the same activations in one launch: out_i = weight_i [m_i, k] * x, layouts and limits
+ * as above. */
+IEX_API int iex_linear_pair_f16(int m0, int m1, int k, int n, const void* weight0, const void* weight1,
+                                const void* x, int x_tokens_major, void* out0, int tokens_major0, void* out1,
+                                int tokens_major1, void* stream);
+
 /* CSR SpMM with 1 to 16 dense columns (decoding steps), fp16, fp32 accumulation, CUDA cores:
  * out(r, t) = sum_p values[p] * x(col[p], t).  The strides are in elements, so x and out may be
  * [k, n] / [m, n] or [n, k] / [n, m].  values 4-byte, column_indices 2 * sizeof(index) aligned. */

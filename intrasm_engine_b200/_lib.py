@@ -69,6 +69,13 @@ SIGNATURES = {
                              c_int, c_int, c_ptr]),
     # m n k b_mn out_transposed
     "iex_gemm_f16_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int, c_int]),
+    # m_sparse m_dense k n nnz row_offsets cols index_bits values weight x x_tokens_major bias
+    # out_sparse sparse_tokens_major out_dense dense_tokens_major stream
+    "iex_spmm_linear_f16_tile": (c_int, [c_int, c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr,
+                                         c_int, c_ptr, c_ptr, c_int, c_ptr, c_int, c_ptr]),
+    # m0 m1 k n weight0 weight1 x x_tokens_major out0 tokens_major0 out1 tokens_major1 stream
+    "iex_linear_pair_f16": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_int, c_ptr, c_int,
+                                    c_ptr]),
     "iex_spmm_f16_skinny_supported": (c_int, [c_int, c_int]),
     # m k n nnz row_offsets cols index_bits values x x_row x_col out out_row out_col stream
     "iex_spmm_f16_skinny": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ll, c_ll,

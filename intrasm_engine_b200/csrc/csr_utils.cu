@@ -158,73 +158,87 @@ csr_to_dense_f16_kernel(int m, int k, int slice, const int* __restrict__ row_off
   }
 }
 
-// The same for matrices of many rows: TPR threads (a warp or a whole block) build a row in shared
-// memory and store it with 16-byte pieces, so the dense row is written once instead of cleared
-// and then scattered into (two-byte stores to global memory cost a 32-byte sector each at low
-// density and one L2 transaction per warp and 64 columns at best).  Neighbouring lanes take
-// neighbouring pairs of nonzeros: the pair loads are coalesced, and because columns ascend the
-// two-byte shared-memory stores of a warp fall into neighbouring banks.  kU pairs per thread are
-// requested before the first store: eight blocks of 256 threads keep about 64 KB in flight per SM,
-// what HBM latency asks for.  11008 x 4096 at 50 %: bound by HBM, 180 MB.
+// The same for matrices of many rows: TPR threads (a warp, or a block where a row needs more shared memory)
+// build a row in shared memory and store it with 16-byte pieces, so the dense row is written once
+// instead of cleared and then scattered into.  Neighbouring lanes take neighbouring pairs of nonzeros:
+// the pair loads are coalesced, and because columns ascend the two-byte shared-memory stores of a warp
+// fall into neighbouring banks.  kU pairs per thread are requested before the first store; a first or last
+// nonzero whose partner belongs to another row is written alone, so the loop has no checks.
+// 11008 x 4096 at 50 %, 180 MB: 63 us as a block per row with a check per pair.
+template <typename IT>
+__device__ __forceinline__ void load_pair(const __half* values, const IT* cols, int p, uint32_t& v, int (&c)[2]) {
+  v = __ldg(reinterpret_cast<const uint32_t*>(values + p));
+  if constexpr (sizeof(IT) == 2) {
+    const uint32_t cc = __ldg(reinterpret_cast<const uint32_t*>(cols + p));
+    c[0] = static_cast<int>(cc & 0xffffu);
+    c[1] = static_cast<int>(cc >> 16);
+  } else {
+    const int2 cc = __ldg(reinterpret_cast<const int2*>(cols + p));
+    c[0] = cc.x;
+    c[1] = cc.y;
+  }
+}
+
 template <typename IT, int TPR>
 __global__ void __launch_bounds__(256)
 csr_expand_rows_kernel(int m, int ld, const int* __restrict__ row_offsets, const IT* __restrict__ cols,
                        const __half* __restrict__ values, __half* __restrict__ out) {
-  constexpr int kU = 4;
+  constexpr int kU = TPR == 32 ? 8 : 4;
   extern __shared__ __align__(16) uint8_t row_smem[];
   const int group = threadIdx.x / TPR, t = threadIdx.x % TPR;
-  constexpr int kGroups = 256 / TPR;
-  const uint32_t row_bytes = static_cast<uint32_t>(ld) * 2u;
-  uint8_t* buf = row_smem + group * row_bytes;
+  const int groups = blockDim.x / TPR;
+  uint8_t* buf = row_smem + group * (static_cast<uint32_t>(ld) * 2u);
   __half* row_buf = reinterpret_cast<__half*>(buf);
   uint4* row_vec = reinterpret_cast<uint4*>(buf);
   const int vecs = ld >> 3;
   auto sync = [] { if constexpr (TPR == 32) __syncwarp(); else __syncthreads(); };
+  auto put = [&](uint32_t v, const int (&c)[2]) {
+    row_buf[c[0]] = __ushort_as_half(static_cast<unsigned short>(v & 0xffffu));
+    row_buf[c[1]] = __ushort_as_half(static_cast<unsigned short>(v >> 16));
+  };
   for (int i = t; i < vecs; i += TPR) row_vec[i] = make_uint4(0u, 0u, 0u, 0u);
   grid_dependency_wait();
   grid_launch_dependents();
-  const int nnz = __ldg(row_offsets + m);
   sync();
-  for (int r = blockIdx.x * kGroups + group; r < m; r += gridDim.x * kGroups) {
-    const int beg = __ldg(row_offsets + r), end = __ldg(row_offsets + r + 1);
-    for (int p0 = (beg & ~1) + 2 * t; p0 < end; p0 += 2 * TPR * kU) {
+  const int step = gridDim.x * groups;
+  int r = blockIdx.x * groups + group;
+  int beg = 0, end = 0;
+  if (r < m) { beg = __ldg(row_offsets + r); end = __ldg(row_offsets + r + 1); }
+  for (; r < m; r += step) {
+    int next_beg = 0, next_end = 0;
+    if (r + step < m) { next_beg = __ldg(row_offsets + r + step); next_end = __ldg(row_offsets + r + step + 1); }
+    const int even_beg = (beg + 1) & ~1, even_end = end & ~1;
+    if (t == 0 && beg < end && (beg & 1)) row_buf[to_index(__ldg(cols + beg))] = __ldg(values + beg);
+    if (t == 1 && beg < end && (end & 1) && end - 1 >= even_beg) row_buf[to_index(__ldg(cols + end - 1))] = __ldg(values + end - 1);
+    int p0 = even_beg;
+    for (; p0 + 2 * TPR * kU <= even_end; p0 += 2 * TPR * kU) {
       uint32_t v[kU];
       int c[kU][2];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int p = p0 + 2 * TPR * u;
-        c[u][0] = c[u][1] = -1;
-        v[u] = 0u;
-        if (p + 1 < nnz && p < end) {
-          v[u] = __ldg(reinterpret_cast<const uint32_t*>(values + p));
-          if constexpr (sizeof(IT) == 2) {
-            const uint32_t cc = __ldg(reinterpret_cast<const uint32_t*>(cols + p));
-            c[u][0] = static_cast<int>(cc & 0xffffu);
-            c[u][1] = static_cast<int>(cc >> 16);
-          } else {
-            const int2 cc = __ldg(reinterpret_cast<const int2*>(cols + p));
-            c[u][0] = cc.x;
-            c[u][1] = cc.y;
-          }
-        } else if (p < end) {  // last nonzero of the arrays
-          v[u] = __half_as_ushort(__ldg(values + p));
-          c[u][0] = to_index(__ldg(cols + p));
-        }
-      }
+      for (int u = 0; u < kU; ++u) load_pair(values, cols, p0 + 2 * TPR * u + 2 * t, v[u], c[u]);
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int p = p0 + 2 * TPR * u;
-        if (p >= beg && p < end) row_buf[c[u][0]] = __ushort_as_half(static_cast<unsigned short>(v[u] & 0xffffu));
-        if (p + 1 < end) row_buf[c[u][1]] = __ushort_as_half(static_cast<unsigned short>(v[u] >> 16));
-      }
+      for (int u = 0; u < kU; ++u) put(v[u], c[u]);
+    }
+    if (p0 < even_end) {
+      uint32_t v[kU];
+      int c[kU][2];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (p0 + 2 * TPR * u + 2 * t < even_end) load_pair(values, cols, p0 + 2 * TPR * u + 2 * t, v[u], c[u]);
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (p0 + 2 * TPR * u + 2 * t < even_end) put(v[u], c[u]);
     }
     sync();
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(r) * ld);
+#pragma unroll 4
     for (int i = t; i < vecs; i += TPR) {
       dst[i] = row_vec[i];
       row_vec[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     sync();
+    beg = next_beg;
+    end = next_end;
   }
 }
 
@@ -364,10 +378,15 @@ int csr_to_dense(int m, int ld, const int* row_offsets, const IT* cols, const __
   const bool pairs = (reinterpret_cast<uintptr_t>(values) & 3u) == 0 &&
                      (reinterpret_cast<uintptr_t>(cols) & (2 * sizeof(IT) - 1)) == 0;
   if (m >= 4 * kNumSMs && ld % 8 == 0 && ld <= 24 * 1024 && pairs && aligned16(out)) {
-    // a warp per row while eight rows of 2 KB fit into a block's default shared memory
-    if (ld <= 2048)
-      return launch_overlapped(csr_expand_rows_kernel<IT, 32>, dim3(m / 8 < 7 * kNumSMs ? (m + 7) / 8 : 7 * kNumSMs),
-                               dim3(256), static_cast<size_t>(ld) * 16, s, m, ld, row_offsets, cols, values, out);
+    // a warp per row while the rows of 24 warps fit into an SM's shared memory, else a block per row
+    if (ld <= 4608) {
+      const int row_bytes = 2 * ld, fit = 48 * 1024 / row_bytes;  // a block's default shared memory
+      const int warps = fit < 8 ? fit : 8;
+      const int per_sm = 220 * 1024 / (row_bytes * warps) < 8 ? 220 * 1024 / (row_bytes * warps) : 8;
+      const int blocks = (m + warps - 1) / warps, most = kNumSMs * per_sm;
+      return launch_overlapped(csr_expand_rows_kernel<IT, 32>, dim3(blocks < most ? blocks : most), dim3(32 * warps),
+                               static_cast<size_t>(ld) * 2 * warps, s, m, ld, row_offsets, cols, values, out);
+    }
     return launch_overlapped(csr_expand_rows_kernel<IT, 256>, dim3(m < 8 * kNumSMs ? m : 8 * kNumSMs), dim3(256),
                              static_cast<size_t>(ld) * 2, s, m, ld, row_offsets, cols, values, out);
   }

@@ -44,7 +44,7 @@ int make_map_f16(CUtensorMap* map, const void* base, long long rows, long long c
 
 namespace {
 
-constexpr int kDecoders = 16;
+constexpr int kDecoders = 20;    // 24 warps' worth of registers: 80 a thread; 16 and 24 decoders measured slower
 constexpr int kThreads = (2 + kDecoders) * 32;
 constexpr int kMaxXSlots = 4;    // sparse units: slots of X
 constexpr int kMaxStages = 8;    // dense units: slots of X and W together
@@ -61,10 +61,11 @@ struct TileParams {
   const float* bias;  // optional: relu(sum + bias[row])
   __half* s_out;
   long long s_row, s_tok;
-  // dense units
-  int d_tiles, d_rows, d_m;
-  __half* d_out;
-  long long d_row, d_tok;
+  // dense units of one or two matrices on the same activations, d_rows rows each
+  int d_rows;
+  int d_tiles[2], d_m[2];
+  __half* d_out[2];
+  long long d_row[2], d_tok[2];
   // shared
   int k, n;
   int x_mn;            // X stored [k, n] (tokens contiguous), else [n, k]
@@ -86,47 +87,69 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
       : "memory");
 }
 
-// U pairs of a lane as loaded, the columns in the matrix's index type.
+// U pairs of a lane as loaded, the columns in the matrix's index type.  A half warp (16 lanes) reads one
+// row: pair u of its lane h are positions base + 32 u + 2 h and the next.
 template <typename IT, int U> struct Window;
 template <int U> struct Window<uint16_t, U> { uint32_t v[U], c[U]; };
 template <int U> struct Window<int, U> { uint32_t v[U]; int2 c[U]; };
 
-// Requests positions [base, base + 64 U) of one row; pairs that start at or past `end` hold an
-// index no block contains.
+// Requests positions [base, base + 32 U) of the arrays, whatever row they belong to.
 template <typename IT, int U>
 __device__ __forceinline__ void load_window(Window<IT, U>& w, const __half* __restrict__ values,
-                                            const IT* __restrict__ cols, int base, int end, int nnz, int lane) {
+                                            const IT* __restrict__ cols, int base, int half_lane) {
+  const __half* pv = values + base + 2 * half_lane;
+  const IT* pc = cols + base + 2 * half_lane;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const int p = base + 64 * u + 2 * lane;
-    if constexpr (sizeof(IT) == 2) w.c[u] = 0xffffffffu; else w.c[u] = make_int2(-1, -1);
-    w.v[u] = 0u;
-    if (p < end) {
-      if (p + 1 < nnz) {
-        w.v[u] = __ldg(reinterpret_cast<const uint32_t*>(values + p));
-        if constexpr (sizeof(IT) == 2) w.c[u] = __ldg(reinterpret_cast<const uint32_t*>(cols + p));
-        else w.c[u] = __ldg(reinterpret_cast<const int2*>(cols + p));
-      } else {  // last nonzero of the arrays
-        w.v[u] = __half_as_ushort(__ldg(values + p));
-        if constexpr (sizeof(IT) == 2) w.c[u] = 0xffff0000u | __ldg(cols + p);
-        else w.c[u] = make_int2(__ldg(cols + p), -1);
-      }
-    }
+    w.v[u] = __ldg(reinterpret_cast<const uint32_t*>(pv + 32 * u));
+    if constexpr (sizeof(IT) == 2) w.c[u] = __ldg(reinterpret_cast<const uint32_t*>(pc + 32 * u));
+    else w.c[u] = __ldg(reinterpret_cast<const int2*>(pc + 32 * u));
   }
 }
-// Both columns of pair u relative to the block's first column, 16 bits each; anything outside the
-// block is at least kb (columns below the block only occur before `cur` and are excluded there).
+// Gives the positions of a window outside [cur, end) an index no block contains.
 template <int U>
-__device__ __forceinline__ uint32_t relative(const Window<uint16_t, U>& w, int u, uint32_t c0, bool skip_first) {
-  uint32_t c = w.c[u];
-  if (skip_first) c = (c & 0xffff0000u) | (c >> 16);  // keeps the packed subtraction free of a borrow
-  return c - (c0 | (c0 << 16));
+__device__ __forceinline__ void cut_window(Window<uint16_t, U>& w, int p0, int cur, int end) {
+  const uint32_t n = static_cast<uint32_t>(end - cur), q = static_cast<uint32_t>(p0 - cur);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    w.c[u] |= q + 32u * u >= n ? 0x0000ffffu : 0u;
+    w.c[u] |= q + 32u * u + 1u >= n ? 0xffff0000u : 0u;
+  }
 }
 template <int U>
-__device__ __forceinline__ uint32_t relative(const Window<int, U>& w, int u, uint32_t c0, bool) {
+__device__ __forceinline__ void cut_window(Window<int, U>& w, int p0, int cur, int end) {
+  const uint32_t n = static_cast<uint32_t>(end - cur), q = static_cast<uint32_t>(p0 - cur);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    w.c[u].x = q + 32u * u >= n ? -1 : w.c[u].x;
+    w.c[u].y = q + 32u * u + 1u >= n ? -1 : w.c[u].y;
+  }
+}
+// Both columns of pair u relative to the block's first column, 16 bits each.  Columns ascend and everything
+// before the row's position is masked (`before`), so no column is below the block's first one.
+template <int U>
+__device__ __forceinline__ uint32_t relative(const Window<uint16_t, U>& w, int u, uint32_t c0c0, uint32_t before) {
+  return (u == 0 ? w.c[0] | before : w.c[u]) - c0c0;
+}
+template <int U>
+__device__ __forceinline__ uint32_t relative(const Window<int, U>& w, int u, uint32_t c0c0, uint32_t before) {
+  const uint32_t c0 = c0c0 & 0xffffu;
   const uint32_t a = min(static_cast<uint32_t>(w.c[u].x) - c0, 0xffffu);
   const uint32_t b = min(static_cast<uint32_t>(w.c[u].y) - c0, 0xffffu);
-  return a | (b << 16);
+  return (u == 0 ? a | before : a) | (b << 16);
+}
+// If key < limit: stores the low half of v at addr and counts it.  Predicated instructions, one
+// comparison for both.
+__device__ __forceinline__ void store_below(uint32_t key, uint32_t limit, uint32_t addr, uint32_t v, uint32_t& count) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b16 h;\n\t"
+      "setp.lt.u32 p, %1, %2;\n\t"
+      "cvt.u16.u32 h, %4;\n\t"
+      "@p st.shared.u16 [%3], h;\n\t"
+      "@p add.u32 %0, %0, 1;\n\t}"
+      : "+r"(count)
+      : "r"(key), "r"(limit), "r"(addr), "r"(v)
+      : "memory");
 }
 
 // Offsets of the mbarriers behind `bar`.
@@ -192,8 +215,8 @@ __device__ __forceinline__ void issue_unit(const TileParams& p, bool sparse, int
 
 template <typename IT, int U>
 __global__ void __launch_bounds__(kThreads, 1)
-spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x_s, const __grid_constant__ CUtensorMap map_w,
-                 const TileParams p) {
+spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
+                 const __grid_constant__ CUtensorMap map_w1, const TileParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -239,23 +262,24 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x_s, const __grid_const
 
   const int k_slots = (p.k + 63) / 64;
   const int blocks = (p.k + p.kb - 1) / p.kb;
-  const int units = p.s_tiles + p.d_tiles;
+  const int units = p.s_tiles + p.d_tiles[0] + p.d_tiles[1];
   uint32_t x_it = 0, d_it = 0, a_it = 0;  // slots / stages / blocks used so far (each role counts alike)
   uint32_t unit_it = 0;
 
   for (int u = blockIdx.x; u < units; u += gridDim.x, ++unit_it) {
     const bool sparse = u < p.s_tiles;
     const int rows = sparse ? p.s_rows : p.d_rows;
-    const int row0 = (sparse ? u : u - p.s_tiles) * rows;
+    const int which = u >= p.s_tiles + p.d_tiles[0] ? 1 : 0;  // dense matrix
+    const int row0 = (sparse ? u : u - p.s_tiles - (which ? p.d_tiles[0] : 0)) * rows;
     if (warp == 0) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
         const int m_atoms = p.inst_m * p.m_blocks / 64;
         auto load_x = [&](uint32_t dst, uint32_t full, int ks) {
           if (p.x_mn) {
-            for (int j = 0; j < m_atoms; ++j) tma_load_2d(dst + j * 8192u, &map_x_s, full, j * 64, ks * 64);
+            for (int j = 0; j < m_atoms; ++j) tma_load_2d(dst + j * 8192u, &map_x, full, j * 64, ks * 64);
           } else {
-            tma_load_2d(dst, &map_x_s, full, ks * 64, 0);
+            tma_load_2d(dst, &map_x, full, ks * 64, 0);
           }
         };
         if (sparse) {
@@ -274,7 +298,7 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x_s, const __grid_const
             if (!mbar_wait(d_empty(s), ph ^ 1u, abort_flag, p.status, 64)) break;
             const uint32_t dst = base + s * stage_bytes;
             mbar_arrive_expect_tx(d_full(s), stage_bytes);
-            tma_load_2d(dst + x_bytes, &map_w, d_full(s), ks * 64, row0);
+            tma_load_2d(dst + x_bytes, which ? &map_w1 : &map_w0, d_full(s), ks * 64, row0);
             load_x(dst, d_full(s), ks);
             if (++s == p.stages) { s = 0; ph ^= 1u; }
           }
@@ -301,114 +325,144 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x_s, const __grid_const
       bool ok = true;
       if (sparse) {
         const IT* cols = static_cast<const IT*>(p.cols);
-        const int nrows = (rows - w + kDecoders - 1) / kDecoders;  // this warp's rows: w, w + 16, ...
-        // lane i holds the position and the end of the warp's row i
+        // The warp's row pairs are w, w + kDecoders, ...: pair d is rows 2 d (lanes 0-15) and 2 d + 1.
+        const int pairs = (rows / 2 - w + kDecoders - 1) / kDecoders;
+        const int hl = lane & 15, hi = lane >> 4;
+        // lane 16 h + i holds the position and the end of row h of the warp's pair i
         int cur_l = 0, end_l = 0;
-        if (lane < nrows) {
-          const int r = row0 + w + kDecoders * lane;
+        if (hl < pairs) {
+          const int r = row0 + 2 * (w + kDecoders * hl) + hi;
           if (r < p.s_m) {
             cur_l = __ldg(p.row_offsets + r);
             end_l = __ldg(p.row_offsets + r + 1);
           }
         }
-        auto prefetch = [&](int from, int end) {  // eight 128-byte lines of values and of indices
-          const int l8 = lane & 7;
-          if (lane < 8) {
-            const int q = from + l8 * 64;
-            if (q < end && 64 * l8 < p.ahead) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.values + q));
-          } else if (lane < 8 + 8 * static_cast<int>(sizeof(IT)) / 2) {
-            constexpr int kPer = 128 / sizeof(IT);
-            const int q = from + (lane - 8) * kPer;
-            if (q < end && kPer * (lane - 8) < p.ahead) asm volatile("prefetch.global.L2 [%0];" ::"l"(cols + q));
+        // Windows are whole pairs inside the arrays: the last ones start early (last_base), and of an odd
+        // number of nonzeros the very last is taken out of its row and written by itself.
+        const int last_base = (p.s_nnz & ~1) - 32 * U;
+        int tail_pair = -1, tail_lane = -1, tail_col = 0;
+        uint32_t tail_val = 0;
+        if (p.s_nnz & 1) {
+          const uint32_t has = __ballot_sync(0xffffffffu, end_l == p.s_nnz && cur_l < end_l);
+          if (has != 0) {
+            tail_lane = (__ffs(has) - 1) & 16;
+            tail_pair = (__ffs(has) - 1) & 15;
+            tail_col = to_index(__ldg(cols + p.s_nnz - 1));
+            tail_val = __half_as_ushort(__ldg(p.values + p.s_nnz - 1));
+            if (hl == tail_pair && hi == tail_lane >> 4) --end_l;
           }
-        };
-        Window<IT, U> win, next;
-        if (nrows > 0) {
-          for (int i = 0; i < nrows; ++i)
-            prefetch(__shfl_sync(0xffffffffu, cur_l, i), __shfl_sync(0xffffffffu, end_l, i));
-          const int c = __shfl_sync(0xffffffffu, cur_l, 0), e = __shfl_sync(0xffffffffu, end_l, 0);
-          load_window<IT, U>(win, p.values, cols, c & ~1, e, p.s_nnz, lane);
         }
-        for (int b = 0; b < blocks; ++b) {
-          const uint32_t ab = a_it + b;
-          const uint32_t buf = base + (ab & 1u) * block_bytes;
-          const uint32_t c0 = static_cast<uint32_t>(b * p.kb);
-          if (!mbar_wait(a_empty(ab & 1u), ((ab >> 1) & 1u) ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
-          // clear this warp's rows: 8 lanes per 128-byte row of an atom, four atoms at a time
-          for (int i = 0; i < nrows; ++i) {
-            const uint32_t r = w + kDecoders * i;
-            const uint32_t dst = buf + (r >> 3) * atoms * 1024u + (r & 7u) * 128u + (lane & 7) * 16u;
-            for (uint32_t j = lane >> 3; j < atoms; j += 4)
-              asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst + j * 1024u), "r"(0u) : "memory");
+        // L2 prefetch: per half warp up to eight 128-byte lines of values and as many of (16-bit) indices
+        const int pf_pos = (lane & 7) * (hl < 8 ? 64 : 128 / static_cast<int>(sizeof(IT)));
+        const char* const pf_base = hl < 8 ? reinterpret_cast<const char*>(p.values) : reinterpret_cast<const char*>(cols);
+        const int pf_size = hl < 8 ? 2 : static_cast<int>(sizeof(IT));
+        const bool pf_on = pf_pos < p.ahead;
+        auto prefetch = [&](int from, int end) {
+          const int q = from + pf_pos;
+          if (pf_on && q < end) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + static_cast<long long>(q) * pf_size));
+        };
+        const uint32_t kb_hi = static_cast<uint32_t>(p.kb) << 16;
+        for (int j = 0; j < pairs; ++j)
+          prefetch(__shfl_sync(0xffffffffu, cur_l, (lane & 16) + j), __shfl_sync(0xffffffffu, end_l, (lane & 16) + j));
+        // Items: the share of block b in the rows of pair i, row pairs inside blocks.  `win` holds the item's
+        // window, `next` the following item's (loaded one item ahead; with a single row pair per warp
+        // its position is not known earlier).  The loop is written to have one copy of every part: its
+        // instructions have to fit the instruction caches that 20 warps at different places share
+        // (two inlined copies of the item: 44 instead of 40 us at 11008 x 4096, 50 %).
+        int b = 0, i = 0, li = 0;
+        uint32_t buf = 0;
+        bool loaded = false;
+        Window<IT, U> win, next;
+        while (pairs > 0 && b < blocks) {
+          if (pairs > 1 || !loaded) {
+            const int c = __shfl_sync(0xffffffffu, cur_l, (lane & 16) + li);
+            load_window<IT, U>(next, p.values, cols, min(c & ~1, last_base), hl);
+            li = li + 1 < pairs ? li + 1 : 0;
           }
-          __syncwarp();
-          for (int i = 0; i < nrows; ++i) {
-            int cur = __shfl_sync(0xffffffffu, cur_l, i);
-            const int end = __shfl_sync(0xffffffffu, end_l, i);
-            const int ni = i + 1 < nrows ? i + 1 : 0;
-            const bool more_items = i + 1 < nrows || b + 1 < blocks;
-            if (nrows > 1 && more_items) {  // the next row's window travels while this one is written
-              const int nc = __shfl_sync(0xffffffffu, cur_l, ni), ne = __shfl_sync(0xffffffffu, end_l, ni);
-              load_window<IT, U>(next, p.values, cols, nc & ~1, ne, p.s_nnz, lane);
-            }
-            prefetch(cur + p.ahead, end);
-            const uint32_t r = w + kDecoders * i;
-            const uint32_t row_base = buf + (r >> 3) * atoms * 1024u + (r & 7u) * 128u;
-            const uint32_t sw = (r & 7u) << 4, sw2 = sw | (sw << 16);
-            const uint32_t kb = static_cast<uint32_t>(p.kb);
-            for (;;) {
-              const int wbase = cur & ~1;
-              uint32_t rel[U];
-              bool v0[U], v1[U];
-              int cnt = 0;
-#pragma unroll
-              for (int q = 0; q < U; ++q) {
-                const int pos = wbase + 64 * q + 2 * lane;
-                rel[q] = relative<U>(win, q, c0, q == 0 && pos < cur);
-                v0[q] = (rel[q] & 0xffffu) < kb && pos < end && (q > 0 || pos >= cur);
-                v1[q] = (rel[q] >> 16) < kb && pos + 1 < end;
-                cnt += __popc(__ballot_sync(0xffffffffu, v0[q])) + __popc(__ballot_sync(0xffffffffu, v1[q]));
-              }
-              cur += cnt;
-              const bool again = cur == wbase + 64 * U && cur < end;  // the whole window fell into the block
-              if (!again) {
-                if (lane == i) cur_l = cur;
-                if (nrows == 1 && more_items) load_window<IT, U>(next, p.values, cols, cur & ~1, end, p.s_nnz, lane);
-              }
-#pragma unroll
-              for (int q = 0; q < U; ++q) {
-                // offset inside the row group: 64-column atom (bits 6-8 of the column) and swizzled byte
-                const uint32_t off = ((rel[q] << 4) & 0x1c001c00u) | (((rel[q] << 1) & 0x007e007eu) ^ sw2);
-                if (v0[q])
-                  asm volatile("st.shared.u16 [%0], %1;" ::"r"(row_base + (off & 0xffffu)),
-                               "h"(static_cast<uint16_t>(win.v[q])) : "memory");
-                if (v1[q])
-                  asm volatile("st.shared.u16 [%0], %1;" ::"r"(row_base + (off >> 16)),
-                               "h"(static_cast<uint16_t>(win.v[q] >> 16)) : "memory");
-              }
-              if (!again) break;
-              load_window<IT, U>(win, p.values, cols, cur, end, p.s_nnz, lane);
-            }
+          if (!loaded) {
             win = next;
+            loaded = true;
+            continue;
           }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          const uint32_t ab = a_it + b;
+          if (i == 0) {
+            buf = base + (ab & 1u) * block_bytes;
+            if (!mbar_wait(a_empty(ab & 1u), ((ab >> 1) & 1u) ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
+          }
+          int cur = __shfl_sync(0xffffffffu, cur_l, (lane & 16) + i);
+          int end = __shfl_sync(0xffffffffu, end_l, (lane & 16) + i);
+          const uint32_t r = 2u * (w + kDecoders * i);
+          const uint32_t pair_base = buf + (r >> 3) * atoms * 1024u + (r & 7u) * 128u;
+          // clear the pair's 256 bytes of every atom: a half warp each, two atoms at a time
+          {
+            const uint32_t dst = pair_base + hi * 1024u + hl * 16u;
+#pragma unroll
+            for (uint32_t t = 0; t < 8; t += 2)
+              if (t + hi < atoms)
+                asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst + t * 1024u), "r"(0u) : "memory");
+          }
+          prefetch(cur + p.ahead, end);
+          const uint32_t row_base = pair_base + hi * 128u;
+          const uint32_t sw2 = (((r & 7u) + hi) << 4) * 0x00010001u;
+          const uint32_t c0 = static_cast<uint32_t>(b * p.kb), c0c0 = c0 * 0x00010001u;
           __syncwarp();
-          if (lane == 0) mbar_arrive(a_full(ab & 1u));
+          if (i == tail_pair && lane == tail_lane && static_cast<uint32_t>(tail_col) - c0 < static_cast<uint32_t>(p.kb)) {
+            uint32_t one = 0;
+            const uint32_t rel = static_cast<uint32_t>(tail_col) - c0;
+            store_below(0u, 1u, row_base + (((rel << 4) & 0x1c00u) | (((rel << 1) & 0x7eu) ^ (sw2 & 0xffffu))), tail_val, one);
+          }
+          for (;;) {
+            const int wbase = min(cur & ~1, last_base);
+            if (__any_sync(0xffffffffu, wbase + 32 * U > end || wbase + 1 < cur)) cut_window<U>(win, wbase + 2 * hl, cur, end);
+            const uint32_t before = (hl == 0 && (cur & 1)) ? 0xffffu : 0u;
+            uint32_t cnt = 0;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+              const uint32_t rel = relative<U>(win, q, c0c0, before);
+              // offset inside the row group: 64-column atom (bits 6-8 of the column) and swizzled byte
+              const uint32_t off = ((rel << 4) & 0x1c001c00u) | (((rel << 1) & 0x007e007eu) ^ sw2);
+              store_below(rel << 16, kb_hi, row_base + (off & 0xffffu), win.v[q], cnt);
+              store_below(rel, kb_hi, row_base + (off >> 16), win.v[q] >> 16, cnt);
+            }
+            // both rows' counts in one reduction: the upper half warp's in the upper 16 bits
+            const uint32_t both = __reduce_add_sync(0xffffffffu, hi ? cnt << 16 : cnt);
+            cur += hi ? both >> 16 : both & 0xffffu;
+            const bool again = cur == wbase + 32 * U && cur < end;  // the whole window fell into the block
+            if (!__any_sync(0xffffffffu, again)) break;
+            load_window<IT, U>(win, p.values, cols, min(cur & ~1, last_base), hl);
+            if (!again) end = cur;  // this row is done with the block: nothing of the window counts
+          }
+          if (hl == i) cur_l = cur;
+          i = i + 1 < pairs ? i + 1 : 0;
+          if (i == 0) {  // the block's last pair of this warp
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(a_full(ab & 1u));
+            ++b;
+          }
+          if (pairs > 1) win = next; else loaded = false;
+        }
+        if (pairs <= 0) {  // no row of the unit for this warp: only its arrivals
+          for (; b < blocks; ++b) {
+            const uint32_t ab = a_it + b;
+            if (!mbar_wait(a_empty(ab & 1u), ((ab >> 1) & 1u) ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
+            if (lane == 0) mbar_arrive(a_full(ab & 1u));
+          }
         }
       }
       // ---------------------------------------------------------------- read-out
       if (ok && mbar_wait(acc_full, unit_it & 1u, abort_flag, p.status, 64)) {
         tcgen05_fence_after();
-        const int q = warp & 3, share = w >> 2;  // tensor-memory quarter; four warps split its columns
+        const int q = warp & 3, share = w >> 2;  // tensor-memory quarter; the warps of a quarter split its columns
         const int t_local = p.inst_m == 64 ? q * 16 + lane : q * 32 + lane;
         const bool lane_ok = p.inst_m == 128 || lane < 16;
-        const int m_rows = sparse ? p.s_m : p.d_m;
-        __half* out = sparse ? p.s_out : p.d_out;
-        const long long st_row = sparse ? p.s_row : p.d_row, st_tok = sparse ? p.s_tok : p.d_tok;
+        const int m_rows = sparse ? p.s_m : p.d_m[which];
+        __half* out = sparse ? p.s_out : p.d_out[which];
+        const long long st_row = sparse ? p.s_row : p.d_row[which], st_tok = sparse ? p.s_tok : p.d_tok[which];
         const bool vec = st_row == 1 && (st_tok & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
         for (int mb = 0; mb < p.m_blocks; ++mb) {
           const int t = mb * p.inst_m + t_local;
-          for (int c = share * 32; c < rows; c += 128) {
+          for (int c = share * 32; c < rows; c += kDecoders * 8) {
             uint32_t r[32];
             tmem_ld32(tmem + (static_cast<uint32_t>(q * 32) << 16) + mb * p.acc_cols + c, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -471,6 +525,9 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x_s, const __grid_const
   }
 }
 
+// Windows a thread holds twice without spilling registers.
+constexpr int kMaxWindows16 = 6, kMaxWindows32 = 4;
+
 struct TilePlan {
   int s_rows, d_rows, kb, windows;
 };
@@ -481,11 +538,12 @@ int round_up(int v, int to) { return (v + to - 1) / to * to; }
 // dense row its bytes; units are sized so that both kinds together occupy the SMs once and end
 // together.  Measured on B200 (one SM): about 0.9 ns per stored position of a row plus 16 ns per
 // row and block; 95 GB/s of dense operand bytes.
-bool plan_tile(int m_sparse, int m_dense, int k, int n, int nnz, int sms, int step, int x_slot_bytes, TilePlan* out) {
+bool plan_tile(int m_sparse, int m_dense, int k, int nnz, int index_bits, int sms, int step, int x_slot_bytes,
+               TilePlan* out) {
   const double per_row = m_sparse > 0 ? static_cast<double>(nnz) / m_sparse : 0.0;
   const double density = k > 0 ? per_row / k : 0.0;
-  const double s_cost = 0.9e-3 * per_row + 0.016 * ((k + 447) / 448);
-  const double d_cost = 2.0 * k / 95e3;
+  const double s_cost = 0.13e-3 * per_row + 0.0166 * ((k + 511) / 512);
+  const double d_cost = 2.0 * k / 80e3;
   int s_ctas = sms;
   if (m_dense > 0) {
     const double total = s_cost * m_sparse + d_cost * m_dense;
@@ -507,25 +565,30 @@ bool plan_tile(int m_sparse, int m_dense, int k, int n, int nnz, int sms, int st
   if (m_sparse > 0) {
     // Columns per block: as many as two buffers leave room for; U windows of 64 nonzeros have to
     // cover a row's share of a block in almost every case.  Cost of a row and block in instructions:
-    // 17 per window and about 45 of its own.
+    // 17 per window and about 110 of its own.
     const int room = kBudget - 2 * x_slot_bytes;
+    const int max_u = index_bits == 16 ? kMaxWindows16 : kMaxWindows32;
     double best = 1e30;
     for (int kb = 64; kb <= 512 && kb <= round_up(k, 64); kb += 64) {
       if (2 * (pl.s_rows / 8) * (kb / 64) * 1024 > room) break;
       const double a = density * kb;
-      int u = static_cast<int>(std::ceil((a + 1.5 * std::sqrt(a) + 2.0) / 64.0));
-      u = u < 1 ? 1 : (u > 5 ? 5 : u);
-      const double cost = ((k + kb - 1) / kb) * (17.0 * u + 45.0) * std::fmax(1.0, a / (64.0 * u));
+      int u = static_cast<int>(std::ceil((a + 1.5 * std::sqrt(a) + 2.0) / 32.0));
+      const int rounds = (u + max_u - 1) / max_u;  // windows a row needs in most blocks
+      u = u < 1 ? 1 : (u > max_u ? max_u : u);
+      const double cost = ((k + kb - 1) / kb) * (17.0 * u * rounds + 110.0);
       if (cost <= best) { best = cost; pl.kb = kb; pl.windows = u; }
     }
     if (best >= 1e30) return false;
+    // windows lie inside the arrays as a whole
+    while (pl.windows > 1 && 32 * pl.windows > (nnz & ~1)) --pl.windows;
+    if (32 * pl.windows > (nnz & ~1)) return false;
   }
   *out = pl;
   return true;
 }
 
 template <typename IT, int U>
-int launch_tile(const CUtensorMap& mx, const CUtensorMap& mw, const TileParams& p, int grid, cudaStream_t stream) {
+int launch_tile(const CUtensorMap& mx, const CUtensorMap (&mw)[2], const TileParams& p, int grid, cudaStream_t stream) {
   auto kern = spmm_tile_kernel<IT, U>;
   static std::mutex mutex;
   static bool configured[64] = {};
@@ -539,43 +602,50 @@ int launch_tile(const CUtensorMap& mx, const CUtensorMap& mw, const TileParams& 
       if (dev >= 0 && dev < 64) configured[dev] = true;
     }
   }
-  return launch_overlapped(kern, dim3(grid), dim3(kThreads), static_cast<size_t>(227 * 1024), stream, mx, mw, p);
+  return launch_overlapped(kern, dim3(grid), dim3(kThreads), static_cast<size_t>(227 * 1024), stream, mx, mw[0], mw[1], p);
 }
 
 template <typename IT>
-int dispatch_tile(int windows, const CUtensorMap& mx, const CUtensorMap& mw, const TileParams& p, int grid,
+int dispatch_tile(int windows, const CUtensorMap& mx, const CUtensorMap (&mw)[2], const TileParams& p, int grid,
                   cudaStream_t stream) {
   switch (windows) {
     case 1: return launch_tile<IT, 1>(mx, mw, p, grid, stream);
     case 2: return launch_tile<IT, 2>(mx, mw, p, grid, stream);
     case 3: return launch_tile<IT, 3>(mx, mw, p, grid, stream);
     case 4: return launch_tile<IT, 4>(mx, mw, p, grid, stream);
-    default: return launch_tile<IT, 5>(mx, mw, p, grid, stream);
+    default: break;
   }
+  if constexpr (sizeof(IT) == 2) {
+    if (windows == 5) return launch_tile<IT, 5>(mx, mw, p, grid, stream);
+    return launch_tile<IT, 6>(mx, mw, p, grid, stream);
+  }
+  return IEX_ERR_UNSUPPORTED;
 }
 
-}  // namespace
-}  // namespace tc
-}  // namespace iex
+// What the outputs and dense matrices of a launch are.
+struct DenseArg {
+  int m;
+  const void* weight;
+  void* out;
+  int tokens_major;
+};
 
-extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n, int nnz, const int32_t* row_offsets,
-                                        const void* column_indices, int index_bits, const void* values,
-                                        const void* weight, const void* x, int x_tokens_major, const float* bias,
-                                        void* out_sparse, int sparse_tokens_major, void* out_dense,
-                                        int dense_tokens_major, void* stream) {
-  using namespace iex;
-  using namespace iex::tc;
-  if (m_sparse < 0 || m_dense < 0 || k < 0 || n < 0 || nnz < 0) return IEX_ERR_BAD_ARG;
+int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets, const void* cols, int index_bits,
+                const void* values, const float* bias, void* out_sparse, int sparse_tokens_major,
+                const DenseArg (&dense)[2], const void* x, int x_tokens_major, void* stream) {
+  const int m_dense = dense[0].m + dense[1].m;
+  if (m_sparse < 0 || dense[0].m < 0 || dense[1].m < 0 || k < 0 || n < 0 || nnz < 0) return IEX_ERR_BAD_ARG;
   if (index_bits != 16 && index_bits != 32) return IEX_ERR_BAD_ARG;
   if ((m_sparse == 0 && m_dense == 0) || n == 0) return IEX_OK;
-  if (!x || (m_sparse > 0 && (!row_offsets || !out_sparse || (nnz > 0 && (!column_indices || !values)))))
-    return IEX_ERR_BAD_ARG;
-  if (m_dense > 0 && (!weight || !out_dense)) return IEX_ERR_BAD_ARG;
+  if (!x || (m_sparse > 0 && (!row_offsets || !out_sparse || (nnz > 0 && (!cols || !values))))) return IEX_ERR_BAD_ARG;
+  for (const auto& d : dense)
+    if (d.m > 0 && (!d.weight || !d.out)) return IEX_ERR_BAD_ARG;
   if (n > 256 || k == 0 || (x_tokens_major ? k : n) % 8 != 0 || (m_dense > 0 && k % 8 != 0)) return IEX_ERR_UNSUPPORTED;
   if (index_bits == 16 && k > 65024) return IEX_ERR_UNSUPPORTED;  // 0xffff marks padding in every block
-  if (!aligned16(x) || (m_dense > 0 && !aligned16(weight))) return IEX_ERR_UNSUPPORTED;
+  if (!aligned16(x) || (dense[0].m > 0 && !aligned16(dense[0].weight)) || (dense[1].m > 0 && !aligned16(dense[1].weight)))
+    return IEX_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(values) & 3u) != 0 ||
-      (reinterpret_cast<uintptr_t>(column_indices) & static_cast<uintptr_t>(index_bits / 4 - 1)) != 0)
+      (reinterpret_cast<uintptr_t>(cols) & static_cast<uintptr_t>(index_bits / 4 - 1)) != 0)
     return IEX_ERR_UNSUPPORTED;  // pairs of nonzeros are loaded together
   TileParams p{};
   p.inst_m = n <= 64 ? 64 : 128;
@@ -584,24 +654,26 @@ extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n,
   const int x_slot = p.inst_m * p.m_blocks * 128;
   const int sms = sm_count();
   TilePlan pl{};
-  if (!plan_tile(m_sparse, m_dense, k, n, nnz, sms, step, x_slot, &pl)) return IEX_ERR_UNSUPPORTED;
+  if (!plan_tile(m_sparse, m_dense, k, nnz, index_bits, sms, step, x_slot, &pl)) return IEX_ERR_UNSUPPORTED;
   p.s_rows = pl.s_rows;
   p.s_tiles = m_sparse > 0 ? (m_sparse + pl.s_rows - 1) / pl.s_rows : 0;
   p.s_m = m_sparse;
   p.s_nnz = nnz;
   p.row_offsets = row_offsets;
-  p.cols = column_indices;
+  p.cols = cols;
   p.values = static_cast<const __half*>(values);
   p.bias = bias;
   p.s_out = static_cast<__half*>(out_sparse);
   p.s_row = sparse_tokens_major ? 1 : n;
   p.s_tok = sparse_tokens_major ? m_sparse : 1;
   p.d_rows = pl.d_rows;
-  p.d_tiles = m_dense > 0 ? (m_dense + pl.d_rows - 1) / pl.d_rows : 0;
-  p.d_m = m_dense;
-  p.d_out = static_cast<__half*>(out_dense);
-  p.d_row = dense_tokens_major ? 1 : n;
-  p.d_tok = dense_tokens_major ? m_dense : 1;
+  for (int i = 0; i < 2; ++i) {
+    p.d_tiles[i] = (dense[i].m + pl.d_rows - 1) / pl.d_rows;
+    p.d_m[i] = dense[i].m;
+    p.d_out[i] = static_cast<__half*>(dense[i].out);
+    p.d_row[i] = dense[i].tokens_major ? 1 : n;
+    p.d_tok[i] = dense[i].tokens_major ? dense[i].m : 1;
+  }
   p.k = k;
   p.n = n;
   p.x_mn = x_tokens_major ? 0 : 1;
@@ -610,7 +682,7 @@ extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n,
   p.acc_cols = round_up(widest, 32);
   p.tmem_cols = 32;
   while (p.tmem_cols < p.acc_cols * p.m_blocks) p.tmem_cols <<= 1;
-  p.ahead = 2 * 64 * pl.windows < 512 ? 2 * 64 * pl.windows : 512;
+  p.ahead = 2 * 32 * pl.windows;
   p.status = status_word();
   p.x_slots = 1;
   if (m_sparse > 0) {
@@ -624,15 +696,39 @@ extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n,
     p.stages = p.stages > kMaxStages ? kMaxStages : p.stages;
     if (p.stages < 2) return IEX_ERR_UNSUPPORTED;
   }
-  CUtensorMap mx, mw;
+  CUtensorMap mx, mw[2];
   int st = p.x_mn ? make_map_f16(&mx, x, k, n, n, 64, 64, true)
                   : make_map_f16(&mx, x, n, k, k, p.inst_m * p.m_blocks, 64, true);
-  if (st == IEX_OK && m_dense > 0) st = make_map_f16(&mw, weight, m_dense, k, k, p.d_rows, 64, true);
+  for (int i = 0; i < 2; ++i) {
+    if (st == IEX_OK && dense[i].m > 0) st = make_map_f16(&mw[i], dense[i].weight, dense[i].m, k, k, p.d_rows, 64, true);
+    if (dense[i].m == 0) mw[i] = mx;
+  }
   if (st != IEX_OK) return st;
-  if (m_dense == 0) mw = mx;
-  const int units = p.s_tiles + p.d_tiles;
+  const int units = p.s_tiles + p.d_tiles[0] + p.d_tiles[1];
   const int grid = units < sms ? units : sms;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (index_bits == 16) return dispatch_tile<uint16_t>(pl.windows, mx, mw, p, grid, s);
   return dispatch_tile<int>(pl.windows, mx, mw, p, grid, s);
+}
+
+}  // namespace
+}  // namespace tc
+}  // namespace iex
+
+extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n, int nnz, const int32_t* row_offsets,
+                                        const void* column_indices, int index_bits, const void* values,
+                                        const void* weight, const void* x, int x_tokens_major, const float* bias,
+                                        void* out_sparse, int sparse_tokens_major, void* out_dense,
+                                        int dense_tokens_major, void* stream) {
+  const iex::tc::DenseArg dense[2] = {{m_dense, weight, out_dense, dense_tokens_major}, {0, nullptr, nullptr, 0}};
+  return iex::tc::tile_launch(m_sparse, k, n, nnz, row_offsets, column_indices, index_bits, values, bias, out_sparse,
+                              sparse_tokens_major, dense, x, x_tokens_major, stream);
+}
+
+extern "C" int iex_linear_pair_f16(int m0, int m1, int k, int n, const void* weight0, const void* weight1, const void* x,
+                                   int x_tokens_major, void* out0, int tokens_major0, void* out1, int tokens_major1,
+                                   void* stream) {
+  const iex::tc::DenseArg dense[2] = {{m0, weight0, out0, tokens_major0}, {m1, weight1, out1, tokens_major1}};
+  return iex::tc::tile_launch(0, k, n, 0, nullptr, nullptr, 16, nullptr, nullptr, nullptr, 0, dense, x, x_tokens_major,
+                              stream);
 }

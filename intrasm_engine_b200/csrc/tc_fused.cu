@@ -1220,6 +1220,22 @@ int linear_impl(int tokens, int in_features, int out_features, const void* input
   return launch_units<0, uint16_t>(ta, tb, tb, p, stages, 1, static_cast<cudaStream_t>(stream));
 }
 
+// The block decoder (spmm_tile.cu) or the slot decoder of this file?  Alone, the block decoder is faster at
+// every density measured (11008 x 4096 x 64, 16-bit indices: 42 against 46 us at 50 %, 23 against 30 us at
+// 90 %).  Beside a dense branch the slot decoder's time hardly depends on the height of its tiles, so it can
+// leave more SMs to the dense units of large layers: with the 12288 x 4096 dense branch 51 against 73 us
+// at 50 %, 40 against 58 at 70 %, 34 against 39 at 90 %; but 70 against 57 us at 256 tokens and 90 %, and
+// 24 against 18 us for 5048 + 1200 rows.  Both estimates are fits to such measurements (microseconds).
+bool prefers_block_decoder(int m_sparse, int m_dense, int k, int n, int nnz) {
+  if (m_sparse == 0 || m_dense == 0) return true;
+  const double per_row = static_cast<double>(nnz) / m_sparse, slots = (k + 63) / 64;
+  double slot = 9.0 + slots * (0.28 + 0.58 * per_row / k) + 5.5 * (static_cast<double>(m_dense) * k / 50e6);
+  if (n > 128 && slot < 9.0 + 0.95 * slots) slot = 9.0 + 0.95 * slots;
+  const double work = m_sparse * (0.13e-3 * per_row + 0.0166 * ((k + 511) / 512)) + m_dense * (2.0 * k / 80e3);
+  const double block = (8.0 + 1.25 * work / sm_count()) * (n <= 64 ? 1.0 : n <= 128 ? 1.15 : 1.35);
+  return block < slot;
+}
+
 int fused_impl(int m_sparse, int m_dense, int k, int n, int nnz, const int32_t* row_offsets,
                const void* column_indices, int index_bits, const void* values, const void* weight,
                const void* x, void* out_sparse, void* out_dense, int dense_out_tokens_major,
@@ -1238,6 +1254,12 @@ int fused_impl(int m_sparse, int m_dense, int k, int n, int nnz, const int32_t* 
   if (st) return st;
   if (m_dense > 0 && (!weight || !out_dense || !aligned16(weight))) return IEX_ERR_BAD_ARG;
   if (m_sparse == 0 && m_dense == 0) return IEX_OK;
+  if (sparse_parts <= 1 && dense_parts <= 1 && prefers_block_decoder(m_sparse, m_dense, k, n, nnz)) {
+    const int done = iex_spmm_linear_f16_tile(m_sparse, m_dense, k, n, nnz, row_offsets, column_indices, index_bits, values,
+                                              weight, x, 0, sparse_bias, out_sparse, 0, out_dense,
+                                              dense_out_tokens_major, stream);
+    if (done != IEX_ERR_UNSUPPORTED) return done;  // fewer nonzeros than a window: the kernel below
+  }
   CUtensorMap ta, tb, tbs;
   st = make_map(&tb, x, k, n, BK);   // dense units: [128 k-rows x 64 cols] boxes of X
   if (st) return st;

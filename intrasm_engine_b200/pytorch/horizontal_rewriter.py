@@ -20,6 +20,7 @@ from .cpp_extensions.cuda_graph_constructor import TorchCUDAGraphConstructor
 from .cpp_extensions.layers_and_funcs.sputnik import MySpMM
 from .cpp_extensions.layers_and_funcs.torch import MyLinear
 from .cpp_extensions.layers_and_funcs.utils import MyAutogradFunc, default_fwd_kwargs
+from .utils import DenseCopy
 
 
 def simple_combine_search_space(space_1: dict, space_2: dict, space_3: dict) -> dict:
@@ -280,7 +281,8 @@ class SparseDenseLayer(ModuleToReplay):
     """SpMM (pruned weight, CSR) and dense linear on the same activation.
 
     ``forward(x)`` with ``x`` ``[k, tokens]`` returns ``(W_sparse @ x, (W_dense @ x).T)``.  With
-    ``mode="fused"`` the pair function issues one fused launch; ``mode="interleaved"`` records
+    ``mode="fused"`` the pair function issues one fused launch (without gradients and with a sparse
+    weight that is kept dense as well, see ``DenseCopy``, one launch over both dense weights); ``mode="interleaved"`` records
     the two library calls on two streams of one constructor (the reference's method);
     ``mode="serial"`` calls them back to back.
     """
@@ -299,6 +301,9 @@ class SparseDenseLayer(ModuleToReplay):
         self.transp_info = tuple(transp_info)
         self.mode = mode
         self.pair = make_kernel_pair_or_triple_autograd_function(MySpMM, MyLinear)
+        self._dense = DenseCopy(self.m, weight_dense.size(1))
+        if mode == "fused":
+            self._dense.current(self.values, self.row_offsets, self.column_indices)
 
     wants_transposed_input = True  # ConstructorEnabledLayer hands over (x, x.t().contiguous())
 
@@ -308,6 +313,9 @@ class SparseDenseLayer(ModuleToReplay):
                                          (x.requires_grad or values.requires_grad or weight.requires_grad)):
             # the pair function's fused launch without its autograd bookkeeping
             if _fused_operands(x, values, self.column_indices, weight):
+                dense = self._dense.current(values, self.row_offsets, self.column_indices)
+                if dense is not None and dense.size(1) == x.size(0):
+                    return ops.native.linear_pair(x, dense, weight)
                 return ops.native.fused_spmm_linear_half(x, self.row_offsets, values, self.column_indices, self.m,
                                                          weight)
         args = (x, self.row_indices, values, self.row_offsets, self.column_indices, self.m,

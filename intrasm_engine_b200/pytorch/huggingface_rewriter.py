@@ -17,7 +17,7 @@ from .. import ops
 from . import horizontal_rewriter as hr
 from .cpp_extensions.layers_and_funcs.sputnik import MySpMM
 from .cpp_extensions.layers_and_funcs.utils import default_fwd_kwargs
-from .utils import dense_to_sparse_cuda, get_transpose_info
+from .utils import DenseCopy, dense_to_sparse_cuda, get_transpose_info
 
 hr.make_single_kernel_autograd_function(MySpMM)
 
@@ -36,8 +36,9 @@ def magnitude_prune(weight: torch.Tensor, sparsity: float) -> torch.Tensor:
 class SparseLinear(nn.Module):
     """``y = x @ W.T (+ bias)`` with ``W`` ``[out_features, in_features]`` stored as CSR (fp16
     values, int16 column indices when they fit).  Without gradients the product is one native
-    call on ``x`` as it lies; otherwise it runs as ``W_csr @ x.T`` through ``MySpMM``, so that
-    gradients reach ``x`` (and ``values``)."""
+    call on ``x`` as it lies, with the dense copy of a not very sparse weight that the layer keeps
+    (``DenseCopy``); otherwise it runs as ``W_csr @ x.T`` through ``MySpMM``, so that gradients reach
+    ``x`` (and ``values``)."""
 
     def __init__(self, weight: torch.Tensor, bias: torch.Tensor | None = None):
         super().__init__()
@@ -54,11 +55,18 @@ class SparseLinear(nn.Module):
         self.register_buffer("column_indices", column_indices)
         self.transp_info = get_transpose_info(self.out_features, self.in_features, row_indices, row_offsets,
                                               column_indices)
+        self._dense = DenseCopy(self.out_features, self.in_features)
+        self.dense_copy()
         self.bias = None if bias is None else nn.Parameter(bias.detach().clone(), requires_grad=False)
 
     @classmethod
     def from_linear(cls, linear: nn.Linear, sparsity: float) -> "SparseLinear":
         return cls(magnitude_prune(linear.weight.detach(), sparsity), linear.bias)
+
+    def dense_copy(self):
+        """The dense weight for inference, or None below ``DENSE_COPY_DENSITY``; follows in-place
+        changes of ``values``."""
+        return self._dense.current(self.values, self.row_offsets, self.column_indices)
 
     def density(self) -> float:
         return self.values.numel() / float(self.out_features * self.in_features)
@@ -70,7 +78,7 @@ class SparseLinear(nn.Module):
             # inference: x is read as it lies and the result written as [tokens, out_features]
             x2 = x if x.dim() == 2 else x.reshape(-1, self.in_features)
             y = ops.native.sparse_linear(x2.contiguous(), self.values, self.row_offsets, self.column_indices,
-                                         self.out_features)
+                                         self.out_features, self.dense_copy())
             if self.bias is not None:
                 y = y + self.bias
             return y if x.dim() == 2 else y.reshape(*lead, self.out_features)

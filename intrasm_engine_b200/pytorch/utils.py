@@ -68,6 +68,33 @@ def sparse_to_dense(values, row_offsets, column_indices, m: int, k: int) -> torc
     return out
 
 
+# A layer whose sparse weight has at least this share of nonzeros also keeps it dense: the copy is then at
+# most twice the CSR arrays (fp16 values, 16-bit indices), and the dense kernels, which stream it at
+# HBM rate, beat every way of decoding (11008 x 4096 at 50 %, 64 tokens: 20 against 42 us).
+DENSE_COPY_DENSITY = 0.25
+
+
+class DenseCopy:
+    """Dense fp16 copy ``[m, k]`` of a layer's CSR weight, laid out once when the layer is built (k a
+    multiple of 8; None for sparser weights) and again when the values have changed since."""
+
+    def __init__(self, m: int, k: int):
+        self.m, self.k = int(m), int(k)
+        self._key, self._weight = None, None
+
+    def current(self, values, row_offsets, column_indices):
+        key = (values.data_ptr(), column_indices.data_ptr(), 0 if values.is_inference() else values._version)
+        if key != self._key:
+            from .. import ops
+            wanted = (values.is_cuda and values.dtype == torch.float16 and self.k % 8 == 0 and self.m > 0
+                      and values.numel() >= DENSE_COPY_DENSITY * self.m * self.k)
+            with torch.no_grad():
+                self._weight = (ops.native.expand_weight(values.detach(), row_offsets, column_indices, self.m, self.k)
+                                if wanted else None)
+            self._key = key
+        return self._weight
+
+
 def swizzle_rows(row_offsets: torch.Tensor) -> torch.Tensor:
     counts = row_offsets[1:] - row_offsets[:-1]
     return torch.argsort(counts, descending=True, stable=True).to(torch.int32)

@@ -61,15 +61,15 @@ void gemm(int64_t m, int64_t n, int64_t k, const at::Tensor& a, bool a_mn, const
 
 // Estimates in microseconds, fitted to measurements on B200.
 //   expand   one pass over the CSR arrays and the dense copy, at 5.5 TB/s
-//   decode   the tile decoder of tc_fused.cu: 9 us + 0.75 us per 64 columns and wave of tiles
+//   decode   the block decoder of spmm_tile.cu: per row, its stored positions and its blocks of columns
 //   cores    CUDA cores: gathered bytes, and the serial walk over an average row
 double expand_us(int64_t m, int64_t k, int64_t nnz, int bits) {
   return 2.5 + (2.0 * m * round8(k) + static_cast<double>(nnz) * (2 + bits / 8)) / 5.5e6;
 }
-double decode_us(int64_t m, int64_t k) {
-  const int64_t sms = 148, full = (m + 127) / 128;
-  const int64_t tiles = full < sms ? std::min<int64_t>(sms, (m + 7) / 8) : full;
-  return 9.0 + 0.75 * ((k + 63) / 64) * std::max<int64_t>(1, (tiles + sms - 1) / sms);
+double block_decode_us(int64_t m, int64_t k, int64_t n, int64_t nnz) {
+  const int64_t rows = round8((m + 147) / 148);
+  const double t = 8.0 + rows * (0.13e-3 * nnz / std::max<int64_t>(m, 1) + 0.0166 * ((k + 511) / 512));
+  return t * (n <= 128 ? 1.0 : 1.25) * std::max<int64_t>(1, (rows + 127) / 128);
 }
 double cores_us(int64_t m, int64_t n, int64_t nnz) {
   return 1.6 + 0.0605e-6 * 2.0 * nnz * n + 0.158 * nnz / std::max<int64_t>(m, 1);
@@ -106,7 +106,7 @@ at::Tensor spmm_half(const at::Tensor& b, const at::Tensor& ri, const at::Tensor
   check_csr_half(b, values, ro, ci, m);
   const double dense = expand_us(m, k, nnz, index_bits(ci)) + iex_gemm_f16_estimate_us(m, n, k, 1, 0) +
                        (n % 8 == 0 ? 0.0 : 2.0);
-  const double decode = decode_supported(b, values, ci) ? decode_us(m, k) : 1e30;
+  const double decode = decode_supported(b, values, ci) ? block_decode_us(m, k, n, nnz) : 1e30;
   if (mode == kAuto && cores_us(m, n, nnz) <= std::min(dense, decode)) return cores();
   if (decode <= dense) return spmm_tc_half(b, ro, values, ci, m);
   c10::cuda::CUDAGuard guard(b.device());
@@ -287,12 +287,37 @@ std::optional<at::Tensor> mylinear(const at::Tensor& input, const at::Tensor& we
 
 // --------------------------------------------------------------------------- inference layers
 
+// The dense fp16 copy [m, k] of a layer's CSR weight.
+at::Tensor expand_weight(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci, int64_t m, int64_t k) {
+  check_common({{"row_offsets", &ro}, {"values", &values}, {"column_indices", &ci}});
+  TORCH_CHECK(values.scalar_type() == at::kHalf && ro.scalar_type() == at::kInt && ro.numel() == m + 1, "not an fp16 CSR matrix");
+  TORCH_CHECK(k % 8 == 0, "in_features must be a multiple of 8");
+  c10::cuda::CUDAGuard guard(values.device());
+  return expand(values, ro, ci, m, k);
+}
+
+// The two branches of a sparse || dense layer with both weights dense: x [k, n] ->
+// (weight0 @ x [m0, n], (weight1 @ x)^T [n, m1]) in one launch.
+std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Tensor& weight0, const at::Tensor& weight1) {
+  check_common({{"x", &x}, {"weight0", &weight0}, {"weight1", &weight1}});
+  const int64_t k = x.size(0), n = x.size(1), m0 = weight0.size(0), m1 = weight1.size(0);
+  TORCH_CHECK(weight0.size(1) == k && weight1.size(1) == k, "weights must be [rows, k]");
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor out0 = empty(x, {m0, n}), out1 = empty(x, {n, m1});
+  check_status(iex_linear_pair_f16(m0, m1, k, n, weight0.data_ptr(), weight1.data_ptr(), x.data_ptr(), 0, out0.data_ptr(), 0,
+                                   out1.data_ptr(), 1, stream_of(x)),
+               "iex_linear_pair_f16");
+  return {out0, out1};
+}
+
 // SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m].
-//   up to 16 tokens   CUDA cores, the CSR arrays read once (spmm_skinny.cu)
-//   more              W expanded, dense GEMM (weight as the 256-row operand or as the other one)
-// Both read x as it lies and write [tokens, m]: no transposed copies of either.
+//   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu)
+//   with `dense`     the layer's dense copy of W and the dense GEMM
+//   up to 256        block decoder on tensor cores (spmm_tile.cu), unless ...
+//   otherwise        ... expanding W for the dense GEMM is estimated faster (many tokens)
+// All read x as it lies and write [tokens, m]: no transposed copies of either.
 at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
-                         int64_t m) {
+                         int64_t m, const std::optional<at::Tensor>& dense_weight) {
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous(), "x must be a contiguous [tokens, in_features] matrix");
   check_common({{"x", &x}, {"row_offsets", &ro}, {"values", &values}, {"column_indices", &ci}});
   TORCH_CHECK(x.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf, "x and values must be float16");
@@ -302,11 +327,32 @@ at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at
   maybe_validate(ro, ci, m, k, nullptr, false);
   at::Tensor out = empty(x, {tokens, m});
   if (tokens == 0 || m == 0) return out;
-  if (iex_spmm_f16_skinny_supported(k, tokens)) {
-    check_status(iex_spmm_f16_skinny(m, k, tokens, values.numel(), ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
+  const int64_t nnz = values.numel();
+  const double gemm_us = std::min(m % 8 == 0 ? iex_gemm_f16_estimate_us(m, tokens, k, 0, 1) : 1e30,
+                                  iex_gemm_f16_estimate_us(tokens, m, k, 0, 0));
+  // 2.5 us + 1.05 ns per nonzero for one token, 9 + 1.15 for two (a gather more for each); at three the
+  // decoder is as fast
+  const double skinny_us = tokens == 1 ? 2.5 + 1.05e-6 * nnz : 3.5 + 6e-6 * m / 11 + 1.15e-6 * nnz;
+  if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) && (!dense_weight.has_value() || skinny_us <= gemm_us)) {
+    check_status(iex_spmm_f16_skinny(m, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
                                      values.data_ptr(), x.data_ptr(), 1, k, out.data_ptr(), 1, m, stream_of(x)),
                  "iex_spmm_f16_skinny");
     return out;
+  }
+  if (dense_weight.has_value()) {
+    const at::Tensor& w = *dense_weight;
+    TORCH_CHECK(w.size(0) == m && w.size(1) == k && w.scalar_type() == at::kHalf && w.is_contiguous(), "dense copy of another shape");
+    check_status(iex_linear_f16_any(tokens, k, m, x.data_ptr(), w.data_ptr(), out.data_ptr(), stream_of(x)),
+                 "iex_linear_f16_any");
+    return out;
+  }
+  const double as_dense = expand_us(m, k, nnz, index_bits(ci)) + gemm_us;
+  if (tokens <= 256 && k % 8 == 0 && block_decode_us(m, k, tokens, nnz) < as_dense) {
+    const int st = iex_spmm_linear_f16_tile(m, 0, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
+                                            values.data_ptr(), nullptr, x.data_ptr(), 1, nullptr, out.data_ptr(), 1,
+                                            nullptr, 0, stream_of(x));
+    if (st == 0) return out;
+    TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_linear_f16_tile failed with status ", st, ": ", iex_error_string(st));
   }
   const at::Tensor dense = expand(values, ro, ci, m, k), xp = tma_rows(x);
   if (m % 8 == 0 && iex_gemm_f16_estimate_us(m, tokens, k, 0, 1) <= iex_gemm_f16_estimate_us(tokens, m, k, 0, 0))
@@ -354,6 +400,8 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
   mod.def("myspmm", &iex_torch::myspmm);
   mod.def("mylinear", &iex_torch::mylinear);
   mod.def("sparse_linear", &iex_torch::sparse_linear);
+  mod.def("expand_weight", &iex_torch::expand_weight);
+  mod.def("linear_pair", &iex_torch::linear_pair);
   mod.def("ffn_down", &iex_torch::ffn_down);
   mod.def("relu_down_proj", &iex_torch::relu_down_proj);
   mod.def("fused_spmm_linear_half", &iex_torch::fused_spmm_linear_half);
