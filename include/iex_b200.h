@@ -172,6 +172,21 @@ IEX_API size_t iex_spmm_f32_tc_workspace_bytes(int m, int k, int n);
 IEX_API int iex_spmm_f32_tc_supported(int m, int k, int n);
 IEX_API int iex_spmm_f32_prefers_tc(int m, int k, int n, int nnz);
 
+/* The SDDMM -> SpMM chain of masked attention over all heads, fp32, scores kept on chip:
+ *   out[h, i] = sum over stored positions (i, j) of dot(q[h, i], k[h, j]) * v[h, j]
+ * q [heads, m, d], k [heads, n, d], v [heads, n, dv], out [heads, m, dv], contiguous and 16-byte
+ * aligned; d and dv multiples of 4 up to 128.  The plan (256-byte aligned, iex_attention_plan_bytes) depends
+ * on the pattern only; its first word is nonzero if the pattern stores a position twice, and the plan must
+ * then not be used.  The workspace holds the operands' TF32 planes. */
+IEX_API int iex_attention_f32_supported(int heads, int m, int n, int d, int dv);
+IEX_API size_t iex_attention_plan_bytes(int m, int n);
+IEX_API int iex_attention_plan_build(int m, int n, const int32_t* row_offsets, const int32_t* column_indices,
+                                     void* plan, size_t bytes, void* stream);
+IEX_API size_t iex_attention_workspace_bytes(int heads, int m, int n, int d, int dv);
+IEX_API int iex_attention_f32(int heads, int m, int n, int d, int dv, const void* plan, const int32_t* row_offsets,
+                              const int32_t* column_indices, const float* q, const float* k, const float* v,
+                              float* out, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------------------------
  * Tensor-core (tcgen05 / TMEM / TMA) entry points, fp16 storage, fp32 accumulate.
  * Shared limits: n (tokens) a multiple of 16 (dense) / 64 (sparse, fused) and <= 256;

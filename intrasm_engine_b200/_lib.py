@@ -57,6 +57,15 @@ SIGNATURES = {
     "iex_sddmm_f32_tc": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_int, c_ptr]),
     "iex_sddmm_f32_tc_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "iex_sddmm_f32_prefers_tc": (c_int, [c_int, c_int, c_int, c_int, c_int]),
+    # heads m n d dv
+    "iex_attention_f32_supported": (c_int, [c_int, c_int, c_int, c_int, c_int]),
+    "iex_attention_plan_bytes": (c_size, [c_int, c_int]),
+    # m n row_offsets cols plan bytes stream
+    "iex_attention_plan_build": (c_int, [c_int, c_int, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
+    "iex_attention_workspace_bytes": (c_size, [c_int, c_int, c_int, c_int, c_int]),
+    # heads m n d dv plan row_offsets cols q k v out workspace workspace_bytes stream
+    "iex_attention_f32": (c_int, [c_int, c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
+                                  c_ptr, c_size, c_ptr]),
     # tokens in_features out_features input weight out stream
     "iex_linear_f16": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_ptr]),
     # tokens in_features out_features grad weight|input dinput|dweight stream

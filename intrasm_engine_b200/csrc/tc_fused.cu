@@ -950,20 +950,18 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// Row-major fp16 matrix [rows, cols] (cols contiguous, rows `ld` elements apart, a multiple of 8);
-// box = [box_rows x box_cols].
-int make_map_f16(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows,
-                 int box_cols, bool swizzle) {
+int encode_map(CUtensorMap* map, CUtensorMapDataType type, int elt, const void* base, long long rows, long long cols,
+               long long ld, int box_rows, int box_cols, bool swizzle) {
   EncodeFn fn = encode_fn();
   if (!fn) return IEX_ERR_DRIVER;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * elt};
   cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1u, 1u};
   auto encode = [&] {
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return fn(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
   CUresult r = encode();
   if (r != CUDA_SUCCESS) {
@@ -973,6 +971,18 @@ int make_map_f16(CUtensorMap* map, const void* base, long long rows, long long c
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
   }
   return r == CUDA_SUCCESS ? IEX_OK : IEX_ERR_DRIVER;
+}
+
+// Row-major fp16 matrix [rows, cols] (cols contiguous, rows `ld` elements apart, a multiple of 8);
+// box = [box_rows x box_cols].
+int make_map_f16(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows,
+                 int box_cols, bool swizzle) {
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, rows, cols, ld, box_rows, box_cols, swizzle);
+}
+
+// Row-major fp32 matrix, boxes of 32 columns (one 128-byte swizzle atom).
+int make_map_f32(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows) {
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, cols, box_rows, 32, true);
 }
 
 // Operand tile: box = [box_rows x 64 cols], 128-byte swizzle.

@@ -9,7 +9,9 @@ with one mask (CSR pattern) shared by the heads, fp32.  This is the reference's 
 no softmax in it, as there is none in the reference's operators.
 
 What the class adds to calling the two operators in a loop:
-  * the mask's pattern-only data (row order, tile plan of the tensor-core SDDMM) is built once;
+  * the mask's pattern-only data (row order, mask bits, tile plan of the tensor-core SDDMM) is built once;
+  * where the scores are not asked for and d, dv <= 128, all heads run as one launch that keeps the
+    scores on chip (csrc/attention_tc.cu); otherwise
   * heads alternate over two CUDA streams.  The tensor-core SDDMM keeps the tensor pipe and
     shared memory busy, the CUDA-core SpMM the load / store path and L2; run side by side for
     different heads they finish 24 heads of the 4096 x 4096 @95 % case in 31 us per head
@@ -34,6 +36,12 @@ class SparseAttentionChain:
         self.row_indices = swizzle_rows(self.row_offsets)
         self.nnz = int(column_indices.numel())
         self.plan = None  # tile plan of the tensor-core SDDMM, built on first use for a given k
+        # the mask's bits for the one-launch kernel, which takes every position once
+        self.bits = None
+        if self.nnz > 0:
+            bits = ops.native.attention_plan(self.row_offsets, self.column_indices, self.m, self.n)
+            if int(bits[:4].view(torch.int32).item()) == 0:
+                self.bits = bits
         self._streams = [torch.cuda.Stream(device=row_offsets.device) for _ in range(max(1, int(streams)))]
 
     def _on_tensor_cores(self, kdim: int) -> bool:
@@ -57,6 +65,10 @@ class SparseAttentionChain:
         heads = q.size(0)
         assert q.shape[1] == self.m and k.shape[1] == self.n and v.shape[1] == self.n and k.size(0) == heads
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        if self.bits is not None and not return_scores and k.dtype == v.dtype == torch.float32:
+            out = ops.native.attention(q, k, v, self.bits, self.row_offsets, self.column_indices)
+            if out is not None:
+                return out
         scores = torch.empty((heads, max(self.nnz, 1)), dtype=torch.float32, device=q.device)
         out = torch.empty((heads, self.m, v.size(2)), dtype=torch.float32, device=q.device)
         if self.nnz == 0:

@@ -362,6 +362,36 @@ at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at
   return out;
 }
 
+// Masked attention over heads (pytorch/attention.py): the mask's bits, and the chain in one launch.
+at::Tensor attention_plan(const at::Tensor& ro, const at::Tensor& ci, int64_t m, int64_t n) {
+  check_common({{"row_offsets", &ro}, {"column_indices", &ci}});
+  TORCH_CHECK(ro.scalar_type() == at::kInt && ci.scalar_type() == at::kInt && ro.numel() == m + 1, "not an int32 CSR pattern");
+  c10::cuda::CUDAGuard guard(ro.device());
+  const size_t bytes = iex_attention_plan_bytes(m, n);
+  at::Tensor plan = empty_bytes(ro, bytes);
+  check_status(iex_attention_plan_build(m, n, ro.data_ptr<int>(), ci.data_ptr<int>(), plan.data_ptr(), bytes, stream_of(ro)),
+               "iex_attention_plan_build");
+  return plan;
+}
+
+// q [heads, m, d], k [heads, n, d], v [heads, n, dv] -> [heads, m, dv]; nothing for shapes the kernel does not take
+std::optional<at::Tensor> attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& plan,
+                                    const at::Tensor& ro, const at::Tensor& ci) {
+  check_common({{"q", &q}, {"k", &k}, {"v", &v}, {"plan", &plan}, {"row_offsets", &ro}, {"column_indices", &ci}});
+  const int64_t heads = q.size(0), m = q.size(1), d = q.size(2), n = k.size(1), dv = v.size(2);
+  if (!iex_attention_f32_supported(heads, m, n, d, dv) || !aligned16(q) || !aligned16(k) || !aligned16(v)) return std::nullopt;
+  TORCH_CHECK(ro.numel() == m + 1 && static_cast<size_t>(plan.numel()) >= iex_attention_plan_bytes(m, n), "plan of another mask");
+  c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor out = empty(q, {heads, m, dv});
+  const size_t bytes = iex_attention_workspace_bytes(heads, m, n, d, dv);
+  at::Tensor workspace = empty_bytes(q, bytes);
+  check_status(iex_attention_f32(heads, m, n, d, dv, plan.data_ptr(), ro.data_ptr<int>(), ci.data_ptr<int>(),
+                                 q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), out.data_ptr<float>(),
+                                 workspace.data_ptr(), bytes, stream_of(q)),
+               "iex_attention_f32");
+  return out;
+}
+
 // ReluSparseDownProj without a gather of its own: CSR activations [tokens, k] (expanded into
 // `dense`) times weight [n, k]^T into `out`.
 void ffn_down(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci, const at::Tensor& weight,
@@ -402,6 +432,8 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
   mod.def("sparse_linear", &iex_torch::sparse_linear);
   mod.def("expand_weight", &iex_torch::expand_weight);
   mod.def("linear_pair", &iex_torch::linear_pair);
+  mod.def("attention_plan", &iex_torch::attention_plan);
+  mod.def("attention", &iex_torch::attention);
   mod.def("ffn_down", &iex_torch::ffn_down);
   mod.def("relu_down_proj", &iex_torch::relu_down_proj);
   mod.def("fused_spmm_linear_half", &iex_torch::fused_spmm_linear_half);
