@@ -232,6 +232,8 @@ IEX_API int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long long
                          void* stream);
 /* Time this library expects iex_gemm_f16 to take on the current device, for choosing between ways. */
 IEX_API double iex_gemm_f16_estimate_us(int m, int n, int k, int b_mn, int out_transposed);
+/* The same for iex_spmm_f16_i16 (index_bits 16) and iex_spmm_f16_i32 (32). */
+IEX_API double iex_spmm_f16_estimate_us(int m, int k, int n, int nnz, int index_bits);
 
 /* CSR SpMM and dense linear on the same activations in one launch, either of them alone with the
  * other's row count 0.  x is [k, n] (n a multiple of 8) or, with x_tokens_major, [n, k] (k a multiple of

@@ -77,6 +77,7 @@ SIGNATURES = {
     "iex_gemm_f16": (c_int, [c_int, c_int, c_int, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll,
                              c_int, c_int, c_ptr]),
     # m n k b_mn out_transposed
+    "iex_spmm_f16_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int, c_int]),
     "iex_gemm_f16_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int, c_int]),
     # m_sparse m_dense k n nnz row_offsets cols index_bits values weight x x_tokens_major bias
     # out_sparse sparse_tokens_major out_dense dense_tokens_major stream

@@ -1,8 +1,8 @@
 // CSR SpMM on CUDA cores (sm_100a): out[z, r, :] = sum_p values[p] * dense[z, col[p], :].
 //
-// The default for fp32 (spmm_tc.cu holds a TF32 head/tail tensor-core kernel that wins at
-// densities of about 10 % and above) and for fp16 at high sparsity or small shapes; the
-// moderate-sparsity fp16 case runs on the tensor-core kernel in tc_fused.cu.
+// For short rows and small products; longer rows and denser matrices go to spmm_slice.cu, which keeps the
+// dense operand in shared memory (spmm_tc.cu holds a TF32 head/tail tensor-core kernel for fp32, tc_fused.cu,
+// spmm_tile.cu and gemm_tc.cu the tensor-core ways for fp16).
 //
 // Work decomposition
 //   * One sub-warp ("row group") of LPR lanes owns one row of A and one tile of
@@ -19,6 +19,15 @@
 #include "common.cuh"
 
 namespace iex {
+
+// spmm_slice.cu: the dense operand in shared memory
+template <typename VT, typename IT>
+int spmm_slice(int m, int k, int n, int nnz, const int* row_indices, const VT* values, long long vstride,
+               const int* row_offsets, const IT* cols, const VT* dense, const float* bias, VT* out, int batch,
+               int accumulate, cudaStream_t stream);
+template <typename VT, typename IT>
+double spmm_slice_us(int m, int k, int n, int nnz, bool vdn, int batch);
+
 namespace {
 
 template <typename VT> struct Elem;
@@ -301,6 +310,16 @@ int dispatch_dense(int m, int k, int n, int nnz, const int* ri, const VT* values
 #undef IEX_GO
 }
 
+// Time of the kernel above, us, fitted on B200: the bytes gathered (vector loads) or the gathers (scalar ones), and the
+// walk along an average row.  The slices of spmm_slice.cu win on longer rows and denser matrices; a few short rows are
+// done here before a slice is filled.
+template <typename VT>
+double rowgroup_us(int m, int n, int nnz, bool vec, int batch) {
+  const double row = m > 0 ? static_cast<double>(nnz) / m : 0.0, all = static_cast<double>(nnz) * batch;
+  if (!vec) return 3.5 + 26e-6 * all * ((n + 31) / 32) + 0.06 * row;
+  return 1.6 + 0.0302e-6 * all * n * sizeof(VT) + row * (n <= 64 && sizeof(VT) == 4 ? 0.07 : 0.12);
+}
+
 template <typename VT, typename IT>
 int spmm_entry(int m, int k, int n, int nnz, const int* ri, const VT* values,
                long long vstride, const int* ro, const IT* cols, const VT* dense,
@@ -313,6 +332,9 @@ int spmm_entry(int m, int k, int n, int nnz, const int* ri, const VT* values,
   // 128-bit loads of the sparse arrays need 16-byte aligned bases for every batch item.
   const bool vs = aligned16(values) && aligned16(cols) &&
                   (vstride * static_cast<long long>(sizeof(VT))) % 16 == 0;
+  const bool vec = n % Elem<VT>::kPerVec == 0 && aligned16(dense) && aligned16(out);
+  if (vs && spmm_slice_us<VT, IT>(m, k, n, nnz, vec, batch) < rowgroup_us<VT>(m, n, nnz, vec, batch))
+    return spmm_slice<VT, IT>(m, k, n, nnz, ri, values, vstride, ro, cols, dense, bias, out, batch, accumulate, s);
   if (vs)
     return dispatch_dense<VT, IT, true>(m, k, n, nnz, ri, values, vstride, ro, cols, dense,
                                         bias, out, batch, accumulate, s);
@@ -352,4 +374,12 @@ extern "C" int iex_spmm_f16_i32(int m, int k, int n, int nnz, const int32_t* row
       m, k, n, nnz, row_indices, static_cast<const __half*>(values), 0, row_offsets,
       column_indices, static_cast<const __half*>(dense), bias, static_cast<__half*>(out),
       batch, 0, stream);
+}
+
+extern "C" double iex_spmm_f16_estimate_us(int m, int k, int n, int nnz, int index_bits) {
+  const bool vec = n % 8 == 0;
+  const double slice = index_bits == 16 ? iex::spmm_slice_us<__half, uint16_t>(m, k, n, nnz, vec, 1)
+                                        : iex::spmm_slice_us<__half, int>(m, k, n, nnz, vec, 1);
+  const double rows = iex::rowgroup_us<__half>(m, n, nnz, vec, 1);
+  return slice < rows ? slice : rows;
 }

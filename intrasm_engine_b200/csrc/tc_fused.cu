@@ -985,6 +985,13 @@ int make_map_f32(CUtensorMap* map, const void* base, long long rows, long long c
   return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, cols, box_rows, 32, true);
 }
 
+// Row-major matrix, boxes of box_cols columns, rows packed one after the other.
+int make_map_slice(CUtensorMap* map, bool half, const void* base, long long rows, long long cols, int box_rows,
+                   int box_cols) {
+  return encode_map(map, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, half ? 2 : 4, base,
+                    rows, cols, cols, box_rows, box_cols, false);
+}
+
 // Operand tile: box = [box_rows x 64 cols], 128-byte swizzle.
 int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows) {
   return make_map_f16(map, base, rows, cols, cols, box_rows, 64, true);

@@ -62,7 +62,6 @@ void gemm(int64_t m, int64_t n, int64_t k, const at::Tensor& a, bool a_mn, const
 // Estimates in microseconds, fitted to measurements on B200.
 //   expand   one pass over the CSR arrays and the dense copy, at 5.5 TB/s
 //   decode   the block decoder of spmm_tile.cu: per row, its stored positions and its blocks of columns
-//   cores    CUDA cores: gathered bytes, and the serial walk over an average row
 double expand_us(int64_t m, int64_t k, int64_t nnz, int bits) {
   return 2.5 + (2.0 * m * round8(k) + static_cast<double>(nnz) * (2 + bits / 8)) / 5.5e6;
 }
@@ -70,9 +69,6 @@ double block_decode_us(int64_t m, int64_t k, int64_t n, int64_t nnz) {
   const int64_t rows = round8((m + 147) / 148);
   const double t = 8.0 + rows * (0.13e-3 * nnz / std::max<int64_t>(m, 1) + 0.0166 * ((k + 511) / 512));
   return t * (n <= 128 ? 1.0 : 1.25) * std::max<int64_t>(1, (rows + 127) / 128);
-}
-double cores_us(int64_t m, int64_t n, int64_t nnz) {
-  return 1.6 + 0.0605e-6 * 2.0 * nnz * n + 0.158 * nnz / std::max<int64_t>(m, 1);
 }
 bool decode_supported(const at::Tensor& b, const at::Tensor& values, const at::Tensor& ci) {
   const int64_t k = b.size(0), n = b.size(1);
@@ -107,7 +103,7 @@ at::Tensor spmm_half(const at::Tensor& b, const at::Tensor& ri, const at::Tensor
   const double dense = expand_us(m, k, nnz, index_bits(ci)) + iex_gemm_f16_estimate_us(m, n, k, 1, 0) +
                        (n % 8 == 0 ? 0.0 : 2.0);
   const double decode = decode_supported(b, values, ci) ? block_decode_us(m, k, n, nnz) : 1e30;
-  if (mode == kAuto && cores_us(m, n, nnz) <= std::min(dense, decode)) return cores();
+  if (mode == kAuto && iex_spmm_f16_estimate_us(m, k, n, nnz, index_bits(ci)) <= std::min(dense, decode)) return cores();
   if (decode <= dense) return spmm_tc_half(b, ro, values, ci, m);
   c10::cuda::CUDAGuard guard(b.device());
   maybe_validate(ro, ci, m, k, nullptr, false);
@@ -160,7 +156,7 @@ at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tens
       k > 0 && nnz > 0) {
     // the expanded matrix read with its row dimension as the contraction: no transposed pattern needed
     const double dense = expand_us(m, k, nnz, index_bits(p.ci)) + iex_gemm_f16_estimate_us(k, n, m, 1, 0);
-    const double cores = cores_us(k, n, nnz) + 5.0;
+    const double cores = iex_spmm_f16_estimate_us(k, m, n, nnz, index_bits(p.ci)) + 5.0;
     if (dense < cores) {
       c10::cuda::CUDAGuard guard(grad.device());
       at::Tensor out = empty(grad, {k, n});
