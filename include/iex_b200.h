@@ -384,6 +384,8 @@ IEX_API int iex_csr_to_dense_f16_ld(int m, int k, int ld, const int32_t* row_off
 /* out[p] = dense[row(p) * ld + column_indices[p]] for every stored position p (fp16). */
 IEX_API int iex_csr_sample_f16(int m, int k, long long ld, const int32_t* row_offsets, const void* column_indices,
                                int index_bits, const void* dense, void* out, void* stream);
+/* out[i] = in[perm[i]] for `count` values of 2 or 4 bytes. */
+IEX_API int iex_gather_values(int count, int elt_bytes, const void* in, const long long* perm, void* out, void* stream);
 /* Copies rows of `cols` fp16 values into rows of `ld` values (a multiple of 8), zero-filled. */
 IEX_API int iex_pad_rows_f16(int rows, int cols, int ld, const void* in, void* out, void* stream);
 /* out = max(in, 0) over `count` fp16 values (a multiple of 8; NaN becomes 0). */

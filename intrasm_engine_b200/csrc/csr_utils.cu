@@ -270,6 +270,26 @@ csr_sample_kernel(int m, long long ld, const int* __restrict__ row_offsets, cons
   }
 }
 
+// out[i] = in[perm[i]]: the values of a pattern in the order of its transpose.  Bound by the sectors of `in` that the
+// gathers touch; four per thread in flight.  234 k fp32 values: 4.6 -> 2.4 us, and 5 us less of host time than the
+// library's indexing.
+template <typename T>
+__global__ void __launch_bounds__(256)
+gather_values_kernel(int count, const T* __restrict__ in, const long long* __restrict__ perm, T* __restrict__ out) {
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const long long base = blockIdx.x * 1024ll + threadIdx.x;
+  long long at[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) at[u] = base + 256 * u < count ? __ldg(perm + base + 256 * u) : 0;
+  T v[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) v[u] = __ldg(in + at[u]);
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (base + 256 * u < count) out[base + 256 * u] = v[u];
+}
+
 // Rows of `cols` fp16 values, any alignment, into rows of `ld` (a multiple of 8), the rest zero.
 __global__ void __launch_bounds__(256)
 pad_rows_kernel(int rows, int cols, int ld, const __half* __restrict__ in, __half* __restrict__ out) {
@@ -437,6 +457,20 @@ extern "C" int iex_csr_sample_f16(int m, int k, long long ld, const int32_t* row
                              static_cast<const uint16_t*>(column_indices), d, static_cast<__half*>(out));
   return launch_overlapped(csr_sample_kernel<int>, dim3(grid), dim3(256), 0, s, m, ld, row_offsets,
                            static_cast<const int*>(column_indices), d, static_cast<__half*>(out));
+}
+
+extern "C" int iex_gather_values(int count, int elt_bytes, const void* in, const long long* perm, void* out, void* stream) {
+  using namespace iex;
+  if (count < 0 || (elt_bytes != 2 && elt_bytes != 4)) return IEX_ERR_BAD_ARG;
+  if (count == 0) return IEX_OK;
+  if (!in || !perm || !out) return IEX_ERR_BAD_ARG;
+  const dim3 grid((static_cast<unsigned>(count) + 1023u) / 1024u);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (elt_bytes == 4)
+    return launch_overlapped(gather_values_kernel<uint32_t>, grid, dim3(256), 0, s, count,
+                             static_cast<const uint32_t*>(in), perm, static_cast<uint32_t*>(out));
+  return launch_overlapped(gather_values_kernel<uint16_t>, grid, dim3(256), 0, s, count, static_cast<const uint16_t*>(in),
+                           perm, static_cast<uint16_t*>(out));
 }
 
 extern "C" int iex_pad_rows_f16(int rows, int cols, int ld, const void* in, void* out, void* stream) {

@@ -165,7 +165,19 @@ at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tens
     }
   }
   // transposing the pattern is bookkeeping done once (get_transpose_info); the values follow it
-  at::Tensor values_t = values.index({p.perm});
+  at::Tensor values_t;
+  if (p.perm.scalar_type() == at::kLong && p.perm.is_contiguous() && values.is_contiguous() && p.perm.dim() == 1 &&
+      p.perm.numel() == nnz && p.perm.device() == values.device() &&
+      (values.scalar_type() == at::kFloat || values.scalar_type() == at::kHalf)) {
+    c10::cuda::CUDAGuard guard(values.device());
+    values_t = empty(values, {nnz});
+    check_status(iex_gather_values(nnz, values.element_size(), values.data_ptr(),
+                                   reinterpret_cast<const long long*>(p.perm.data_ptr<int64_t>()), values_t.data_ptr(),
+                                   stream_of(values)),
+                 "iex_gather_values");
+  } else {
+    values_t = values.index({p.perm});
+  }
   if (values.scalar_type() == at::kFloat)
     return spmm_sputnik_reuse_weight(grad.unsqueeze(0), p.ri_t, values_t, p.ro_t, p.ci_t, k).squeeze(0);
   return spmm_sputnik_reuse_weight_half(grad.unsqueeze(0), p.ri_t, values_t, p.ro_t, p.ci_t, k).squeeze(0);

@@ -150,3 +150,13 @@ def test_dense_copy_follows_the_values():
     sparse = _ints((64, 64), 6, 1, 3, density=0.1)
     values, _ri, ro, ci = dense_to_sparse_cuda(_dev(sparse))
     assert copy.current(values, ro, ci) is None
+
+
+@pytest.mark.parametrize("count", [1, 255, 1024, 1025, 70001])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_gather_values(count, dtype):
+    v = torch.randn(count, device=DEV).to(dtype)
+    perm = torch.randperm(count, device=DEV)
+    out = torch.full((count + 1,), 9.0, dtype=dtype, device=DEV)
+    _lib.call("iex_gather_values", count, v.element_size(), v.data_ptr(), perm.data_ptr(), out.data_ptr(), _stream())
+    assert torch.equal(out[:-1], v[perm]) and float(out[-1]) == 9.0
