@@ -24,6 +24,8 @@
 // Every mbarrier wait is bounded, as in tc_fused.cu.
 #include <cuda.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "common.cuh"
@@ -117,6 +119,40 @@ __device__ __forceinline__ void tile_of(int t, const GemmParams& p, int& tm, int
   const int r = t - g * per_group;
   tm = first + r % rows;
   tn = r / rows;
+}
+
+// Sums of the P partial tiles of a cluster, in part order, from the CTAs' shared memory.  A load from another CTA takes
+// about 0.4 us and this is all that is left to do, so a thread keeps 8 to 12 of them in flight: with one vector at a time
+// the
+// exchange of a 256 x 256 tile between two pairs took 8 us, now 3 us (256 x 4096 x 11008: 39.5 -> 34.4 us, with 128-wide
+// tiles 27.2 -> 25.2 us).
+template <int P, typename Write>
+__device__ __forceinline__ void add_parts(uint32_t base, int l0, int vecs, uint32_t vec_inv, uint32_t line_bytes, int total,
+                                          int half, const Write& write) {
+  constexpr int U = P == 2 ? 6 : P == 3 ? 4 : 3;
+  for (int f0 = threadIdx.x; f0 < total; f0 += U * kThreads) {
+    float4 x[U][P];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int f = min(f0 + u * kThreads, total - 1);
+      const uint32_t line = (static_cast<uint32_t>(f) * vec_inv) >> 20;
+      const uint32_t off = base + (l0 + line) * line_bytes + (f - line * vecs) * 16u;
+#pragma unroll
+      for (int q = 0; q < P; ++q)
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(x[u][q].x), "=f"(x[u][q].y), "=f"(x[u][q].z), "=f"(x[u][q].w)
+                     : "r"(map_to_rank(off, 2 * q + half)));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float4 sum = x[u][0];
+#pragma unroll
+      for (int q = 1; q < P; ++q) {
+        sum.x += x[u][q].x; sum.y += x[u][q].y; sum.z += x[u][q].z; sum.w += x[u][q].w;
+      }
+      if (f0 + u * kThreads < total) write(f0 + u * kThreads, sum);
+    }
+  }
 }
 
 // The operands' storage orders are template parameters for the sake of the one thread that issues the
@@ -369,17 +405,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int lines = p.out_t ? p.bn : kHalfM;                   // lines of the partial tile
     const uint32_t line_bytes = (p.out_t ? kHalfM : p.bn + 4) * 4u;
     const int l0 = part * lines / p.parts, l1 = (part + 1) * lines / p.parts;
-    for (int f = threadIdx.x; f < (l1 - l0) * vecs; f += kThreads) {
-      const int line = l0 + f / vecs, v = f % vecs;
-      const uint32_t off = base + line * line_bytes + v * 16u;
-      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int q = 0; q < p.parts; ++q) {
-        float4 x;
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                     : "r"(map_to_rank(off, 2 * q + half)));
-        sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
-      }
+    const uint32_t vec_inv = ((1u << 20) + vecs - 1) / vecs;  // f / vecs: f is below 4096, vecs 8 to 64
+    auto write = [&](int f, const float4& sum) {
+      const int line = l0 + static_cast<int>((static_cast<uint32_t>(f) * vec_inv) >> 20);
+      const int v = f - (line - l0) * vecs;
       uint2 pk;
       __half2* hh = reinterpret_cast<__half2*>(&pk);
       hh[0] = __floats2half2_rn(sum.x, sum.y);
@@ -396,7 +425,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           for (int e = 0; e < 4 && inner + e < n_inner; ++e) dst[e] = hv[e];
         }
       }
-    }
+    };
+    const int total = (l1 - l0) * vecs;
+    if (p.parts == 2) add_parts<2>(base, l0, vecs, vec_inv, line_bytes, total, half, write);
+    else if (p.parts == 3) add_parts<3>(base, l0, vecs, vec_inv, line_bytes, total, half, write);
+    else add_parts<4>(base, l0, vecs, vec_inv, line_bytes, total, half, write);
   }
   // nobody leaves while the other CTAs may still read its shared memory or write its tensor memory
   tcgen05_fence_before();
@@ -423,25 +456,29 @@ int stages_for(int bn, bool b_mn) {
 // belong to one GPC, so large clusters leave some SMs out.
 constexpr int kResident[5] = {0, 74, 33, 22, 15};
 
-// Tile width and K split for the smallest estimated time, in microseconds.  Measured on B200: a
-// k-block costs 0.23 us + 0.0005 us per tile column (256 wide: bound by the tensor pipe, narrow:
-// by the operands' way into shared memory), a launch has about 5 us of its own (first loads,
-// read-out), a split 2 us more for the exchange; HBM bounds what is left.
+// Tile width and K split for the smallest estimated time, in microseconds.  Fitted to a sweep over shapes on B200,
+// within about 5 %: a k-block takes 0.155 us + 0.0001 us per tile column, or 0.00118 us per column where the tensor pipe bounds
+// it (from 144 columns), or what L2 delivers to all CTAs together (17.5 TB/s); rows of B that run along n cost 0.02 us
+// more.  HBM gives 5.8 TB/s; where the two bounds are close they add up rather than hide each other.  A launch has
+// 5.3 us of its own (first loads, read-out), an exchange between the parts 0.3 us and 0.0095 us per column.
 double plan_gemm(int m, int n, int k, bool b_mn, bool out_t, int sms, GemmPlan* plan) {
   const int kb = (k + kBK - 1) / kBK, tm = (m + 255) / 256;
-  const double dram = (static_cast<double>(m) * k + static_cast<double>(n) * k + static_cast<double>(m) * n) * 2.0 / 6.5e6;
+  const double dram = (static_cast<double>(m) * k + static_cast<double>(n) * k + static_cast<double>(m) * n) * 2.0 / 5.8e6;
   double best = 1e30;
   for (int bn = 256; bn >= 32; bn -= 32) {
     if ((b_mn || !out_t) && bn % 64 != 0) continue;  // 64-column atoms / output boxes
     if (bn >= n + 64) continue;                      // columns nobody asked for
     const int tiles = tm * ((n + bn - 1) / bn);
-    const double block = 0.23 + 0.0005 * bn;
+    const double alone = std::max(0.155 + 0.0001 * bn, 0.00118 * bn) + (b_mn ? 0.02 : 0.0);
     for (int parts = 1; parts <= 4; ++parts) {
       const int resident = parts == 1 ? sms / 2 : kResident[parts];
       if (parts > 1 && (tiles > resident || kb < 4 * parts)) continue;
       const int waves = (tiles + resident - 1) / resident;
-      double t = waves * (((kb + parts - 1) / parts) * block + 0.4);
-      t = (t > dram ? t : dram) + 5.0 + bn / 256.0 + (parts > 1 ? 1.0 + bn / 256.0 : 0.0);
+      const int ctas = 2 * parts * std::min(tiles, resident);
+      const double block = std::max(alone, ctas * (kABytes + 64.0 * bn) / 17.5e6);
+      const double loop = waves * ((kb + parts - 1) / parts * block + 0.3);
+      const double l2 = loop * loop, d2 = dram * dram;
+      const double t = std::sqrt(std::sqrt(l2 * l2 + d2 * d2)) + 5.0 + 0.5 * bn / 256 + (parts > 1 ? 0.3 + 0.0095 * bn : 0.0);
       if (t < best) { best = t; *plan = {bn, parts}; }
     }
   }
