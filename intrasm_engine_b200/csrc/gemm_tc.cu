@@ -21,6 +21,10 @@
 // its P pairs and adds the fp32 partial tiles through distributed shared memory, in part order
 // (deterministic, no workspace and no second launch).
 //
+// Measured against the one-CTA kernel: 2048 x 4096 -> 12288, forward and backward, 1245 -> 452-520 us (the power limit
+// moves it; the three products alone 146 / 148 / 144 us, 1.41 PFLOP/s); 256 x 11008 -> 4096 35.3 -> 26.1 us; 64 x 4096 ->
+// 12288 23.4 us, where HBM bounds both.
+//
 // Every mbarrier wait is bounded, as in tc_fused.cu.
 #include <cuda.h>
 
