@@ -25,8 +25,8 @@
 //                    registers.  Two warps per tensor-memory quarter share a tile's columns: the tensor pipe
 //                    only has S(t + 1) to do until P(t) is there, so the time from S to P is what counts
 //                    (one warp per quarter and tile, taking turns: 2900 cycles a tile)
-// The runs are equal shares of all tiles; a band cut between two CTAs is added to zeroed rows by both (two
-// addends: the order does not matter).
+// The runs are equal shares of all tiles; the pieces of a band that is cut between CTAs meet in a workspace and are
+// added in order by whichever comes last.
 //
 // Values of v at masked-out positions must not count even if they are not finite.  Zero times such a value is
 // not zero, so the prepare kernel looks for them and the (rare) heads that have some are summed position
@@ -35,6 +35,8 @@
 // Every mbarrier wait is bounded, as in tc_fused.cu.
 #include <cuda.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "common.cuh"
@@ -67,6 +69,8 @@ struct AttnParams {
   float* out;
   const int* row_offsets;
   const int* cols;
+  float4* partials;              // [2 * CTAs][dvp / 4][128]: sums of a CTA's first and last band where they are cut
+  int* counters;                 // [bands of all heads and parts][8]: pieces of a band that are there, per warp
   const int* flags;              // [heads][flag_blocks]: values of v that are not finite
   int flag_blocks;
   int* status;
@@ -74,6 +78,11 @@ struct AttnParams {
 
 __device__ __forceinline__ int range_begin(int c, int total, int ctas) {
   return static_cast<int>(static_cast<long long>(c) * total / ctas);
+}
+
+// The CTA whose range holds tile t.
+__device__ __forceinline__ int cta_of(int t, int total, int ctas) {
+  return static_cast<int>(((t + 1ll) * ctas - 1) / total);
 }
 
 // TF32 head of x, rounded half away from zero, by integer arithmetic on the sign-magnitude bits.
@@ -384,15 +393,49 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       bool finite = true;
       for (int i = lane; i < p.flag_blocks; i += 32) finite = finite && __ldg(p.flags + head * p.flag_blocks + i) == 0;
       finite = __all_sync(0xffffffffu, finite);
-      const bool whole = tiles_here == p.tiles;
-      if (row < p.m && finite) {
+      bool write = finite;
+      if (finite && tiles_here != p.tiles) {
+        // A band cut between CTAs: this piece goes to the workspace, and the warp that finds all the others there adds them
+        // up in the order of the keys.
+        constexpr int kQuads = kCols / 4;
+        const int first_tile = item * p.tiles;
+        const int first = cta_of(first_tile, p.total, gridDim.x), last = cta_of(first_tile + p.tiles - 1, p.total, gridDim.x);
+        const size_t mine = static_cast<size_t>(wg) * kQuads * 128 + row_local;
+        float4* to = p.partials + (2 * blockIdx.x + (r == r0 ? 0 : 1)) * static_cast<size_t>(DVP / 4 * 128) + mine;
+#pragma unroll
+        for (int j = 0; j < kQuads; ++j)
+          __stcg(to + j * 128, make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]));
+        __threadfence();
+        __syncwarp();
+        int there = 0;
+        if (lane == 0) there = atomicAdd(p.counters + item * 8 + wg * 4 + q4, 1);
+        write = __shfl_sync(0xffffffffu, there, 0) == last - first;
+        if (write) {
+          __threadfence();
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
+          for (int c = first; c <= last; ++c) {
+            const int slot = 2 * c + (range_begin(c, p.total, gridDim.x) < first_tile ? 1 : 0);
+            const float4* from = p.partials + slot * static_cast<size_t>(DVP / 4 * 128) + mine;
+            float4 x[kQuads];
+#pragma unroll
+            for (int j = 0; j < kQuads; ++j) x[j] = __ldcg(from + j * 128);
+#pragma unroll
+            for (int j = 0; j < kQuads; ++j) {
+              acc[4 * j] += x[j].x;
+              acc[4 * j + 1] += x[j].y;
+              acc[4 * j + 2] += x[j].z;
+              acc[4 * j + 3] += x[j].w;
+            }
+          }
+        }
+      }
+      if (write && row < p.m) {
         float* dst = p.out + (static_cast<size_t>(head) * p.m + row) * p.dv + col0 + wg * kCols;
 #pragma unroll
         for (int j = 0; j < kCols / 4; ++j)
-          if (col0 + wg * kCols + 4 * j < p.dv) {
-            const float4 f = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-            if (whole) reinterpret_cast<float4*>(dst)[j] = f; else atomicAdd(reinterpret_cast<float4*>(dst) + j, f);
-          }
+          if (col0 + wg * kCols + 4 * j < p.dv)
+            reinterpret_cast<float4*>(dst)[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
       }
       if (!finite && t_begin == 0 && wg == 0 && col0 == 0) rows_by_position(p, head, band * 128 + q4 * 32, lane);
       r = seg_end;
@@ -409,23 +452,16 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
 constexpr int kPrepKeys = 64;
 
 // Block (x, h): keys [64 x, +64) of head h as hi / lo planes.  k planes [2][heads * n][dp], v planes transposed,
-// [2][heads * dvt][np].  The blocks of the last y zero the rows of bands that two CTAs of the main kernel share.
+// [2][heads * dvt][np].  The blocks of the last y zero the main kernel's counters.
 __global__ void __launch_bounds__(256)
-attention_prepare_kernel(const AttnParams p, int dp, int ctas, float* __restrict__ k_planes, float* __restrict__ v_planes,
+attention_prepare_kernel(const AttnParams p, int dp, float* __restrict__ k_planes, float* __restrict__ v_planes,
                          int* __restrict__ flags) {
   extern __shared__ float v_tile[];  // [64][dv + 1]
   grid_dependency_wait();
   grid_launch_dependents();
   if (static_cast<int>(blockIdx.y) == p.heads) {
-    for (int c = 1 + blockIdx.x; c < ctas; c += gridDim.x) {
-      const int b = range_begin(c, p.total, ctas), item = b / p.tiles;
-      if (b % p.tiles == 0) continue;
-      const int unit = item / p.bands, row0 = (item - unit * p.bands) * 128, rows = min(128, p.m - row0);
-      const int head = unit / p.parts, dvp = p.dvt / p.parts, col0 = (unit - head * p.parts) * dvp;
-      const int width = min(dvp, p.dv - col0);
-      float* dst = p.out + (static_cast<size_t>(head) * p.m + row0) * p.dv + col0;
-      for (int i = threadIdx.x; i < rows * width; i += 256) dst[static_cast<size_t>(i / width) * p.dv + i % width] = 0.f;
-    }
+    const int counters = p.heads * p.parts * p.bands * 8;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < counters; i += gridDim.x * 256) p.counters[i] = 0;
     return;
   }
   const int head = blockIdx.y, key0 = blockIdx.x * kPrepKeys;
@@ -570,7 +606,8 @@ extern "C" size_t iex_attention_workspace_bytes(int heads, int m, int n, int d, 
   Shape s;
   if (!attention_shape(heads, m, n, d, dv, &s)) return 0;
   return round256(2ull * heads * n * s.dp * 4) + round256(2ull * heads * s.dvt * s.np * 4) +
-         round256(4ull * heads * flag_blocks_of(s.np));
+         round256(4ull * heads * flag_blocks_of(s.np)) + round256(2ull * kNumSMs * 128 * s.dvp * 4) +
+         round256(32ull * heads * s.parts * ((m + 127) / 128));
 }
 
 extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const void* plan, const int32_t* row_offsets,
@@ -588,7 +625,10 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   float* k_planes = reinterpret_cast<float*>(ws);
   float* v_planes = reinterpret_cast<float*>(ws + round256(2ull * heads * n * s.dp * 4));
   int* flags = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(v_planes) + round256(2ull * heads * s.dvt * s.np * 4));
+  uint8_t* after = reinterpret_cast<uint8_t*>(flags) + round256(4ull * heads * flag_blocks_of(s.np));
   AttnParams p{};
+  p.partials = reinterpret_cast<float4*>(after);
+  p.counters = reinterpret_cast<int*>(after + round256(2ull * kNumSMs * 128 * s.dvp * 4));
   p.heads = heads; p.m = m; p.n = n; p.d = d; p.dv = dv;
   p.parts = s.parts;
   p.dvt = s.dvt;
@@ -604,17 +644,28 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   p.flags = flags;
   p.flag_blocks = flag_blocks_of(s.np);
   p.status = status_word();
-  // One CTA per SM with an equal share of the tiles, unless that would cut a band in three: then half a
-  // band per CTA (or a whole one, if the halves would not fit on the chip at once).
-  const int items = heads * s.parts * p.bands, sms = sm_count();
-  int ctas = items >= sms ? sms : (2 * items <= sms && p.tiles > 1 ? 2 * items : items);
+  // One CTA per SM with an equal share of the tiles; with fewer bands than SMs, as many equal pieces of every band as
+  // fit on the chip, for a CTA that works on two bands pays for a second start (5 us), and no more than this
+  // root, since whoever comes last adds the pieces up alone.
+  const int items = heads * s.parts * p.bands, sms = std::min(sm_count(), kNumSMs);
+  const int pieces = std::max(1, static_cast<int>(std::sqrt(1.5 * p.tiles)));
+  const int ctas = items >= sms ? sms : items * std::min(pieces, sms / items);
   CUtensorMap mk, mv;
   int st = make_map_f32(&mk, k_planes, 2ll * heads * n, s.dp, s.kt);
   if (st == IEX_OK) st = make_map_f32(&mv, v_planes, 2ll * heads * s.dvt, s.np, s.dvp);
   if (st != IEX_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  st = launch_overlapped(attention_prepare_kernel, dim3(p.flag_blocks, heads + 1), dim3(256),
-                         static_cast<size_t>(kPrepKeys) * (dv + 1) * 4, cs, p, s.dp, ctas, k_planes, v_planes, flags);
+  // The prepare kernel of a call usually follows the main kernel of the one before.  Launched ahead of that kernel's end its
+  // blocks would crowd on the few SMs that are free (6 heads x 1003, d 80: 42 us a call instead of 31), so that is
+  // done only where main kernels leave a third of the chip free (then it saves 1 to 2 us).
+  const dim3 prep_grid(p.flag_blocks, heads + 1);
+  const size_t prep_smem = static_cast<size_t>(kPrepKeys) * (dv + 1) * 4;
+  if (3 * ctas <= 2 * sms) {
+    st = launch_overlapped(attention_prepare_kernel, prep_grid, dim3(256), prep_smem, cs, p, s.dp, k_planes, v_planes, flags);
+  } else {
+    attention_prepare_kernel<<<prep_grid, 256, prep_smem, cs>>>(p, s.dp, k_planes, v_planes, flags);
+    st = launch_status();
+  }
   if (st != 0) return st;
   const int which = s.da * 10 + s.dvp / 16;
   switch (which) {
