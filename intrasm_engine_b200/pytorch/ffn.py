@@ -53,16 +53,22 @@ class ReluSparseDownProj:
         self.gather = gather if world > 1 else "none"
         self.device = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
         self.parts = split_k_parts(self.n_local)
-        self.workspace = None
+        self._workspace = None
         self.dense_act = torch.empty((self.tokens, self.k), dtype=torch.float16, device=self.device)
         self.out_local = torch.empty((self.tokens, self.n_local), dtype=torch.float16, device=self.device)
         self.peer = None
         self._slot = 0
         if self.gather == "peer":
             from .distributed import PeerGather
-            need = _lib.lib.iex_tc_workspace_bytes(0, 1, self.n_local, self.parts, self.tokens)
-            self.workspace = torch.empty(max(int(need), 256), dtype=torch.uint8, device=self.device)
             self.peer = PeerGather(self.tokens, self.n, rank, world, self.device, group=group)
+
+    @property
+    def workspace(self) -> torch.Tensor:
+        """Scratch of the split-K entry points, allocated when first asked for: the CTA-pair GEMM needs none."""
+        if self._workspace is None:
+            need = _lib.lib.iex_tc_workspace_bytes(0, 1, self.n_local, self.parts, self.tokens)
+            self._workspace = torch.empty(max(int(need), 256), dtype=torch.uint8, device=self.device)
+        return self._workspace
 
     # -- pieces ---------------------------------------------------------------------------
     def expand(self, values, row_offsets, column_indices, stream=None) -> torch.Tensor:
