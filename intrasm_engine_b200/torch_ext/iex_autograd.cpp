@@ -97,7 +97,7 @@ enum Mode { kCudaCores = 0, kTensorCores = 1, kAuto = 2 };
 at::Tensor spmm_half(const at::Tensor& b, const at::Tensor& ri, const at::Tensor& values, const at::Tensor& ro,
                      const at::Tensor& ci, int64_t m, int mode) {
   const int64_t k = b.size(0), n = b.size(1), nnz = values.numel();
-  auto cores = [&] { return spmm_sputnik_reuse_weight_half(b.unsqueeze(0), ri, values, ro, ci, m).squeeze(0); };
+  auto cores = [&] { return spmm_matrix(b, ri, values, ro, ci, m); };
   if (mode == kCudaCores || m == 0 || k == 0 || n == 0) return cores();
   check_csr_half(b, values, ro, ci, m);
   const double dense = expand_us(m, k, nnz, index_bits(ci)) + iex_gemm_f16_estimate_us(m, n, k, 1, 0) +
@@ -125,13 +125,13 @@ struct SpmmArgs {
 
 at::Tensor spmm_forward(const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
   if (values.scalar_type() == at::kFloat)
-    return spmm_sputnik_reuse_weight(b.unsqueeze(0), p.ri, values, p.ro, p.ci, p.m).squeeze(0);
+    return spmm_matrix(b, p.ri, values, p.ro, p.ci, p.m);
   return spmm_half(b, p.ri, values, p.ro, p.ci, p.m, p.mode);
 }
 
 at::Tensor grad_of_values(const at::Tensor& grad, const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
   if (grad.scalar_type() != at::kHalf)
-    return sddmm_sputnik_atomic_upd_weight(grad.unsqueeze(0), b.unsqueeze(0), p.ri, p.ro, p.ci.to(at::kInt));
+    return sddmm_matrix(grad, b, p.ri, p.ro, p.ci.scalar_type() == at::kInt ? p.ci : p.ci.to(at::kInt));
   const int64_t m = grad.size(0), n = grad.size(1), k = b.size(0), nnz = values.numel();
   if (p.mode != kCudaCores && b.scalar_type() == at::kHalf && m > 0 && n > 0 && k > 0 && nnz > 0) {
     // every product of the dense matrix, of which the stored positions are kept, against one
@@ -149,7 +149,7 @@ at::Tensor grad_of_values(const at::Tensor& grad, const at::Tensor& b, const at:
       return out;
     }
   }
-  return sddmm_sputnik_half(grad.unsqueeze(0), b.to(at::kHalf).unsqueeze(0), p.ri, p.ro, p.ci);
+  return sddmm_matrix(grad, b.scalar_type() == at::kHalf ? b : b.to(at::kHalf), p.ri, p.ro, p.ci);
 }
 
 at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
@@ -180,9 +180,7 @@ at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tens
   } else {
     values_t = values.index({p.perm});
   }
-  if (values.scalar_type() == at::kFloat)
-    return spmm_sputnik_reuse_weight(grad.unsqueeze(0), p.ri_t, values_t, p.ro_t, p.ci_t, k).squeeze(0);
-  return spmm_sputnik_reuse_weight_half(grad.unsqueeze(0), p.ri_t, values_t, p.ro_t, p.ci_t, k).squeeze(0);
+  return spmm_matrix(grad, p.ri_t, values_t, p.ro_t, p.ci_t, k);
 }
 
 struct MySpMMBackward : public Node {

@@ -74,8 +74,8 @@ void maybe_validate(const at::Tensor& row_offsets, const at::Tensor& column_indi
 
 void check_spmm(const at::Tensor& b, const at::Tensor& row_indices, const at::Tensor& values,
                 const at::Tensor& row_offsets, const at::Tensor& column_indices, int64_t m,
-                bool per_batch_values) {
-  TORCH_CHECK(b.dim() == 3, "b must be [batch, k, n]");
+                bool per_batch_values, bool batched) {
+  TORCH_CHECK(b.dim() == (batched ? 3 : 2), "b must be ", batched ? "[batch, k, n]" : "[k, n]");
   if (per_batch_values) {
     TORCH_CHECK(values.dim() == 2, "values must be [batch, nnz]");
     TORCH_CHECK(b.size(0) == values.size(0), "values and b disagree on the batch size");
@@ -92,21 +92,23 @@ void check_spmm(const at::Tensor& b, const at::Tensor& row_indices, const at::Te
               "row_indices and row_offsets must be int32");
   TORCH_CHECK(row_indices.size(0) == m && row_offsets.size(0) == m + 1,
               "row_indices must have m entries and row_offsets m + 1");
-  TORCH_CHECK(b.size(0) == 1 || column_indices.size(0) % 4 == 0,
+  TORCH_CHECK(!batched || b.size(0) == 1 || column_indices.size(0) % 4 == 0,
               "If batch size > 1 then number of nonzeros should be a multiple of 4");
 }
 
 at::Tensor spmm_f32(const at::Tensor& b, const at::Tensor& row_indices, const at::Tensor& values,
                     const at::Tensor& row_offsets, const at::Tensor& column_indices, int64_t m,
-                    bool per_batch_values) {
-  check_spmm(b, row_indices, values, row_offsets, column_indices, m, per_batch_values);
+                    bool per_batch_values, bool batched = true) {
+  check_spmm(b, row_indices, values, row_offsets, column_indices, m, per_batch_values, batched);
   TORCH_CHECK(b.scalar_type() == at::kFloat && values.scalar_type() == at::kFloat,
               "b and values must be float32");
   TORCH_CHECK(column_indices.scalar_type() == at::kInt, "column_indices must be int32");
   c10::cuda::CUDAGuard guard(b.device());
-  const int batch = b.size(0), k = b.size(1), n = b.size(2), nnz = column_indices.size(0);
+  const int batch = batched ? b.size(0) : 1, k = b.size(-2), n = b.size(-1), nnz = column_indices.size(0);
   maybe_validate(row_offsets, column_indices, m, k, &row_indices, false);
-  at::Tensor out = per_batch_values ? at::zeros({batch, m, n}, b.options()) : empty(b, {batch, m, n});
+  at::Tensor out = per_batch_values ? at::zeros({batch, m, n}, b.options())
+                   : batched        ? empty(b, {batch, m, n})
+                                    : empty(b, {m, n});
   check_status(iex_spmm_f32(m, k, n, nnz, row_indices.data_ptr<int>(), values.data_ptr<float>(),
                             per_batch_values ? nnz : 0, row_offsets.data_ptr<int>(),
                             column_indices.data_ptr<int>(), b.data_ptr<float>(), nullptr,
@@ -129,19 +131,17 @@ at::Tensor spmm_sputnik_atomic(const at::Tensor& b, const at::Tensor& row_indice
   return spmm_f32(b, row_indices, values, row_offsets, column_indices, m, true);
 }
 
-// fp16 storage, fp32 accumulate, int16 or int32 column indices (sputnik_kernels.cpp:179-181)
-at::Tensor spmm_sputnik_reuse_weight_half(const at::Tensor& b, const at::Tensor& row_indices,
-                                          const at::Tensor& values, const at::Tensor& row_offsets,
-                                          const at::Tensor& column_indices, int64_t m) {
-  check_spmm(b, row_indices, values, row_offsets, column_indices, m, false);
+at::Tensor spmm_f16(const at::Tensor& b, const at::Tensor& row_indices, const at::Tensor& values,
+                    const at::Tensor& row_offsets, const at::Tensor& column_indices, int64_t m, bool batched) {
+  check_spmm(b, row_indices, values, row_offsets, column_indices, m, false, batched);
   TORCH_CHECK(b.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf,
               "b and values must be float16");
   const bool i16 = column_indices.scalar_type() == at::kShort;
   TORCH_CHECK(i16 || column_indices.scalar_type() == at::kInt, "column_indices must be int16 or int32");
   c10::cuda::CUDAGuard guard(b.device());
-  const int batch = b.size(0), k = b.size(1), n = b.size(2), nnz = column_indices.size(0);
+  const int batch = batched ? b.size(0) : 1, k = b.size(-2), n = b.size(-1), nnz = column_indices.size(0);
   maybe_validate(row_offsets, column_indices, m, k, &row_indices, false);
-  at::Tensor out = empty(b, {batch, m, n});
+  at::Tensor out = batched ? empty(b, {batch, m, n}) : empty(b, {m, n});
   const int st = i16 ? iex_spmm_f16_i16(m, k, n, nnz, row_indices.data_ptr<int>(), values.data_ptr(),
                                         row_offsets.data_ptr<int>(),
                                         reinterpret_cast<const uint16_t*>(column_indices.data_ptr()),
@@ -153,13 +153,27 @@ at::Tensor spmm_sputnik_reuse_weight_half(const at::Tensor& b, const at::Tensor&
   return out;
 }
 
+// fp16 storage, fp32 accumulate, int16 or int32 column indices (sputnik_kernels.cpp:179-181)
+at::Tensor spmm_sputnik_reuse_weight_half(const at::Tensor& b, const at::Tensor& row_indices,
+                                          const at::Tensor& values, const at::Tensor& row_offsets,
+                                          const at::Tensor& column_indices, int64_t m) {
+  return spmm_f16(b, row_indices, values, row_offsets, column_indices, m, true);
+}
+
+// The same for one [k, n] matrix, without the views (1 us of host time each) that make it a batch of one.
+at::Tensor spmm_matrix(const at::Tensor& b, const at::Tensor& row_indices, const at::Tensor& values,
+                       const at::Tensor& row_offsets, const at::Tensor& column_indices, int64_t m) {
+  return values.scalar_type() == at::kFloat ? spmm_f32(b, row_indices, values, row_offsets, column_indices, m, false, false)
+                                            : spmm_f16(b, row_indices, values, row_offsets, column_indices, m, false);
+}
+
 // fp32 SDDMM, batch items summed into one [nnz] vector (sputnik_kernels.cpp:182-184)
-at::Tensor sddmm_sputnik_atomic_upd_weight(const at::Tensor& a, const at::Tensor& b,
+at::Tensor sddmm_f32(const at::Tensor& a, const at::Tensor& b,
                                            const at::Tensor& row_indices, const at::Tensor& row_offsets,
-                                           const at::Tensor& column_indices) {
-  TORCH_CHECK(a.dim() == b.dim() && a.dim() == 3, "a and b must be [batch, rows, k]");
-  TORCH_CHECK(a.size(0) == b.size(0), "a and b disagree on the batch size");
-  TORCH_CHECK(a.size(2) == b.size(2), "a and b disagree on k");
+                                           const at::Tensor& column_indices, bool batched) {
+  TORCH_CHECK(a.dim() == b.dim() && a.dim() == (batched ? 3 : 2), "a and b must be ", batched ? "[batch, rows, k]" : "[rows, k]");
+  TORCH_CHECK(!batched || a.size(0) == b.size(0), "a and b disagree on the batch size");
+  TORCH_CHECK(a.size(-1) == b.size(-1), "a and b disagree on k");
   TORCH_CHECK(row_indices.dim() == 1 && row_offsets.dim() == 1 && column_indices.dim() == 1,
               "row_indices, row_offsets and column_indices must be 1-D");
   check_common({{"a", &a}, {"b", &b}, {"row_indices", &row_indices}, {"row_offsets", &row_offsets},
@@ -168,7 +182,7 @@ at::Tensor sddmm_sputnik_atomic_upd_weight(const at::Tensor& a, const at::Tensor
   TORCH_CHECK(row_indices.scalar_type() == at::kInt && row_offsets.scalar_type() == at::kInt &&
                   column_indices.scalar_type() == at::kInt,
               "index tensors must be int32");
-  const int batch = a.size(0), m = a.size(1), k = a.size(2), n = b.size(1);
+  const int batch = batched ? a.size(0) : 1, m = a.size(-2), k = a.size(-1), n = b.size(-2);
   TORCH_CHECK(row_indices.size(0) == m && row_offsets.size(0) == m + 1,
               "row_indices must have m entries and row_offsets m + 1");
   const int nnz = column_indices.size(0);
@@ -182,12 +196,18 @@ at::Tensor sddmm_sputnik_atomic_upd_weight(const at::Tensor& a, const at::Tensor
   return out;
 }
 
+at::Tensor sddmm_sputnik_atomic_upd_weight(const at::Tensor& a, const at::Tensor& b,
+                                           const at::Tensor& row_indices, const at::Tensor& row_offsets,
+                                           const at::Tensor& column_indices) {
+  return sddmm_f32(a, b, row_indices, row_offsets, column_indices, true);
+}
+
 // fp16 SDDMM (the instantiation the reference leaves commented out, sputnik_kernels.cpp:185-187):
 // a [batch, m, k] and b [batch, n, k] fp16 -> fp16 [nnz]; int16 or int32 column indices
-at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
-                              const at::Tensor& row_offsets, const at::Tensor& column_indices) {
-  TORCH_CHECK(a.dim() == b.dim() && a.dim() == 3, "a and b must be [batch, rows, k]");
-  TORCH_CHECK(a.size(0) == b.size(0) && a.size(2) == b.size(2), "a and b disagree on batch size or k");
+at::Tensor sddmm_f16(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
+                              const at::Tensor& row_offsets, const at::Tensor& column_indices, bool batched) {
+  TORCH_CHECK(a.dim() == b.dim() && a.dim() == (batched ? 3 : 2), "a and b must be ", batched ? "[batch, rows, k]" : "[rows, k]");
+  TORCH_CHECK((!batched || a.size(0) == b.size(0)) && a.size(-1) == b.size(-1), "a and b disagree on batch size or k");
   check_common({{"a", &a}, {"b", &b}, {"row_indices", &row_indices}, {"row_offsets", &row_offsets},
                 {"column_indices", &column_indices}});
   TORCH_CHECK(a.scalar_type() == at::kHalf && b.scalar_type() == at::kHalf, "a and b must be float16");
@@ -195,7 +215,7 @@ at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at
               "row_indices and row_offsets must be int32");
   const bool i16 = column_indices.scalar_type() == at::kShort;
   TORCH_CHECK(i16 || column_indices.scalar_type() == at::kInt, "column_indices must be int16 or int32");
-  const int batch = a.size(0), m = a.size(1), k = a.size(2), n = b.size(1);
+  const int batch = batched ? a.size(0) : 1, m = a.size(-2), k = a.size(-1), n = b.size(-2);
   TORCH_CHECK(row_indices.size(0) == m && row_offsets.size(0) == m + 1,
               "row_indices must have m entries and row_offsets m + 1");
   const int nnz = column_indices.size(0);
@@ -207,6 +227,17 @@ at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at
                              out.data_ptr(), batch, stream_of(a)),
                "iex_sddmm_f16");
   return out;
+}
+
+at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
+                              const at::Tensor& row_offsets, const at::Tensor& column_indices) {
+  return sddmm_f16(a, b, row_indices, row_offsets, column_indices, true);
+}
+
+at::Tensor sddmm_matrix(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
+                        const at::Tensor& row_offsets, const at::Tensor& column_indices) {
+  return a.scalar_type() == at::kHalf ? sddmm_f16(a, b, row_indices, row_offsets, column_indices, false)
+                                      : sddmm_f32(a, b, row_indices, row_offsets, column_indices, false);
 }
 
 // Dense branch on tensor cores: input @ weight^T (layers_and_funcs/torch.py:17), any number of tokens.

@@ -35,15 +35,10 @@ inline void check_common(std::initializer_list<std::pair<const char*, const at::
 }
 
 // Operator implementations (iex_torch_ext.cpp)
-at::Tensor spmm_sputnik_reuse_weight(const at::Tensor& b, const at::Tensor& row_indices, const at::Tensor& values,
-                                     const at::Tensor& row_offsets, const at::Tensor& column_indices, int64_t m);
-at::Tensor spmm_sputnik_reuse_weight_half(const at::Tensor& b, const at::Tensor& row_indices,
-                                          const at::Tensor& values, const at::Tensor& row_offsets,
-                                          const at::Tensor& column_indices, int64_t m);
-at::Tensor sddmm_sputnik_atomic_upd_weight(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
-                                           const at::Tensor& row_offsets, const at::Tensor& column_indices);
-at::Tensor sddmm_sputnik_half(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
-                              const at::Tensor& row_offsets, const at::Tensor& column_indices);
+at::Tensor spmm_matrix(const at::Tensor& b, const at::Tensor& row_indices, const at::Tensor& values,
+                       const at::Tensor& row_offsets, const at::Tensor& column_indices, int64_t m);
+at::Tensor sddmm_matrix(const at::Tensor& a, const at::Tensor& b, const at::Tensor& row_indices,
+                        const at::Tensor& row_offsets, const at::Tensor& column_indices);
 at::Tensor spmm_tc_half(const at::Tensor& x, const at::Tensor& row_offsets, const at::Tensor& values,
                         const at::Tensor& column_indices, int64_t m);
 at::Tensor linear_fp16(const at::Tensor& input, const at::Tensor& weight);
