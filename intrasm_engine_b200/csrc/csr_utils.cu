@@ -394,12 +394,14 @@ namespace {
 template <typename IT>
 int csr_to_dense(int m, int ld, const int* row_offsets, const IT* cols, const __half* values, __half* out,
                  cudaStream_t s) {
-  // Many rows: one pass through shared memory.  Fewer rows than a wave of blocks: column slices.
+  // Many rows, or short ones: one pass through shared memory.  A few long rows: column slices, since a block that clears
+  // and stores a long row alone takes longer than the second pass (256 x 11008 before a product: 30.6 us in slices, 31.3
+  // us by rows; 128 x 6000: 20.4 and 18.3 us).
   const bool pairs = (reinterpret_cast<uintptr_t>(values) & 3u) == 0 &&
                      (reinterpret_cast<uintptr_t>(cols) & (2 * sizeof(IT) - 1)) == 0;
-  if (m >= 4 * kNumSMs && ld % 8 == 0 && ld <= 24 * 1024 && pairs && aligned16(out)) {
+  if (ld % 8 == 0 && ld <= (m >= 4 * kNumSMs ? 24 * 1024 : 6144) && pairs && aligned16(out)) {
     // a warp per row while the rows of 24 warps fit into an SM's shared memory, else a block per row
-    if (ld <= 4608) {
+    if (ld <= 4608 && m >= 4 * kNumSMs) {
       const int row_bytes = 2 * ld, fit = 48 * 1024 / row_bytes;  // a block's default shared memory
       const int warps = fit < 8 ? fit : 8;
       const int per_sm = 220 * 1024 / (row_bytes * warps) < 8 ? 220 * 1024 / (row_bytes * warps) : 8;

@@ -123,7 +123,7 @@ def test_spmm_few_tokens(n, m, k, density, index):
 
 
 @pytest.mark.parametrize("m,k,density", [(592, 8, 0.5), (700, 1600, 0.5), (700, 4608, 0.1), (600, 4616, 0.9),
-                                         (1500, 33, 0.3), (3, 100, 1.0)])
+                                         (1500, 33, 0.3), (3, 100, 1.0), (1, 8, 1.0), (200, 6144, 0.05), (200, 6152, 0.05)])
 @pytest.mark.parametrize("index", [torch.int16, torch.int32])
 def test_csr_expansion_and_sampling(m, k, density, index):
     a = _ints((m, k), m + k, density=density)
