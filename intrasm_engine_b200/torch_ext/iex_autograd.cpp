@@ -136,8 +136,10 @@ at::Tensor grad_of_values(const at::Tensor& grad, const at::Tensor& b, const at:
   if (p.mode != kCudaCores && b.scalar_type() == at::kHalf && m > 0 && n > 0 && k > 0 && nnz > 0) {
     // every product of the dense matrix, of which the stored positions are kept, against one
     // gathered row of b per stored position
-    const double dense = iex_gemm_f16_estimate_us(m, k, n, 0, 0) + 3.0 + 6.0e-6 * nnz;
-    const double cores = 2.0 + 0.19e-6 * 2.0 * nnz * n;
+    // (bytes, and a chain of L2 latencies for every 256 or, unaligned, 32 columns)
+    const double dense = iex_gemm_f16_estimate_us(m, k, n, 0, 0) + 3.0 + 6.0e-6 * nnz + (n % 8 == 0 ? 0.0 : 4.0);
+    const double chain = n % 8 == 0 ? 4.0 * ((n + 255) / 256) : 3.5 * ((n + 31) / 32);
+    const double cores = 2.0 + 0.19e-6 * 2.0 * nnz * n + chain;
     if (dense < cores) {
       c10::cuda::CUDAGuard guard(grad.device());
       at::Tensor all = empty(grad, {m, round8(k)});
