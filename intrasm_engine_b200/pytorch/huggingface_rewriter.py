@@ -10,6 +10,8 @@ the matching linears -- e.g. ``up_proj`` / ``gate_proj`` of every ``LlamaMLP``.
 """
 from __future__ import annotations
 
+import math
+
 import torch
 from torch import nn
 
@@ -73,12 +75,16 @@ class SparseLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
+        if math.prod(lead) * self.in_features != x.numel():
+            # a narrower x would send column indices past its rows, a wider one be cut off
+            raise RuntimeError(f"SparseLinear expects {self.in_features} input features, got an input of shape "
+                               f"{tuple(x.shape)}")
         if x.is_cuda and x.dtype == torch.float16 and not (torch.is_grad_enabled() and
                                                            (x.requires_grad or self.values.requires_grad)):
             # inference: x is read as it lies and the result written as [tokens, out_features]
-            x2 = x if x.dim() == 2 else x.reshape(-1, self.in_features)
+            x2 = x if x.dim() == 2 and x.size(1) == self.in_features else x.reshape(-1, self.in_features)
             y = ops.native.sparse_linear(x2.contiguous(), self.values, self.row_offsets, self.column_indices,
-                                         self.out_features, self.dense_copy())
+                                         self.out_features, self.in_features, self.dense_copy())
             if self.bias is not None:
                 y = y + self.bias
             return y if x.dim() == 2 else y.reshape(*lead, self.out_features)

@@ -320,19 +320,23 @@ std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Te
   return {out0, out1};
 }
 
-// SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m].
+// SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m], W_csr [m, k].
 //   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu)
 //   with `dense`     the layer's dense copy of W and the dense GEMM
 //   up to 256        block decoder on tensor cores (spmm_tile.cu), unless ...
 //   otherwise        ... expanding W for the dense GEMM is estimated faster (many tokens)
 // All read x as it lies and write [tokens, m]: no transposed copies of either.
 at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
-                         int64_t m, const std::optional<at::Tensor>& dense_weight) {
+                         int64_t m, int64_t k, const std::optional<at::Tensor>& dense_weight) {
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous(), "x must be a contiguous [tokens, in_features] matrix");
+  TORCH_CHECK(x.size(1) == k, "x has ", x.size(1), " columns, the weight ", k);
+  TORCH_CHECK(values.dim() == 1 && ci.dim() == 1 && values.size(0) == ci.size(0),
+              "values and column_indices must be 1-D with nnz entries");
   check_common({{"x", &x}, {"row_offsets", &ro}, {"values", &values}, {"column_indices", &ci}});
   TORCH_CHECK(x.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf, "x and values must be float16");
   TORCH_CHECK(ro.scalar_type() == at::kInt && ro.numel() == m + 1, "row_offsets must be int32 with m + 1 entries");
-  const int64_t tokens = x.size(0), k = x.size(1);
+  TORCH_CHECK(ci.scalar_type() == at::kShort || ci.scalar_type() == at::kInt, "column_indices must be int16 or int32");
+  const int64_t tokens = x.size(0);
   c10::cuda::CUDAGuard guard(x.device());
   maybe_validate(ro, ci, m, k, nullptr, false);
   at::Tensor out = empty(x, {tokens, m});
