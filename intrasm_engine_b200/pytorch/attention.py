@@ -61,11 +61,15 @@ class SparseAttentionChain:
     def forward(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, return_scores: bool = False):
         """``q [heads, m, d]``, ``k [heads, n, d]``, ``v [heads, n, dv]`` fp32 contiguous ->
         ``out [heads, m, dv]`` (and ``scores [heads, nnz]``)."""
-        assert q.dim() == 3 and k.dim() == 3 and v.dim() == 3 and q.dtype == torch.float32
+        assert q.dim() == 3 and k.dim() == 3 and v.dim() == 3
+        assert q.dtype == k.dtype == v.dtype == torch.float32
+        assert q.device == k.device == v.device == self.row_offsets.device
         heads = q.size(0)
-        assert q.shape[1] == self.m and k.shape[1] == self.n and v.shape[1] == self.n and k.size(0) == heads
+        assert q.shape[1] == self.m and k.shape[1] == self.n and v.shape[1] == self.n
+        assert k.size(0) == heads and v.size(0) >= heads  # heads of v past those of q are not read
+        assert k.size(2) == q.size(2)
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        if self.bits is not None and not return_scores and k.dtype == v.dtype == torch.float32:
+        if self.bits is not None and not return_scores:
             out = ops.native.attention(q, k, v, self.bits, self.row_offsets, self.column_indices)
             if out is not None:
                 return out
