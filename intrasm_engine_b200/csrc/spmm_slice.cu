@@ -171,7 +171,8 @@ spmm_slice_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant
           const bool val = i < kVP;
           const int e = base + (val ? i * VN : (i - kVP) * (16 / static_cast<int>(sizeof(IT))));
           const int size = val ? static_cast<int>(sizeof(VT)) : static_cast<int>(sizeof(IT));
-          const int rest = e < gend ? min((q.nnz - e) * size, 16) : 0;  // past the arrays: zeros
+          // past the arrays: zeros (the minimum first: the bytes that are left can be more than an int holds)
+          const int rest = e < gend ? min(q.nnz - e, 16 / size) * size : 0;
           const char* src = val ? reinterpret_cast<const char*>(vals + e) : reinterpret_cast<const char*>(cols + e);
           asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(to + i * 16u),
                        "l"(rest > 0 ? src : reinterpret_cast<const char*>(cols)), "r"(rest)

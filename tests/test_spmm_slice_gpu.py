@@ -2,8 +2,9 @@
 the edges of its slices, windows and shared-memory limits."""
 import numpy as np
 import pytest
+import torch
 
-from intrasm_engine_b200 import _lib, synthetic as syn
+from intrasm_engine_b200 import _lib, ops, synthetic as syn  # noqa: F401  (ops registers torch.ops.iex_ops)
 from . import gpu_util as G
 
 pytestmark = pytest.mark.gpu
@@ -62,3 +63,22 @@ def test_slices_leave_out_other_rows(oracle):
     got = G.spmm_f32(G.DevCSR(a), G.dev(b)[None])[0].cpu().numpy()
     ref = oracle.spmm(a.row_indices, a.values, a.row_offsets, a.column_indices, b, 150)[0]
     np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("dtype,idx,log2_nnz", [(torch.float32, torch.int32, 29), (torch.float16, torch.int16, 30)])
+def test_slices_of_two_gigabytes_of_values(dtype, idx, log2_nnz):
+    """A little more than 2^31 bytes of values: the bytes behind a nonzero do not fit an int.  Every row is
+    full of ones, so that every row of the result is the sum of the dense operand's rows, exactly."""
+    k, n = 1024, 3
+    m = (1 << log2_nnz) // k + 5
+    values = torch.ones(m * k, dtype=dtype, device=G.DEV)
+    cols = torch.arange(k, device=G.DEV, dtype=idx).repeat(m)
+    offsets = torch.arange(m + 1, device=G.DEV, dtype=torch.int32) * k
+    order = torch.arange(m, device=G.DEV, dtype=torch.int32)
+    dense = torch.randint(0, 3, (1, k, n), device=G.DEV).to(dtype)
+    ref = dense[0].float().sum(0)
+    assert float(ref.max()) < 2048
+    op = torch.ops.iex_ops.spmm_sputnik_reuse_weight if dtype == torch.float32 else torch.ops.iex_ops.spmm_sputnik_reuse_weight_half
+    out = op(dense, order, values, offsets, cols, m)
+    assert out.shape == (1, m, n) and torch.equal(out[0].float(), ref.expand(m, n))
+    assert _lib.lib.iex_last_device_status(1) == 0
