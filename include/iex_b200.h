@@ -388,7 +388,8 @@ IEX_API int iex_csr_sample_f16(int m, int k, long long ld, const int32_t* row_of
 IEX_API int iex_gather_values(int count, int elt_bytes, const void* in, const long long* perm, void* out, void* stream);
 /* Copies rows of `cols` fp16 values into rows of `ld` values (a multiple of 8), zero-filled. */
 IEX_API int iex_pad_rows_f16(int rows, int cols, int ld, const void* in, void* out, void* stream);
-/* out = max(in, 0) over `count` fp16 values (a multiple of 8; NaN becomes 0). */
+/* out = max(in, 0) over `count` fp16 values (a multiple of 8; NaN becomes 0).  out is 16-byte aligned, in aligned to
+ * its elements. */
 IEX_API int iex_relu_f16(long long count, const void* in, void* out, void* stream);
 
 /* Dense matrix -> CSR on the device, in two calls, for the conversions the reference

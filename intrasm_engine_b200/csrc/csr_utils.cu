@@ -308,15 +308,23 @@ pad_rows_kernel(int rows, int cols, int ld, const __half* __restrict__ in, __hal
   }
 }
 
-// max(x, 0) on 16-byte pieces (NaN and negative values become 0, as in the ReLU of the converter)
+// max(x, 0) on 16-byte pieces (NaN and negative values become 0, as in the ReLU of the converter).  An input that is only
+// aligned to its elements (a view into a larger buffer) is read value by value.
+template <bool kVec>
 __global__ void __launch_bounds__(256)
-relu_f16_kernel(long long vecs, const uint4* __restrict__ in, uint4* __restrict__ out) {
+relu_f16_kernel(long long vecs, const __half* __restrict__ in, uint4* __restrict__ out) {
   grid_dependency_wait();
   grid_launch_dependents();
   const __half zero = __float2half(0.f);
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < vecs; i += gridDim.x * 256ll) {
-    uint4 v = __ldg(in + i);
+    uint4 v;
     __half* h = reinterpret_cast<__half*>(&v);
+    if constexpr (kVec) {
+      v = __ldg(reinterpret_cast<const uint4*>(in) + i);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) h[e] = __ldg(in + 8 * i + e);
+    }
 #pragma unroll
     for (int e = 0; e < 8; ++e) h[e] = __hgt(h[e], zero) ? h[e] : zero;
     out[i] = v;
@@ -490,10 +498,11 @@ extern "C" int iex_relu_f16(long long count, const void* in, void* out, void* st
   using namespace iex;
   if (count < 0 || count % 8 != 0) return IEX_ERR_BAD_ARG;
   if (count == 0) return IEX_OK;
-  if (!in || !out || !aligned16(in) || !aligned16(out)) return IEX_ERR_BAD_ARG;
+  if (!in || !out || !aligned16(out)) return IEX_ERR_BAD_ARG;
   const long long blocks = (count / 8 + 255) / 256;
-  return launch_overlapped(relu_f16_kernel, dim3(static_cast<unsigned>(blocks < 8 * kNumSMs ? blocks : 8 * kNumSMs)),
-                           dim3(256), 0, static_cast<cudaStream_t>(stream), count / 8, static_cast<const uint4*>(in),
+  return launch_overlapped(aligned16(in) ? relu_f16_kernel<true> : relu_f16_kernel<false>,
+                           dim3(static_cast<unsigned>(blocks < 8 * kNumSMs ? blocks : 8 * kNumSMs)), dim3(256), 0,
+                           static_cast<cudaStream_t>(stream), count / 8, static_cast<const __half*>(in),
                            static_cast<uint4*>(out));
 }
 

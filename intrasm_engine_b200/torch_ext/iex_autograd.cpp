@@ -348,15 +348,17 @@ at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at
   // decoder is as fast
   const double skinny_us = tokens == 1 ? 2.5 + 1.05e-6 * nnz : 3.5 + 6e-6 * m / 11 + 1.15e-6 * nnz;
   if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) && (!dense_weight.has_value() || skinny_us <= gemm_us)) {
-    check_status(iex_spmm_f16_skinny(m, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
-                                     values.data_ptr(), x.data_ptr(), 1, k, out.data_ptr(), 1, m, stream_of(x)),
-                 "iex_spmm_f16_skinny");
-    return out;
+    const int st = iex_spmm_f16_skinny(m, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
+                                       values.data_ptr(), x.data_ptr(), 1, k, out.data_ptr(), 1, m, stream_of(x));
+    if (st == 0) return out;
+    // pairs of nonzeros are loaded together; a matrix that is not aligned for that takes the ways below
+    TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_f16_skinny failed with status ", st, ": ", iex_error_string(st));
   }
   if (dense_weight.has_value()) {
     const at::Tensor& w = *dense_weight;
     TORCH_CHECK(w.size(0) == m && w.size(1) == k && w.scalar_type() == at::kHalf && w.is_contiguous(), "dense copy of another shape");
-    check_status(iex_linear_f16_any(tokens, k, m, x.data_ptr(), w.data_ptr(), out.data_ptr(), stream_of(x)),
+    const at::Tensor xp = tma_rows(x);
+    check_status(iex_linear_f16_any(tokens, k, m, xp.data_ptr(), w.data_ptr(), out.data_ptr(), stream_of(x)),
                  "iex_linear_f16_any");
     return out;
   }
