@@ -66,9 +66,17 @@ class SparseLinear(nn.Module):
         return cls(magnitude_prune(linear.weight.detach(), sparsity), linear.bias)
 
     def dense_copy(self):
-        """The dense weight for inference, or None below ``DENSE_COPY_DENSITY``; follows in-place
-        changes of ``values``."""
+        """The dense weight for inference, or None (``DenseCopy``); follows changes of the CSR tensors, except
+        writes through ``.data``, after which ``reset_dense_copy`` has to be called."""
         return self._dense.current(self.values, self.row_offsets, self.column_indices)
+
+    def reset_dense_copy(self):
+        self._dense.reset()
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        if "_dense" not in self.__dict__:  # saved before the layer kept a copy
+            self._dense = DenseCopy(self.out_features, self.in_features)
 
     def density(self) -> float:
         return self.values.numel() / float(self.out_features * self.in_features)

@@ -307,13 +307,14 @@ at::Tensor expand_weight(const at::Tensor& values, const at::Tensor& ro, const a
 }
 
 // The two branches of a sparse || dense layer with both weights dense: x [k, n] ->
-// (weight0 @ x [m0, n], (weight1 @ x)^T [n, m1]) in one launch.
+// (weight0 @ x [m0, n], (weight1 @ x)^T [n, m1]) in one launch.  weight0 is the layer's dense copy.
 std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Tensor& weight0, const at::Tensor& weight1) {
   check_common({{"x", &x}, {"weight0", &weight0}, {"weight1", &weight1}});
   const int64_t k = x.size(0), n = x.size(1), m0 = weight0.size(0), m1 = weight1.size(0);
   TORCH_CHECK(weight0.size(1) == k && weight1.size(1) == k, "weights must be [rows, k]");
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor out0 = empty(x, {m0, n}), out1 = empty(x, {n, m1});
+  mark_stream(weight0);
   check_status(iex_linear_pair_f16(m0, m1, k, n, weight0.data_ptr(), weight1.data_ptr(), x.data_ptr(), 0, out0.data_ptr(), 0,
                                    out1.data_ptr(), 1, stream_of(x)),
                "iex_linear_pair_f16");
@@ -357,6 +358,7 @@ at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at
   if (dense_weight.has_value()) {
     const at::Tensor& w = *dense_weight;
     TORCH_CHECK(w.size(0) == m && w.size(1) == k && w.scalar_type() == at::kHalf && w.is_contiguous(), "dense copy of another shape");
+    mark_stream(w);
     const at::Tensor xp = tma_rows(x);
     check_status(iex_linear_f16_any(tokens, k, m, xp.data_ptr(), w.data_ptr(), out.data_ptr(), stream_of(x)),
                  "iex_linear_f16_any");
@@ -453,6 +455,7 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
   mod.def("mylinear", &iex_torch::mylinear);
   mod.def("sparse_linear", &iex_torch::sparse_linear);
   mod.def("expand_weight", &iex_torch::expand_weight);
+  mod.def("stream_capturing", [](const at::Tensor& t) { return iex_stream_is_capturing(iex_torch::stream_of(t)) != 0; });
   mod.def("linear_pair", &iex_torch::linear_pair);
   mod.def("attention_plan", &iex_torch::attention_plan);
   mod.def("attention", &iex_torch::attention);

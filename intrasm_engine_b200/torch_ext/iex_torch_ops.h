@@ -3,6 +3,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/ops/empty.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include <tuple>
@@ -32,6 +33,12 @@ inline void check_common(std::initializer_list<std::pair<const char*, const at::
     if (first == nullptr) first = t;
     TORCH_CHECK(t->device() == first->device(), name, " should be in the same device as the first argument");
   }
+}
+
+// `t` is read on the current stream although its owner may let go of it at any time (nothing to do on the stream it was
+// allocated on).
+inline void mark_stream(const at::Tensor& t) {
+  c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), at::cuda::getCurrentCUDAStream(t.get_device()));
 }
 
 // Operator implementations (iex_torch_ext.cpp)
