@@ -179,6 +179,10 @@ IEX_API int iex_spmm_f32_prefers_tc(int m, int k, int n, int nnz);
  * on the pattern only; its first word is nonzero if the pattern stores a position twice, and the plan must
  * then not be used.  The workspace holds the operands' TF32 planes. */
 IEX_API int iex_attention_f32_supported(int heads, int m, int n, int d, int dv);
+/* Whether this call is expected to beat SDDMM and SpMM head by head: its time follows m * n, theirs the nnz
+ * stored positions, so it is not the way for large, very sparse masks (whose plan of m * n / 8 bytes need not
+ * be built then either). */
+IEX_API int iex_attention_f32_prefers(int heads, int m, int n, int d, int dv, int nnz);
 IEX_API size_t iex_attention_plan_bytes(int m, int n);
 IEX_API int iex_attention_plan_build(int m, int n, const int32_t* row_offsets, const int32_t* column_indices,
                                      void* plan, size_t bytes, void* stream);

@@ -542,6 +542,36 @@ bool attention_shape(int heads, int m, int n, int d, int dv, Shape* s) {
   return tiles < (1ll << 30) && 2ll * heads * n < (1ll << 30) && 2ll * heads * s->dvt < (1ll << 30) && heads <= 65000;
 }
 
+// One CTA per SM with an equal share of the tiles; with fewer bands than SMs, as many equal pieces of every band as
+// fit on the chip, for a CTA that works on two bands pays for a second start (5 us), and no more than this
+// root, since whoever comes last adds the pieces up alone.
+int cta_count(int items, int tiles, int sms) {
+  const int pieces = std::max(1, static_cast<int>(std::sqrt(1.5 * tiles)));
+  return items >= sms ? sms : items * std::min(pieces, sms / items);
+}
+
+// Times in microseconds, fitted on B200 to 578 measurements: 1 to 32 heads, 256 to 16384 rows and keys, 32 to 128 columns,
+// masks of 0.05 to 23 % stored positions, scattered or in a band.
+//
+// This kernel multiplies every tile, empty or not: m * n counts, not the positions.
+double one_launch_us(int heads, int m, int n, const Shape& s, int sms) {
+  const int bands = (m + 127) / 128, tiles = (n + s.kt - 1) / s.kt, items = heads * s.parts * bands;
+  const int ctas = cta_count(items, tiles, sms);
+  const double tile = (0.40 + 0.0032 * (s.da * s.kt + s.kt * s.dvp / 32)) * (s.kt == 32 ? 1.12 : 1.0);
+  const double planes = static_cast<double>(heads) * n * (s.dp + s.dvt) * 12 / 6e6;
+  return 13.0 + planes + (static_cast<long long>(items) * tiles + ctas - 1) / ctas * tile;
+}
+
+// SDDMM and SpMM head by head over two streams (pytorch/attention.py): 20 us of host time a head for the two launches, or
+// what their gathers take, which follows the positions (a row of q.k and of v for each), and the dense tiles of the SDDMM
+// where that is the tensor-core one.
+double head_by_head_us(int heads, int m, int n, int d, int dv, int nnz) {
+  auto row = [](int cols) { return cols <= 32 ? 32 : cols <= 64 ? 64 : 128; };
+  double head = (0.6e-5 + 0.235e-6 * (row(d) + row(dv))) * nnz;
+  if (iex_sddmm_f32_prefers_tc(m, d, n, nnz, 1)) head += 0.4e-6 * m * n;
+  return std::max(28.0 + 19.5 * heads, 10.0 + heads * head);
+}
+
 size_t round256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 int flag_blocks_of(int np) { return (np + kPrepKeys - 1) / kPrepKeys; }
 
@@ -581,6 +611,17 @@ using namespace iex::tc;
 extern "C" int iex_attention_f32_supported(int heads, int m, int n, int d, int dv) {
   Shape s;
   return attention_shape(heads, m, n, d, dv, &s) ? 1 : 0;
+}
+
+// One launch unless the operators are estimated a sixth shorter.  Where the line lies, measured (us, one launch / head by
+// head): 4096 x 4096, 12 heads, d 80: 367 / 257 at 1 %, 367 / 307 at 2 %, 371 / 712 at 5 %; d 64: 211 / 265 from 0.05 to 2 %
+// (the launches), 211 / 375 at 5 %; d 128: 741 / 256 at 1 %, 755 / 755 at 5 %, 761 / 1554 at 10 %.  16384 x 16384 with a band
+// of 256, 8 heads, d 64: 2260 / 1425; with one of 1024: 2236 / 5026.  Of the 578 measurements the choice is the slower one by
+// more than 10 % in three (14 % at most).
+extern "C" int iex_attention_f32_prefers(int heads, int m, int n, int d, int dv, int nnz) {
+  Shape s;
+  if (!attention_shape(heads, m, n, d, dv, &s)) return 0;
+  return one_launch_us(heads, m, n, s, std::min(sm_count(), kNumSMs)) <= 1.2 * head_by_head_us(heads, m, n, d, dv, nnz);
 }
 
 // Plan: one word (nonzero if a position is stored twice), then, 256 bytes on, the mask's bits.
@@ -644,12 +685,7 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   p.flags = flags;
   p.flag_blocks = flag_blocks_of(s.np);
   p.status = status_word();
-  // One CTA per SM with an equal share of the tiles; with fewer bands than SMs, as many equal pieces of every band as
-  // fit on the chip, for a CTA that works on two bands pays for a second start (5 us), and no more than this
-  // root, since whoever comes last adds the pieces up alone.
-  const int items = heads * s.parts * p.bands, sms = std::min(sm_count(), kNumSMs);
-  const int pieces = std::max(1, static_cast<int>(std::sqrt(1.5 * p.tiles)));
-  const int ctas = items >= sms ? sms : items * std::min(pieces, sms / items);
+  const int sms = std::min(sm_count(), kNumSMs), ctas = cta_count(heads * s.parts * p.bands, p.tiles, sms);
   CUtensorMap mk, mv;
   int st = make_map_f32(&mk, k_planes, 2ll * heads * n, s.dp, s.kt);
   if (st == IEX_OK) st = make_map_f32(&mv, v_planes, 2ll * heads * s.dvt, s.np, s.dvp);

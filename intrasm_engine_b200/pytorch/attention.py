@@ -11,7 +11,8 @@ no softmax in it, as there is none in the reference's operators.
 What the class adds to calling the two operators in a loop:
   * the mask's pattern-only data (row order, mask bits, tile plan of the tensor-core SDDMM) is built once;
   * where the scores are not asked for and d, dv <= 128, all heads run as one launch that keeps the
-    scores on chip (csrc/attention_tc.cu); otherwise
+    scores on chip (csrc/attention_tc.cu), unless the mask is so sparse, or the matrix so large, that the
+    operators are estimated faster (``iex_attention_f32_prefers``); otherwise
   * heads alternate over two CUDA streams.  The tensor-core SDDMM keeps the tensor pipe and
     shared memory busy, the CUDA-core SpMM the load / store path and L2; run side by side for
     different heads they finish 24 heads of the 4096 x 4096 @95 % case in 31 us per head
@@ -36,9 +37,11 @@ class SparseAttentionChain:
         self.row_indices = swizzle_rows(self.row_offsets)
         self.nnz = int(column_indices.numel())
         self.plan = None  # tile plan of the tensor-core SDDMM, built on first use for a given k
-        # the mask's bits for the one-launch kernel, which takes every position once
+        # the mask's bits (m * n / 8 bytes) for the one-launch kernel, if any width and number of heads would
+        # prefer it; it takes every position once, which is read back here (not while a stream is recorded)
         self.bits = None
-        if self.nnz > 0:
+        if (self.nnz > 0 and any(_lib.lib.iex_attention_f32_prefers(h, self.m, self.n, 4, 4, self.nnz) for h in (1, 64))
+                and not ops.native.stream_capturing(self.row_offsets)):
             bits = ops.native.attention_plan(self.row_offsets, self.column_indices, self.m, self.n)
             if int(bits[:4].view(torch.int32).item()) == 0:
                 self.bits = bits

@@ -392,7 +392,8 @@ at::Tensor attention_plan(const at::Tensor& ro, const at::Tensor& ci, int64_t m,
   return plan;
 }
 
-// q [heads, m, d], k [heads, n, d], v [heads, n, dv] -> [heads, m, dv]; nothing for shapes the kernel does not take
+// q [heads, m, d], k [heads, n, d], v [heads, n, dv] -> [heads, m, dv]; nothing for shapes the kernel does not take or is
+// not the faster way for
 std::optional<at::Tensor> attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& plan,
                                     const at::Tensor& ro, const at::Tensor& ci) {
   check_common({{"q", &q}, {"k", &k}, {"v", &v}, {"plan", &plan}, {"row_offsets", &ro}, {"column_indices", &ci}});
@@ -402,7 +403,7 @@ std::optional<at::Tensor> attention(const at::Tensor& q, const at::Tensor& k, co
   TORCH_CHECK(k.size(0) == q.size(0) && v.size(0) >= q.size(0), "k and v have fewer heads than q");
   TORCH_CHECK(k.size(2) == q.size(2) && v.size(1) == k.size(1), "q and k disagree on d, or k and v on n");
   const int64_t heads = q.size(0), m = q.size(1), d = q.size(2), n = k.size(1), dv = v.size(2);
-  if (!iex_attention_f32_supported(heads, m, n, d, dv) || !aligned16(q) || !aligned16(k) || !aligned16(v)) return std::nullopt;
+  if (!iex_attention_f32_prefers(heads, m, n, d, dv, ci.numel()) || !aligned16(q) || !aligned16(k) || !aligned16(v)) return std::nullopt;
   TORCH_CHECK(ro.scalar_type() == at::kInt && ci.scalar_type() == at::kInt, "row_offsets and column_indices must be int32");
   TORCH_CHECK(ro.numel() == m + 1 && static_cast<size_t>(plan.nbytes()) >= iex_attention_plan_bytes(m, n), "plan of another mask");
   c10::cuda::CUDAGuard guard(q.device());

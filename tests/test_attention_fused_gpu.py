@@ -68,3 +68,48 @@ def test_repeated_position_takes_the_operators():
     q, k, v = _qkv(1, 1, 4, 32, 32, 1)
     ref = 2 * (q[0] @ k[0, 1]) * v[0, 1]
     assert torch.allclose(chain(q, k, v)[0, 0], ref, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("heads,m,d,width", [(2, 16384, 64, 32), (3, 4096, 128, 64), (1, 8192, 80, 16)])
+def test_sparse_bands_take_the_operators(heads, m, d, width):
+    """Large masks with few positions: no launch over every tile and, where no width of q and v would want one,
+    no bits of the whole matrix."""
+    rows = torch.arange(m, device=DEV)[:, None]
+    cols = rows + torch.arange(-width // 2, width // 2, device=DEV)[None, :]
+    inside = (cols >= 0) & (cols < m)
+    ro = torch.zeros(m + 1, dtype=torch.int32, device=DEV)
+    ro[1:] = torch.cumsum(inside.sum(1), 0)
+    ci = cols[inside].to(torch.int32)
+    nnz = ci.numel()
+    before = torch.cuda.memory_allocated()
+    chain = SparseAttentionChain(ro, ci, m, m)
+    assert not _lib.lib.iex_attention_f32_prefers(heads, m, m, d, d, nnz)
+    if m == 16384:
+        assert chain.bits is None and torch.cuda.memory_allocated() - before < m * m // 16
+    q, k, v = _qkv(heads, m, m, d, d, m)
+    out = chain(q, k, v)
+    index = cols.clamp(0, m - 1)
+    for h in range(heads):
+        s = torch.einsum("rd,rwd->rw", q[h].double(), k[h].double()[index]) * inside
+        ref = torch.einsum("rw,rwd->rd", s, v[h].double()[index])
+        assert float((out[h].double() - ref).norm() / ref.norm()) < 1e-6
+    scored, scores = chain(q, k, v, return_scores=True)
+    assert torch.equal(out, scored) and scores.shape == (heads, nnz)
+
+
+def test_chain_made_while_a_stream_is_recorded():
+    """Making a chain reads nothing back then; it works without the bits."""
+    mask, ro, ci = _mask(200, 300, 0.1, 5)
+    q, k, v = _qkv(2, 200, 300, 64, 64, 1)
+    ref = SparseAttentionChain(ro, ci, 200, 300)(q, k, v)
+    SparseAttentionChain(ro, ci, 200, 300)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain = SparseAttentionChain(ro, ci, 200, 300)
+        out = chain(q, k, v)
+    assert chain.bits is None
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.allclose(out, ref, rtol=1e-5, atol=1e-3)
+    del graph
