@@ -255,7 +255,7 @@ IEX_API int iex_linear_pair_f16(int m0, int m1, int k, int n, const void* weight
                                 const void* x, int x_tokens_major, void* out0, int tokens_major0, void* out1,
                                 int tokens_major1, void* stream);
 
-/* CSR SpMM with 1 to 16 dense columns (decoding steps), fp16, fp32 accumulation, CUDA cores:
+/* CSR SpMM with 1 to 16 dense columns (decoding steps; one launch up to 8, else two), fp16, fp32 accumulation, CUDA cores:
  * out(r, t) = sum_p values[p] * x(col[p], t).  The strides are in elements, so x and out may be
  * [k, n] / [m, n] or [n, k] / [n, m].  values 4-byte, column_indices 2 * sizeof(index) aligned. */
 IEX_API int iex_spmm_f16_skinny_supported(int k, int n);

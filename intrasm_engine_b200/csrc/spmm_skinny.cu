@@ -1,5 +1,5 @@
-// fp16 CSR SpMM with a handful of dense columns (1 to 16: decoding steps of a pruned projection) on
-// CUDA cores: out[r, t] = sum_p values[p] * x[col[p], t], fp32 accumulation.
+// fp16 CSR SpMM with a handful of dense columns (decoding steps of a pruned projection) on CUDA cores:
+// out[r, t] = sum_p values[p] * x[col[p], t], fp32 accumulation.
 //
 // With so few columns the product is bound by reading the CSR arrays once (11008 x 4096 at 50 %
 // with 16-bit indices: 90 MB, 14 us at the measured copy bandwidth).  The general CUDA-core kernel
@@ -8,6 +8,11 @@
 // nonzeros per step (one 4-byte load of values, one of indices, kU steps requested together), and
 // the dense operand, interleaved by column, is gathered from shared memory: because columns
 // ascend, neighbouring lanes gather from neighbouring words.  A butterfly adds the lanes' sums.
+//
+// Reached from MySpMM for 1 to 8 columns (x [k, n]; where the line lies stands at spmm_half in torch_ext/iex_autograd.cpp)
+// and from SparseLinear for 1 and 2 tokens (x [n, k]; interleaving more of those on the way in costs as much as the product: 4096
+// x 4096 at 10 %, 3 tokens: 33 us, the block decoder 27).  A kernel for 16 columns was no faster than the
+// wide kernels (6 to 101 us against 5 to 55); 9 to 16 columns are two launches.
 #include "common.cuh"
 
 namespace iex {
@@ -19,13 +24,12 @@ constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 
 // The N columns of one row of x as they lie in shared memory: fp32 for N <= 4 (no conversion per
-// nonzero), fp16 for 8 and 16 (half the shared-memory traffic, which is what bounds these).
+// nonzero), fp16 for 8 (half the shared-memory traffic, which is what bounds it).
 template <int N> struct Slot;
 template <> struct Slot<1> { using T = float; };
 template <> struct Slot<2> { using T = float; };
 template <> struct Slot<4> { using T = float; };
 template <> struct Slot<8> { using T = __half; };
-template <> struct Slot<16> { using T = __half; };
 
 template <int N>
 __device__ __forceinline__ void accumulate(float (&acc)[N], float v, const typename Slot<N>::T* row) {
@@ -42,16 +46,13 @@ __device__ __forceinline__ void accumulate(float (&acc)[N], float v, const typen
     acc[2] = fmaf(v, x.z, acc[2]);
     acc[3] = fmaf(v, x.w, acc[3]);
   } else {
+    const uint4 x = *reinterpret_cast<const uint4*>(row);
+    const __half2* h = reinterpret_cast<const __half2*>(&x);
 #pragma unroll
-    for (int q = 0; q < N / 8; ++q) {
-      const uint4 x = *(reinterpret_cast<const uint4*>(row) + q);
-      const __half2* h = reinterpret_cast<const __half2*>(&x);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = __half22float2(h[i]);
-        acc[8 * q + 2 * i] = fmaf(v, f.x, acc[8 * q + 2 * i]);
-        acc[8 * q + 2 * i + 1] = fmaf(v, f.y, acc[8 * q + 2 * i + 1]);
-      }
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __half22float2(h[i]);
+      acc[2 * i] = fmaf(v, f.x, acc[2 * i]);
+      acc[2 * i + 1] = fmaf(v, f.y, acc[2 * i + 1]);
     }
   }
 }
@@ -193,10 +194,11 @@ int dispatch(int m, int k, int n, const int* ro, const IT* cols, const __half* v
   if (n == 2) return launch<IT, 2>(m, k, n, ro, cols, values, x, xr, xc, out, orow, ocol, s);
   if (n <= 4) return launch<IT, 4>(m, k, n, ro, cols, values, x, xr, xc, out, orow, ocol, s);
   if (n <= 8) return launch<IT, 8>(m, k, n, ro, cols, values, x, xr, xc, out, orow, ocol, s);
-  return launch<IT, 16>(m, k, n, ro, cols, values, x, xr, xc, out, orow, ocol, s);
+  const int st = launch<IT, 8>(m, k, 8, ro, cols, values, x, xr, xc, out, orow, ocol, s);
+  return st != 0 ? st : dispatch<IT>(m, k, n - 8, ro, cols, values, x + 8 * xc, xr, xc, out + 8 * ocol, orow, ocol, s);
 }
 
-int slot_bytes(int n) { return n == 1 ? 4 : n == 2 ? 8 : n <= 8 ? 16 : 32; }
+int slot_bytes(int n) { return n == 1 ? 4 : n == 2 ? 8 : 16; }
 
 }  // namespace
 }  // namespace iex

@@ -160,3 +160,27 @@ def test_gather_values(count, dtype):
     out = torch.full((count + 1,), 9.0, dtype=dtype, device=DEV)
     _lib.call("iex_gather_values", count, v.element_size(), v.data_ptr(), perm.data_ptr(), out.data_ptr(), _stream())
     assert torch.equal(out[:-1], v[perm]) and float(out[-1]) == 9.0
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("m,k,density", [(300, 1000, 0.3), (300, 1000, 0.09), (67, 2050, 0.45), (40, 14001, 0.03), (30, 60000, 0.05),
+                                         (900, 192, 0.5), (64, 640, 0.6)])
+@pytest.mark.parametrize("index", [torch.int16, torch.int32])
+def test_few_columns_take_the_same_sum(n, m, k, density, index):
+    """use_tensor_cores="auto" on both sides of the rule for few columns (row length, share stored, shared
+    memory), with uneven rows, an empty one and arrays off the alignment of pair loads, against the sums of the
+    CUDA cores: one fp16 rounding of fp32 sums in another order."""
+    if index == torch.int16 and k > 32767:
+        index = torch.int32
+    rng = np.random.default_rng(m + k + n)
+    a = (rng.standard_normal((m, k)) * 0.1).astype(np.float16) * (rng.random((m, k)) < density)
+    a[1], a[2, : k // 2] = 0, 1
+    values, ri, ro, ci = dense_to_sparse_cuda(_dev(a), index_dtype=index)
+    b = torch.randn(k, n, device=DEV).half()
+    terms = torch.as_tensor(np.abs(a.astype(np.float64))).to(DEV) @ b.double().abs()
+    ref = torch.ops.iex_ops.spmm_sputnik_reuse_weight_half(b[None], ri, values, ro, ci, m)[0].double()
+    shifted = torch.empty(values.numel() + 1, dtype=values.dtype, device=DEV)[1:]
+    shifted.copy_(values)
+    for v in (values, shifted):
+        out = ops.native.myspmm(b, ri, v, ro, ci, m, [], 2)
+        assert bool(((out.double() - ref).abs() <= 2.0 ** -10 * ref.abs() + 2e-5 * terms + 2.0 ** -24).all())
