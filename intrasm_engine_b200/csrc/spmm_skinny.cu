@@ -9,7 +9,7 @@
 // the dense operand, interleaved by column, is gathered from shared memory: because columns
 // ascend, neighbouring lanes gather from neighbouring words.  A butterfly adds the lanes' sums.
 //
-// Reached from MySpMM for 1 to 8 columns (x [k, n]; where the line lies stands at spmm_half in torch_ext/iex_autograd.cpp)
+// Reached from MySpMM for 1 to 8 columns (x [k, n]; where the line lies stands at spmm_half_way in torch_ext/iex_autograd.cpp)
 // and from SparseLinear for 1 and 2 tokens (x [n, k]; interleaving more of those on the way in costs as much as the product: 4096
 // x 4096 at 10 %, 3 tokens: 33 us, the block decoder 27).  A kernel for 16 columns was no faster than the
 // wide kernels (6 to 101 us against 5 to 55); 9 to 16 columns are two launches.

@@ -6,9 +6,10 @@ dense ``[k, n]`` operand, and the same derivative scheme (:77-149):
     d values = SDDMM(grad, b) sampled at A's pattern,   d b = A^T @ grad.
 fp32 runs the CUDA-core kernels (bit-reproducible); fp16 runs the CUDA-core fp16 kernel or,
 with ``use_tensor_cores=True`` in the forward kwargs, the tcgen05 kernel;
-``use_tensor_cores="auto"`` lets a cost model choose.  ``run`` is native unless a graph
-constructor is recording: there ``use_tensor_cores`` also covers the backward pass and any n,
-because the matrix may be expanded and multiplied as a dense one (torch_ext/iex_autograd.cpp).
+``use_tensor_cores="auto"`` lets estimates choose.  ``run`` is native unless a graph
+constructor is recording: the native calls' ``use_tensor_cores`` also covers the backward pass and any
+n, because the matrix may be expanded and multiplied as a dense one (torch_ext/iex_autograd.cpp); a
+recorded call has the two kernels that need no scratch, chosen by the same estimates.
 """
 from __future__ import annotations
 
@@ -26,7 +27,7 @@ def _spmm(b2d, row_indices, values, row_offsets, column_indices, m, use_tc=False
     if values.dtype == torch.float32:
         return torch.ops.iex_ops.spmm_sputnik_reuse_weight(b2d.unsqueeze(0), row_indices, values,
                                                            row_offsets, column_indices, m)[0]
-    if use_tc == "auto":  # cost model fitted to measurements (pytorch/tuning.py)
+    if use_tc == "auto":  # the estimates of the eager path, between the two kernels that need no scratch (pytorch/tuning.py)
         use_tc = choose_spmm_kernel(m, b2d.size(0), b2d.size(1), values.numel(), 16,
                                     16 if column_indices.dtype == torch.int16 else 32) == "tensor_core"
     if use_tc:

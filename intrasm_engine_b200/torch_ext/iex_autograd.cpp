@@ -7,7 +7,7 @@
 // graph constructor is recording, `run` comes here instead: the same kernels in the same order,
 // with the autograd node, its saved tensors and its backward pass in C++.
 //
-// It also holds the choice between the ways to multiply an fp16 CSR matrix (spmm_half_auto).
+// It also holds the choice between the ways to multiply an fp16 CSR matrix (spmm_half_way).
 #include "iex_torch_ops.h"
 
 #include <torch/csrc/autograd/edge.h>
@@ -61,19 +61,49 @@ void gemm(int64_t m, int64_t n, int64_t k, const at::Tensor& a, bool a_mn, const
 
 // Estimates in microseconds, fitted to measurements on B200.
 //   expand   one pass over the CSR arrays and the dense copy, at 5.5 TB/s
-//   decode   the block decoder of spmm_tile.cu: per row, its stored positions and its blocks of columns
+//   decode   the block decoder of spmm_tile.cu: a chain of blocks of 512 columns, and per row of a unit its stored
+//            positions and its part of a block.  Within -16 and +23 % of 504 measurements (256 to 11008 rows, 512 to 4096
+//            columns, 2 to 70 % stored, 64 to 256 tokens), where the choice of spmm_half_way takes 4 % longer than the fastest way on
+//            (geometric) average, 1.7 x at worst: short rows of large matrices, whose time on CUDA cores is underestimated
 double expand_us(int64_t m, int64_t k, int64_t nnz, int bits) {
   return 2.5 + (2.0 * m * round8(k) + static_cast<double>(nnz) * (2 + bits / 8)) / 5.5e6;
 }
 double block_decode_us(int64_t m, int64_t k, int64_t n, int64_t nnz) {
-  const int64_t rows = round8((m + 147) / 148);
-  const double t = 8.0 + rows * (0.13e-3 * nnz / std::max<int64_t>(m, 1) + 0.0166 * ((k + 511) / 512));
-  return t * (n <= 128 ? 1.0 : 1.25) * std::max<int64_t>(1, (rows + 127) / 128);
+  const int64_t step = n <= 64 ? 8 : 16, rows = ((m + 147) / 148 + step - 1) / step * step;  // of an SM's unit
+  const double blocks = static_cast<double>((k + 511) / 512), waves = static_cast<double>(std::max<int64_t>(1, (rows + 127) / 128));
+  const bool wide = n > 128;
+  return (wide ? 6.2 : 4.85) + waves * blocks * (wide ? 1.75 : 1.6) +
+         rows * (0.155e-3 * nnz / std::max<int64_t>(m, 1) + (wide ? 0.02 : 0.006) * blocks);
 }
-bool decode_supported(const at::Tensor& b, const at::Tensor& values, const at::Tensor& ci) {
-  const int64_t k = b.size(0), n = b.size(1);
-  return n % 64 == 0 && n > 0 && n <= 256 && k % 8 == 0 && k > 0 && (index_bits(ci) == 32 || k <= 65280) &&
-         aligned16(b) && aligned16(values) && aligned16(ci);
+bool decode_supported(int64_t k, int64_t n, int bits) {
+  return n % 64 == 0 && n > 0 && n <= 256 && k % 8 == 0 && k > 0 && (bits == 32 || k <= 65280);
+}
+
+enum Mode { kCudaCores = 0, kTensorCores = 1, kAuto = 2 };
+enum Way { kRows = 0, kDecode = 1, kExpand = 2, kFewColumns = 3 };
+
+// How an fp16 CSR product [m, k] x [k, n] runs.  On tensor cores the matrix is either decoded tile by tile inside the
+// product (tc_fused.cu) or expanded once and multiplied as a dense matrix: the decoder needs no scratch and no second pass,
+// the expansion costs the dense copy's traffic but then runs at the dense kernel's rate, for any n.
+//   aligned   operands start on 16-byte boundaries
+//   eager     scratch may be used; not in a graph constructor's recording, where it would be handed out again before the
+//             graph runs, and which knows the registered operators only: there the choice is between kRows and kDecode
+Way spmm_half_way(int64_t m, int64_t k, int64_t n, int64_t nnz, int bits, int mode, bool aligned, bool eager) {
+  if (mode == kCudaCores || m == 0 || k == 0 || n == 0) return kRows;
+  // Up to 8 columns one lane per nonzero (spmm_skinny.cu) instead of one per column: 4096 x 4096 at 10 %, 4 columns 12 us
+  // against 21, at 30 % 23 against 27.  Not for rows of less than 96 nonzeros, or 2 % of the columns, which do not pay for
+  // a row's start or for x in every block's shared memory (32768 x 256 at 30 %: 17 us against 13; 2048 x 14000 at 0.5 %: 11
+  // against 8), and not above one half stored (2048 x 14000 at 90 %: 58 against 52).
+  if (mode == kAuto && eager && n <= 8 && nnz >= 96 * m && 50 * nnz >= m * k && 2 * nnz <= m * k &&
+      iex_spmm_f16_skinny_supported(k, n))
+    return kFewColumns;
+  const double expand = eager ? expand_us(m, k, nnz, bits) + iex_gemm_f16_estimate_us(m, n, k, 1, 0) + (n % 8 == 0 ? 0.0 : 2.0)
+                              : 1e30;
+  const double decode = decode_supported(k, n, bits) && aligned ? block_decode_us(m, k, n, nnz) : 1e30;
+  // Tensor cores where the estimates are close: they are good to 10 %, and the walk along the longest row, which only
+  // the CUDA cores pay for, is estimated from the average one.
+  if (mode == kAuto && 1.15 * iex_spmm_f16_estimate_us(m, k, n, nnz, bits) <= std::min(expand, decode)) return kRows;
+  return decode <= expand ? kDecode : kExpand;
 }
 
 void check_csr_half(const at::Tensor& b, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
@@ -88,41 +118,25 @@ void check_csr_half(const at::Tensor& b, const at::Tensor& values, const at::Ten
   TORCH_CHECK(ci.scalar_type() == at::kShort || ci.scalar_type() == at::kInt, "column_indices must be int16 or int32");
 }
 
-enum Mode { kCudaCores = 0, kTensorCores = 1, kAuto = 2 };
-
-// A_csr [m, k] @ b [k, n], fp16.  On tensor cores the matrix is either decoded tile by tile inside the
-// product (tc_fused.cu) or expanded once and multiplied as a dense matrix: the decoder needs no
-// scratch and no second pass, the expansion costs the dense copy's traffic but then runs at the
-// dense kernel's rate, for any n.
+// A_csr [m, k] @ b [k, n], fp16
 at::Tensor spmm_half(const at::Tensor& b, const at::Tensor& ri, const at::Tensor& values, const at::Tensor& ro,
                      const at::Tensor& ci, int64_t m, int mode) {
   const int64_t k = b.size(0), n = b.size(1), nnz = values.numel();
-  auto cores = [&] { return spmm_matrix(b, ri, values, ro, ci, m); };
-  if (mode == kCudaCores || m == 0 || k == 0 || n == 0) return cores();
+  const bool aligned = aligned16(b) && aligned16(values) && aligned16(ci);
+  const Way way = spmm_half_way(m, k, n, nnz, index_bits(ci), mode, aligned, true);
+  if (way == kRows) return spmm_matrix(b, ri, values, ro, ci, m);
   check_csr_half(b, values, ro, ci, m);
-  // Up to 8 columns one lane per nonzero (spmm_skinny.cu) instead of one per column: 4096 x 4096 at 10 %, 4 columns 12 us
-  // against 21, at 30 % 23 against 27.  Not for rows of less than 96 nonzeros, or 2 % of the columns, which do not pay for
-  // a row's start or for x in every block's shared memory (32768 x 256 at 30 %: 17 us against 13; 2048 x 14000 at 0.5 %: 11
-  // against 8), and not above one half stored (2048 x 14000 at 90 %: 58 against 52).
-  if (mode == kAuto && n <= 8 && nnz >= 96 * m && 50 * nnz >= m * k && 2 * nnz <= m * k && iex_spmm_f16_skinny_supported(k, n)) {
-    c10::cuda::CUDAGuard guard(b.device());
-    maybe_validate(ro, ci, m, k, nullptr, false);
-    at::Tensor out = empty(b, {m, n});
-    const int st = iex_spmm_f16_skinny(m, k, n, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(),
-                                       b.data_ptr(), n, 1, out.data_ptr(), n, 1, stream_of(b));
-    if (st == 0) return out;
-    TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_f16_skinny failed with status ", st, ": ", iex_error_string(st));
-  }
-  const double dense = expand_us(m, k, nnz, index_bits(ci)) + iex_gemm_f16_estimate_us(m, n, k, 1, 0) +
-                       (n % 8 == 0 ? 0.0 : 2.0);
-  const double decode = decode_supported(b, values, ci) ? block_decode_us(m, k, n, nnz) : 1e30;
-  // Tensor cores where the estimates are close: they are good to 10 %, and the walk along the longest row, which only
-  // the CUDA cores pay for, is estimated from the average one.
-  if (mode == kAuto && 1.15 * iex_spmm_f16_estimate_us(m, k, n, nnz, index_bits(ci)) <= std::min(dense, decode)) return cores();
-  if (decode <= dense) return spmm_tc_half(b, ro, values, ci, m);
+  if (way == kDecode) return spmm_tc_half(b, ro, values, ci, m);
   c10::cuda::CUDAGuard guard(b.device());
   maybe_validate(ro, ci, m, k, nullptr, false);
   at::Tensor out = empty(b, {m, n});
+  if (way == kFewColumns) {
+    const int st = iex_spmm_f16_skinny(m, k, n, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(),
+                                       b.data_ptr(), n, 1, out.data_ptr(), n, 1, stream_of(b));
+    if (st == 0) return out;
+    // pairs of nonzeros are loaded together; a matrix that is not aligned for that is expanded
+    TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_f16_skinny failed with status ", st, ": ", iex_error_string(st));
+  }
   gemm(m, n, k, expand(values, ro, ci, m, k), false, tma_rows(b), true, out, false);
   return out;
 }
@@ -466,6 +480,9 @@ at::Tensor relu_down_proj(const at::Tensor& hidden, const at::Tensor& weight) {
 
 PYBIND11_MODULE(iex_torch_ext, mod) {
   mod.def("myspmm", &iex_torch::myspmm);
+  mod.def("spmm_half_way", [](int64_t m, int64_t k, int64_t n, int64_t nnz, int bits, bool eager) {
+    return static_cast<int>(iex_torch::spmm_half_way(m, k, n, nnz, bits, iex_torch::kAuto, true, eager));
+  });
   mod.def("mylinear", &iex_torch::mylinear);
   mod.def("sparse_linear", &iex_torch::sparse_linear);
   mod.def("expand_weight", &iex_torch::expand_weight);

@@ -1,5 +1,6 @@
 """CPU: the kernel-selection cost model reproduces the measured winners and respects the
 tensor-core kernel's shape limits."""
+from intrasm_engine_b200 import ops
 from intrasm_engine_b200.pytorch import tuning
 
 
@@ -12,12 +13,27 @@ def test_measured_cases():
         assert tuning.choose_spmm_kernel(m, k, n, nnz) == want, (m, k, n, sp)
 
 
-def test_model_against_measured_times():
-    assert abs(tuning.tensor_core_us(11008, 4096) - 57.0) < 10     # 49-58 us measured
-    assert abs(tuning.tensor_core_us(2048, 512) - 15.0) < 4        # 12.4 us measured
-    for (m, nnz, n), measured in (((2048, 315538, 128), 30.8), ((512, 52418, 128), 18.5),
-                                  ((512, 25390, 256), 10.3), ((11008, 22544909, 64), 450.0)):
-        assert abs(tuning.cuda_core_us(m, nnz, n) - measured) < 0.15 * measured
+def test_eager_and_recorded_calls_share_the_model():
+    """Where an eager call takes one of the two kernels that a recorded one has, both take the same."""
+    ways = set()
+    for m, k in ((256, 512), (2048, 512), (512, 2048), (1024, 1024), (4096, 4096), (11008, 4096)):
+        for n in (64, 128, 256, 48, 100):
+            for sp in (0.5, 0.7, 0.8, 0.9, 0.95, 0.98):
+                nnz = int(m * k * (1 - sp))
+                eager = ops.native.spmm_half_way(m, k, n, nnz, 16, True)
+                recorded = ops.native.spmm_half_way(m, k, n, nnz, 16, False)
+                ways.add(eager)
+                assert recorded in (0, 1)
+                if eager != 2:  # not expanded
+                    assert eager == recorded
+                assert tuning.choose_spmm_kernel(m, k, n, nnz) == ("tensor_core" if recorded == 1 else "cuda_core")
+    assert ways == {0, 1, 2}
+
+
+def test_few_columns_are_an_eager_way():
+    assert ops.native.spmm_half_way(4096, 4096, 4, 1677721, 16, True) == 3
+    assert ops.native.spmm_half_way(4096, 4096, 4, 1677721, 16, False) == 0
+    assert ops.native.spmm_half_way(4096, 4096, 9, 1677721, 16, True) != 3
 
 
 def test_shape_limits():
