@@ -83,21 +83,24 @@ class SparseLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
-        if math.prod(lead) * self.in_features != x.numel():
+        flat = x.dim() == 2 and x.size(1) == self.in_features
+        if not flat and math.prod(lead) * self.in_features != x.numel():
             # a narrower x would send column indices past its rows, a wider one be cut off
             raise RuntimeError(f"SparseLinear expects {self.in_features} input features, got an input of shape "
                                f"{tuple(x.shape)}")
+        values = self.values
         if x.is_cuda and x.dtype == torch.float16 and not (torch.is_grad_enabled() and
-                                                           (x.requires_grad or self.values.requires_grad)):
+                                                           (x.requires_grad or values.requires_grad)):
             # inference: x is read as it lies and the result written as [tokens, out_features]
-            x2 = x if x.dim() == 2 and x.size(1) == self.in_features else x.reshape(-1, self.in_features)
-            y = ops.native.sparse_linear(x2.contiguous(), self.values, self.row_offsets, self.column_indices,
-                                         self.out_features, self.in_features, self.dense_copy())
+            x2 = x if flat else x.reshape(-1, self.in_features)
+            row_offsets, column_indices = self.row_offsets, self.column_indices
+            y = ops.native.sparse_linear(x2.contiguous(), values, row_offsets, column_indices, self.out_features,
+                                         self.in_features, self._dense.current(values, row_offsets, column_indices))
             if self.bias is not None:
                 y = y + self.bias
-            return y if x.dim() == 2 else y.reshape(*lead, self.out_features)
+            return y if flat else y.reshape(*lead, self.out_features)
         b = x.reshape(-1, self.in_features).t().contiguous()  # [in_features, tokens]
-        out = MySpMM.run(b, self.row_indices, self.values, self.row_offsets, self.column_indices,
+        out = MySpMM.run(b, self.row_indices, values, self.row_offsets, self.column_indices,
                          self.out_features, self.transp_info,
                          fwd_kwargs_1=default_fwd_kwargs(use_tensor_cores="auto"))
         y = out.t()

@@ -11,6 +11,8 @@ from __future__ import annotations
 
 import torch
 
+from .. import ops
+
 
 def dense_to_sparse(matrix: torch.Tensor, device=None, index_dtype=torch.int32):
     """Dense 2-D matrix -> ``(values, row_indices, row_offsets, column_indices)``.
@@ -74,7 +76,7 @@ def sparse_to_dense(values, row_offsets, column_indices, m: int, k: int) -> torc
 DENSE_COPY_DENSITY = 0.25
 
 
-class DenseCopy:
+class DenseCopy(ops.native.KeptCopy):
     """Dense fp16 copy ``[m, k]`` of a layer's CSR weight, laid out once when the layer is built (k a
     multiple of 8; None for sparser weights) and again when one of the three CSR tensors has been replaced,
     moved or changed in place since.
@@ -84,40 +86,17 @@ class DenseCopy:
     by the tensors' version counters.  What leaves no trace there gets no copy, or has to be told:
       * inference tensors have no counter: no copy;
       * a call that is recorded into a CUDA graph: no copy, since the values may change between replays;
-      * writes through ``.data`` or raw pointers: call ``reset``.
+      * writes through ``.data`` or raw pointers: call ``reset()``; ``current`` then makes a new one.
     A copy is complete before another stream or thread can see it, and the native calls that read it mark
     their stream, so that it can be replaced while they run.  It is left out of pickles and deep copies."""
 
     def __init__(self, m: int, k: int):
-        self.m, self.k = int(m), int(k)
-        self._state = None  # (the three tensors, views that hold their storage, key, copy), replaced as a whole
+        super().__init__(int(m), int(k), DENSE_COPY_DENSITY)
 
     def __reduce__(self):
         return DenseCopy, (self.m, self.k)
 
-    def reset(self):
-        """Forgets the copy; the next call makes one from the values as they are then."""
-        self._state = None
-
-    def current(self, values, row_offsets, column_indices):
-        from .. import ops
-        if (not values.is_cuda or values.dtype != torch.float16 or self.k % 8 != 0 or self.m == 0
-                or values.numel() < DENSE_COPY_DENSITY * self.m * self.k
-                or values.is_inference() or row_offsets.is_inference() or column_indices.is_inference()
-                or ops.native.stream_capturing(values)):
-            return None
-        state = self._state
-        key = (values.data_ptr(), values.numel(), values._version, row_offsets.data_ptr(), row_offsets._version,
-               column_indices.data_ptr(), column_indices._version)
-        if (state is not None and state[0] is values and state[1] is row_offsets and state[2] is column_indices
-                and state[4] == key):
-            return state[5]
-        with torch.no_grad():
-            held = tuple(t.detach() for t in (values, row_offsets, column_indices))
-            weight = ops.native.expand_weight(*held, self.m, self.k)
-        torch.cuda.current_stream(values.device).synchronize()
-        self._state = (values, row_offsets, column_indices, held, key, weight)
-        return weight
+    # current(values, row_offsets, column_indices) and reset(): KeptCopy in torch_ext/iex_autograd.cpp
 
 
 def swizzle_rows(row_offsets: torch.Tensor) -> torch.Tensor:

@@ -17,6 +17,7 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
+#include <array>
 #include <optional>
 
 namespace iex_torch {
@@ -333,6 +334,58 @@ at::Tensor expand_weight(const at::Tensor& values, const at::Tensor& ro, const a
   return expand(values, ro, ci, m, k);
 }
 
+// The dense copy a layer keeps of its CSR weight (pytorch/utils.py: DenseCopy, which says what it follows).  Asked for on
+// every inference call, so the comparison is done here: 0.3 us, 3 us in Python.
+class KeptCopy {
+ public:
+  KeptCopy(int64_t m, int64_t k, double density) : m_(m), k_(k), density_(density) {}
+  int64_t rows() const { return m_; }
+  int64_t columns() const { return k_; }
+  void reset() {
+    weight_.reset();
+    held_ = {};
+  }
+
+  // Called with the interpreter lock held, which is what makes the members' update atomic.
+  std::optional<at::Tensor> current(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci) {
+    if (!values.is_cuda() || values.scalar_type() != at::kHalf || k_ % 8 != 0 || m_ == 0 ||
+        static_cast<double>(values.numel()) < density_ * m_ * k_ || values.is_inference() || ro.is_inference() ||
+        ci.is_inference() || iex_stream_is_capturing(stream_of(values)))
+      return std::nullopt;
+    const std::array<const at::Tensor*, 3> now = {&values, &ro, &ci};
+    bool same = weight_.has_value();
+    for (int i = 0; i < 3 && same; ++i) same = held_[i].is(*now[i]);
+    if (same) return weight_;
+    std::array<Held, 3> held = {Held(values), Held(ro), Held(ci)};
+    at::Tensor weight = expand_weight(values, ro, ci, m_, k_);
+    {
+      pybind11::gil_scoped_release unlocked;
+      at::cuda::getCurrentCUDAStream(values.get_device()).synchronize();
+    }
+    held_ = std::move(held);
+    weight_ = std::move(weight);
+    return weight_;
+  }
+
+ private:
+  struct Held {
+    at::Tensor tensor;      // the object itself ...
+    c10::Storage storage;   // ... and what it lay in, so that its address cannot come back as something else
+    const void* data = nullptr;
+    int64_t count = 0, version = 0;
+    Held() = default;
+    explicit Held(const at::Tensor& t)
+        : tensor(t), storage(t.storage()), data(t.data_ptr()), count(t.numel()), version(t._version()) {}
+    bool is(const at::Tensor& t) const {
+      return tensor.is_same(t) && data == t.data_ptr() && count == t.numel() && version == t._version();
+    }
+  };
+  const int64_t m_, k_;
+  const double density_;
+  std::array<Held, 3> held_;
+  std::optional<at::Tensor> weight_;
+};
+
 // The two branches of a sparse || dense layer with both weights dense: x [k, n] ->
 // (weight0 @ x [m0, n], (weight1 @ x)^T [n, m1]) in one launch.  weight0 is the layer's dense copy.
 std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Tensor& weight0, const at::Tensor& weight1) {
@@ -486,6 +539,13 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
   mod.def("mylinear", &iex_torch::mylinear);
   mod.def("sparse_linear", &iex_torch::sparse_linear);
   mod.def("expand_weight", &iex_torch::expand_weight);
+  pybind11::class_<iex_torch::KeptCopy>(mod, "KeptCopy")
+      .def(pybind11::init<int64_t, int64_t, double>())
+      .def_property_readonly("m", &iex_torch::KeptCopy::rows)
+      .def_property_readonly("k", &iex_torch::KeptCopy::columns)
+      .def("reset", &iex_torch::KeptCopy::reset)
+      .def("current", &iex_torch::KeptCopy::current, pybind11::arg("values"), pybind11::arg("row_offsets"),
+           pybind11::arg("column_indices"));
   mod.def("stream_capturing", [](const at::Tensor& t) { return iex_stream_is_capturing(iex_torch::stream_of(t)) != 0; });
   mod.def("linear_pair", &iex_torch::linear_pair);
   mod.def("attention_plan", &iex_torch::attention_plan);
