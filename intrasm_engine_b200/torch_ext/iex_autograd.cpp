@@ -72,9 +72,9 @@ double expand_us(int64_t m, int64_t k, int64_t nnz, int bits) {
 double block_decode_us(int64_t m, int64_t k, int64_t n, int64_t nnz) {
   const int64_t step = n <= 64 ? 8 : 16, rows = ((m + 147) / 148 + step - 1) / step * step;  // of an SM's unit
   const double blocks = static_cast<double>((k + 511) / 512), waves = static_cast<double>(std::max<int64_t>(1, (rows + 127) / 128));
-  const bool wide = n > 128;
-  return (wide ? 6.2 : 4.85) + waves * blocks * (wide ? 1.75 : 1.6) +
-         rows * (0.155e-3 * nnz / std::max<int64_t>(m, 1) + (wide ? 0.02 : 0.006) * blocks);
+  const double wide = std::clamp((n - 128) / 128.0, 0.0, 1.0);
+  return 4.85 + 1.35 * wide + waves * blocks * (1.6 + 0.15 * wide) +
+         rows * (0.155e-3 * nnz / std::max<int64_t>(m, 1) + (0.006 + 0.014 * wide) * blocks);
 }
 bool decode_supported(int64_t k, int64_t n, int bits) {
   return n % 64 == 0 && n > 0 && n <= 256 && k % 8 == 0 && k > 0 && (bits == 32 || k <= 65280);
@@ -444,7 +444,8 @@ at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at
                  "iex_linear_f16_any");
     return out;
   }
-  const double as_dense = expand_us(m, k, nnz, index_bits(ci)) + gemm_us;
+  // a launch and a buffer more than the decoder: 13 us a call from the host, 10 with the decoder, where kernels are short
+  const double as_dense = std::max(13.0, expand_us(m, k, nnz, index_bits(ci)) + gemm_us);
   if (tokens <= 256 && k % 8 == 0 && block_decode_us(m, k, tokens, nnz) < as_dense) {
     const int st = iex_spmm_linear_f16_tile(m, 0, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
                                             values.data_ptr(), nullptr, x.data_ptr(), 1, nullptr, out.data_ptr(), 1,
