@@ -52,7 +52,9 @@ class MySpMM(MyAutogradFunc):
             b, ri, values, ro, ci, m, transp = args
             if (b.is_cuda and b.dim() == 2 and values.dtype in (torch.float32, torch.float16)
                     and (len(transp) == 4 or not b.requires_grad)):
-                return ops.native.myspmm(b, ri, values, ro, ci, m, transp, _MODES[kw.get("use_tensor_cores", False)])
+                out = ops.native.myspmm(b, ri, values, ro, ci, m, transp, _MODES[kw.get("use_tensor_cores", False)])
+                if out is not None:
+                    return out
         return super().run(*args, **fwd_kwargs)
 
     @staticmethod

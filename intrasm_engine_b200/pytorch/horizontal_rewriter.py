@@ -312,7 +312,7 @@ class SparseDenseLayer(ModuleToReplay):
         if self.mode == "fused" and not (torch.is_grad_enabled() and
                                          (x.requires_grad or values.requires_grad or weight.requires_grad)):
             # the pair function's fused launch without its autograd bookkeeping
-            if _fused_operands(x, values, self.column_indices, weight):
+            if ops.native.plain(x, values, weight) and _fused_operands(x, values, self.column_indices, weight):
                 dense = self._dense.current(values, self.row_offsets, self.column_indices)
                 if dense is not None and dense.size(1) == x.size(0):
                     return ops.native.linear_pair(x, dense, weight)

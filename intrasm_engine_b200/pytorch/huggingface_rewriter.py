@@ -96,9 +96,10 @@ class SparseLinear(nn.Module):
             row_offsets, column_indices = self.row_offsets, self.column_indices
             y = ops.native.sparse_linear(x2.contiguous(), values, row_offsets, column_indices, self.out_features,
                                          self.in_features, self._dense.current(values, row_offsets, column_indices))
-            if self.bias is not None:
-                y = y + self.bias
-            return y if flat else y.reshape(*lead, self.out_features)
+            if y is not None:  # else the call is being traced, or carries tangents
+                if self.bias is not None:
+                    y = y + self.bias
+                return y if flat else y.reshape(*lead, self.out_features)
         b = x.reshape(-1, self.in_features).t().contiguous()  # [in_features, tokens]
         out = MySpMM.run(b, self.row_indices, values, self.row_offsets, self.column_indices,
                          self.out_features, self.transp_info,

@@ -10,10 +10,13 @@
 // It also holds the choice between the ways to multiply an fp16 CSR matrix (spmm_half_way).
 #include "iex_torch_ops.h"
 
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <torch/csrc/autograd/edge.h>
 #include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
@@ -30,6 +33,34 @@ using torch::autograd::variable_list;
 int index_bits(const at::Tensor& ci) { return ci.scalar_type() == at::kShort ? 16 : 32; }
 int64_t round8(int64_t v) { return (v + 7) / 8 * 8; }
 bool aligned16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+
+// Whether a call may go past the dispatcher: nobody records the operators (torch.jit.trace, a dispatch mode such as
+// make_fx or FakeTensorMode), and the operands are ordinary tensors without tangents.  Otherwise the callers in Python go on to the
+// autograd functions and registered operators, which a recorder sees and which refuse what they have no rule for.
+bool plain(std::initializer_list<const at::Tensor*> operands) {
+  if (torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;
+  constexpr c10::DispatchKeySet special({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot,
+                                         c10::DispatchKey::Functionalize, c10::DispatchKey::Conjugate,
+                                         c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor,
+                                         c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::BatchedNestedTensor,
+                                         c10::DispatchKey::FuncTorchGradWrapper});
+  for (const at::Tensor* t : operands)
+    if (!t->defined() || t->key_set().has_any(special) || t->_fw_grad(/*level=*/0).defined()) return false;
+  return true;
+}
+
+// First-order gradients of a backward pass that is itself recorded (create_graph): differentiating them again is an error,
+// as the kernels have no second derivative.
+variable_list once_differentiable(variable_list&& grads, const at::Tensor& grad, const at::Tensor& a, const at::Tensor& b,
+                                  const char* what) {
+  if (torch::autograd::compute_requires_grad(grad, a, b)) {
+    auto error = std::make_shared<torch::autograd::Error>(std::string(what) + " cannot be differentiated twice",
+                                                          torch::autograd::collect_next_edges(grad, a, b));
+    for (at::Tensor& g : grads)
+      if (g.defined()) torch::autograd::set_history(g, error);
+  }
+  return std::move(grads);
+}
 
 // ---------------------------------------------------------------------------- fp16 CSR products
 
@@ -214,31 +245,38 @@ at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tens
 }
 
 struct MySpMMBackward : public Node {
-  SavedVariable b_, values_;
-  SpmmArgs args;
+  // b, values and the pattern: hooks on saved tensors see all of them, and changing one in place before the backward
+  // pass is an error
+  std::array<SavedVariable, 9> saved_;
+  int64_t m_ = 0;
+  int mode_ = kCudaCores;
   std::string name() const override { return "MySpMMBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    b_.reset_data();
-    values_.reset_data();
+    for (SavedVariable& v : saved_) v.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(2);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView below;
-    const at::Tensor b = b_.unpack(), values = values_.unpack();
-    const at::Tensor grad = grads[0].contiguous();
-    if (task_should_compute_output(1)) out[1] = grad_of_values(grad, b, values, args);
-    if (task_should_compute_output(0)) out[0] = grad_of_b(grad, b, values, args);
-    return out;
+    std::array<at::Tensor, 9> t;
+    for (int i = 0; i < 9; ++i) t[i] = saved_[i].unpack();
+    const SpmmArgs args{t[2], t[3], t[4], t[5], t[6], t[7], t[8], m_, mode_};
+    {
+      at::AutoDispatchBelowADInplaceOrView below;
+      const at::Tensor grad = grads[0].contiguous();
+      if (task_should_compute_output(1)) out[1] = grad_of_values(grad, t[0], t[1], args);
+      if (task_should_compute_output(0)) out[0] = grad_of_b(grad, t[0], t[1], args);
+    }
+    return once_differentiable(std::move(out), grads[0], t[0], t[1], "MySpMM");
   }
 };
 
-// MySpMM.run without a graph constructor.  `transp` is (row_indices_t, row_offsets_t,
-// column_indices_t, perm) or empty; without it b must not require a gradient.
-at::Tensor myspmm(const at::Tensor& b_in, const at::Tensor& ri, const at::Tensor& values, const at::Tensor& ro,
-                  const at::Tensor& ci, int64_t m, const std::vector<at::Tensor>& transp, int mode) {
+// MySpMM.run without a graph constructor; nothing for calls that have to go through the dispatcher.  `transp` is
+// (row_indices_t, row_offsets_t, column_indices_t, perm) or empty; without it b must not require a gradient.
+std::optional<at::Tensor> myspmm(const at::Tensor& b_in, const at::Tensor& ri, const at::Tensor& values, const at::Tensor& ro,
+                                 const at::Tensor& ci, int64_t m, const std::vector<at::Tensor>& transp, int mode) {
+  if (!plain({&b_in, &values, &ri, &ro, &ci})) return std::nullopt;
   SpmmArgs p;
   p.ri = ri;
   p.ro = ro;
@@ -261,9 +299,10 @@ at::Tensor myspmm(const at::Tensor& b_in, const at::Tensor& ri, const at::Tensor
   if (needs_grad) {
     auto node = std::shared_ptr<MySpMMBackward>(new MySpMMBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(b, values));
-    node->b_ = SavedVariable(b, false);
-    node->values_ = SavedVariable(values, false);
-    node->args = std::move(p);
+    const std::array<const at::Tensor*, 9> saved = {&b, &values, &p.ri, &p.ro, &p.ci, &p.ri_t, &p.ro_t, &p.ci_t, &p.perm};
+    for (int i = 0; i < 9; ++i) node->saved_[i] = SavedVariable(*saved[i], false);
+    node->m_ = m;
+    node->mode_ = mode;
     torch::autograd::set_history(out, node);
   }
   return out;
@@ -283,16 +322,19 @@ struct MyLinearBackward : public Node {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(2);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView below;
     const at::Tensor input = input_.unpack(), weight = weight_.unpack();
     const at::Tensor& grad = grads[0];
     const bool own = grad.scalar_type() == at::kHalf && grad.is_cuda() && weight.size(0) % 8 == 0 &&
                      weight.size(1) % 8 == 0;
     if (own) {
-      const at::Tensor g = grad.contiguous();
-      if (task_should_compute_output(0)) out[0] = linear_fp16_dgrad(g, weight);
-      if (task_should_compute_output(1)) out[1] = linear_fp16_wgrad(g, input);
-    } else {
+      {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const at::Tensor g = grad.contiguous();
+        if (task_should_compute_output(0)) out[0] = linear_fp16_dgrad(g, weight);
+        if (task_should_compute_output(1)) out[1] = linear_fp16_wgrad(g, input);
+      }
+      return once_differentiable(std::move(out), grad, input, weight, "MyLinear's tensor-core path");
+    } else {  // differentiable products
       if (task_should_compute_output(0)) out[0] = grad.mm(weight);
       if (task_should_compute_output(1)) out[1] = grad.t().mm(input);
     }
@@ -301,8 +343,9 @@ struct MyLinearBackward : public Node {
 };
 
 // MyLinear.run without a graph constructor; nothing for operands the tensor-core kernel does not
-// take (tc_linear_eligible in layers_and_funcs/torch.py).
+// take (tc_linear_eligible in layers_and_funcs/torch.py) and for calls that have to go through the dispatcher.
 std::optional<at::Tensor> mylinear(const at::Tensor& input, const at::Tensor& weight) {
+  if (!plain({&input, &weight})) return std::nullopt;
   const bool eligible = input.is_cuda() && weight.is_cuda() && input.scalar_type() == at::kHalf &&
                         weight.scalar_type() == at::kHalf && input.dim() == 2 && weight.dim() == 2 &&
                         input.size(0) > 0 && input.size(1) % 8 == 0 && input.is_contiguous() &&
@@ -348,7 +391,7 @@ class KeptCopy {
 
   // Called with the interpreter lock held, which is what makes the members' update atomic.
   std::optional<at::Tensor> current(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci) {
-    if (!values.is_cuda() || values.scalar_type() != at::kHalf || k_ % 8 != 0 || m_ == 0 ||
+    if (!plain({&values, &ro, &ci}) || !values.is_cuda() || values.scalar_type() != at::kHalf || k_ % 8 != 0 || m_ == 0 ||
         static_cast<double>(values.numel()) < density_ * m_ * k_ || values.is_inference() || ro.is_inference() ||
         ci.is_inference() || iex_stream_is_capturing(stream_of(values)))
       return std::nullopt;
@@ -406,9 +449,11 @@ std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Te
 //   with `dense`     the layer's dense copy of W and the dense GEMM
 //   up to 256        block decoder on tensor cores (spmm_tile.cu), unless ...
 //   otherwise        ... expanding W for the dense GEMM is estimated faster (many tokens)
-// All read x as it lies and write [tokens, m]: no transposed copies of either.
-at::Tensor sparse_linear(const at::Tensor& x, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
+// All read x as it lies and write [tokens, m]: no transposed copies of either.  Nothing for calls that have to go through the
+// dispatcher.
+std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
                          int64_t m, int64_t k, const std::optional<at::Tensor>& dense_weight) {
+  if (!plain({&x, &values, &ro, &ci})) return std::nullopt;
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous(), "x must be a contiguous [tokens, in_features] matrix");
   TORCH_CHECK(x.size(1) == k, "x has ", x.size(1), " columns, the weight ", k);
   TORCH_CHECK(values.dim() == 1 && ci.dim() == 1 && values.size(0) == ci.size(0),
@@ -548,6 +593,7 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
       .def("current", &iex_torch::KeptCopy::current, pybind11::arg("values"), pybind11::arg("row_offsets"),
            pybind11::arg("column_indices"));
   mod.def("stream_capturing", [](const at::Tensor& t) { return iex_stream_is_capturing(iex_torch::stream_of(t)) != 0; });
+  mod.def("plain", [](const at::Tensor& a, const at::Tensor& b, const at::Tensor& c) { return iex_torch::plain({&a, &b, &c}); });
   mod.def("linear_pair", &iex_torch::linear_pair);
   mod.def("attention_plan", &iex_torch::attention_plan);
   mod.def("attention", &iex_torch::attention);
