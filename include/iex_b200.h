@@ -234,6 +234,15 @@ IEX_API int iex_linear_f16_wgrad(int tokens, int in_features, int out_features, 
 IEX_API int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long long lda, const void* b, int b_mn,
                          long long ldb, void* out, int out_transposed, long long ldo, int tile_n, int k_parts,
                          void* stream);
+/* The same where one operand (sparse_operand 0: a, 1: b) is the dense copy of a CSR matrix, given beside it with its rows
+ * along the product's rows (a) or columns (b); value p is values[p] or, with perm, values[perm[p]].  A position that is
+ * not stored is a zero in the copy, and zero times an infinity or NaN of the other operand is NaN in every row: outputs
+ * that come out NaN are summed again from the stored positions alone, as a CSR product has them (the CUDA-core kernels'
+ * sums).  Takes longer only then. */
+IEX_API int iex_gemm_f16_csr(int m, int n, int k, const void* a, int a_mn, long long lda, const void* b, int b_mn,
+                             long long ldb, void* out, int out_transposed, long long ldo, int sparse_operand,
+                             const int32_t* row_offsets, const void* column_indices, int index_bits,
+                             const void* values, const long long* perm, int tile_n, int k_parts, void* stream);
 /* Time this library expects iex_gemm_f16 to take on the current device, for choosing between ways. */
 IEX_API double iex_gemm_f16_estimate_us(int m, int n, int k, int b_mn, int out_transposed);
 /* The same for iex_spmm_f16_i16 (index_bits 16) and iex_spmm_f16_i32 (32). */
@@ -242,7 +251,8 @@ IEX_API double iex_spmm_f16_estimate_us(int m, int k, int n, int nnz, int index_
 /* CSR SpMM and dense linear on the same activations in one launch, either of them alone with the
  * other's row count 0.  x is [k, n] (n a multiple of 8) or, with x_tokens_major, [n, k] (k a multiple of
  * 8); n <= 256.  Each output is [rows, n] or, with its tokens-major flag, [n, rows].  `bias`
- * (nullable) makes the sparse output relu(sum + bias[row]).  Columns ascend within a row. */
+ * (nullable) makes the sparse output relu(sum + bias[row]).  Columns ascend within a row.  Sparse outputs that come out
+ * NaN are summed again from the stored positions alone (see iex_gemm_f16_csr). */
 IEX_API int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n, int nnz, const int32_t* row_offsets,
                                      const void* column_indices, int index_bits, const void* values,
                                      const void* weight, const void* x, int x_tokens_major, const float* bias,

@@ -77,6 +77,9 @@ SIGNATURES = {
     # m n k a a_mn lda b b_mn ldb out out_transposed ldo tile_n k_parts stream
     "iex_gemm_f16": (c_int, [c_int, c_int, c_int, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll,
                              c_int, c_int, c_ptr]),
+    # ... sparse_operand row_offsets cols index_bits values perm tile_n k_parts stream
+    "iex_gemm_f16_csr": (c_int, [c_int, c_int, c_int, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll, c_ptr, c_int, c_ll,
+                                 c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_int, c_int, c_ptr]),
     # m n k b_mn out_transposed
     "iex_spmm_f16_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int, c_int]),
     "iex_gemm_f16_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int, c_int]),

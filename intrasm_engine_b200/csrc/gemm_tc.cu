@@ -33,6 +33,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "csr_terms.cuh"
 #include "tc_ptx.cuh"
 
 namespace iex {
@@ -63,6 +64,7 @@ struct GemmParams {
   int tma_out;             // rows of the output are multiples of 16 bytes: TMA stores
   __half* out;
   long long ldo;           // elements between rows of the stored output
+  CsrTerms terms;          // kStored: one operand is the dense copy of this CSR matrix
   int* status;
 };
 
@@ -160,11 +162,12 @@ __device__ __forceinline__ void add_parts(uint32_t base, int l0, int vecs, uint3
 }
 
 // The operands' storage orders are template parameters for the sake of the one thread that issues the
-// MMAs: its descriptors then advance by constants.
-template <bool kAMn, bool kBMn>
+// MMAs: its descriptors then advance by constants.  kStored: p.terms says which CSR matrix an operand is the dense copy of
+// (a parameter too, since the path that sums outputs again costs every launch 0.2 us, by its registers and stack).
+template <bool kAMn, bool kBMn, bool kStored>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap map_out, const __grid_constant__ GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -268,7 +271,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       uint32_t ph = 0;
       for (int t = unit0; t < tiles && ok; t += unit_step, ++u) {
         const int acc = u & 1;
-        if (!mbar_wait(acc_empty(acc), ((u >> 1) & 1u) ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
+        // an accumulator whose outputs are summed again (csr_terms.cuh) may take tens of ms to read out
+        if (!mbar_wait(acc_empty(acc), ((u >> 1) & 1u) ^ 1u, abort_flag, p.status, kStored ? 512 : 32)) {
+          ok = false;
+          break;
+        }
         tcgen05_fence_after();
         const uint32_t d = tmem + acc * kAccumCols;
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -313,6 +320,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           uint32_t r[32];
           tmem_ld32(taddr + c + h * 32, r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if constexpr (kStored) {
+            const int row = row0 + lane, col = tn * p.bn + c + h * 32;
+            if (p.terms.sparse_is_a) repair(p.terms, row, col, 0, 1, r);
+            else repair(p.terms, col, row, 1, 0, r);
+            __syncwarp();
+          }
           if (p.out_t) {  // [N, M]: 32 columns of D x 64 bytes of rows
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -410,9 +423,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t line_bytes = (p.out_t ? kHalfM : p.bn + 4) * 4u;
     const int l0 = part * lines / p.parts, l1 = (part + 1) * lines / p.parts;
     const uint32_t vec_inv = ((1u << 20) + vecs - 1) / vecs;  // f / vecs: f is below 4096, vecs 8 to 64
-    auto write = [&](int f, const float4& sum) {
+    auto write = [&](int f, const float4& total) {
       const int line = l0 + static_cast<int>((static_cast<uint32_t>(f) * vec_inv) >> 20);
       const int v = f - (line - l0) * vecs;
+      float4 sum = total;
+      if constexpr (kStored) {
+        uint32_t r[4] = {__float_as_uint(sum.x), __float_as_uint(sum.y), __float_as_uint(sum.z), __float_as_uint(sum.w)};
+        const int row = row0 + (p.out_t ? v * 4 : line), col = col0 + (p.out_t ? line : v * 4);
+        const int row_step = p.out_t ? 1 : 0;
+        if (p.terms.sparse_is_a) repair(p.terms, row, col, row_step, 1 - row_step, r);
+        else repair(p.terms, col, row, 1 - row_step, row_step, r);
+        sum = make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
+      }
       uint2 pk;
       __half2* hh = reinterpret_cast<__half2*>(&pk);
       hh[0] = __floats2half2_rn(sum.x, sum.y);
@@ -494,7 +516,8 @@ double plan_gemm(int m, int n, int k, bool b_mn, bool out_t, int sms, GemmPlan* 
 // lda, ldb, ldo: elements between consecutive rows of the stored arrays (multiples of 8 for the
 // operands; any for a row-major output).
 int gemm_f16(int m, int n, int k, const void* a, bool a_mn, long long lda, const void* b, bool b_mn, long long ldb,
-             void* out, bool out_t, long long ldo, int force_bn, int force_parts, cudaStream_t stream) {
+             void* out, bool out_t, long long ldo, int force_bn, int force_parts, cudaStream_t stream,
+             const CsrTerms* terms = nullptr) {
   if (m < 0 || n < 0 || k < 0) return IEX_ERR_BAD_ARG;
   if (m == 0 || n == 0) return IEX_OK;
   if (!out || (k > 0 && (!a || !b))) return IEX_ERR_BAD_ARG;
@@ -529,14 +552,17 @@ int gemm_f16(int m, int n, int k, const void* a, bool a_mn, long long lda, const
   p.tma_out = tma_out;
   p.out = static_cast<__half*>(out);
   p.ldo = ldo;
+  if (terms != nullptr) p.terms = *terms;
   p.status = status_word();
   constexpr size_t smem = 227 * 1024;
-  auto kern = a_mn ? (b_mn ? gemm_pair_kernel<true, true> : gemm_pair_kernel<true, false>)
-                   : (b_mn ? gemm_pair_kernel<false, true> : gemm_pair_kernel<false, false>);
+  auto kern = terms == nullptr ? (a_mn ? (b_mn ? gemm_pair_kernel<true, true, false> : gemm_pair_kernel<true, false, false>)
+                                       : (b_mn ? gemm_pair_kernel<false, true, false> : gemm_pair_kernel<false, false, false>))
+                               : (a_mn ? (b_mn ? gemm_pair_kernel<true, true, true> : gemm_pair_kernel<true, false, true>)
+                                       : (b_mn ? gemm_pair_kernel<false, true, true> : gemm_pair_kernel<false, false, true>));
   {
     static std::mutex mutex;
-    static bool configured[64][4] = {};
-    const int which = (a_mn ? 2 : 0) + (b_mn ? 1 : 0);
+    static bool configured[64][8] = {};
+    const int which = (terms ? 4 : 0) + (a_mn ? 2 : 0) + (b_mn ? 1 : 0);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
     std::lock_guard<std::mutex> lock(mutex);
@@ -583,6 +609,31 @@ extern "C" int iex_gemm_f16(int m, int n, int k, const void* a, int a_mn, long l
                             void* stream) {
   return iex::tc::gemm_f16(m, n, k, a, a_mn != 0, lda, b, b_mn != 0, ldb, out, out_transposed != 0, ldo, tile_n,
                            k_parts, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int iex_gemm_f16_csr(int m, int n, int k, const void* a, int a_mn, long long lda, const void* b, int b_mn,
+                                long long ldb, void* out, int out_transposed, long long ldo, int sparse_operand,
+                                const int32_t* row_offsets, const void* column_indices, int index_bits, const void* values,
+                                const long long* perm, int tile_n, int k_parts, void* stream) {
+  if (sparse_operand < 0 || sparse_operand > 1 || (index_bits != 16 && index_bits != 32)) return IEX_ERR_BAD_ARG;
+  if (m > 0 && n > 0 && (!row_offsets || (k > 0 && (!column_indices || !values)))) return IEX_ERR_BAD_ARG;
+  iex::tc::CsrTerms t{};
+  t.row_offsets = row_offsets;
+  t.cols = column_indices;
+  t.values = static_cast<const __half*>(values);
+  t.perm = perm;
+  t.index_bits = index_bits;
+  t.sparse_is_a = sparse_operand == 0;
+  t.rows = t.sparse_is_a ? m : n;
+  t.columns = t.sparse_is_a ? n : m;
+  // the other operand: its k dimension runs along rows (strides 1, ld) or down them (ld, 1)
+  t.dense = static_cast<const __half*>(t.sparse_is_a ? b : a);
+  const bool mn = (t.sparse_is_a ? b_mn : a_mn) != 0;
+  const long long ld = t.sparse_is_a ? ldb : lda;
+  t.dense_c = mn ? ld : 1;
+  t.dense_t = mn ? 1 : ld;
+  return iex::tc::gemm_f16(m, n, k, a, a_mn != 0, lda, b, b_mn != 0, ldb, out, out_transposed != 0, ldo, tile_n, k_parts,
+                           static_cast<cudaStream_t>(stream), &t);
 }
 
 extern "C" double iex_gemm_f16_estimate_us(int m, int n, int k, int b_mn, int out_transposed) {

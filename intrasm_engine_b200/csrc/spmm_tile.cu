@@ -35,6 +35,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "csr_terms.cuh"
 #include "tc_ptx.cuh"
 
 namespace iex {
@@ -76,6 +77,7 @@ struct TileParams {
   int x_slots, stages;
   int acc_cols, tmem_cols;
   int ahead;           // nonzeros of L2 prefetch distance
+  CsrTerms terms;      // of the sparse units
   int* status;
 };
 
@@ -86,6 +88,21 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
       : "memory");
+}
+
+// This thread's outputs of a sparse unit, for token t_local and, if the bits say so, the one inst_m further: summed again
+// (csr_terms.cuh) and stored over what is there.  Called with next to nothing live: the decoders have no registers to spare.
+__device__ __noinline__ void store_again(const TileParams& p, int row0, int rows, int first, int t_local, uint32_t blocks) {
+  for (int mb = 0; mb < p.m_blocks; ++mb) {
+    const int t = mb * p.inst_m + t_local;
+    if (!(blocks >> mb & 1u) || t >= p.n) continue;
+    for (int c = first; c < rows; c += kDecoders * 8)
+      for (int row = row0 + c; row < min(row0 + min(c + 32, rows), p.s_m); ++row) {
+        float v = sum_stored(p.terms, row, t);
+        if (p.bias != nullptr) v = fmaxf(v + __ldg(p.bias + row), 0.f);
+        p.s_out[row * p.s_row + t * p.s_tok] = __float2half_rn(v);
+      }
+  }
 }
 
 // U pairs of a lane as loaded, the columns in the matrix's index type.  A half warp (16 lanes) reads one
@@ -214,10 +231,11 @@ __device__ __forceinline__ void issue_unit(const TileParams& p, bool sparse, int
   umma_commit(bar + kAccFull);
 }
 
-template <typename IT, int U>
+// kSparse false: a launch of dense units only
+template <typename IT, int U, bool kSparse = true>
 __global__ void __launch_bounds__(kThreads, 1)
 spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
-                 const __grid_constant__ CUtensorMap map_w1, const TileParams p) {
+                 const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ TileParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -268,7 +286,7 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   uint32_t unit_it = 0;
 
   for (int u = blockIdx.x; u < units; u += gridDim.x, ++unit_it) {
-    const bool sparse = u < p.s_tiles;
+    const bool sparse = kSparse && u < p.s_tiles;
     const int rows = sparse ? p.s_rows : p.d_rows;
     const int which = u >= p.s_tiles + p.d_tiles[0] ? 1 : 0;  // dense matrix
     const int row0 = (sparse ? u : u - p.s_tiles - (which ? p.d_tiles[0] : 0)) * rows;
@@ -461,12 +479,15 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __half* out = sparse ? p.s_out : p.d_out[which];
         const long long st_row = sparse ? p.s_row : p.d_row[which], st_tok = sparse ? p.s_tok : p.d_tok[which];
         const bool vec = st_row == 1 && (st_tok & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+        uint32_t again = 0;
         for (int mb = 0; mb < p.m_blocks; ++mb) {
           const int t = mb * p.inst_m + t_local;
           for (int c = share * 32; c < rows; c += kDecoders * 8) {
             uint32_t r[32];
             tmem_ld32(tmem + (static_cast<uint32_t>(q * 32) << 16) + mb * p.acc_cols + c, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int left = min(min(rows - c, 32), m_rows - row0 - c);  // what the unit has of these rows
+            if (sparse && lane_ok && t < p.n && any_nan(r, left)) again |= 1u << mb;
             if (sparse && p.bias != nullptr) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
@@ -476,7 +497,6 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
               }
             }
             if (!lane_ok || t >= p.n) continue;
-            const int left = min(min(rows - c, 32), m_rows - row0 - c);
             __half* dst = out + static_cast<long long>(row0 + c) * st_row + t * st_tok;
             if (vec) {
 #pragma unroll
@@ -502,6 +522,7 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             }
           }
         }
+        if (again != 0) store_again(p, row0, rows, share * 32, t_local, again);
       }
       __syncwarp();
     }
@@ -588,9 +609,9 @@ bool plan_tile(int m_sparse, int m_dense, int k, int nnz, int index_bits, int sm
   return true;
 }
 
-template <typename IT, int U>
+template <typename IT, int U, bool kSparse = true>
 int launch_tile(const CUtensorMap& mx, const CUtensorMap (&mw)[2], const TileParams& p, int grid, cudaStream_t stream) {
-  auto kern = spmm_tile_kernel<IT, U>;
+  auto kern = spmm_tile_kernel<IT, U, kSparse>;
   static std::mutex mutex;
   static bool configured[64] = {};
   {
@@ -678,6 +699,15 @@ int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets,
   p.k = k;
   p.n = n;
   p.x_mn = x_tokens_major ? 0 : 1;
+  p.terms.row_offsets = row_offsets;
+  p.terms.cols = cols;
+  p.terms.values = p.values;
+  p.terms.dense = static_cast<const __half*>(x);
+  p.terms.dense_c = p.x_mn ? n : 1;
+  p.terms.dense_t = p.x_mn ? 1 : k;
+  p.terms.rows = m_sparse;
+  p.terms.columns = n;
+  p.terms.index_bits = index_bits;
   p.kb = pl.kb;
   const int widest = (m_sparse > 0 && p.s_rows > p.d_rows) || m_dense == 0 ? p.s_rows : p.d_rows;
   p.acc_cols = round_up(widest, 32);
@@ -708,6 +738,7 @@ int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets,
   const int units = p.s_tiles + p.d_tiles[0] + p.d_tiles[1];
   const int grid = units < sms ? units : sms;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (m_sparse == 0) return launch_tile<uint16_t, 1, false>(mx, mw, p, grid, s);
   if (index_bits == 16) return dispatch_tile<uint16_t>(pl.windows, mx, mw, p, grid, s);
   return dispatch_tile<int>(pl.windows, mx, mw, p, grid, s);
 }

@@ -84,6 +84,25 @@ at::Tensor tma_rows(const at::Tensor& x) {
   return padded;
 }
 
+// The CSR matrix that one operand of a product is the dense copy of; `perm` (optional) gives each position's value.
+struct Stored {
+  int operand;  // 0: a, 1: b
+  const at::Tensor &ro, &ci, &values;
+  const at::Tensor* perm = nullptr;
+};
+
+// The dense product.  Outputs that come out NaN are summed again from the stored positions, so that an infinity or NaN in the
+// other operand reaches only the outputs that have a position there, as in a CSR product.
+void gemm(int64_t m, int64_t n, int64_t k, const at::Tensor& a, bool a_mn, const at::Tensor& b, bool b_mn,
+          const at::Tensor& out, bool out_t, const Stored& s) {
+  check_status(iex_gemm_f16_csr(m, n, k, a.data_ptr(), a_mn, a.size(1), b.data_ptr(), b_mn, b.size(1), out.data_ptr(), out_t,
+                                out.size(1), s.operand, s.ro.data_ptr<int>(), s.ci.data_ptr(), index_bits(s.ci),
+                                s.values.data_ptr(),
+                                s.perm ? reinterpret_cast<const long long*>(s.perm->data_ptr<int64_t>()) : nullptr, 0, 0,
+                                stream_of(a)),
+               "iex_gemm_f16_csr");
+}
+// The same for dense operands.
 void gemm(int64_t m, int64_t n, int64_t k, const at::Tensor& a, bool a_mn, const at::Tensor& b, bool b_mn,
           const at::Tensor& out, bool out_t) {
   check_status(iex_gemm_f16(m, n, k, a.data_ptr(), a_mn, a.size(1), b.data_ptr(), b_mn, b.size(1), out.data_ptr(), out_t,
@@ -169,7 +188,7 @@ at::Tensor spmm_half(const at::Tensor& b, const at::Tensor& ri, const at::Tensor
     // pairs of nonzeros are loaded together; a matrix that is not aligned for that is expanded
     TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_f16_skinny failed with status ", st, ": ", iex_error_string(st));
   }
-  gemm(m, n, k, expand(values, ro, ci, m, k), false, tma_rows(b), true, out, false);
+  gemm(m, n, k, expand(values, ro, ci, m, k), false, tma_rows(b), true, out, false, Stored{0, ro, ci, values});
   return out;
 }
 
@@ -215,23 +234,27 @@ at::Tensor grad_of_values(const at::Tensor& grad, const at::Tensor& b, const at:
 
 at::Tensor grad_of_b(const at::Tensor& grad, const at::Tensor& b, const at::Tensor& values, const SpmmArgs& p) {
   const int64_t m = grad.size(0), n = grad.size(1), k = b.size(0), nnz = values.numel();
+  const bool perm_ok = p.perm.scalar_type() == at::kLong && p.perm.is_contiguous() && values.is_contiguous() &&
+                       p.perm.dim() == 1 && p.perm.numel() == nnz && p.perm.device() == values.device();
   if (p.mode != kCudaCores && grad.scalar_type() == at::kHalf && values.scalar_type() == at::kHalf && m > 0 && n > 0 &&
-      k > 0 && nnz > 0) {
-    // the expanded matrix read with its row dimension as the contraction: no transposed pattern needed
+      k > 0 && nnz > 0 && perm_ok && p.ro_t.scalar_type() == at::kInt && p.ro_t.is_contiguous() && p.ro_t.numel() == k + 1 &&
+      p.ci_t.is_contiguous() && p.ci_t.numel() == nnz && p.ro_t.device() == values.device() &&
+      p.ci_t.device() == values.device() && (p.ci_t.scalar_type() == at::kShort || p.ci_t.scalar_type() == at::kInt)) {
+    // the expanded matrix read with its row dimension as the contraction; the transposed pattern is for outputs that
+    // have to be summed again
     const double dense = expand_us(m, k, nnz, index_bits(p.ci)) + iex_gemm_f16_estimate_us(k, n, m, 1, 0);
     const double cores = iex_spmm_f16_estimate_us(k, m, n, nnz, index_bits(p.ci)) + 5.0;
     if (dense < cores) {
       c10::cuda::CUDAGuard guard(grad.device());
       at::Tensor out = empty(grad, {k, n});
-      gemm(k, n, m, expand(values, p.ro, p.ci, m, k), true, tma_rows(grad), true, out, false);
+      gemm(k, n, m, expand(values, p.ro, p.ci, m, k), true, tma_rows(grad), true, out, false,
+           Stored{0, p.ro_t, p.ci_t, values, &p.perm});
       return out;
     }
   }
   // transposing the pattern is bookkeeping done once (get_transpose_info); the values follow it
   at::Tensor values_t;
-  if (p.perm.scalar_type() == at::kLong && p.perm.is_contiguous() && values.is_contiguous() && p.perm.dim() == 1 &&
-      p.perm.numel() == nnz && p.perm.device() == values.device() &&
-      (values.scalar_type() == at::kFloat || values.scalar_type() == at::kHalf)) {
+  if (perm_ok && (values.scalar_type() == at::kFloat || values.scalar_type() == at::kHalf)) {
     c10::cuda::CUDAGuard guard(values.device());
     values_t = empty(values, {nnz});
     check_status(iex_gather_values(nnz, values.element_size(), values.data_ptr(),
@@ -480,29 +503,30 @@ std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& v
     // pairs of nonzeros are loaded together; a matrix that is not aligned for that takes the ways below
     TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_f16_skinny failed with status ", st, ": ", iex_error_string(st));
   }
+  at::Tensor dense;
   if (dense_weight.has_value()) {
-    const at::Tensor& w = *dense_weight;
-    TORCH_CHECK(w.size(0) == m && w.size(1) == k && w.scalar_type() == at::kHalf && w.is_contiguous(), "dense copy of another shape");
-    mark_stream(w);
-    const at::Tensor xp = tma_rows(x);
-    check_status(iex_linear_f16_any(tokens, k, m, xp.data_ptr(), w.data_ptr(), out.data_ptr(), stream_of(x)),
-                 "iex_linear_f16_any");
-    return out;
+    dense = *dense_weight;
+    TORCH_CHECK(dense.dim() == 2 && dense.size(0) == m && dense.size(1) == k && k % 8 == 0 && dense.scalar_type() == at::kHalf &&
+                    dense.is_contiguous() && dense.device() == x.device(),
+                "dense copy of another shape");
+    mark_stream(dense);
+  } else {
+    // a launch and a buffer more than the decoder: 13 us a call from the host, 10 with the decoder, where kernels are short
+    const double as_dense = std::max(13.0, expand_us(m, k, nnz, index_bits(ci)) + gemm_us);
+    if (tokens <= 256 && k % 8 == 0 && block_decode_us(m, k, tokens, nnz) < as_dense) {
+      const int st = iex_spmm_linear_f16_tile(m, 0, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
+                                              values.data_ptr(), nullptr, x.data_ptr(), 1, nullptr, out.data_ptr(), 1,
+                                              nullptr, 0, stream_of(x));
+      if (st == 0) return out;
+      TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_linear_f16_tile failed with status ", st, ": ", iex_error_string(st));
+    }
+    dense = expand(values, ro, ci, m, k);
   }
-  // a launch and a buffer more than the decoder: 13 us a call from the host, 10 with the decoder, where kernels are short
-  const double as_dense = std::max(13.0, expand_us(m, k, nnz, index_bits(ci)) + gemm_us);
-  if (tokens <= 256 && k % 8 == 0 && block_decode_us(m, k, tokens, nnz) < as_dense) {
-    const int st = iex_spmm_linear_f16_tile(m, 0, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
-                                            values.data_ptr(), nullptr, x.data_ptr(), 1, nullptr, out.data_ptr(), 1,
-                                            nullptr, 0, stream_of(x));
-    if (st == 0) return out;
-    TORCH_CHECK(st == IEX_ERR_UNSUPPORTED, "iex_spmm_linear_f16_tile failed with status ", st, ": ", iex_error_string(st));
-  }
-  const at::Tensor dense = expand(values, ro, ci, m, k), xp = tma_rows(x);
+  const at::Tensor xp = tma_rows(x);
   if (m % 8 == 0 && iex_gemm_f16_estimate_us(m, tokens, k, 0, 1) <= iex_gemm_f16_estimate_us(tokens, m, k, 0, 0))
-    gemm(m, tokens, k, dense, false, xp, false, out, true);
+    gemm(m, tokens, k, dense, false, xp, false, out, true, Stored{0, ro, ci, values});
   else
-    gemm(tokens, m, k, xp, false, dense, false, out, false);
+    gemm(tokens, m, k, xp, false, dense, false, out, false, Stored{1, ro, ci, values});
   return out;
 }
 
