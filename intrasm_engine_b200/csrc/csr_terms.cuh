@@ -46,16 +46,22 @@ static __device__ __noinline__ float sum_stored(const CsrTerms& q, int s, int t)
   return acc;
 }
 
-// Whether one of the first `count` accumulator words is NaN.  Their sum is NaN then (or by infinities of both signs): short
-// chains of packed adds, where a comparison for each word is one long chain.
+// The sum of accumulator words, NaN if one of them is (or by infinities of both signs): short chains of packed adds, where a
+// comparison for each word is one long chain.
 template <int N>
-__device__ __forceinline__ bool any_nan(const uint32_t (&r)[N], int count) {
+__device__ __forceinline__ float sum_words(const uint32_t (&r)[N]) {
   float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
   for (int j = 0; j < N; j += 2)
     sum[j / 2 % 2] = ffma2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), make_float2(1.f, 1.f), sum[j / 2 % 2]);
-  const float all = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
-  if (all == all) return false;
+  return (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+}
+
+// Whether one of the first `count` accumulator words is NaN.
+template <int N>
+__device__ __forceinline__ bool any_nan(const uint32_t (&r)[N], int count) {
+  const float sum = sum_words(r);
+  if (sum == sum) return false;
   bool any = false;
 #pragma unroll
   for (int j = 0; j < N; ++j) any = any || (j < count && __uint_as_float(r[j]) != __uint_as_float(r[j]));

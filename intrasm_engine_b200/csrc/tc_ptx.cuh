@@ -53,12 +53,13 @@ __device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity
 }
 // Bounded wait with back-off.  A waiting warp sleeps `sleep_ns` between polls so that it
 // does not take issue slots from the warps doing the work.  Returns false when the wait
-// gave up or another role already aborted.
+// gave up or another role already aborted.  `late_ns`: the pause from the 16384th poll on, for a
+// wait that may rightly take long.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status, unsigned sleep_ns) {
+                                          int* status, unsigned sleep_ns, unsigned late_ns = 0) {
   for (uint32_t i = 0; i < kSpinLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (i >= 2u) __nanosleep(sleep_ns);
+    if (i >= 2u) __nanosleep(late_ns != 0 && i >= 1u << 14 ? late_ns : sleep_ns);
     if ((i & 63u) == 63u && *abort_flag) return false;
   }
   *abort_flag = 1;
