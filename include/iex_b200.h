@@ -395,6 +395,11 @@ IEX_API int iex_csr_to_dense_f16(int m, int k, const int32_t* row_offsets, const
 /* The same with `ld` >= k elements between the dense rows (the columns past k become zero). */
 IEX_API int iex_csr_to_dense_f16_ld(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices,
                                     int index_bits, const void* values, void* out, void* stream);
+/* The same for an operand of iex_gemm_f16_csr: columns may come in any order and more than once.  The plain copy holds one
+ * value of a column that a row stores twice; here it holds NaN, so that the product's outputs there are summed from the
+ * positions, all of them (a row whose order is broken may be marked as a whole). */
+IEX_API int iex_csr_expand_f16(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices,
+                               int index_bits, const void* values, void* out, void* stream);
 /* out[p] = dense[row(p) * ld + column_indices[p]] for every stored position p (fp16). */
 IEX_API int iex_csr_sample_f16(int m, int k, long long ld, const int32_t* row_offsets, const void* column_indices,
                                int index_bits, const void* dense, void* out, void* stream);

@@ -96,6 +96,7 @@ SIGNATURES = {
                                     c_ptr, c_ll, c_ll, c_ptr]),
     # m k ld row_offsets cols index_bits values out stream
     "iex_csr_to_dense_f16_ld": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
+    "iex_csr_expand_f16": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
     # m k ld row_offsets cols index_bits dense out stream
     "iex_csr_sample_f16": (c_int, [c_int, c_int, c_ll, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
     "iex_gather_values": (c_int, [c_int, c_int, c_ptr, c_ptr, c_ptr, c_ptr]),

@@ -123,7 +123,7 @@ row_fill_kernel(int m, int k, const T* __restrict__ dense, int relu, const int* 
 template <typename IT>
 __global__ void __launch_bounds__(256)
 csr_to_dense_f16_kernel(int m, int k, int slice, const int* __restrict__ row_offsets, const IT* __restrict__ cols,
-                        const __half* __restrict__ values, __half* __restrict__ out) {
+                        const __half* __restrict__ values, __half* __restrict__ out, int mark) {
   grid_dependency_wait();  // `out` may still be read by the kernel before this one
   grid_launch_dependents();
   const int c0 = blockIdx.y * slice;
@@ -146,15 +146,26 @@ csr_to_dense_f16_kernel(int m, int k, int slice, const int* __restrict__ row_off
       for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) row[i] = __float2half(0.f);
     }
     __syncthreads();
+    bool unordered = false;
     while (p < end) {
       if (c >= c0 && c < c1) row[c] = v;
+      if (mark && p > beg && to_index(__ldg(cols + p - 1)) >= c) unordered = true;
       p += blockDim.x;
       if (p < end) {
         c = to_index(__ldg(cols + p));
         v = __ldg(values + p);
       }
     }
-    __syncthreads();
+    if (!mark) {
+      __syncthreads();
+    } else if (__syncthreads_or(unordered ? 1 : 0)) {
+      // a column may be there twice: all that the row stores is marked, and summed from the positions
+      for (p = beg + threadIdx.x; p < end; p += blockDim.x) {
+        c = to_index(__ldg(cols + p));
+        if (c >= c0 && c < c1) row[c] = __ushort_as_half(0x7fff);
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -179,7 +190,31 @@ __device__ __forceinline__ void load_pair(const __half* values, const IT* cols, 
   }
 }
 
-template <typename IT, int TPR>
+// A row that is not strictly ascending, built again (all TPR threads): NaN where a column is stored twice.  Two bits per
+// column first (seen, seen again), then the marks, then the values of the other columns.
+template <typename IT, int TPR, typename Sync>
+__device__ __noinline__ void mark_repeats(uint32_t* words, int ld, int beg, int end, int t, const IT* cols, const __half* values,
+                                          const Sync& sync) {
+  for (int i = t; i < ld / 2; i += TPR) words[i] = 0u;
+  sync();
+  for (int p = beg + t; p < end; p += TPR) {
+    const int c = to_index(__ldg(cols + p)), at = 16 * (c & 1);
+    if (atomicOr(words + (c >> 1), 1u << at) >> at & 1u) atomicOr(words + (c >> 1), 2u << at);
+  }
+  sync();
+  for (int i = t; i < ld / 2; i += TPR) words[i] = (words[i] & 2u ? 0x7fffu : 0u) | (words[i] & 0x20000u ? 0x7fff0000u : 0u);
+  sync();
+  unsigned short* row = reinterpret_cast<unsigned short*>(words);
+  for (int p = beg + t; p < end; p += TPR) {
+    const int c = to_index(__ldg(cols + p));
+    if (row[c] != 0x7fffu) row[c] = __half_as_ushort(__ldg(values + p));
+  }
+  sync();
+}
+
+// kMark: the copy is for a product that sums NaN outputs again from the stored positions (csr_terms.cuh).  A column that a row
+// stores twice, of which only one value would be in the copy, becomes NaN, so that its outputs are.
+template <typename IT, int TPR, bool kMark>
 __global__ void __launch_bounds__(256)
 csr_expand_rows_kernel(int m, int ld, const int* __restrict__ row_offsets, const IT* __restrict__ cols,
                        const __half* __restrict__ values, __half* __restrict__ out) {
@@ -208,6 +243,21 @@ csr_expand_rows_kernel(int m, int ld, const int* __restrict__ row_offsets, const
     int next_beg = 0, next_end = 0;
     if (r + step < m) { next_beg = __ldg(row_offsets + r + step); next_end = __ldg(row_offsets + r + step + 1); }
     const int even_beg = (beg + 1) & ~1, even_end = end & ~1;
+    // A pair against itself and the position before it, which the lane before has; lane 0 has it from the window before, or,
+    // where another warp has that, loads it.  Called by whole warps.
+    bool unordered = false;
+    int before = kMark && (beg & 1) && beg < end ? to_index(__ldg(cols + beg)) : -1;
+    auto check = [&](int p, bool on, const int (&c)[2]) {
+      if constexpr (kMark) {
+        const int lane = threadIdx.x & 31;
+        const int rotated = __shfl_sync(0xffffffffu, c[1], (lane + 31) & 31);
+        int prev = rotated;
+        if (lane == 0) prev = TPR == 32 || p == even_beg ? before : on ? to_index(__ldg(cols + p - 1)) : -1;
+        unordered = unordered || (on && (prev >= c[0] || c[0] >= c[1]));
+        if (TPR == 32) before = rotated;
+      }
+    };
+    if (kMark && t == 1 && (end & 1) && end - 1 > beg) unordered = to_index(__ldg(cols + end - 2)) >= to_index(__ldg(cols + end - 1));
     if (t == 0 && beg < end && (beg & 1)) row_buf[to_index(__ldg(cols + beg))] = __ldg(values + beg);
     if (t == 1 && beg < end && (end & 1) && end - 1 >= even_beg) row_buf[to_index(__ldg(cols + end - 1))] = __ldg(values + end - 1);
     int p0 = even_beg;
@@ -217,17 +267,30 @@ csr_expand_rows_kernel(int m, int ld, const int* __restrict__ row_offsets, const
 #pragma unroll
       for (int u = 0; u < kU; ++u) load_pair(values, cols, p0 + 2 * TPR * u + 2 * t, v[u], c[u]);
 #pragma unroll
-      for (int u = 0; u < kU; ++u) put(v[u], c[u]);
+      for (int u = 0; u < kU; ++u) {
+        put(v[u], c[u]);
+        check(p0 + 2 * TPR * u + 2 * t, true, c[u]);
+      }
     }
     if (p0 < even_end) {
       uint32_t v[kU];
-      int c[kU][2];
+      int c[kU][2] = {};
 #pragma unroll
       for (int u = 0; u < kU; ++u)
         if (p0 + 2 * TPR * u + 2 * t < even_end) load_pair(values, cols, p0 + 2 * TPR * u + 2 * t, v[u], c[u]);
 #pragma unroll
       for (int u = 0; u < kU; ++u)
-        if (p0 + 2 * TPR * u + 2 * t < even_end) put(v[u], c[u]);
+      {
+        const int p = p0 + 2 * TPR * u + 2 * t;
+        if (p < even_end) put(v[u], c[u]);
+        check(p, p < even_end, c[u]);
+      }
+    }
+    if constexpr (kMark) {
+      bool again;
+      if constexpr (TPR == 32) again = __any_sync(0xffffffffu, unordered);
+      else again = __syncthreads_or(unordered ? 1 : 0) != 0;
+      if (again) mark_repeats<IT, TPR>(reinterpret_cast<uint32_t*>(buf), ld, beg, end, t, cols, values, sync);
     }
     sync();
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(r) * ld);
@@ -400,7 +463,7 @@ namespace iex {
 namespace {
 
 template <typename IT>
-int csr_to_dense(int m, int ld, const int* row_offsets, const IT* cols, const __half* values, __half* out,
+int csr_to_dense(int m, int ld, const int* row_offsets, const IT* cols, const __half* values, __half* out, bool mark,
                  cudaStream_t s) {
   // Many rows, or short ones: one pass through shared memory.  A few long rows: column slices, since a block that clears
   // and stores a long row alone takes longer than the second pass (256 x 11008 before a product: 30.6 us in slices, 31.3
@@ -414,10 +477,10 @@ int csr_to_dense(int m, int ld, const int* row_offsets, const IT* cols, const __
       const int warps = fit < 8 ? fit : 8;
       const int per_sm = 220 * 1024 / (row_bytes * warps) < 8 ? 220 * 1024 / (row_bytes * warps) : 8;
       const int blocks = (m + warps - 1) / warps, most = kNumSMs * per_sm;
-      return launch_overlapped(csr_expand_rows_kernel<IT, 32>, dim3(blocks < most ? blocks : most), dim3(32 * warps),
+      return launch_overlapped(mark ? csr_expand_rows_kernel<IT, 32, true> : csr_expand_rows_kernel<IT, 32, false>, dim3(blocks < most ? blocks : most), dim3(32 * warps),
                                static_cast<size_t>(ld) * 2 * warps, s, m, ld, row_offsets, cols, values, out);
     }
-    return launch_overlapped(csr_expand_rows_kernel<IT, 256>, dim3(m < 8 * kNumSMs ? m : 8 * kNumSMs), dim3(256),
+    return launch_overlapped(mark ? csr_expand_rows_kernel<IT, 256, true> : csr_expand_rows_kernel<IT, 256, false>, dim3(m < 8 * kNumSMs ? m : 8 * kNumSMs), dim3(256),
                              static_cast<size_t>(ld) * 2, s, m, ld, row_offsets, cols, values, out);
   }
   // about eight CTAs of 256 threads per SM in all: rows first, then up to eight column slices
@@ -428,24 +491,34 @@ int csr_to_dense(int m, int ld, const int* row_offsets, const IT* cols, const __
   int slice = ((ld + slices - 1) / slices + 7) & ~7;
   if (slice < 256) slice = 256 < ld ? 256 : ((ld + 7) & ~7);
   return launch_overlapped(csr_to_dense_f16_kernel<IT>, dim3(gx, (ld + slice - 1) / slice), dim3(256), 0, s, m, ld,
-                           slice, row_offsets, cols, values, out);
+                           slice, row_offsets, cols, values, out, mark ? 1 : 0);
 }
 
 }  // namespace
 }  // namespace iex
 
-extern "C" int iex_csr_to_dense_f16_ld(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices,
-                                       int index_bits, const void* values, void* out, void* stream) {
+static int csr_to_dense_any(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices, int index_bits,
+                            const void* values, void* out, bool mark, void* stream) {
   using namespace iex;
   if (m < 0 || k < 0 || ld < k || (index_bits != 16 && index_bits != 32)) return IEX_ERR_BAD_ARG;
   if (m == 0 || k == 0) return IEX_OK;
   if (!row_offsets || !out) return IEX_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const __half* v = static_cast<const __half*>(values);
+  __half* o = static_cast<__half*>(out);
   if (index_bits == 16)
-    return csr_to_dense<uint16_t>(m, ld, row_offsets, static_cast<const uint16_t*>(column_indices), v,
-                                  static_cast<__half*>(out), s);
-  return csr_to_dense<int>(m, ld, row_offsets, static_cast<const int*>(column_indices), v, static_cast<__half*>(out), s);
+    return csr_to_dense<uint16_t>(m, ld, row_offsets, static_cast<const uint16_t*>(column_indices), v, o, mark, s);
+  return csr_to_dense<int>(m, ld, row_offsets, static_cast<const int*>(column_indices), v, o, mark, s);
+}
+
+extern "C" int iex_csr_to_dense_f16_ld(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices,
+                                       int index_bits, const void* values, void* out, void* stream) {
+  return csr_to_dense_any(m, k, ld, row_offsets, column_indices, index_bits, values, out, false, stream);
+}
+
+extern "C" int iex_csr_expand_f16(int m, int k, int ld, const int32_t* row_offsets, const void* column_indices,
+                                  int index_bits, const void* values, void* out, void* stream) {
+  return csr_to_dense_any(m, k, ld, row_offsets, column_indices, index_bits, values, out, true, stream);
 }
 
 extern "C" int iex_csr_to_dense_f16(int m, int k, const int32_t* row_offsets, const void* column_indices,

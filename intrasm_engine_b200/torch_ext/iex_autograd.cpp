@@ -64,13 +64,13 @@ variable_list once_differentiable(variable_list&& grads, const at::Tensor& grad,
 
 // ---------------------------------------------------------------------------- fp16 CSR products
 
-// The dense fp16 copy [m, round8(k)] of a CSR matrix.
+// The dense fp16 copy [m, round8(k)] of a CSR matrix, as an operand of the products below that sum NaN outputs again.
 at::Tensor expand(const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci, int64_t m, int64_t k) {
   const int64_t ld = round8(k);
   at::Tensor dense = empty(values, {m, ld});
-  check_status(iex_csr_to_dense_f16_ld(m, k, ld, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(),
-                                       dense.data_ptr(), stream_of(values)),
-               "iex_csr_to_dense_f16_ld");
+  check_status(iex_csr_expand_f16(m, k, ld, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(),
+                                  dense.data_ptr(), stream_of(values)),
+               "iex_csr_expand_f16");
   return dense;
 }
 

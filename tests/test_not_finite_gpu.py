@@ -127,3 +127,38 @@ def test_everything_not_finite_ends():
     out = layer(x)
     assert bool(torch.isnan(out[:, 1:]).all()) and not bool(out[:, 0].any())
     assert _lib.lib.iex_last_device_status(1) == 0
+
+
+@pytest.mark.parametrize("m,k", [(700, 300), (700, 4608), (600, 4616), (40, 200), (300, 6144), (30, 6152), (900, 25000)])
+@pytest.mark.parametrize("index", [torch.int16, torch.int32])
+def test_columns_out_of_order_and_stored_twice(m, k, index):
+    """Rows in falling order, rows with repeated columns next to each other, far apart and three times, odd starts and
+    lengths: the sums over all positions, forward and backward, for every way of expanding a matrix."""
+    rng = np.random.default_rng(m + k)
+    rows = []
+    for r in range(m):
+        cols = np.sort(rng.choice(k, size=int(rng.integers(0, min(k, 200))), replace=False))
+        if r % 4 == 1:
+            cols = cols[::-1]
+        elif r % 4 == 2 and len(cols) > 2:
+            cols = np.concatenate([cols, cols[-1:]])
+        elif r % 4 == 3 and len(cols) > 2:
+            cols = np.concatenate([cols[:1], cols, cols[:1]])
+        rows.append(cols)
+    counts = [len(c) for c in rows]
+    ro = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device=DEV)
+    ci = torch.tensor(np.concatenate(rows).astype(np.int32), device=DEV).to(index)
+    values = torch.randint(1, 4, (ci.numel(),), device=DEV).half()
+    ri = torch.arange(m, dtype=torch.int32, device=DEV)
+    info = get_transpose_info(m, k, ri, ro, ci)
+    where = torch.repeat_interleave(torch.arange(m, device=DEV), (ro[1:] - ro[:-1]).long())
+    dense = torch.zeros(m, k, dtype=torch.float64, device=DEV).index_put((where, ci.long()), values.double(), accumulate=True)
+    n = 72 if m > 100 else 300
+    x = torch.randint(-1, 2, (k, n), device=DEV).half().requires_grad_(True)
+    grad = torch.randint(-1, 2, (m, n), device=DEV).half()
+    for auto in ("auto", True):
+        out = MySpMM.run(x, ri, values, ro, ci, m, info, fwd_kwargs_1=default_fwd_kwargs(use_tensor_cores=auto))
+        assert torch.equal(out.detach().double(), dense @ x.detach().double())
+        (gx,) = torch.autograd.grad(out, x, grad)
+        assert torch.equal(gx.double(), dense.t() @ grad.double())
+    assert _lib.lib.iex_last_device_status(1) == 0
