@@ -12,8 +12,8 @@
 // a sum over thousands of positions (2e-6 of the result, measured); a tile's 64 keys are therefore added to
 // fp32 registers with ordinary rounding before the next tile: as accurate as the CUDA-core sum (2.6e-7).
 //
-//   prepare kernel   k and v (transposed) as hi / lo planes that TMA can load; zeroes the output rows that
-//                    two CTAs share
+//   prepare kernel   k and v (transposed) as hi / lo planes that TMA can load; looks for values of v that are not
+//                    finite and clears the counters of the bands' pieces
 //   main kernel      one persistent CTA per SM over a contiguous run of (head, 128-row band, key tile)
 //     warp 0         TMA producer: k planes and v planes of a key tile in two rings (k is free again after S, a
 //                    tile earlier than v: one ring for both left loads too little time, 2600 cycles a tile)
@@ -25,8 +25,12 @@
 //                    registers.  Two warps per tensor-memory quarter share a tile's columns: the tensor pipe
 //                    only has S(t + 1) to do until P(t) is there, so the time from S to P is what counts
 //                    (one warp per quarter and tile, taking turns: 2900 cycles a tile)
-// The runs are equal shares of all tiles; the pieces of a band that is cut between CTAs meet in a workspace and are
-// added in order by whichever comes last.
+// The runs are equal shares of all tiles; with fewer bands than SMs, every band is cut into the same number of equal pieces
+// instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
+//
+// 24 heads x 4096 x 4096 at 5 %, d 64: 499 us in the first tenth of a second (1965 MHz), 547 to 565 us sustained (1430 to 1470
+// MHz, at the power limit); head by head over two streams 723 us.  6 heads x 1003 x 1003 at 10 %, d 80: 30.7 us against 147.
+// Which masks are faster one way or the other: iex_attention_f32_prefers below.
 //
 // Values of v at masked-out positions must not count even if they are not finite.  Zero times such a value is
 // not zero, so the prepare kernel looks for them and the (rare) heads that have some are summed position

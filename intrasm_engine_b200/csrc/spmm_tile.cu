@@ -558,8 +558,8 @@ int round_up(int v, int to) { return (v + to - 1) / to * to; }
 
 // Rows per unit and columns per block.  A sparse row costs its share of decoder instructions, a
 // dense row its bytes; units are sized so that both kinds together occupy the SMs once and end
-// together.  Measured on B200 (one SM): about 0.9 ns per stored position of a row plus 16 ns per
-// row and block; 95 GB/s of dense operand bytes.
+// together.  Measured on B200 (one SM): about 0.13 ns per stored position of a row plus 16.6 ns per
+// row and block of 512 columns; 80 GB/s of dense operand bytes.
 bool plan_tile(int m_sparse, int m_dense, int k, int nnz, int index_bits, int sms, int step, int x_slot_bytes,
                TilePlan* out) {
   const double per_row = m_sparse > 0 ? static_cast<double>(nnz) / m_sparse : 0.0;
@@ -585,7 +585,7 @@ bool plan_tile(int m_sparse, int m_dense, int k, int nnz, int index_bits, int sm
     if (pl.d_rows > 256) pl.d_rows = 256;
   }
   if (m_sparse > 0) {
-    // Columns per block: as many as two buffers leave room for; U windows of 64 nonzeros have to
+    // Columns per block: as many as two buffers leave room for; U windows of 32 nonzeros have to
     // cover a row's share of a block in almost every case.  Cost of a row and block in instructions:
     // 17 per window and about 110 of its own.
     const int room = kBudget - 2 * x_slot_bytes;
