@@ -177,7 +177,8 @@ IEX_API int iex_spmm_f32_prefers_tc(int m, int k, int n, int nnz);
  * q [heads, m, d], k [heads, n, d], v [heads, n, dv], out [heads, m, dv], contiguous and 16-byte
  * aligned; d and dv multiples of 4 up to 128.  The plan (256-byte aligned, iex_attention_plan_bytes) depends
  * on the pattern only; its first word is nonzero if the pattern stores a position twice, and the plan must
- * then not be used.  The workspace holds the operands' TF32 planes. */
+ * then not be used.  The workspace holds k and v as fp16 head and tail planes
+ * (22 bits; rows and tiles scaled by powers of two). */
 IEX_API int iex_attention_f32_supported(int heads, int m, int n, int d, int dv);
 /* Whether this call is expected to beat SDDMM and SpMM head by head: its time follows m * n, theirs the nnz
  * stored positions, so it is not the way for large, very sparse masks (whose plan of m * n / 8 bytes need not

@@ -7,34 +7,39 @@
 // the tensor cores and the mask is applied in between, in tensor memory, flash-attention style: scores
 // never leave the SM and v is read once per 128 rows.
 //
-// fp32 accuracy: operands are split into TF32 head and tail (x = hi + lo) and three of the four products
-// are kept, as in sddmm_tc.cu.  The tensor core truncates when it adds to an accumulator, which would bias
-// a sum over thousands of positions (2e-6 of the result, measured); a tile's 64 keys are therefore added to
-// fp32 registers with ordinary rounding before the next tile: as accurate as the CUDA-core sum (2.6e-7).
+// fp32 accuracy: operands are split into fp16 head and tail (x = hi + lo, 22 bits) and three of the four products are kept,
+// at twice the rate of the TF32 planes that an earlier version used and with the same number of bits.  What fp16 lacks is
+// range, so everything is scaled by powers of two, exactly: a row of q or k to a largest magnitude in [8, 16) (then |S| <
+// 2^15 for up to 128 columns), v by the factor its key's row of k lost and by one of its tile (64 or 128 keys), both given
+// back when a tile of O is added up.  Tails are stored 2^11 times as large, so that they run out of exponents no sooner than
+// the heads; the first head * head instruction scales what the tails' products have summed up back (scale-input-d).  The
+// error of a score is about 2^-22 sum |q_i k_i| + 2^-39 (max |q| sum |k_i| + max |k| sum |q_i|); in normally distributed data the result is 2.0e-7
+// off (2-norm), the TF32 planes gave 2.6e-7.  A tile whose keys' (or columns') largest magnitudes lie 2^28 and more apart, or
+// that has values of v that are not finite, does not suit the planes; its head is summed position by position (rare).
+// The tensor core truncates when it adds to an accumulator, which would bias a sum over thousands of positions (2e-6 of the
+// result, measured); a tile's keys are therefore added to fp32 registers with ordinary rounding before the next tile.
 //
-//   prepare kernel   k and v (transposed) as hi / lo planes that TMA can load; looks for values of v that are not
-//                    finite and clears the counters of the bands' pieces
+//   prepare kernel   k and v as hi / lo planes that TMA can load; marks the tiles that do not suit and clears the counters
+//                    of the bands' pieces (24 heads x 4096 x 64: 21 us, 100 MB)
 //   main kernel      one persistent CTA per SM over a contiguous run of (head, 128-row band, key tile)
-//     warp 0         TMA producer: k planes and v planes of a key tile in two rings (k is free again after S, a
-//                    tile earlier than v: one ring for both left loads too little time, 2600 cycles a tile)
-//     warp 1         issues S(t) = Q K(t)^T, warp 2 O(t) = P(t) V(t); A operands (Q, P) in tensor memory.  Two
-//                    warps because a thread that issues for a busy tensor pipe pays 200-300 cycles for every
-//                    barrier it waits on, completed or not, and 100 for a commit: one for both products took
-//                    2740 cycles a tile, of which the pipe needs 1540
+//     warp 0         TMA producer: k and v planes of the next key tiles, q's rows of the next band
+//     warp 1         issues S(t) = Q K(t)^T, warp 2 O(t) = P(t) V(t); A operands (Q, P) in tensor memory.  A thread that
+//                    issues for a busy tensor pipe pays 200-300 cycles for every barrier it waits on, completed or not, and
+//                    70 for a commit.  So there are two of them, each waits once a tile (the barrier of K(t) also counts
+//                    the PV that used up the score tile, that of V(t) the warps that wrote P), and a tile has 128 keys where
+//                    they fit (1536 cycles of the pipe; with 64 and separate barriers: 313 us instead of 288)
 //     warps 4-11     read S, keep the mask's positions, write P hi / lo over it; add the O of the tile before to
-//                    registers.  Two warps per tensor-memory quarter share a tile's columns: the tensor pipe
-//                    only has S(t + 1) to do until P(t) is there, so the time from S to P is what counts
-//                    (one warp per quarter and tile, taking turns: 2900 cycles a tile)
+//                    registers.  Two warps per tensor-memory quarter share a tile's columns: the tensor pipe has little else
+//                    to do until P(t) is there.  Four per quarter: 294 us, short sequences 25.1 instead of 23.2 us.
+//                    They also convert q, from shared memory, under the last PV of the band before (each thread loading its
+//                    row from global memory took 7500 cycles a band).
 // The runs are equal shares of all tiles; with fewer bands than SMs, every band is cut into the same number of equal pieces
 // instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
 //
-// 24 heads x 4096 x 4096 at 5 %, d 64: 499 us in the first tenth of a second (1965 MHz), 547 to 565 us sustained (1430 to 1470
-// MHz, at the power limit); head by head over two streams 723 us.  6 heads x 1003 x 1003 at 10 %, d 80: 30.7 us against 147.
+// 24 heads x 4096 x 4096 at 5 %, d 64: 255 us in the first tenths of a second (1965 MHz), 288 us sustained (1590 MHz, at the
+// power limit), with TF32 planes 499 and 548 us; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys
+// of which the pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 23.2 us, before 30.7.
 // Which masks are faster one way or the other: iex_attention_f32_prefers below.
-//
-// Values of v at masked-out positions must not count even if they are not finite.  Zero times such a value is
-// not zero, so the prepare kernel looks for them and the (rare) heads that have some are summed position
-// by position.
 //
 // Every mbarrier wait is bounded, as in tc_fused.cu.
 #include <cuda.h>
@@ -50,22 +55,31 @@ namespace iex {
 namespace tc {
 
 int make_map_f32(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows);  // tc_fused.cu
+int make_map_f16(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows,
+                 int box_cols, bool swizzle);  // tc_fused.cu
 
 namespace {
 
-constexpr int kThreads = 384;
-constexpr int kMaxStages = 6;      // of either ring
-constexpr int kBars = 4 * kMaxStages + 8;
-constexpr int kBarBytes = 8 * kBars + 16;
+constexpr int kGroups = 2;         // warps that share a quarter of tensor memory: keys and output columns are split between them
+constexpr int kThreads = 128 + 128 * kGroups;
+constexpr int kMaxTiles = 4;       // tiles at a time: in shared memory and, as scores, in tensor memory
+constexpr int kBars = 4 * kMaxTiles + 4;
+constexpr int kBarBytes = 8 * kBars + 8;
+constexpr int kExpBytes = kGroups * 128;  // exponents of the parts of a band's rows of q
 constexpr int kBudget = (227 * 1024 - 1024 - kBarBytes) & ~1023;
+constexpr int kRing = kBudget - ((kExpBytes + 1023) & ~1023);  // for the rings and q
+
+constexpr int kTail = 11;      // tails are stored 2^11 times as large: their exponents are then those of the heads
+constexpr int kRowExp = 3;     // rows of q and k are scaled to a largest magnitude in [2^3, 2^4): scores stay below 2^15
+constexpr int kTileExp = 14;   // a tile of v to [2^14, 2^15)
+constexpr int kSpread = 28;    // a key's or a column's largest magnitude this far (in powers of two) below the tile's
+constexpr int kOdd = 1 << 20;  // added to the exponent of a tile that has to be summed position by position
 
 struct AttnParams {
   int heads, m, n, d, dv;
-  int parts, dvt;                // a head's columns of v in parts of DVP (wide heads: two), dvt = parts * DVP
-  int bands, tiles, mp;          // 128-row bands, key tiles per band, rows of the mask words
-  int np;                        // row length of the transposed v planes
-  int total;                     // heads * parts * bands * tiles
-  int k_stages, v_stages;
+  int bands, tiles, mp;          // 128-row bands, key tiles of a head, rows of the mask words
+  int np, words;                 // keys of a head in the planes (whole tiles), mask words of a row
+  int total;                     // heads * bands * tiles
   const uint32_t* bits;          // [key words][mp]
   const float* q;
   const float* k;
@@ -74,9 +88,8 @@ struct AttnParams {
   const int* row_offsets;
   const int* cols;
   float4* partials;              // [2 * CTAs][dvp / 4][128]: sums of a CTA's first and last band where they are cut
-  int* counters;                 // [bands of all heads and parts][8]: pieces of a band that are there, per warp
-  const int* flags;              // [heads][flag_blocks]: values of v that are not finite
-  int flag_blocks;
+  int* counters;                 // [bands of all heads][4 * kGroups]: pieces of a band that are there, per warp
+  const int* exponents;          // [heads][tiles]: v's rows times k's scales are stored times 2^-this (+ kOdd)
   int* status;
 };
 
@@ -89,17 +102,67 @@ __device__ __forceinline__ int cta_of(int t, int total, int ctas) {
   return static_cast<int>(((t + 1ll) * ctas - 1) / total);
 }
 
-// TF32 head of x, rounded half away from zero, by integer arithmetic on the sign-magnitude bits.
-__device__ __forceinline__ uint32_t tf32_head(uint32_t x) { return (x + 0x1000u) & 0xffffe000u; }
+// floor(log2 |x|) from the bits of |x| (not 0, finite)
+__device__ __forceinline__ int exponent_of(uint32_t bits) {
+  return bits >= 0x00800000u ? static_cast<int>(bits >> 23) - 127 : -118 - __clz(bits);
+}
+// 2^e; 0 below the smallest subnormal, 2^127 above it
+__device__ __forceinline__ float power_of_two(int e) {
+  if (e >= -126) return __uint_as_float(static_cast<uint32_t>(min(e, 127) + 127) << 23);
+  return e < -149 ? 0.f : __uint_as_float(1u << (149 + e));
+}
+// x * 2^e, in two steps since 2^e alone may be out of range
+struct Scale {
+  float a, b;
+  __device__ __forceinline__ explicit Scale(int e) {
+    e = max(-250, min(250, e));
+    a = power_of_two(e >> 1);
+    b = power_of_two(e - (e >> 1));
+  }
+  __device__ __forceinline__ float operator()(float x) const { return x * a * b; }
+};
+// The largest |x| of the finite ones, as bits
+__device__ __forceinline__ uint32_t finite_max(uint32_t so_far, float x) {
+  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+  return b < 0x7f800000u ? max(so_far, b) : so_far;
+}
+// Two numbers as fp16 heads and tails, the tails times 2^11
+__device__ __forceinline__ void split2(float2 x, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x.x, x.y);
+  constexpr float kUp = static_cast<float>(1 << kTail);
+  float2 t = __fmul2_rn(x, make_float2(kUp, kUp));
+  // x * 2^11 - h * 2^11 straight from the fp16 numbers
+  asm("{\n\t.reg .b16 a, b, c;\n\tmov.b32 {a, b}, %2;\n\tmov.b16 c, %3;\n\t"
+      "fma.rn.f32.f16 %0, a, c, %0;\n\tfma.rn.f32.f16 %1, b, c, %1;\n\t}"
+      : "+f"(t.x), "+f"(t.y)
+      : "r"(*reinterpret_cast<const uint32_t*>(&h)), "n"(0xe800));  // -2^11
+  const __half2 l = __floats2half2_rn(t.x, t.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
 
-__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// D = A B + D * 2^-kTail
+__device__ __forceinline__ void umma_f16_ts_scaled(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "n"(kTail)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
@@ -108,6 +171,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
       "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -121,7 +190,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Rows [row0, row0 + 32) of one head, position by position (a warp; see the note on values that are not finite).
+// Rows [row0, row0 + 32) of one head, position by position (a warp; for tiles that do not suit the planes).
 __device__ __noinline__ void rows_by_position(const AttnParams& p, int head, int row0, int lane) {
   const float* q = p.q + static_cast<size_t>(head) * p.m * p.d;
   const float* k = p.k + static_cast<size_t>(head) * p.n * p.d;
@@ -141,44 +210,56 @@ __device__ __noinline__ void rows_by_position(const AttnParams& p, int head, int
   }
 }
 
-// kDA: 32-float atoms of d (rounded up); KT: keys per tile; kOut: 16-float pieces of dv (rounded up)
-template <int kDA, int KT, int kOut>
+// kQ: columns of q and k (d rounded up to 64 or 128), KT: keys per tile, DVP: columns of v (dv rounded up)
+template <int kQ, int KT, int DVP>
+struct Layout {
+  static constexpr int kKAtoms = kQ / 64, kVAtoms = (DVP + 63) / 64;  // 64 fp16 numbers: one 128-byte swizzle atom
+  static constexpr int kKPlane = KT * 128 * kKAtoms, kVPlane = KT * 128 * kVAtoms;
+  static constexpr int kQBytes = kQ / 32 * 16384;
+  static constexpr int kTensor = (512 - kQ - 2 * DVP) / KT, kShared = (kRing - kQBytes) / (2 * (kKPlane + kVPlane));
+  static constexpr int kFit = kTensor < kShared ? kTensor : kShared, kTiles = kFit < kMaxTiles ? kFit : kMaxTiles;
+  static_assert(kTiles >= 2, "two tiles at a time");
+};
+
+template <int kQ, int KT, int DVP>
 __global__ void __launch_bounds__(kThreads, 1)
-attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
-  constexpr int DP = kDA * 32, DVP = kOut * 16;
-  constexpr uint32_t kQHi = 0, kQLo = DP, kS = 2 * DP, kO = 2 * DP + 4 * KT;
-  static_assert(2 * DP + 4 * KT + 2 * DVP <= 512, "tensor memory");
-  constexpr uint32_t kKPlane = KT * DP * 4, kVPlane = KT * DVP * 4;
+attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                 const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
+  using L = Layout<kQ, KT, DVP>;
+  constexpr int kKAtoms = L::kKAtoms, kVAtoms = L::kVAtoms, kTiles = L::kTiles;
+  constexpr uint32_t kKPlane = L::kKPlane, kVPlane = L::kVPlane;
+  constexpr uint32_t kQHi = 0, kQLo = kQ / 2, kS = kQ, kO = kQ + kTiles * KT;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar = base + kBudget;
-  auto k_full = [&](int s) { return bar + 8u * s; };
-  auto k_empty = [&](int s) { return bar + 8u * (kMaxStages + s); };
-  auto v_full = [&](int s) { return bar + 8u * (2 * kMaxStages + s); };
-  auto v_empty = [&](int s) { return bar + 8u * (3 * kMaxStages + s); };
-  const uint32_t v_base = base + p.k_stages * 2u * kKPlane;
-  constexpr uint32_t kB0 = 32u * kMaxStages;
-  auto s_full = [&](int b) { return bar + kB0 + 8u * b; };
-  auto p_full = [&](int b) { return bar + kB0 + 16u + 8u * b; };
-  auto pv_done = [&](int b) { return bar + kB0 + 32u + 8u * b; };
-  const uint32_t q_full = bar + kB0 + 48u, seg_done = bar + kB0 + 56u;
+  // Of tile t, with b = t % kTiles: K(t) is there and P(t - kTiles) used up; S(t); P(t) and V(t) are there; O(t)
+  auto k_full = [&](int b) { return bar + 8u * b; };
+  auto s_full = [&](int b) { return bar + 8u * (kMaxTiles + b); };
+  auto p_full = [&](int b) { return bar + 8u * (2 * kMaxTiles + b); };
+  auto pv_done = [&](int b) { return bar + 8u * (3 * kMaxTiles + b); };
+  const uint32_t v_base = base + kTiles * 2u * kKPlane, q_base = v_base + kTiles * 2u * kVPlane;
+  constexpr uint32_t kB1 = 32u * kMaxTiles;
+  const uint32_t q_full = bar + kB1, raw_full = bar + kB1 + 8u, raw_empty = bar + kB1 + 16u, exps_there = bar + kB1 + 24u;
   volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kBudget + 8 * kBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 4 * kMaxStages; ++s) mbar_init(bar + 8u * s, 1);
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kMaxTiles; ++b) {
+      mbar_init(k_full(b), 2);
       mbar_init(s_full(b), 1);
-      mbar_init(p_full(b), 8);
+      mbar_init(p_full(b), 4 * kGroups + 1);
       mbar_init(pv_done(b), 1);
     }
-    mbar_init(q_full, 8);
-    mbar_init(seg_done, 1);
+    mbar_init(q_full, 4 * kGroups);
+    mbar_init(raw_full, 1);
+    mbar_init(raw_empty, 4 * kGroups);
+    mbar_init(exps_there, 4 * kGroups);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int b = 0; b < kTiles; ++b) mbar_arrive(k_full(b));  // nothing to use up before the first tiles
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bar + 8u * kBars), "r"(512u)
@@ -197,30 +278,38 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
-      int sk = 0, sv = 0;
-      uint32_t phk = 0, phv = 0;
+      int b = 0;
+      uint32_t ph = 0, seg = 0;
+      const int q_atoms = (p.d + 31) / 32;
       for (int r = r0; r < r1; ++r) {
-        const int item = r / p.tiles, t = r - item * p.tiles, unit = item / p.bands, head = unit / p.parts;
-        if (!mbar_wait(k_empty(sk), phk ^ 1u, abort_flag, p.status, 32)) break;
-        mbar_arrive_expect_tx(k_full(sk), 2 * kKPlane);
+        const int item = r / p.tiles, t = r - item * p.tiles, head = item / p.bands;
+        if (r == r0 || t == 0) {  // the band's rows of q as they are
+          if (!mbar_wait(raw_empty, (seg & 1u) ^ 1u, abort_flag, p.status, 32)) break;
+          mbar_arrive_expect_tx(raw_full, q_atoms * 16384u);
+          for (int a = 0; a < q_atoms; ++a)
+            tma_load_2d(q_base + a * 16384u, &map_q, raw_full, a * 32, head * p.m + (item - head * p.bands) * 128);
+          ++seg;
+        }
+        if (!mbar_wait(s_full(b), ph ^ 1u, abort_flag, p.status, 32)) break;
+        mbar_arrive_expect_tx(k_full(b), 2 * kKPlane);
 #pragma unroll
         for (int pl = 0; pl < 2; ++pl)
 #pragma unroll
-          for (int a = 0; a < kDA; ++a)
-            tma_load_2d(base + (2 * sk + pl) * kKPlane + a * (KT * 128), &map_k, k_full(sk), a * 32,
-                        (pl * p.heads + head) * p.n + t * KT);
-        if (!mbar_wait(v_empty(sv), phv ^ 1u, abort_flag, p.status, 32)) break;
-        mbar_arrive_expect_tx(v_full(sv), 2 * kVPlane);
+          for (int a = 0; a < kKAtoms; ++a)
+            tma_load_2d(base + (2 * b + pl) * kKPlane + a * (KT * 128), &map_k, k_full(b), a * 64,
+                        (pl * p.heads + head) * p.np + t * KT);
+        if (!mbar_wait(pv_done(b), ph ^ 1u, abort_flag, p.status, 32)) break;
+        mbar_arrive_expect_tx(p_full(b), 2 * kVPlane);
 #pragma unroll
         for (int pl = 0; pl < 2; ++pl)
 #pragma unroll
-          for (int a = 0; a < KT / 32; ++a)
-            tma_load_2d(v_base + (2 * sv + pl) * kVPlane + a * (DVP * 128), &map_v, v_full(sv), t * KT + a * 32,
-                        pl * p.heads * p.dvt + unit * DVP);
-        if (++sk == p.k_stages) { sk = 0; phk ^= 1u; }
-        if (++sv == p.v_stages) { sv = 0; phv ^= 1u; }
+          for (int a = 0; a < kVAtoms; ++a)
+            tma_load_2d(v_base + (2 * b + pl) * kVPlane + a * (KT * 128), &map_v, p_full(b), a * 64,
+                        (pl * p.heads + head) * p.np + t * KT);
+        if (++b == kTiles) { b = 0; ph ^= 1u; }
       }
       if (*abort_flag)
         for (uint32_t i = 0; i < 2048u; ++i) __nanosleep(100);
@@ -229,33 +318,34 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------------------------------------------ S = Q K^T
     if (elect_one()) {
-      constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(KT >> 3) << 17) | (8u << 24);
-      int st = 0;
+      constexpr uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(KT >> 3) << 17) | (8u << 24);
+      const int steps = (p.d + 15) / 16;
+      int b = 0;
       uint32_t ph = 0, seg = 0;
       bool ok = true;
       for (int r = r0; r < r1 && ok; ++seg) {
         const int seg_end = min(r1, (r / p.tiles + 1) * p.tiles);
         if (!mbar_wait(q_full, seg & 1u, abort_flag, p.status, 20)) break;
         for (; r < seg_end; ++r) {
-          const int g = r - r0, b = g & 1;
-          if (!mbar_wait(k_full(st), ph, abort_flag, p.status, 20) ||
-              !mbar_wait(pv_done(b), ((g >> 1) & 1u) ^ 1u, abort_flag, p.status, 20)) { ok = false; break; }
+          if (!mbar_wait(k_full(b), ph, abort_flag, p.status, 20)) { ok = false; break; }
           tcgen05_fence_after();
-          const uint32_t k_hi = base + 2 * st * kKPlane, d = tmem + kS + b * 2 * KT;
-          // small terms first: lo * hi', hi * lo', then hi * hi'
+          const uint32_t k_hi = base + 2 * b * kKPlane, d = tmem + kS + b * KT;
+          // small terms first: tail * head', head * tail', then, with those scaled back, head * head'
 #pragma unroll
           for (int pr = 0; pr < 3; ++pr)
 #pragma unroll
-            for (int a = 0; a < kDA; ++a) {
+            for (int a = 0; a < kKAtoms; ++a) {
               const uint64_t bd = smem_desc(k_hi + (pr == 1 ? kKPlane : 0u) + a * (KT * 128), 16, 1024);
 #pragma unroll
-              for (int ks = 0; ks < 4; ++ks)
-                umma_tf32_ts(d, tmem + (pr == 0 ? kQLo : kQHi) + a * 32 + ks * 8, desc_advance(bd, ks * 32), idesc,
-                             (pr | a | ks) != 0 ? 1u : 0u);
+              for (int ks = 0; ks < 4; ++ks) {
+                if (a * 4 + ks >= steps) continue;
+                const uint32_t qa = tmem + (pr == 0 ? kQLo : kQHi) + a * 32 + ks * 8;
+                if (pr == 2 && a == 0 && ks == 0) umma_f16_ts_scaled(d, qa, bd, idesc);
+                else umma_f16_ts(d, qa, desc_advance(bd, ks * 32), idesc, (pr | a | ks) != 0 ? 1u : 0u);
+              }
             }
           umma_commit(s_full(b));
-          umma_commit(k_empty(st));
-          if (++st == p.k_stages) { st = 0; ph ^= 1u; }
+          if (++b == kTiles) { b = 0; ph ^= 1u; }
         }
       }
     }
@@ -263,142 +353,176 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   } else if (warp == 2) {
     // ------------------------------------------------------------------ O = P V
     if (elect_one()) {
-      constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(DVP >> 3) << 17) | (8u << 24);
-      int st = 0;
+      const uint32_t idesc = (1u << 4) | (1u << 16) | (static_cast<uint32_t>((p.dv + 15) / 16 * 2) << 17) | (8u << 24);
+      int b = 0;
       uint32_t ph = 0;
       for (int r = r0; r < r1; ++r) {
-        const int g = r - r0, b = g & 1;
         // P(g) also says that O(g - 2) has been read: every warp adds it before it writes P(g)
-        if (!mbar_wait(v_full(st), ph, abort_flag, p.status, 20) ||
-            !mbar_wait(p_full(b), (g >> 1) & 1u, abort_flag, p.status, 20)) break;
+        if (!mbar_wait(p_full(b), ph, abort_flag, p.status, 20)) break;
         tcgen05_fence_after();
-        const uint32_t v_hi = v_base + 2 * st * kVPlane, d = tmem + kO + b * DVP, pp = tmem + kS + b * 2 * KT;
+        const uint32_t v_hi = v_base + 2 * b * kVPlane, d = tmem + kO + ((r - r0) & 1) * DVP, pp = tmem + kS + b * KT;
 #pragma unroll
-        for (int pr = 0; pr < 3; ++pr)
+        for (int pr = 0; pr < 3; ++pr) {
+          const uint64_t bd = smem_desc(v_hi + (pr == 1 ? kVPlane : 0u), KT * 128, 1024);
 #pragma unroll
-          for (int a = 0; a < KT / 32; ++a) {
-            const uint64_t bd = smem_desc(v_hi + (pr == 1 ? kVPlane : 0u) + a * (DVP * 128), 16, 1024);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              umma_tf32_ts(d, pp + (pr == 0 ? KT : 0) + a * 32 + ks * 8, desc_advance(bd, ks * 32), idesc,
-                           (pr | a | ks) != 0 ? 1u : 0u);
+          for (int ks = 0; ks < KT / 16; ++ks) {  // 16 keys of P: 8 columns of heads, 8 of tails
+            const uint32_t pa = pp + ks * 16 + (pr == 0 ? 8 : 0);
+            if (pr == 2 && ks == 0) umma_f16_ts_scaled(d, pa, bd, idesc);
+            else umma_f16_ts(d, pa, desc_advance(bd, ks * (16 * 128)), idesc, (pr | ks) != 0 ? 1u : 0u);
           }
+        }
         umma_commit(pv_done(b));
-        umma_commit(v_empty(st));
-        if (r + 1 == r1 || (r + 1) % p.tiles == 0) umma_commit(seg_done);  // a band's last tile
-        if (++st == p.v_stages) { st = 0; ph ^= 1u; }
+        if (r + kTiles < r1) umma_commit(k_full(b));
+        if (++b == kTiles) { b = 0; ph ^= 1u; }
       }
     }
     __syncwarp();
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ mask and sums
-    const int wg = warp >= 8 ? 1 : 0, q4 = warp & 3;
+    const int wg = (warp >> 2) - 1, q4 = warp & 3;
     const uint32_t lanes = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
     const int row_local = q4 * 32 + lane;
-    bool ok = true;
-    uint32_t seg = 0;
+    // This warp group's share of a band's q columns into tensor memory; the band's sums are those of O times 2^row_exp, and the
+    // tile's exponent.
+    const uint8_t* q_ptr = base_ptr + (q_base - base);
+    volatile uint8_t* exp_ptr = base_ptr + kRing;
+    auto put_q = [&](uint32_t seg, int& row_exp) -> bool {
+      constexpr int kShare = kQ / kGroups;
+      if (!mbar_wait(raw_full, seg & 1u, abort_flag, p.status, 20)) return false;
+      float4 x[kShare / 4];
+      uint32_t top = 0;
+#pragma unroll
+      for (int j = 0; j < kShare / 4; ++j) {
+        const int c = wg * kShare + 4 * j;  // 128-byte swizzle; whole 32-column atoms are there
+        x[j] = *reinterpret_cast<const float4*>(q_ptr + (c >> 5) * 16384 + row_local * 128 + ((((c >> 2) & 7) ^ (row_local & 7)) << 4));
+        if (c >= p.d) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        top = finite_max(finite_max(finite_max(finite_max(top, x[j].x), x[j].y), x[j].z), x[j].w);
+      }
+      exp_ptr[wg * 128 + row_local] = static_cast<uint8_t>(top >> 23);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(exps_there);
+      if (!mbar_wait(exps_there, seg & 1u, abort_flag, p.status, 20)) return false;
+      int e = 0;
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) e = max(e, static_cast<int>(exp_ptr[i * 128 + row_local]));
+      e = max(e, 1) - 127;  // of the whole row; of subnormal ones as of 2^-126
+      const Scale scale(kRowExp - e);
+      row_exp = e - 2 * kRowExp;
+#pragma unroll
+      for (int h = 0; h < kShare / 16; ++h) {
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 f = x[4 * h + j];
+          split2(make_float2(scale(f.x), scale(f.y)), hi[2 * j], lo[2 * j]);
+          split2(make_float2(scale(f.z), scale(f.w)), hi[2 * j + 1], lo[2 * j + 1]);
+        }
+        tmem_st8(lanes + kQHi + wg * (kShare / 2) + h * 8, hi);
+        tmem_st8(lanes + kQLo + wg * (kShare / 2) + h * 8, lo);
+      }
+      tmem_wait_st();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(q_full);
+        mbar_arrive(raw_empty);
+      }
+      return true;
+    };
+    int row_exp = 0, row_exp_next = 0;
+    bool ok = r0 >= r1 || put_q(0, row_exp_next);
+    uint32_t seg = 0, ph_b = 0, ph_add = 0;  // of the score tile that is next, and of the one whose O is
+    int b = 0, b_add = 0;
     for (int r = r0; r < r1 && ok; ++seg) {
-      const int item = r / p.tiles, unit = item / p.bands, band = item - unit * p.bands;
-      const int head = unit / p.parts, col0 = (unit - head * p.parts) * DVP;
+      const int item = r / p.tiles, head = item / p.bands, band = item - head * p.bands;
       const int t_begin = r - item * p.tiles;
       const int seg_end = min(r1, (item + 1) * p.tiles);
       const int row = band * 128 + row_local;
-      {  // this warp group's half of the band's q columns into tensor memory
-        constexpr int kHalf = DP / 2;
-        const float* src = p.q + (static_cast<size_t>(head) * p.m + row) * p.d + wg * kHalf;
-        uint32_t x[kHalf];
+      row_exp = row_exp_next;
+      // this warp group's share of a tile's keys and of the output columns
+      constexpr int kKeys = KT / kGroups, kCols = DVP / kGroups, kWords = (kKeys + 31) / 32;
+      float2 acc2[kCols / 2];
 #pragma unroll
-        for (int j = 0; j < kHalf / 4; ++j) {
-          float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (row < p.m && wg * kHalf + 4 * j < p.d) f = __ldg(reinterpret_cast<const float4*>(src) + j);
-          x[4 * j] = __float_as_uint(f.x);
-          x[4 * j + 1] = __float_as_uint(f.y);
-          x[4 * j + 2] = __float_as_uint(f.z);
-          x[4 * j + 3] = __float_as_uint(f.w);
-        }
-        // the tensor core is done with the previous band (all its tiles, both groups')
-        if (seg > 0 && !mbar_wait(seg_done, (seg - 1u) & 1u, abort_flag, p.status, 32)) { ok = false; break; }
+      for (int j = 0; j < kCols / 2; ++j) acc2[j] = make_float2(0.f, 0.f);
+      auto add_tile = [&](int g, int e) -> bool {  // O of tile g, whose v has the exponent e
+        if (!mbar_wait(pv_done(b_add), ph_add, abort_flag, p.status, 20)) return false;
+        if (++b_add == kTiles) { b_add = 0; ph_add ^= 1u; }
         __syncwarp();
         tcgen05_fence_after();
-#pragma unroll
-        for (int h = 0; h < kHalf / 16; ++h) {
-          uint32_t hi[16], lo[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            hi[j] = tf32_head(x[16 * h + j]);
-            lo[j] = __float_as_uint(__uint_as_float(x[16 * h + j]) - __uint_as_float(hi[j]));
-          }
-          tmem_st16(lanes + kQHi + wg * kHalf + h * 16, hi);
-          tmem_st16(lanes + kQLo + wg * kHalf + h * 16, lo);
-        }
-        tmem_wait_st();
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(q_full);
-      }
-      // this warp group's half of a tile's keys and of the output columns
-      constexpr int kKeys = KT / 2, kCols = DVP / 2;
-      float acc[kCols];
-#pragma unroll
-      for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
-      auto add_tile = [&](int g) -> bool {  // O of tile g
-        const int b = g & 1;
-        if (!mbar_wait(pv_done(b), (g >> 1) & 1u, abort_flag, p.status, 20)) return false;
-        __syncwarp();
-        tcgen05_fence_after();
+        const float f = power_of_two(row_exp + e);
         uint32_t o[kCols];
 #pragma unroll
-        for (int h = 0; h < kCols / 16; ++h) tmem_ld16(lanes + kO + b * DVP + wg * kCols + h * 16, &o[16 * h]);
+        for (int h = 0; h < kCols / 8; ++h) tmem_ld8(lanes + kO + (g & 1) * DVP + wg * kCols + h * 8, &o[8 * h]);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < kCols; ++j) acc[j] += __uint_as_float(o[j]);
+        for (int j = 0; j < kCols / 2; ++j)
+          acc2[j] = ffma2(make_float2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])), make_float2(f, f), acc2[j]);
         tcgen05_fence_before();
         return true;
       };
       const int tiles_here = seg_end - r, g0 = r - r0;
-      // the row's mask bits of this half of a tile: a word, or half of one
-      const uint32_t* bits = p.bits + static_cast<size_t>(t_begin) * (KT / 32) * p.mp + (KT == 64 ? wg * p.mp : 0) + band * 128 + row_local;
-      auto mask_of = [&](int t) -> uint32_t {
-        const uint32_t w = t < tiles_here ? __ldg(bits + static_cast<size_t>(t) * (KT / 32) * p.mp) : 0u;
-        return KT == 64 ? w : w >> (wg * 16);
+      // the row's mask bits of this share of a tile
+      const uint32_t* bits = p.bits + band * 128 + row_local;
+      auto mask_of = [&](int t, int i) -> uint32_t {
+        const int key = (t_begin + t) * KT + wg * kKeys + 32 * i, word = key >> 5;
+        return t < tiles_here && word < p.words ? __ldg(bits + static_cast<size_t>(word) * p.mp) >> (key & 31) : 0u;
       };
-      uint32_t w = mask_of(0);
+      const int* exponents = p.exponents + head * p.tiles + t_begin;
+      uint32_t w[kWords];
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) w[i] = mask_of(0, i);
+      int e_before = 0, e_now = __ldg(exponents);
+      bool odd = false;
       for (int t = 0; t < tiles_here; ++t) {
-        const int g = g0 + t, b = g & 1;
-        const uint32_t next = mask_of(t + 1);
-        if (!mbar_wait(s_full(b), (g >> 1) & 1u, abort_flag, p.status, 20)) { ok = false; break; }
+        const int g = g0 + t;
+        uint32_t next[kWords];
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) next[i] = mask_of(t + 1, i);
+        const int e_next = __ldg(exponents + min(t + 1, tiles_here - 1));
+        if (!mbar_wait(s_full(b), ph_b, abort_flag, p.status, 20)) { ok = false; break; }
         __syncwarp();
         tcgen05_fence_after();
-        const uint32_t s_addr = lanes + kS + b * 2 * KT + wg * kKeys;
+        const uint32_t s_addr = lanes + kS + b * KT + wg * kKeys;
         uint32_t x[kKeys];
 #pragma unroll
         for (int h = 0; h < kKeys / 16; ++h) tmem_ld16(s_addr + h * 16, &x[16 * h]);
         tmem_wait_ld();
 #pragma unroll
-        for (int h = 0; h < kKeys / 16; ++h) {
-          uint32_t hi[16], lo[16];
+        for (int h = 0; h < kKeys / 16; ++h) {  // over 16 columns of S: 8 of heads, 8 of tails
+          uint32_t r[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const uint32_t v = (w & (1u << (16 * h + j))) ? x[16 * h + j] : 0u;
-            hi[j] = tf32_head(v);
-            lo[j] = __float_as_uint(__uint_as_float(v) - __uint_as_float(hi[j]));
+          for (int j = 0; j < 8; ++j) {
+            const int c = 16 * h + 2 * j;
+            const uint32_t bit = 1u << (c & 31);
+            const float a0 = (w[h / 2] & bit) ? __uint_as_float(x[c]) : 0.f;
+            const float a1 = (w[h / 2] & (2 * bit)) ? __uint_as_float(x[c + 1]) : 0.f;
+            split2(make_float2(a0, a1), r[j], r[8 + j]);
           }
-          tmem_st16(s_addr + h * 16, hi);
-          tmem_st16(s_addr + KT + h * 16, lo);
+          tmem_st16(s_addr + h * 16, r);
         }
         tmem_wait_st();
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full(b));
-        if (t > 0 && !add_tile(g - 1)) { ok = false; break; }
-        w = next;
+        if (++b == kTiles) { b = 0; ph_b ^= 1u; }
+        // q has been read when the band's last S is there: the next band's goes in under the last PV
+        if (t + 1 == tiles_here && seg_end < r1 && !put_q(seg + 1, row_exp_next)) { ok = false; break; }
+        if (t > 0 && !add_tile(g - 1, e_before)) { ok = false; break; }
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] = next[i];
+        odd = odd || e_now >= kOdd / 2;
+        e_before = e_now;
+        e_now = e_next;
       }
-      if (!ok || !add_tile(g0 + tiles_here - 1)) { ok = false; break; }
-      bool finite = true;
-      for (int i = lane; i < p.flag_blocks; i += 32) finite = finite && __ldg(p.flags + head * p.flag_blocks + i) == 0;
-      finite = __all_sync(0xffffffffu, finite);
-      bool write = finite;
-      if (finite && tiles_here != p.tiles) {
+      if (!ok || !add_tile(g0 + tiles_here - 1, e_before)) { ok = false; break; }
+      float acc[kCols];
+#pragma unroll
+      for (int j = 0; j < kCols / 2; ++j) {
+        acc[2 * j] = acc2[j].x;
+        acc[2 * j + 1] = acc2[j].y;
+      }
+      bool write = true;
+      if (tiles_here != p.tiles) {
         // A band cut between CTAs: this piece goes to the workspace, and the warp that finds all the others there adds them
         // up in the order of the keys.
         constexpr int kQuads = kCols / 4;
@@ -412,9 +536,11 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         __threadfence();
         __syncwarp();
         int there = 0;
-        if (lane == 0) there = atomicAdd(p.counters + item * 8 + wg * 4 + q4, 1);
-        write = __shfl_sync(0xffffffffu, there, 0) == last - first;
-        if (write) {
+        if (lane == 0) there = atomicAdd(p.counters + item * 4 * kGroups + wg * 4 + q4, odd ? 0x10001 : 1);
+        there = __shfl_sync(0xffffffffu, there, 0);
+        write = (there & 0xffff) == last - first;
+        odd = odd || there > 0xffff;
+        if (write && !odd) {
           __threadfence();
 #pragma unroll
           for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
@@ -434,14 +560,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
           }
         }
       }
-      if (write && row < p.m) {
-        float* dst = p.out + (static_cast<size_t>(head) * p.m + row) * p.dv + col0 + wg * kCols;
+      if (write && !odd && row < p.m) {
+        float* dst = p.out + (static_cast<size_t>(head) * p.m + row) * p.dv + wg * kCols;
 #pragma unroll
         for (int j = 0; j < kCols / 4; ++j)
-          if (col0 + wg * kCols + 4 * j < p.dv)
+          if (wg * kCols + 4 * j < p.dv)
             reinterpret_cast<float4*>(dst)[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
       }
-      if (!finite && t_begin == 0 && wg == 0 && col0 == 0) rows_by_position(p, head, band * 128 + q4 * 32, lane);
+      if (write && odd && wg == 0) rows_by_position(p, head, band * 128 + q4 * 32, lane);
       r = seg_end;
     }
   }
@@ -453,59 +579,115 @@ attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   }
 }
 
-constexpr int kPrepKeys = 64;
-
-// Block (x, h): keys [64 x, +64) of head h as hi / lo planes.  k planes [2][heads * n][dp], v planes transposed,
-// [2][heads * dvt][np].  The blocks of the last y zero the main kernel's counters.
+// Block (x, h): key tile x of head h as head / tail planes, [2][heads * np][dk] and [2][heads * np][dvk], zeros past n, d and
+// dv.  16 threads a row, everything read once and kept in registers.  A row of k is scaled to a largest magnitude in
+// [2^kRowExp, 2^(kRowExp + 1)); v takes the factor that k's row lost, and the tile's rows of v together another (exponents).
+// Tiles where that leaves a key or a column of v too few bits, or that have values of v that are not finite, are marked.
+// The blocks of the last y zero the main kernel's counters.
+template <int kVecs, int KT>
 __global__ void __launch_bounds__(256)
-attention_prepare_kernel(const AttnParams p, int dp, float* __restrict__ k_planes, float* __restrict__ v_planes,
-                         int* __restrict__ flags) {
-  extern __shared__ float v_tile[];  // [64][dv + 1]
+attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict__ k_planes, __half* __restrict__ v_planes,
+                         int* __restrict__ exponents) {
+  constexpr int kRows = KT / 16, kNone = -100000;
+  __shared__ int top_exp, low_exp;
+  __shared__ uint32_t column_top[64 * kVecs];
+  if (threadIdx.x == 0) { top_exp = kNone; low_exp = -kNone; }
+  for (int i = threadIdx.x; i < 64 * kVecs; i += 256) column_top[i] = 0;
   grid_dependency_wait();
   grid_launch_dependents();
   if (static_cast<int>(blockIdx.y) == p.heads) {
-    const int counters = p.heads * p.parts * p.bands * 8;
+    const int counters = p.heads * p.bands * 4 * kGroups;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < counters; i += gridDim.x * 256) p.counters[i] = 0;
     return;
   }
-  const int head = blockIdx.y, key0 = blockIdx.x * kPrepKeys;
-  const int keys = min(kPrepKeys, p.n - key0);  // may be <= 0 in the padding of the v planes
-  const float* k = p.k + (static_cast<size_t>(head) * p.n + key0) * p.d;
-  const float* v = p.v + (static_cast<size_t>(head) * p.n + key0) * p.dv;
-  const size_t k_plane = static_cast<size_t>(p.heads) * p.n * dp;
-  float* kd = k_planes + (static_cast<size_t>(head) * p.n + key0) * dp;
-  const int d4 = dp / 4;
-  for (int i = threadIdx.x; i < keys * d4; i += 256) {
-    const int r = i / d4, c = (i - r * d4) * 4;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), lo;
-    if (c < p.d) x = __ldg(reinterpret_cast<const float4*>(k + static_cast<size_t>(r) * p.d + c));
-    float4 hi = make_float4(__uint_as_float(tf32_head(__float_as_uint(x.x))), __uint_as_float(tf32_head(__float_as_uint(x.y))),
-                            __uint_as_float(tf32_head(__float_as_uint(x.z))), __uint_as_float(tf32_head(__float_as_uint(x.w))));
-    lo = make_float4(x.x - hi.x, x.y - hi.y, x.z - hi.z, x.w - hi.w);
-    reinterpret_cast<float4*>(kd)[i] = hi;
-    reinterpret_cast<float4*>(kd + k_plane)[i] = lo;
+  const int head = blockIdx.y, key0 = blockIdx.x * KT, group = threadIdx.x >> 4, lane16 = threadIdx.x & 15;
+  const float* k = p.k + static_cast<size_t>(head) * p.n * p.d;
+  const float* v = p.v + static_cast<size_t>(head) * p.n * p.dv;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 xk[kRows][kVecs], xv[kRows][kVecs];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int key = key0 + group + 16 * i;
+#pragma unroll
+    for (int j = 0; j < kVecs; ++j) {
+      const int c = (lane16 + 16 * j) * 4;
+      xk[i][j] = key < p.n && c < p.d ? __ldg(reinterpret_cast<const float4*>(k + static_cast<size_t>(key) * p.d + c)) : zero;
+      xv[i][j] = key < p.n && c < p.dv ? __ldg(reinterpret_cast<const float4*>(v + static_cast<size_t>(key) * p.dv + c)) : zero;
+    }
   }
-  bool odd = false;  // a value whose head or product is not finite
-  const int pitch = p.dv + 1;
-  for (int i = threadIdx.x; i < keys * p.dv; i += 256) {
-    const float x = __ldg(v + i);
-    odd = odd || !(fabsf(x) < 1.7e38f);
-    const int r = i / p.dv;
-    v_tile[r * pitch + (i - r * p.dv)] = x;
+  __syncthreads();
+  int ek[kRows], top = kNone, low = -kNone;
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    uint32_t bk = 0, bv = 0;
+#pragma unroll
+    for (int j = 0; j < kVecs; ++j) {
+      const float4 a = xk[i][j], b = xv[i][j];
+      bk = finite_max(finite_max(finite_max(finite_max(bk, a.x), a.y), a.z), a.w);
+      bv = finite_max(finite_max(finite_max(finite_max(bv, b.x), b.y), b.z), b.w);
+      odd = odd || !(isfinite(b.x) && isfinite(b.y) && isfinite(b.z) && isfinite(b.w));
+    }
+#pragma unroll
+    for (int s = 8; s >= 1; s >>= 1) {
+      bk = max(bk, __shfl_xor_sync(0xffffffffu, bk, s));
+      bv = max(bv, __shfl_xor_sync(0xffffffffu, bv, s));
+    }
+    ek[i] = bk != 0u ? exponent_of(bk) : kNone;
+    if (bk != 0u && bv != 0u) {
+      const int e = ek[i] + exponent_of(bv);
+      top = max(top, e);
+      low = min(low, e);
+    }
   }
-  const int any = __syncthreads_or(odd ? 1 : 0);
-  if (threadIdx.x == 0) flags[head * gridDim.x + blockIdx.x] = any;
-  const size_t v_plane = static_cast<size_t>(p.heads) * p.dvt * p.np;
-  const int width = min(kPrepKeys, p.np - key0);
-  for (int i = threadIdx.x; i < p.dvt * kPrepKeys; i += 256) {
-    const int c = i / kPrepKeys, key = i % kPrepKeys;
-    if (key >= width) continue;
-    const float x = key < keys && c < p.dv ? v_tile[key * pitch + c] : 0.f;
-    const float hi = __uint_as_float(tf32_head(__float_as_uint(x)));
-    float* dst = v_planes + (static_cast<size_t>(head) * p.dvt + c) * p.np + key0 + key;
-    dst[0] = hi;
-    dst[v_plane] = x - hi;
+  if (lane16 == 0 && top != kNone) {
+    atomicMax(&top_exp, top);
+    atomicMin(&low_exp, low);
   }
+  __syncthreads();
+  const int exponent = top_exp == kNone ? 0 : top_exp - kTileExp;
+  odd = odd || top_exp - low_exp >= kSpread;
+  const size_t row0 = static_cast<size_t>(head) * p.np + key0, rows = static_cast<size_t>(p.heads) * p.np;
+  auto put = [&](__half* planes, int width, int row, int c, const float4& x) {
+    if (c >= width) return;
+    uint2 hi, lo;
+    split2(make_float2(x.x, x.y), hi.x, lo.x);
+    split2(make_float2(x.z, x.w), hi.y, lo.y);
+    __half* dst = planes + (row0 + row) * width + c;
+    *reinterpret_cast<uint2*>(dst) = hi;
+    *reinterpret_cast<uint2*>(dst + rows * width) = lo;
+  };
+#pragma unroll
+  for (int j = 0; j < kVecs; ++j) {
+    const int c = (lane16 + 16 * j) * 4;
+    uint32_t columns[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const Scale scale_k(kRowExp - ek[i]), scale_v(ek[i] - exponent);
+      const float4 a = xk[i][j], b = xv[i][j];
+      put(k_planes, dk, group + 16 * i, c, make_float4(scale_k(a.x), scale_k(a.y), scale_k(a.z), scale_k(a.w)));
+      const bool none = ek[i] == kNone;  // a row of k that is zero: nothing of v's counts
+      const float4 w = none ? zero : make_float4(scale_v(b.x), scale_v(b.y), scale_v(b.z), scale_v(b.w));
+      put(v_planes, dvk, group + 16 * i, c, w);
+      auto seen = [&](float scaled, float as_it_is) -> uint32_t {  // at least 1 where there is something
+        return max(__float_as_uint(fabsf(scaled)), as_it_is != 0.f && !none ? 1u : 0u);
+      };
+      columns[0] = max(columns[0], seen(w.x, b.x));
+      columns[1] = max(columns[1], seen(w.y, b.y));
+      columns[2] = max(columns[2], seen(w.z, b.z));
+      columns[3] = max(columns[3], seen(w.w, b.w));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      columns[i] = max(columns[i], __shfl_xor_sync(0xffffffffu, columns[i], 16));
+      if ((threadIdx.x & 16) == 0) atomicMax(&column_top[c + i], columns[i]);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 64 * kVecs; i += 256)
+    odd = odd || (column_top[i] != 0u && exponent_of(column_top[i]) <= kTileExp - kSpread);
+  odd = __syncthreads_or(odd ? 1 : 0) != 0;
+  if (threadIdx.x == 0) exponents[head * p.tiles + blockIdx.x] = exponent + (odd ? kOdd : 0);
 }
 
 // bits[column / 32][row]; a position stored twice (a sum in the operators' terms) sets *repeated.
@@ -522,28 +704,23 @@ attention_bits_kernel(int m, int mp, const int* __restrict__ row_offsets, const 
 }
 
 struct Shape {
-  int da, kt, dp, dvp, parts, dvt, np, mp;
+  int q, kt, dvp;      // the kernel's template arguments
+  int dk, dvk, np, mp;  // row lengths of the planes, keys of a head in them, rows of the mask words
+  int tiles;
 };
 
-// Tensor memory holds q's planes (2 dp columns), two score tiles with their tails (4 kt) and two output
-// tiles (2 dvp).
 bool attention_shape(int heads, int m, int n, int d, int dv, Shape* s) {
   if (heads < 1 || m < 1 || n < 1 || d < 4 || dv < 4 || d % 4 != 0 || dv % 4 != 0 || d > 128 || dv > 128) return false;
-  s->da = (d + 31) / 32;
-  s->dvp = dv <= 32 ? 32 : dv <= 64 ? 64 : 96;
-  s->parts = 1;
-  if (s->da == 4 || dv > 96) {  // wide heads: v in parts of 64 columns, scores formed for each
-    s->dvp = dv <= 32 ? 32 : 64;
-    s->parts = (dv + s->dvp - 1) / s->dvp;
-  }
-  if (s->dvp == 96 && s->da < 3) s->da = 3;
-  s->kt = s->da <= 2 ? 64 : 32;
-  s->dp = s->da * 32;
-  s->dvt = s->parts * s->dvp;
-  s->np = (n + 31) / 32 * 32;
+  s->q = d <= 64 ? 64 : 128;
+  s->dvp = (dv + 31) / 32 * 32;
+  s->kt = s->q == 64 && s->dvp <= 64 ? 128 : 64;
+  s->dk = (d + 15) / 16 * 16;
+  s->dvk = (dv + 15) / 16 * 16;
+  s->tiles = (n + s->kt - 1) / s->kt;
+  s->np = s->tiles * s->kt;
   s->mp = (m + 127) / 128 * 128;
-  const long long tiles = static_cast<long long>(heads) * s->parts * ((m + 127) / 128) * ((n + s->kt - 1) / s->kt);
-  return tiles < (1ll << 30) && 2ll * heads * n < (1ll << 30) && 2ll * heads * s->dvt < (1ll << 30) && heads <= 65000;
+  const long long tiles = static_cast<long long>(heads) * ((m + 127) / 128) * s->tiles;
+  return tiles < (1ll << 30) && 2ll * heads * s->np < (1ll << 30) && heads <= 65000;
 }
 
 // One CTA per SM with an equal share of the tiles; with fewer bands than SMs, as many equal pieces of every band as
@@ -554,19 +731,20 @@ int cta_count(int items, int tiles, int sms) {
   return items >= sms ? sms : items * std::min(pieces, sms / items);
 }
 
-// Times in microseconds, fitted on B200 to 578 measurements: 1 to 32 heads, 256 to 16384 rows and keys, 32 to 128 columns,
-// masks of 0.05 to 23 % stored positions, scattered or in a band.
+// Times in microseconds, fitted on B200 to 70 measurements: 1 to 32 heads, 256 to 16384 rows and keys, 32 to 128 columns;
+// within 18 %, launches of more than 100 us within 8 %.
 //
 // This kernel multiplies every tile, empty or not: m * n counts, not the positions.
 double one_launch_us(int heads, int m, int n, const Shape& s, int sms) {
-  const int bands = (m + 127) / 128, tiles = (n + s.kt - 1) / s.kt, items = heads * s.parts * bands;
-  const int ctas = cta_count(items, tiles, sms);
-  const double tile = (0.40 + 0.0032 * (s.da * s.kt + s.kt * s.dvp / 32)) * (s.kt == 32 ? 1.12 : 1.0);
-  const double planes = static_cast<double>(heads) * n * (s.dp + s.dvt) * 12 / 6e6;
-  return 13.0 + planes + (static_cast<long long>(items) * tiles + ctas - 1) / ctas * tile;
+  const int bands = (m + 127) / 128, items = heads * bands;
+  const int ctas = cta_count(items, s.tiles, sms);
+  const double tile = 0.58 + 2.87e-5 * (s.dk + s.dvk) * s.kt + (s.q == 128 ? 0.13 : 0.0);
+  const double planes = 1.8e-6 * heads * n * (s.dk + s.dvk);
+  return 14.0 + planes + (static_cast<long long>(items) * s.tiles + ctas - 1) / ctas * tile;
 }
 
-// SDDMM and SpMM head by head over two streams (pytorch/attention.py): 20 us of host time a head for the two launches, or
+// SDDMM and SpMM head by head over two streams (pytorch/attention.py), fitted to 578 measurements with masks of 0.05 to
+// 23 % stored positions, scattered or in a band: 20 us of host time a head for the two launches, or
 // what their gathers take, which follows the positions (a row of q.k and of v for each), and the dense tiles of the SDDMM
 // where that is the tensor-core one.
 double head_by_head_us(int heads, int m, int n, int d, int dv, int nnz) {
@@ -577,19 +755,11 @@ double head_by_head_us(int heads, int m, int n, int d, int dv, int nnz) {
 }
 
 size_t round256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
-int flag_blocks_of(int np) { return (np + kPrepKeys - 1) / kPrepKeys; }
 
-template <int kDA, int KT, int kOut>
-int launch_attention(const CUtensorMap& mk, const CUtensorMap& mv, AttnParams p, int ctas, cudaStream_t s) {
-  constexpr int k_bytes = 2 * KT * kDA * 32 * 4, v_bytes = 2 * KT * kOut * 16 * 4;
-  static_assert(2 * (k_bytes + v_bytes) <= kBudget, "two stages of each");
-  p.k_stages = p.v_stages = 2;
-  for (int left = kBudget - 2 * (k_bytes + v_bytes);;) {  // k first: it is asked for earlier
-    if (p.k_stages <= p.v_stages && p.k_stages < kMaxStages && left >= k_bytes) { ++p.k_stages; left -= k_bytes; }
-    else if (p.v_stages < kMaxStages && left >= v_bytes) { ++p.v_stages; left -= v_bytes; }
-    else break;
-  }
-  auto kern = attention_kernel<kDA, KT, kOut>;
+template <int kQ, int KT, int DVP>
+int launch_attention(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int ctas,
+                     cudaStream_t s) {
+  auto kern = attention_kernel<kQ, KT, DVP>;
   static std::mutex mutex;
   static bool configured[64] = {};
   {
@@ -602,7 +772,7 @@ int launch_attention(const CUtensorMap& mk, const CUtensorMap& mv, AttnParams p,
       if (dev >= 0 && dev < 64) configured[dev] = true;
     }
   }
-  return launch_overlapped(kern, dim3(ctas), dim3(kThreads), static_cast<size_t>(227 * 1024), s, mk, mv, p);
+  return launch_overlapped(kern, dim3(ctas), dim3(kThreads), static_cast<size_t>(227 * 1024), s, mq, mk, mv, p);
 }
 
 }  // namespace
@@ -617,15 +787,15 @@ extern "C" int iex_attention_f32_supported(int heads, int m, int n, int d, int d
   return attention_shape(heads, m, n, d, dv, &s) ? 1 : 0;
 }
 
-// One launch unless the operators are estimated a sixth shorter.  Where the line lies, measured (us, one launch / head by
-// head): 4096 x 4096, 12 heads, d 80: 367 / 257 at 1 %, 367 / 307 at 2 %, 371 / 712 at 5 %; d 64: 211 / 265 from 0.05 to 2 %
-// (the launches), 211 / 375 at 5 %; d 128: 741 / 256 at 1 %, 755 / 755 at 5 %, 761 / 1554 at 10 %.  16384 x 16384 with a band
-// of 256, 8 heads, d 64: 2260 / 1425; with one of 1024: 2236 / 5026.  Of the 578 measurements the choice is the slower one by
-// more than 10 % in three (14 % at most).
+// One launch where it is estimated 1.4 times as fast as the operators.  Below that the two are within their estimates' errors
+// of one another, and the operators, which give the same bits as a call that returns the scores, keep the masks they were
+// measured faster for when the launch took TF32 planes.  Measured (us, one launch / head by head): 4096 x 4096, 12 heads,
+// d 64: 129 / 265 from 0.05 to 2 %, / 375 at 5 %; 32 heads, d 128: about 600 / 1075 at 2 % (estimated 1.2 times: operators), /
+// 4330 at 10 %; 16384 x 16384, 1 head, d 64: 156 / 49 for a band of 32; 32 heads x 8192, d 64: 1000 / 640 at 0.2 %.
 extern "C" int iex_attention_f32_prefers(int heads, int m, int n, int d, int dv, int nnz) {
   Shape s;
   if (!attention_shape(heads, m, n, d, dv, &s)) return 0;
-  return one_launch_us(heads, m, n, s, std::min(sm_count(), kNumSMs)) <= 1.2 * head_by_head_us(heads, m, n, d, dv, nnz);
+  return 1.4 * one_launch_us(heads, m, n, s, std::min(sm_count(), kNumSMs)) <= head_by_head_us(heads, m, n, d, dv, nnz);
 }
 
 // Plan: one word (nonzero if a position is stored twice), then, 256 bytes on, the mask's bits.
@@ -647,12 +817,28 @@ extern "C" int iex_attention_plan_build(int m, int n, const int32_t* row_offsets
   return launch_status();
 }
 
+namespace {
+
+// Sections of the workspace, each on 256 bytes.
+struct Sections {
+  size_t k, v, exponents, partials, counters, end;
+  Sections(int heads, int m, const Shape& s) {
+    const size_t rows = 2ull * heads * s.np, tiles = 4ull * heads * s.tiles;
+    k = 0;
+    v = k + round256(rows * s.dk * 2);
+    exponents = v + round256(rows * s.dvk * 2);
+    partials = exponents + round256(tiles);
+    counters = partials + round256(2ull * kNumSMs * 128 * s.dvp * 4);
+    end = counters + round256(16ull * kGroups * heads * ((m + 127) / 128));
+  }
+};
+
+}  // namespace
+
 extern "C" size_t iex_attention_workspace_bytes(int heads, int m, int n, int d, int dv) {
   Shape s;
   if (!attention_shape(heads, m, n, d, dv, &s)) return 0;
-  return round256(2ull * heads * n * s.dp * 4) + round256(2ull * heads * s.dvt * s.np * 4) +
-         round256(4ull * heads * flag_blocks_of(s.np)) + round256(2ull * kNumSMs * 128 * s.dvp * 4) +
-         round256(32ull * heads * s.parts * ((m + 127) / 128));
+  return Sections(heads, m, s).end;
 }
 
 extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const void* plan, const int32_t* row_offsets,
@@ -663,61 +849,59 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   Shape s;
   if (!attention_shape(heads, m, n, d, dv, &s)) return IEX_ERR_UNSUPPORTED;
   if (!plan || !row_offsets || !column_indices || !q || !k || !v || !out || !workspace) return IEX_ERR_BAD_ARG;
-  if (workspace_bytes < iex_attention_workspace_bytes(heads, m, n, d, dv)) return IEX_ERR_TOO_LARGE;
+  const Sections at(heads, m, s);
+  if (workspace_bytes < at.end) return IEX_ERR_TOO_LARGE;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
     return IEX_ERR_UNSUPPORTED;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  float* k_planes = reinterpret_cast<float*>(ws);
-  float* v_planes = reinterpret_cast<float*>(ws + round256(2ull * heads * n * s.dp * 4));
-  int* flags = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(v_planes) + round256(2ull * heads * s.dvt * s.np * 4));
-  uint8_t* after = reinterpret_cast<uint8_t*>(flags) + round256(4ull * heads * flag_blocks_of(s.np));
+  __half* k_planes = reinterpret_cast<__half*>(ws + at.k);
+  __half* v_planes = reinterpret_cast<__half*>(ws + at.v);
+  int* exponents = reinterpret_cast<int*>(ws + at.exponents);
   AttnParams p{};
-  p.partials = reinterpret_cast<float4*>(after);
-  p.counters = reinterpret_cast<int*>(after + round256(2ull * kNumSMs * 128 * s.dvp * 4));
+  p.partials = reinterpret_cast<float4*>(ws + at.partials);
+  p.counters = reinterpret_cast<int*>(ws + at.counters);
   p.heads = heads; p.m = m; p.n = n; p.d = d; p.dv = dv;
-  p.parts = s.parts;
-  p.dvt = s.dvt;
   p.bands = (m + 127) / 128;
-  p.tiles = (n + s.kt - 1) / s.kt;
+  p.tiles = s.tiles;
   p.mp = s.mp;
   p.np = s.np;
-  p.total = heads * s.parts * p.bands * p.tiles;
+  p.words = (n + 31) / 32;
+  p.total = heads * p.bands * p.tiles;
   p.bits = static_cast<const uint32_t*>(plan) + 64;
   p.q = q; p.k = k; p.v = v; p.out = out;
   p.row_offsets = row_offsets;
   p.cols = column_indices;
-  p.flags = flags;
-  p.flag_blocks = flag_blocks_of(s.np);
+  p.exponents = exponents;
   p.status = status_word();
-  const int sms = std::min(sm_count(), kNumSMs), ctas = cta_count(heads * s.parts * p.bands, p.tiles, sms);
-  CUtensorMap mk, mv;
-  int st = make_map_f32(&mk, k_planes, 2ll * heads * n, s.dp, s.kt);
-  if (st == IEX_OK) st = make_map_f32(&mv, v_planes, 2ll * heads * s.dvt, s.np, s.dvp);
+  const int sms = std::min(sm_count(), kNumSMs), ctas = cta_count(heads * p.bands, p.tiles, sms);
+  CUtensorMap mq, mk, mv;
+  int st = make_map_f32(&mq, q, static_cast<long long>(heads) * m, d, 128);
+  if (st == IEX_OK) st = make_map_f16(&mk, k_planes, 2ll * heads * s.np, s.dk, s.dk, s.kt, 64, true);
+  if (st == IEX_OK) st = make_map_f16(&mv, v_planes, 2ll * heads * s.np, s.dvk, s.dvk, s.kt, 64, true);
   if (st != IEX_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   // The prepare kernel of a call usually follows the main kernel of the one before.  Launched ahead of that kernel's end its
   // blocks would crowd on the few SMs that are free (6 heads x 1003, d 80: 42 us a call instead of 31), so that is
   // done only where main kernels leave a third of the chip free (then it saves 1 to 2 us).
-  const dim3 prep_grid(p.flag_blocks, heads + 1);
-  const size_t prep_smem = static_cast<size_t>(kPrepKeys) * (dv + 1) * 4;
+  const dim3 prep_grid(p.tiles, heads + 1);
+  auto prepare = s.kt == 128 ? attention_prepare_kernel<1, 128> : attention_prepare_kernel<2, 64>;
   if (3 * ctas <= 2 * sms) {
-    st = launch_overlapped(attention_prepare_kernel, prep_grid, dim3(256), prep_smem, cs, p, s.dp, k_planes, v_planes, flags);
+    st = launch_overlapped(prepare, prep_grid, dim3(256), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, exponents);
   } else {
-    attention_prepare_kernel<<<prep_grid, 256, prep_smem, cs>>>(p, s.dp, k_planes, v_planes, flags);
+    prepare<<<prep_grid, 256, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, exponents);
     st = launch_status();
   }
   if (st != 0) return st;
-  const int which = s.da * 10 + s.dvp / 16;
+  const int which = s.q + s.dvp / 32;
   switch (which) {
-    case 12: return launch_attention<1, 64, 2>(mk, mv, p, ctas, cs);
-    case 14: return launch_attention<1, 64, 4>(mk, mv, p, ctas, cs);
-    case 22: return launch_attention<2, 64, 2>(mk, mv, p, ctas, cs);
-    case 24: return launch_attention<2, 64, 4>(mk, mv, p, ctas, cs);
-    case 32: return launch_attention<3, 32, 2>(mk, mv, p, ctas, cs);
-    case 34: return launch_attention<3, 32, 4>(mk, mv, p, ctas, cs);
-    case 36: return launch_attention<3, 32, 6>(mk, mv, p, ctas, cs);
-    case 42: return launch_attention<4, 32, 2>(mk, mv, p, ctas, cs);
-    case 44: return launch_attention<4, 32, 4>(mk, mv, p, ctas, cs);
+    case 65: return launch_attention<64, 128, 32>(mq, mk, mv, p, ctas, cs);
+    case 66: return launch_attention<64, 128, 64>(mq, mk, mv, p, ctas, cs);
+    case 67: return launch_attention<64, 64, 96>(mq, mk, mv, p, ctas, cs);
+    case 68: return launch_attention<64, 64, 128>(mq, mk, mv, p, ctas, cs);
+    case 129: return launch_attention<128, 64, 32>(mq, mk, mv, p, ctas, cs);
+    case 130: return launch_attention<128, 64, 64>(mq, mk, mv, p, ctas, cs);
+    case 131: return launch_attention<128, 64, 96>(mq, mk, mv, p, ctas, cs);
+    case 132: return launch_attention<128, 64, 128>(mq, mk, mv, p, ctas, cs);
     default: return IEX_ERR_UNSUPPORTED;
   }
 }

@@ -1,0 +1,107 @@
+"""GPU: the fp16 head / tail planes of masked attention: every width class at tile and band edges, scales far from one,
+tiles that do not suit the planes (summed position by position), rows and columns that are zero or not finite."""
+import numpy as np
+import pytest
+import torch
+
+from intrasm_engine_b200 import _lib, ops
+from intrasm_engine_b200.pytorch.attention import SparseAttentionChain
+from intrasm_engine_b200.pytorch.utils import dense_to_sparse_cuda
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _case(heads, m, n, d, dv, seed=0, density=0.1):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    mask = torch.rand((m, n), generator=g, device=DEV) < density
+    _values, _ri, ro, ci = dense_to_sparse_cuda(mask.to(torch.float16))
+    q, k, v = (torch.randn(s, generator=g, device=DEV) for s in ((heads, m, d), (heads, n, d), (heads, n, dv)))
+    return mask, SparseAttentionChain(ro, ci, m, n), q, k, v, g
+
+
+def _run(chain, q, k, v):
+    out = ops.native.attention(q, k, v, chain.bits, chain.row_offsets, chain.column_indices)
+    torch.cuda.synchronize()
+    assert _lib.lib.iex_last_device_status(1) == 0
+    return out
+
+
+def _check(out, mask, q, k, v, bound=2e-6):
+    """Per element against fp64.  Heads and tails leave 2^-22 of each of the three factors, a tile's 24 accumulations
+    in the tensor core 2^-23 each at most: 2e-6 of the sum of the terms' magnitudes is twice that."""
+    zero = torch.zeros((), dtype=torch.float64, device=DEV)
+    q, k, v = q.double(), k.double(), v.double()
+    ref = torch.where(mask, q @ k.transpose(1, 2), zero) @ v
+    terms = torch.where(mask, q.abs() @ k.abs().transpose(1, 2), zero) @ v.abs()
+    assert bool(((out.double() - ref).abs() <= bound * terms + 1e-44).all())
+
+
+@pytest.mark.parametrize("d,dv", [(4, 4), (32, 64), (64, 32), (64, 68), (60, 128), (68, 32), (128, 64), (80, 80), (128, 128)])
+@pytest.mark.parametrize("m,n", [(1, 1), (129, 65), (255, 129), (300, 640)])
+def test_width_classes_at_tile_edges(d, dv, m, n):
+    mask, chain, q, k, v, _g = _case(3, m, n, d, dv, d + dv + m, density=0.3 if m > 1 else 2.0)
+    _check(_run(chain, q, k, v), mask, q, k, v)
+
+
+@pytest.mark.parametrize("d", [64, 96])
+@pytest.mark.parametrize("scale", [1e-30, 1e-12, 1e12, 1e18])
+def test_scales_far_from_one(d, scale):
+    mask, chain, q, k, v, g = _case(2, 200, 300, d, d, 5)
+    _check(_run(chain, q * scale, k / scale, v), mask, q * scale, k / scale, v)
+    if scale > 1:
+        _check(_run(chain, q / scale, k, v * scale), mask, q / scale, k, v * scale)
+    rows = torch.exp2(torch.randint(-6, 7, (300, 1), generator=g, device=DEV).float())
+    columns = torch.exp2(torch.randint(-6, 7, (d,), generator=g, device=DEV).float())
+    q2, k2, v2 = q * columns, k * rows, v * columns / rows
+    _check(_run(chain, q2, k2, v2), mask, q2, k2, v2)
+
+
+@pytest.mark.parametrize("d", [64, 96])
+@pytest.mark.parametrize("what", ["key of k", "key of v", "column of v"])
+def test_tiles_that_do_not_suit_the_planes(d, what):
+    mask, chain, q, k, v, _g = _case(2, 300, 200, d, d, 7)
+    for exponent in (-20, -32, 40):
+        k2, v2 = k.clone(), v.clone()
+        if what == "key of k":
+            k2[1, 70] *= 2.0 ** exponent
+        elif what == "key of v":
+            v2[1, 70] *= 2.0 ** exponent
+        else:
+            v2[1, :, 3] *= 2.0 ** exponent
+        out = _run(chain, q, k2, v2)
+        _check(out, mask, q, k2, v2)
+        assert torch.equal(out[0], _run(chain, q, k, v)[0])
+
+
+def test_band_cut_between_blocks_that_does_not_suit():
+    mask, chain, q, k, v, _g = _case(1, 130, 3000, 64, 64, 8, density=0.05)
+    v[0, 2900] = 0
+    v[0, 2900, 5] = 1e-30
+    v[0, 17] *= 1e20
+    _check(_run(chain, q, k, v), mask, q, k, v)
+
+
+def test_zero_rows_and_values_that_are_not_finite():
+    mask, chain, q, k, v, _g = _case(2, 260, 200, 64, 64, 9)
+    k[0, 11] = 0
+    v[0, 11] = 3e38  # a key that gives nothing
+    v[1, 64:128] = 0
+    q[1, 5] = 0
+    q[0, 9] = 1e-41
+    _check(_run(chain, q, k, v), mask, q, k, v)
+    clean = _run(chain, q, k, v)
+    for value in (float("inf"), float("nan"), torch.finfo(torch.float32).min):
+        k2 = k.clone()
+        k2[0, 20, 7] = value
+        out = _run(chain, q, k2, v)
+        seen = mask[:, 20]
+        assert torch.allclose(out[0, ~seen], clean[0, ~seen], rtol=1e-5, atol=1e-4) and torch.equal(out[1], clean[1])
+        if not np.isfinite(value):
+            assert bool((~torch.isfinite(out[0, seen & (q[0, :, 7] != 0)])).all())
+    q2 = q.clone()
+    q2[0, 33, 1] = float("nan")
+    out = _run(chain, q2, k, v)
+    others = torch.arange(260, device=DEV) != 33
+    assert torch.equal(out[0, others], clean[0, others]) and bool(torch.isnan(out[0, 33]).all() == mask[33].any())
