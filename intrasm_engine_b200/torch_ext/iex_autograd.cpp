@@ -468,8 +468,8 @@ std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Te
 }
 
 // SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m], W_csr [m, k].
-//   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu)
-//   with `dense`     the layer's dense copy of W and the dense GEMM
+//   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu), where they are smaller than a dense copy
+//   with `dense`     the layer's dense copy of W: on CUDA cores for a handful of tokens (linear_few.cu), else the dense GEMM
 //   up to 256        block decoder on tensor cores (spmm_tile.cu), unless ...
 //   otherwise        ... expanding W for the dense GEMM is estimated faster (many tokens)
 // All read x as it lies and write [tokens, m]: no transposed copies of either.  Nothing for calls that have to go through the
@@ -495,8 +495,9 @@ std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& v
                                   iex_gemm_f16_estimate_us(tokens, m, k, 0, 0));
   // 2.5 us + 1.05 ns per nonzero for one token, 9 + 1.15 for two (a gather more for each); at three the
   // decoder is as fast
+  const double few_us = dense_weight.has_value() ? iex_linear_f16_few_estimate_us(tokens, k, m) : 1e30;
   const double skinny_us = tokens == 1 ? 2.5 + 1.05e-6 * nnz : 3.5 + 6e-6 * m / 11 + 1.15e-6 * nnz;
-  if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) && (!dense_weight.has_value() || skinny_us <= gemm_us)) {
+  if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) && (!dense_weight.has_value() || skinny_us <= std::min(gemm_us, few_us))) {
     const int st = iex_spmm_f16_skinny(m, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
                                        values.data_ptr(), x.data_ptr(), 1, k, out.data_ptr(), 1, m, stream_of(x));
     if (st == 0) return out;
@@ -523,6 +524,12 @@ std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& v
     dense = expand(values, ro, ci, m, k);
   }
   const at::Tensor xp = tma_rows(x);
+  if (1.25 * few_us <= gemm_us) {
+    check_status(iex_linear_f16_few(tokens, k, m, xp.data_ptr(), dense.data_ptr(), out.data_ptr(), ro.data_ptr<int>(),
+                                    ci.data_ptr(), index_bits(ci), values.data_ptr(), stream_of(x)),
+                 "iex_linear_f16_few");
+    return out;
+  }
   if (m % 8 == 0 && iex_gemm_f16_estimate_us(m, tokens, k, 0, 1) <= iex_gemm_f16_estimate_us(tokens, m, k, 0, 0))
     gemm(m, tokens, k, dense, false, xp, false, out, true, Stored{0, ro, ci, values});
   else
