@@ -172,14 +172,15 @@ IEX_API size_t iex_spmm_f32_tc_workspace_bytes(int m, int k, int n);
 IEX_API int iex_spmm_f32_tc_supported(int m, int k, int n);
 IEX_API int iex_spmm_f32_prefers_tc(int m, int k, int n, int nnz);
 
-/* out [tokens, out] = input [tokens, in] * weight [out, in]^T for up to 8 tokens on CUDA cores (fp32 accumulation), the weight
- * read once.  input and weight 16-byte aligned, in a multiple of 8 and tokens (rounded up to 1, 2, 4 or 8) * in up to 32768
- * (else IEX_ERR_UNSUPPORTED).  With row_offsets the weight is the dense copy of that CSR matrix, and outputs that come out NaN
+/* out [tokens, out] = input [tokens, in] * weight [out, in]^T for up to 16 tokens (fp32 accumulation), the weight read once.
+ * input and weight 16-byte aligned, in a multiple of 8 (else IEX_ERR_UNSUPPORTED).  weight_settled: nonzero if nothing that was
+ * launched before and may still run writes the weight; the first part of it is then requested while the kernel in front on
+ * the stream still runs.  With row_offsets the weight is the dense copy of that CSR matrix, and outputs that come out NaN
  * are summed again from the stored positions.  The estimate is 1e30 for what the kernel does not take. */
 IEX_API int iex_linear_f16_few(int tokens, int in_features, int out_features, const void* input, const void* weight,
-                               void* out, const int32_t* row_offsets, const void* column_indices, int index_bits,
-                               const void* values, void* stream);
-IEX_API double iex_linear_f16_few_estimate_us(int tokens, int in_features, int out_features);
+                               void* out, int weight_settled, const int32_t* row_offsets, const void* column_indices,
+                               int index_bits, const void* values, void* stream);
+IEX_API double iex_linear_f16_few_estimate_us(int tokens, int in_features, int out_features, int weight_settled);
 IEX_API int iex_linear_f16_few_supported(int tokens, int in_features);
 
 /* The SDDMM -> SpMM chain of masked attention over all heads, fp32, scores kept on chip:

@@ -57,9 +57,9 @@ SIGNATURES = {
     "iex_sddmm_f32_tc": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_int, c_ptr]),
     "iex_sddmm_f32_tc_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "iex_sddmm_f32_prefers_tc": (c_int, [c_int, c_int, c_int, c_int, c_int]),
-    # tokens in out input weight out row_offsets cols index_bits values stream
-    "iex_linear_f16_few": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr]),
-    "iex_linear_f16_few_estimate_us": (ctypes.c_double, [c_int, c_int, c_int]),
+    # tokens in out input weight out weight_settled row_offsets cols index_bits values stream
+    "iex_linear_f16_few": (c_int, [c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr]),
+    "iex_linear_f16_few_estimate_us": (ctypes.c_double, [c_int, c_int, c_int, c_int]),
     "iex_linear_f16_few_supported": (c_int, [c_int, c_int]),
     # heads m n d dv
     "iex_attention_f32_supported": (c_int, [c_int, c_int, c_int, c_int, c_int]),

@@ -471,14 +471,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       uint32_t w[kWords];
 #pragma unroll
       for (int i = 0; i < kWords; ++i) w[i] = mask_of(0, i);
-      int e_before = 0, e_now = __ldg(exponents);
+      int e_before = 0, e_now = __ldcg(exponents);
       bool odd = false;
       for (int t = 0; t < tiles_here; ++t) {
         const int g = g0 + t;
         uint32_t next[kWords];
 #pragma unroll
         for (int i = 0; i < kWords; ++i) next[i] = mask_of(t + 1, i);
-        const int e_next = __ldg(exponents + min(t + 1, tiles_here - 1));
+        const int e_next = __ldcg(exponents + min(t + 1, tiles_here - 1));
         if (!mbar_wait(s_full(b), ph_b, abort_flag, p.status, 20)) { ok = false; break; }
         __syncwarp();
         tcgen05_fence_after();

@@ -619,8 +619,8 @@ int gemm_f16(int m, int n, int k, const void* a, bool a_mn, long long lda, const
 }
 
 int linear_few(int tokens, int in_features, int out_features, const void* x, long long ldx, const void* w, long long ldw,
-               void* out, long long ldo, const CsrTerms* terms, cudaStream_t stream);  // linear_few.cu
-double linear_few_us(int tokens, int in_features, int out_features);
+               void* out, long long ldo, bool settled, const CsrTerms* terms, cudaStream_t stream);  // linear_few.cu
+double linear_few_us(int tokens, int in_features, int out_features, bool settled);
 
 // The weight can be A (256-row tiles of features, the tokens as tile columns, result transposed) or
 // B (tiles of 256 tokens): few tokens want the former, many the latter; whichever the estimate favours.
@@ -680,10 +680,10 @@ extern "C" int iex_linear_f16_any(int tokens, int in_features, int out_features,
   using namespace iex::tc;
   const int t = tokens, i = in_features, o = out_features;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (t > 0 && t <= 8 && o > 0 && iex::aligned16(input) && iex::aligned16(weight)) {  // a handful of tokens: HBM, on CUDA cores
+  if (t > 0 && o > 0 && linear_few_us(t, i, o, false) < 1e30 && iex::aligned16(input) && iex::aligned16(weight)) {  // a handful of tokens
     GemmPlan plan{};
     const double gemm = std::min(plan_gemm(o, t, i, false, true, sm_count(), &plan), plan_gemm(t, o, i, false, false, sm_count(), &plan));
-    if (1.25 * linear_few_us(t, i, o) <= gemm) return linear_few(t, i, o, input, i, weight, i, out, o, nullptr, s);
+    if (1.15 * linear_few_us(t, i, o, false) <= gemm) return linear_few(t, i, o, input, i, weight, i, out, o, false, nullptr, s);
   }
   if (o % 8 == 0 && iex::aligned16(out) && weight_as_a(t, o, i, false))
     return gemm_f16(o, t, i, weight, false, i, input, false, i, out, true, o, 0, 0, s);

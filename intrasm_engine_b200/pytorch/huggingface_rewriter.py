@@ -95,7 +95,8 @@ class SparseLinear(nn.Module):
             x2 = x if flat else x.reshape(-1, self.in_features)
             row_offsets, column_indices = self.row_offsets, self.column_indices
             y = ops.native.sparse_linear(x2.contiguous(), values, row_offsets, column_indices, self.out_features,
-                                         self.in_features, self._dense.current(values, row_offsets, column_indices))
+                                         self.in_features, self._dense.current(values, row_offsets, column_indices),
+                                         True)
             if y is not None:  # else the call is being traced, or carries tangents
                 if self.bias is not None:
                     y = y + self.bias

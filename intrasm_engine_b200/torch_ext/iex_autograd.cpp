@@ -469,13 +469,14 @@ std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Te
 
 // SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m], W_csr [m, k].
 //   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu), where they are smaller than a dense copy
-//   with `dense`     the layer's dense copy of W: on CUDA cores for a handful of tokens (linear_few.cu), else the dense GEMM
+//   with `dense`     the layer's dense copy of W: for a handful of tokens linear_few.cu, else the dense GEMM
 //   up to 256        block decoder on tensor cores (spmm_tile.cu), unless ...
 //   otherwise        ... expanding W for the dense GEMM is estimated faster (many tokens)
+// `settled`: the dense copy was complete before the call and nothing writes it (a KeptCopy).
 // All read x as it lies and write [tokens, m]: no transposed copies of either.  Nothing for calls that have to go through the
 // dispatcher.
 std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& values, const at::Tensor& ro, const at::Tensor& ci,
-                         int64_t m, int64_t k, const std::optional<at::Tensor>& dense_weight) {
+                         int64_t m, int64_t k, const std::optional<at::Tensor>& dense_weight, bool settled) {
   if (!plain({&x, &values, &ro, &ci})) return std::nullopt;
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous(), "x must be a contiguous [tokens, in_features] matrix");
   TORCH_CHECK(x.size(1) == k, "x has ", x.size(1), " columns, the weight ", k);
@@ -495,7 +496,7 @@ std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& v
                                   iex_gemm_f16_estimate_us(tokens, m, k, 0, 0));
   // 2.5 us + 1.05 ns per nonzero for one token, 9 + 1.15 for two (a gather more for each); at three the
   // decoder is as fast
-  const double few_us = dense_weight.has_value() ? iex_linear_f16_few_estimate_us(tokens, k, m) : 1e30;
+  const double few_us = dense_weight.has_value() ? iex_linear_f16_few_estimate_us(tokens, k, m, settled) : 1e30;
   const double skinny_us = tokens == 1 ? 2.5 + 1.05e-6 * nnz : 3.5 + 6e-6 * m / 11 + 1.15e-6 * nnz;
   if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) && (!dense_weight.has_value() || skinny_us <= std::min(gemm_us, few_us))) {
     const int st = iex_spmm_f16_skinny(m, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
@@ -524,9 +525,9 @@ std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& v
     dense = expand(values, ro, ci, m, k);
   }
   const at::Tensor xp = tma_rows(x);
-  if (1.25 * few_us <= gemm_us) {
-    check_status(iex_linear_f16_few(tokens, k, m, xp.data_ptr(), dense.data_ptr(), out.data_ptr(), ro.data_ptr<int>(),
-                                    ci.data_ptr(), index_bits(ci), values.data_ptr(), stream_of(x)),
+  if (1.15 * few_us <= gemm_us) {
+    check_status(iex_linear_f16_few(tokens, k, m, xp.data_ptr(), dense.data_ptr(), out.data_ptr(), settled ? 1 : 0,
+                                    ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci), values.data_ptr(), stream_of(x)),
                  "iex_linear_f16_few");
     return out;
   }
@@ -614,7 +615,9 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
     return static_cast<int>(iex_torch::spmm_half_way(m, k, n, nnz, bits, iex_torch::kAuto, true, eager));
   });
   mod.def("mylinear", &iex_torch::mylinear);
-  mod.def("sparse_linear", &iex_torch::sparse_linear);
+  mod.def("sparse_linear", &iex_torch::sparse_linear, pybind11::arg("x"), pybind11::arg("values"), pybind11::arg("row_offsets"),
+          pybind11::arg("column_indices"), pybind11::arg("out_features"), pybind11::arg("in_features"),
+          pybind11::arg("dense_weight"), pybind11::arg("settled") = false);
   mod.def("expand_weight", &iex_torch::expand_weight);
   pybind11::class_<iex_torch::KeptCopy>(mod, "KeptCopy")
       .def(pybind11::init<int64_t, int64_t, double>())
