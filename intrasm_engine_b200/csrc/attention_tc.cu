@@ -20,7 +20,7 @@
 // result, measured); a tile's keys are therefore added to fp32 registers with ordinary rounding before the next tile.
 //
 //   prepare kernel   k and v as hi / lo planes that TMA can load; marks the tiles that do not suit and clears the counters
-//                    of the bands' pieces (24 heads x 4096 x 64: 21 us, 100 MB)
+//                    of the bands' pieces (24 heads x 4096 x 64: 17 us, 100 MB)
 //   main kernel      one persistent CTA per SM over a contiguous run of (head, 128-row band, key tile)
 //     warp 0         TMA producer: k and v planes of the next key tiles, q's rows of the next band
 //     warp 1         issues S(t) = Q K(t)^T, warp 2 O(t) = P(t) V(t); A operands (Q, P) in tensor memory.  A thread that
@@ -36,9 +36,9 @@
 // The runs are equal shares of all tiles; with fewer bands than SMs, every band is cut into the same number of equal pieces
 // instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
 //
-// 24 heads x 4096 x 4096 at 5 %, d 64: 255 us in the first tenths of a second (1965 MHz), 288 us sustained (1590 MHz, at the
+// 24 heads x 4096 x 4096 at 5 %, d 64: 251 us in the first tenths of a second (1965 MHz), 284 us sustained (1590 MHz, at the
 // power limit), with TF32 planes 499 and 548 us; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys
-// of which the pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 23.2 us, before 30.7.
+// of which the pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.5 us, before 30.7.
 // Which masks are faster one way or the other: iex_attention_f32_prefers below.
 //
 // Every mbarrier wait is bounded, as in tc_fused.cu.
@@ -579,25 +579,30 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   }
 }
 
+// 512 threads hold 2 (64 keys) to 4 rows of 16 bytes of k and of v each: with 256 the loads of a block's second half wait behind
+// its first (24 heads x 4096, d 64, whole call 283 us, with 512 279, with 1024 284; 6 x 1003, d 80 23.5 and 22.5; 12 x 300 x
+// 3000, d 128 47.0, 44.9 and 49.1).
+constexpr int kPrepThreads = 512;
+
 // Block (x, h): key tile x of head h as head / tail planes, [2][heads * np][dk] and [2][heads * np][dvk], zeros past n, d and
 // dv.  16 threads a row, everything read once and kept in registers.  A row of k is scaled to a largest magnitude in
 // [2^kRowExp, 2^(kRowExp + 1)); v takes the factor that k's row lost, and the tile's rows of v together another (exponents).
 // Tiles where that leaves a key or a column of v too few bits, or that have values of v that are not finite, are marked.
 // The blocks of the last y zero the main kernel's counters.
 template <int kVecs, int KT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kPrepThreads)
 attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict__ k_planes, __half* __restrict__ v_planes,
                          int* __restrict__ exponents) {
-  constexpr int kRows = KT / 16, kNone = -100000;
+  constexpr int kSide = kPrepThreads / 16, kRows = KT / kSide, kNone = -100000;
   __shared__ int top_exp, low_exp;
   __shared__ uint32_t column_top[64 * kVecs];
   if (threadIdx.x == 0) { top_exp = kNone; low_exp = -kNone; }
-  for (int i = threadIdx.x; i < 64 * kVecs; i += 256) column_top[i] = 0;
+  for (int i = threadIdx.x; i < 64 * kVecs; i += kPrepThreads) column_top[i] = 0;
   grid_dependency_wait();
   grid_launch_dependents();
   if (static_cast<int>(blockIdx.y) == p.heads) {
     const int counters = p.heads * p.bands * 4 * kGroups;
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < counters; i += gridDim.x * 256) p.counters[i] = 0;
+    for (int i = blockIdx.x * kPrepThreads + threadIdx.x; i < counters; i += gridDim.x * kPrepThreads) p.counters[i] = 0;
     return;
   }
   const int head = blockIdx.y, key0 = blockIdx.x * KT, group = threadIdx.x >> 4, lane16 = threadIdx.x & 15;
@@ -607,7 +612,7 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
   float4 xk[kRows][kVecs], xv[kRows][kVecs];
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
-    const int key = key0 + group + 16 * i;
+    const int key = key0 + group + kSide * i;
 #pragma unroll
     for (int j = 0; j < kVecs; ++j) {
       const int c = (lane16 + 16 * j) * 4;
@@ -665,10 +670,10 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
     for (int i = 0; i < kRows; ++i) {
       const Scale scale_k(kRowExp - ek[i]), scale_v(ek[i] - exponent);
       const float4 a = xk[i][j], b = xv[i][j];
-      put(k_planes, dk, group + 16 * i, c, make_float4(scale_k(a.x), scale_k(a.y), scale_k(a.z), scale_k(a.w)));
+      put(k_planes, dk, group + kSide * i, c, make_float4(scale_k(a.x), scale_k(a.y), scale_k(a.z), scale_k(a.w)));
       const bool none = ek[i] == kNone;  // a row of k that is zero: nothing of v's counts
       const float4 w = none ? zero : make_float4(scale_v(b.x), scale_v(b.y), scale_v(b.z), scale_v(b.w));
-      put(v_planes, dvk, group + 16 * i, c, w);
+      put(v_planes, dvk, group + kSide * i, c, w);
       auto seen = [&](float scaled, float as_it_is) -> uint32_t {  // at least 1 where there is something
         return max(__float_as_uint(fabsf(scaled)), as_it_is != 0.f && !none ? 1u : 0u);
       };
@@ -684,7 +689,7 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 64 * kVecs; i += 256)
+  for (int i = threadIdx.x; i < 64 * kVecs; i += kPrepThreads)
     odd = odd || (column_top[i] != 0u && exponent_of(column_top[i]) <= kTileExp - kSpread);
   odd = __syncthreads_or(odd ? 1 : 0) != 0;
   if (threadIdx.x == 0) exponents[head * p.tiles + blockIdx.x] = exponent + (odd ? kOdd : 0);
@@ -886,9 +891,9 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   const dim3 prep_grid(p.tiles, heads + 1);
   auto prepare = s.kt == 128 ? attention_prepare_kernel<1, 128> : attention_prepare_kernel<2, 64>;
   if (3 * ctas <= 2 * sms) {
-    st = launch_overlapped(prepare, prep_grid, dim3(256), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, exponents);
+    st = launch_overlapped(prepare, prep_grid, dim3(kPrepThreads), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, exponents);
   } else {
-    prepare<<<prep_grid, 256, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, exponents);
+    prepare<<<prep_grid, kPrepThreads, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, exponents);
     st = launch_status();
   }
   if (st != 0) return st;
