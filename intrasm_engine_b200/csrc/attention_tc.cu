@@ -20,7 +20,7 @@
 // result, measured); a tile's keys are therefore added to fp32 registers with ordinary rounding before the next tile.
 //
 //   prepare kernel   k and v as hi / lo planes that TMA can load; marks the tiles that do not suit and clears the counters
-//                    of the bands' pieces (24 heads x 4096 x 64: 17 us, 100 MB)
+//                    of the bands' pieces (24 heads x 4096 x 64: 100 MB, 20 us cold)
 //   main kernel      one persistent CTA per SM over a contiguous run of (head, 128-row band, key tile)
 //     warp 0         TMA producer: k and v planes of the next key tiles, q's rows of the next band
 //     warp 1         issues S(t) = Q K(t)^T, warp 2 O(t) = P(t) V(t); A operands (Q, P) in tensor memory.  A thread that
@@ -36,9 +36,9 @@
 // The runs are equal shares of all tiles; with fewer bands than SMs, every band is cut into the same number of equal pieces
 // instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
 //
-// 24 heads x 4096 x 4096 at 5 %, d 64: 251 us in the first tenths of a second (1965 MHz), 284 us sustained (1590 MHz, at the
-// power limit), with TF32 planes 499 and 548 us; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys
-// of which the pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.5 us, before 30.7.
+// 24 heads x 4096 x 4096 at 5 %, d 64: 280 us back to back at the power limit (1590 MHz), about 250 on a cool chip (1965 MHz); with
+// TF32 planes 532 to 554 and 499; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys, of which the
+// pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.5 us, with TF32 planes 30.7.
 // Which masks are faster one way or the other: iex_attention_f32_prefers below.
 //
 // Every mbarrier wait is bounded, as in tc_fused.cu.

@@ -166,8 +166,10 @@ template <int NT, int MT>
 int launch_mma(const FewParams& p, int blocks, bool stored, cudaStream_t stream) {
   constexpr int smem = kWarps * MT * kTileRows * (8 * NT + 4) * 4;
   auto kern = stored ? linear_few_mma_kernel<NT, MT, true> : linear_few_mma_kernel<NT, MT, false>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return static_cast<int>(e);
+  if constexpr (smem > 48 * 1024) {  // what a block may have without asking
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
   return launch_overlapped(kern, dim3(blocks), dim3(kThreads), static_cast<size_t>(smem), stream, p);
 }
 
