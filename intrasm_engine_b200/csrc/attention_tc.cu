@@ -36,7 +36,7 @@
 // The runs are equal shares of all tiles; with fewer bands than SMs, every band is cut into the same number of equal pieces
 // instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
 //
-// 24 heads x 4096 x 4096 at 5 %, d 64: 280 us back to back at the power limit (1590 MHz), about 250 on a cool chip (1965 MHz); with
+// 24 heads x 4096 x 4096 at 5 %, d 64: 278 us back to back at the power limit (1590 MHz), about 250 on a cool chip (1965 MHz); with
 // TF32 planes 532 to 554 and 499; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys, of which the
 // pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.5 us, with TF32 planes 30.7.
 // Which masks are faster one way or the other: iex_attention_f32_prefers below.
@@ -483,22 +483,27 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         __syncwarp();
         tcgen05_fence_after();
         const uint32_t s_addr = lanes + kS + b * KT + wg * kKeys;
-        uint32_t x[kKeys];
+        // 32 keys at a time, over their columns of S: 8 of heads, 8 of tails, twice.  A loop: the warps wait for instructions too
+        // (half a warp per issue), and the 64 keys of a tile in one run are 1 to 2 % slower (24 heads x 4096, d 64: 283.4 us a
+        // call, 278.5 so).
+#pragma unroll 1
+        for (int i = 0; i < kWords; ++i) {
+          uint32_t x[32];
+          tmem_ld32(s_addr + i * 32, x);
+          const uint32_t word = i == 0 ? w[0] : w[kWords - 1];
+          tmem_wait_ld();
 #pragma unroll
-        for (int h = 0; h < kKeys / 16; ++h) tmem_ld16(s_addr + h * 16, &x[16 * h]);
-        tmem_wait_ld();
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[16];
 #pragma unroll
-        for (int h = 0; h < kKeys / 16; ++h) {  // over 16 columns of S: 8 of heads, 8 of tails
-          uint32_t r[16];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int c = 16 * h + 2 * j;
-            const uint32_t bit = 1u << (c & 31);
-            const float a0 = (w[h / 2] & bit) ? __uint_as_float(x[c]) : 0.f;
-            const float a1 = (w[h / 2] & (2 * bit)) ? __uint_as_float(x[c + 1]) : 0.f;
-            split2(make_float2(a0, a1), r[j], r[8 + j]);
+            for (int j = 0; j < 8; ++j) {
+              const int c = 16 * h + 2 * j;
+              const float a0 = (word & (1u << c)) ? __uint_as_float(x[c]) : 0.f;
+              const float a1 = (word & (2u << c)) ? __uint_as_float(x[c + 1]) : 0.f;
+              split2(make_float2(a0, a1), r[j], r[8 + j]);
+            }
+            tmem_st16(s_addr + i * 32 + h * 16, r);
           }
-          tmem_st16(s_addr + h * 16, r);
         }
         tmem_wait_st();
         tcgen05_fence_before();
