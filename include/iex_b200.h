@@ -186,7 +186,7 @@ IEX_API int iex_linear_f16_few_supported(int tokens, int in_features);
 /* The SDDMM -> SpMM chain of masked attention over all heads, fp32, scores kept on chip:
  *   out[h, i] = sum over stored positions (i, j) of dot(q[h, i], k[h, j]) * v[h, j]
  * q [heads, m, d], k [heads, n, d], v [heads, n, dv], out [heads, m, dv], contiguous and 16-byte
- * aligned; d and dv multiples of 4 up to 128.  The plan (256-byte aligned, iex_attention_plan_bytes) depends
+ * aligned; d and dv multiples of 4 up to 128; heads * m below 2^31 - 128.  The plan (256-byte aligned, iex_attention_plan_bytes) depends
  * on the pattern only; its first word is nonzero if the pattern stores a position twice, and the plan must
  * then not be used.  The workspace holds k and v as fp16 head and tail planes
  * (22 bits; rows and tiles scaled by powers of two). */

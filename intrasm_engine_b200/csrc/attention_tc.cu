@@ -721,6 +721,8 @@ struct Shape {
 
 bool attention_shape(int heads, int m, int n, int d, int dv, Shape* s) {
   if (heads < 1 || m < 1 || n < 1 || d < 4 || dv < 4 || d % 4 != 0 || dv % 4 != 0 || d > 128 || dv > 128) return false;
+  // A row of all heads' q is a TMA coordinate, a 32-bit integer, and so is the last row of a band that starts inside.
+  if (static_cast<long long>(heads) * m > 0x7fffffffll - 128) return false;
   s->q = d <= 64 ? 64 : 128;
   s->dvp = (dv + 31) / 32 * 32;
   s->kt = s->q == 64 && s->dvp <= 64 ? 128 : 64;

@@ -25,3 +25,14 @@ def test_shapes_the_kernel_does_not_take():
     for shape in ((0, 64, 64, 64, 64), (1, 64, 64, 132, 64), (1, 64, 64, 64, 132), (1, 64, 64, 62, 64)):
         assert not _lib.lib.iex_attention_f32_supported(*shape)
         assert not _lib.lib.iex_attention_f32_prefers(*shape, 1000)
+
+
+def test_rows_of_q_stay_below_what_a_tma_coordinate_holds():
+    """64 x 40 M rows of q would wrap into negative rows, which read as zeros."""
+    last = 2 ** 31 - 129
+    for heads, m, taken in ((64, 40_000_000, 0), (54, 40_000_000, 0), (53, 40_000_000, 1), (1, last, 1), (1, last + 1, 0), (3, last // 3, 1),
+                            (3, last // 3 + 1, 0)):
+        assert _lib.lib.iex_attention_f32_supported(heads, m, 128, 4, 4) == taken, (heads, m)
+        if not taken:
+            assert not _lib.lib.iex_attention_f32_prefers(heads, m, 128, 4, 4, 2 ** 31 - 1)
+            assert _lib.lib.iex_attention_workspace_bytes(heads, m, 128, 4, 4) == 0
