@@ -14,12 +14,13 @@
 // back when a tile of O is added up.  Tails are stored 2^11 times as large, so that they run out of exponents no sooner than
 // the heads; the first head * head instruction scales what the tails' products have summed up back (scale-input-d).  The
 // error of a score is about 2^-22 sum |q_i k_i| + 2^-39 (max |q| sum |k_i| + max |k| sum |q_i|); in normally distributed data the result is 2.0e-7
-// off (2-norm), the TF32 planes gave 2.6e-7.  A tile whose keys' (or columns') largest magnitudes lie 2^28 and more apart, or
-// that has values of v that are not finite, does not suit the planes; its head is summed position by position (rare).
+// off (2-norm), the TF32 planes gave 2.6e-7.  A key with values of v that are not finite, or that would leave fp16's normal range
+// and lose more than 2^-20 of themselves, does not suit the planes: rows of the mask that store it are summed position by
+// position (normally distributed data: for one element of v in 170 million).
 // The tensor core truncates when it adds to an accumulator, which would bias a sum over thousands of positions (2e-6 of the
 // result, measured); a tile's keys are therefore added to fp32 registers with ordinary rounding before the next tile.
 //
-//   prepare kernel   k and v as hi / lo planes that TMA can load; marks the tiles that do not suit and clears the counters
+//   prepare kernel   k and v as hi / lo planes that TMA can load; marks the keys that do not suit and clears the counters
 //                    of the bands' pieces (24 heads x 4096 x 64: 100 MB, 20 us cold)
 //   main kernel      one persistent CTA per SM over a contiguous run of (head, 128-row band, key tile)
 //     warp 0         TMA producer: k and v planes of the next key tiles, q's rows of the next band
@@ -63,17 +64,20 @@ namespace {
 constexpr int kGroups = 2;         // warps that share a quarter of tensor memory: keys and output columns are split between them
 constexpr int kThreads = 128 + 128 * kGroups;
 constexpr int kMaxTiles = 4;       // tiles at a time: in shared memory and, as scores, in tensor memory
-constexpr int kBars = 4 * kMaxTiles + 4;
+constexpr int kBars = 4 * kMaxTiles + 5;
 constexpr int kBarBytes = 8 * kBars + 8;
 constexpr int kExpBytes = kGroups * 128;  // exponents of the parts of a band's rows of q
+constexpr int kShareBytes = kExpBytes + 2 * kGroups * 4 * 4;  // and, for two bands, which rows are to be summed by position
 constexpr int kBudget = (227 * 1024 - 1024 - kBarBytes) & ~1023;
-constexpr int kRing = kBudget - ((kExpBytes + 1023) & ~1023);  // for the rings and q
+constexpr int kRing = kBudget - ((kShareBytes + 1023) & ~1023);  // for the rings and q
 
 constexpr int kTail = 11;      // tails are stored 2^11 times as large: their exponents are then those of the heads
 constexpr int kRowExp = 3;     // rows of q and k are scaled to a largest magnitude in [2^3, 2^4): scores stay below 2^15
 constexpr int kTileExp = 14;   // a tile of v to [2^14, 2^15)
-constexpr int kSpread = 28;    // a key's or a column's largest magnitude this far (in powers of two) below the tile's
-constexpr int kOdd = 1 << 20;  // added to the exponent of a tile that has to be summed position by position
+// Scaled elements of v from here on keep all but 2^-20 of themselves: a tail is 2^-36 off at most where it has no more
+// exponents, and as much is lost with the product of the tails.
+constexpr float kSmallV = 1.f / (1 << 15);
+constexpr int kOdd = 1 << 20;  // added to the exponent of a tile with keys that do not suit the planes
 
 struct AttnParams {
   int heads, m, n, d, dv;
@@ -88,8 +92,10 @@ struct AttnParams {
   const int* row_offsets;
   const int* cols;
   float4* partials;              // [2 * CTAs][dvp / 4][128]: sums of a CTA's first and last band where they are cut
-  int* counters;                 // [bands of all heads][4 * kGroups]: pieces of a band that are there, per warp
+  int* counters;                 // [bands of all heads][4 * kGroups]: pieces of a band that are there, per warp ...
+  uint32_t* odd_rows;            // ... and the warps' rows that have to be summed by position
   const int* exponents;          // [heads][tiles]: v's rows times k's scales are stored times 2^-this (+ kOdd)
+  const uint32_t* odd_keys;      // [heads][np / 32]: keys that do not suit the planes
   int* status;
 };
 
@@ -178,35 +184,48 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
                : "r"(taddr)
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Rows [row0, row0 + 32) of one head, position by position (a warp; for tiles that do not suit the planes).
-__device__ __noinline__ void rows_by_position(const AttnParams& p, int head, int row0, int lane) {
-  const float* q = p.q + static_cast<size_t>(head) * p.m * p.d;
+// Of rows [row0, row0 + 32) of one head those set in `rows` position by position, every kGroups-th by this warp: 32 positions'
+// scores at a time, a lane each, then their rows of v one after the other, 4 columns a lane.
+__device__ __noinline__ void rows_by_position(const AttnParams& p, int head, int row0, uint32_t rows, int share, int lane) {
   const float* k = p.k + static_cast<size_t>(head) * p.n * p.d;
   const float* v = p.v + static_cast<size_t>(head) * p.n * p.dv;
-  for (int r = row0; r < row0 + 32 && r < p.m; ++r) {
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};  // dv <= 128
-    for (int e = p.row_offsets[r]; e < p.row_offsets[r + 1]; ++e) {
-      const int j = p.cols[e];
-      float s = 0.f;
-      for (int c = lane; c < p.d; c += 32) s = fmaf(q[static_cast<size_t>(r) * p.d + c], k[static_cast<size_t>(j) * p.d + c], s);
-      for (int x = 16; x >= 1; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
-      for (int i = 0; i < 4; ++i)
-        if (lane + 32 * i < p.dv) acc[i] = fmaf(s, v[static_cast<size_t>(j) * p.dv + lane + 32 * i], acc[i]);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = 0; rows != 0; ++i, rows &= rows - 1) {
+    if (i % kGroups != share) continue;
+    const int r = row0 + __ffs(rows) - 1, end = __ldg(p.row_offsets + r + 1);
+    const float4* q = reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(head) * p.m + r) * p.d);
+    float4 acc = zero;
+    for (int e0 = __ldg(p.row_offsets + r); e0 < end; e0 += 32) {
+      const int j = e0 + lane < end ? __ldg(p.cols + e0 + lane) : 0;
+      float4 s = zero;
+      if (e0 + lane < end) {
+        const float4* kj = reinterpret_cast<const float4*>(k + static_cast<size_t>(j) * p.d);
+#pragma unroll 8
+        for (int c = 0; c < p.d / 4; ++c) {
+          const float4 a = __ldg(q + c), b = __ldg(kj + c);
+          s.x = fmaf(a.x, b.x, s.x);
+          s.y = fmaf(a.y, b.y, s.y);
+          s.z = fmaf(a.z, b.z, s.z);
+          s.w = fmaf(a.w, b.w, s.w);
+        }
+      }
+      const float score = (s.x + s.y) + (s.z + s.w);
+      const int here = min(32, end - e0);
+#pragma unroll 8
+      for (int u = 0; u < here; ++u) {
+        const float f = __shfl_sync(0xffffffffu, score, u);
+        const int key = __shfl_sync(0xffffffffu, j, u);
+        const float4 x = 4 * lane < p.dv ? __ldg(reinterpret_cast<const float4*>(v + static_cast<size_t>(key) * p.dv) + lane) : zero;
+        acc.x = fmaf(f, x.x, acc.x);
+        acc.y = fmaf(f, x.y, acc.y);
+        acc.z = fmaf(f, x.z, acc.z);
+        acc.w = fmaf(f, x.w, acc.w);
+      }
     }
-    for (int i = 0; i < 4; ++i)
-      if (lane + 32 * i < p.dv) p.out[(static_cast<size_t>(head) * p.m + r) * p.dv + lane + 32 * i] = acc[i];
+    if (4 * lane < p.dv) reinterpret_cast<float4*>(p.out + (static_cast<size_t>(head) * p.m + r) * p.dv)[lane] = acc;
   }
 }
 
@@ -224,7 +243,7 @@ struct Layout {
 template <int kQ, int KT, int DVP>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                 const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
+                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ AttnParams p) {
   using L = Layout<kQ, KT, DVP>;
   constexpr int kKAtoms = L::kKAtoms, kVAtoms = L::kVAtoms, kTiles = L::kTiles;
   constexpr uint32_t kKPlane = L::kKPlane, kVPlane = L::kVPlane;
@@ -240,7 +259,8 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   auto pv_done = [&](int b) { return bar + 8u * (3 * kMaxTiles + b); };
   const uint32_t v_base = base + kTiles * 2u * kKPlane, q_base = v_base + kTiles * 2u * kVPlane;
   constexpr uint32_t kB1 = 32u * kMaxTiles;
-  const uint32_t q_full = bar + kB1, raw_full = bar + kB1 + 8u, raw_empty = bar + kB1 + 16u, exps_there = bar + kB1 + 24u;
+  const uint32_t q_full = bar + kB1, raw_full = bar + kB1 + 8u, raw_empty = bar + kB1 + 16u, exps_there = bar + kB1 + 24u,
+                 odd_there = bar + kB1 + 32u;
   volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kBudget + 8 * kBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
@@ -256,6 +276,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     mbar_init(raw_full, 1);
     mbar_init(raw_empty, 4 * kGroups);
     mbar_init(exps_there, 4 * kGroups);
+    mbar_init(odd_there, 4 * kGroups);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -386,6 +407,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     // tile's exponent.
     const uint8_t* q_ptr = base_ptr + (q_base - base);
     volatile uint8_t* exp_ptr = base_ptr + kRing;
+    volatile uint32_t* odd_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kRing + kExpBytes);
     auto put_q = [&](uint32_t seg, int& row_exp) -> bool {
       constexpr int kShare = kQ / kGroups;
       if (!mbar_wait(raw_full, seg & 1u, abort_flag, p.status, 20)) return false;
@@ -472,7 +494,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
       for (int i = 0; i < kWords; ++i) w[i] = mask_of(0, i);
       int e_before = 0, e_now = __ldcg(exponents);
-      bool odd = false;
+      bool odd_row = false;
       for (int t = 0; t < tiles_here; ++t) {
         const int g = g0 + t;
         uint32_t next[kWords];
@@ -513,13 +535,27 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         // q has been read when the band's last S is there: the next band's goes in under the last PV
         if (t + 1 == tiles_here && seg_end < r1 && !put_q(seg + 1, row_exp_next)) { ok = false; break; }
         if (t > 0 && !add_tile(g - 1, e_before)) { ok = false; break; }
+        if (e_now >= kOdd / 2) {
+          const uint32_t* keys = p.odd_keys + ((head * p.tiles + t_begin + t) * KT + wg * kKeys) / 32;
+#pragma unroll
+          for (int i = 0; i < kWords; ++i) odd_row = odd_row || (w[i] & __ldcg(keys + i)) != 0;
+          e_now -= kOdd;
+        }
 #pragma unroll
         for (int i = 0; i < kWords; ++i) w[i] = next[i];
-        odd = odd || e_now >= kOdd / 2;
         e_before = e_now;
         e_now = e_next;
       }
-      if (!ok || !add_tile(g0 + tiles_here - 1, e_before)) { ok = false; break; }
+      if (!ok) break;
+      uint32_t odd = __ballot_sync(0xffffffffu, odd_row);
+      if (lane == 0) {  // the warps of a quarter have seen different keys
+        odd_ptr[((seg & 1u) * kGroups + wg) * 4 + q4] = odd;
+        mbar_arrive(odd_there);
+      }
+      if (!add_tile(g0 + tiles_here - 1, e_before)) { ok = false; break; }
+      if (!mbar_wait(odd_there, seg & 1u, abort_flag, p.status, 20)) { ok = false; break; }
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) odd |= odd_ptr[((seg & 1u) * kGroups + i) * 4 + q4];
       float acc[kCols];
 #pragma unroll
       for (int j = 0; j < kCols / 2; ++j) {
@@ -538,15 +574,17 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
         for (int j = 0; j < kQuads; ++j)
           __stcg(to + j * 128, make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]));
+        const int counter = item * 4 * kGroups + wg * 4 + q4;
+        if (lane == 0 && odd != 0) atomicOr(p.odd_rows + counter, odd);
         __threadfence();
         __syncwarp();
         int there = 0;
-        if (lane == 0) there = atomicAdd(p.counters + item * 4 * kGroups + wg * 4 + q4, odd ? 0x10001 : 1);
+        if (lane == 0) there = atomicAdd(p.counters + counter, 1);
         there = __shfl_sync(0xffffffffu, there, 0);
-        write = (there & 0xffff) == last - first;
-        odd = odd || there > 0xffff;
-        if (write && !odd) {
+        write = there == last - first;
+        if (write) {
           __threadfence();
+          odd = __ldcg(p.odd_rows + counter);
 #pragma unroll
           for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
           for (int c = first; c <= last; ++c) {
@@ -565,14 +603,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           }
         }
       }
-      if (write && !odd && row < p.m) {
+      if (write && row < p.m && !(odd >> lane & 1u)) {
         float* dst = p.out + (static_cast<size_t>(head) * p.m + row) * p.dv + wg * kCols;
 #pragma unroll
         for (int j = 0; j < kCols / 4; ++j)
           if (wg * kCols + 4 * j < p.dv)
             reinterpret_cast<float4*>(dst)[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
       }
-      if (write && odd && wg == 0) rows_by_position(p, head, band * 128 + q4 * 32, lane);
+      if (write && odd != 0) rows_by_position(p, head, band * 128 + q4 * 32, odd, wg, lane);
       r = seg_end;
     }
   }
@@ -592,22 +630,26 @@ constexpr int kPrepThreads = 512;
 // Block (x, h): key tile x of head h as head / tail planes, [2][heads * np][dk] and [2][heads * np][dvk], zeros past n, d and
 // dv.  16 threads a row, everything read once and kept in registers.  A row of k is scaled to a largest magnitude in
 // [2^kRowExp, 2^(kRowExp + 1)); v takes the factor that k's row lost, and the tile's rows of v together another (exponents).
-// Tiles where that leaves a key or a column of v too few bits, or that have values of v that are not finite, are marked.
-// The blocks of the last y zero the main kernel's counters.
+// Keys where that leaves an element of v too few bits, or that have values of v that are not finite, which are stored as zeros, are
+// marked.  The blocks of the last y zero the main kernel's counters.
 template <int kVecs, int KT>
 __global__ void __launch_bounds__(kPrepThreads)
 attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict__ k_planes, __half* __restrict__ v_planes,
-                         int* __restrict__ exponents) {
+                         int* __restrict__ exponents, uint32_t* __restrict__ odd_keys) {
   constexpr int kSide = kPrepThreads / 16, kRows = KT / kSide, kNone = -100000;
-  __shared__ int top_exp, low_exp;
-  __shared__ uint32_t column_top[64 * kVecs];
-  if (threadIdx.x == 0) { top_exp = kNone; low_exp = -kNone; }
-  for (int i = threadIdx.x; i < 64 * kVecs; i += kPrepThreads) column_top[i] = 0;
+  static_assert(kSide == 32, "the keys of a block's i-th rows are a word of odd_keys");
+  __shared__ int top_exp;
+  __shared__ uint32_t odd_words[kRows];
+  if (threadIdx.x == 0) top_exp = kNone;
+  if (threadIdx.x < kRows) odd_words[threadIdx.x] = 0;
   grid_dependency_wait();
   grid_launch_dependents();
   if (static_cast<int>(blockIdx.y) == p.heads) {
     const int counters = p.heads * p.bands * 4 * kGroups;
-    for (int i = blockIdx.x * kPrepThreads + threadIdx.x; i < counters; i += gridDim.x * kPrepThreads) p.counters[i] = 0;
+    for (int i = blockIdx.x * kPrepThreads + threadIdx.x; i < counters; i += gridDim.x * kPrepThreads) {
+      p.counters[i] = 0;
+      p.odd_rows[i] = 0;
+    }
     return;
   }
   const int head = blockIdx.y, key0 = blockIdx.x * KT, group = threadIdx.x >> 4, lane16 = threadIdx.x & 15;
@@ -626,8 +668,7 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
     }
   }
   __syncthreads();
-  int ek[kRows], top = kNone, low = -kNone;
-  bool odd = false;
+  int ek[kRows], top = kNone;
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
     uint32_t bk = 0, bv = 0;
@@ -636,7 +677,6 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
       const float4 a = xk[i][j], b = xv[i][j];
       bk = finite_max(finite_max(finite_max(finite_max(bk, a.x), a.y), a.z), a.w);
       bv = finite_max(finite_max(finite_max(finite_max(bv, b.x), b.y), b.z), b.w);
-      odd = odd || !(isfinite(b.x) && isfinite(b.y) && isfinite(b.z) && isfinite(b.w));
     }
 #pragma unroll
     for (int s = 8; s >= 1; s >>= 1) {
@@ -644,19 +684,11 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
       bv = max(bv, __shfl_xor_sync(0xffffffffu, bv, s));
     }
     ek[i] = bk != 0u ? exponent_of(bk) : kNone;
-    if (bk != 0u && bv != 0u) {
-      const int e = ek[i] + exponent_of(bv);
-      top = max(top, e);
-      low = min(low, e);
-    }
+    if (bk != 0u && bv != 0u) top = max(top, ek[i] + exponent_of(bv));
   }
-  if (lane16 == 0 && top != kNone) {
-    atomicMax(&top_exp, top);
-    atomicMin(&low_exp, low);
-  }
+  if (lane16 == 0 && top != kNone) atomicMax(&top_exp, top);
   __syncthreads();
   const int exponent = top_exp == kNone ? 0 : top_exp - kTileExp;
-  odd = odd || top_exp - low_exp >= kSpread;
   const size_t row0 = static_cast<size_t>(head) * p.np + key0, rows = static_cast<size_t>(p.heads) * p.np;
   auto put = [&](__half* planes, int width, int row, int c, const float4& x) {
     if (c >= width) return;
@@ -668,36 +700,37 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
     *reinterpret_cast<uint2*>(dst + rows * width) = lo;
   };
 #pragma unroll
-  for (int j = 0; j < kVecs; ++j) {
-    const int c = (lane16 + 16 * j) * 4;
-    uint32_t columns[4] = {0, 0, 0, 0};
+  for (int i = 0; i < kRows; ++i) {
+    const Scale scale_k(kRowExp - ek[i]), scale_v(ek[i] - exponent);
+    const bool none = ek[i] == kNone;  // a row of k that is zero: nothing of v's counts, if it is finite
+    bool odd = false;
+    auto scaled = [&](float x) -> float {
+      const float w = none ? 0.f : scale_v(x);
+      const bool finite = isfinite(x);
+      odd = odd || !finite || (fabsf(w) < kSmallV && x != 0.f && !none);
+      return finite ? w : 0.f;
+    };
 #pragma unroll
-    for (int i = 0; i < kRows; ++i) {
-      const Scale scale_k(kRowExp - ek[i]), scale_v(ek[i] - exponent);
+    for (int j = 0; j < kVecs; ++j) {
+      const int c = (lane16 + 16 * j) * 4, row = group + kSide * i;
       const float4 a = xk[i][j], b = xv[i][j];
-      put(k_planes, dk, group + kSide * i, c, make_float4(scale_k(a.x), scale_k(a.y), scale_k(a.z), scale_k(a.w)));
-      const bool none = ek[i] == kNone;  // a row of k that is zero: nothing of v's counts
-      const float4 w = none ? zero : make_float4(scale_v(b.x), scale_v(b.y), scale_v(b.z), scale_v(b.w));
-      put(v_planes, dvk, group + kSide * i, c, w);
-      auto seen = [&](float scaled, float as_it_is) -> uint32_t {  // at least 1 where there is something
-        return max(__float_as_uint(fabsf(scaled)), as_it_is != 0.f && !none ? 1u : 0u);
-      };
-      columns[0] = max(columns[0], seen(w.x, b.x));
-      columns[1] = max(columns[1], seen(w.y, b.y));
-      columns[2] = max(columns[2], seen(w.z, b.z));
-      columns[3] = max(columns[3], seen(w.w, b.w));
+      put(k_planes, dk, row, c, make_float4(scale_k(a.x), scale_k(a.y), scale_k(a.z), scale_k(a.w)));
+      put(v_planes, dvk, row, c, make_float4(scaled(b.x), scaled(b.y), scaled(b.z), scaled(b.w)));
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      columns[i] = max(columns[i], __shfl_xor_sync(0xffffffffu, columns[i], 16));
-      if ((threadIdx.x & 16) == 0) atomicMax(&column_top[c + i], columns[i]);
-    }
+    const uint32_t both = __ballot_sync(0xffffffffu, odd);  // two keys a warp
+    if (both != 0 && (threadIdx.x & 31) == 0)
+      atomicOr(&odd_words[i], (both & 0xffffu ? 1u << group : 0u) | (both >> 16 ? 2u << group : 0u));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 64 * kVecs; i += kPrepThreads)
-    odd = odd || (column_top[i] != 0u && exponent_of(column_top[i]) <= kTileExp - kSpread);
-  odd = __syncthreads_or(odd ? 1 : 0) != 0;
-  if (threadIdx.x == 0) exponents[head * p.tiles + blockIdx.x] = exponent + (odd ? kOdd : 0);
+  if (threadIdx.x == 0) {
+    uint32_t any = 0;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      odd_keys[(head * p.np + key0) / 32 + i] = odd_words[i];
+      any |= odd_words[i];
+    }
+    exponents[head * p.tiles + blockIdx.x] = exponent + (any != 0 ? kOdd : 0);
+  }
 }
 
 // bits[column / 32][row]; a position stored twice (a sum in the operators' terms) sets *repeated.
@@ -833,15 +866,17 @@ namespace {
 
 // Sections of the workspace, each on 256 bytes.
 struct Sections {
-  size_t k, v, exponents, partials, counters, end;
+  size_t k, v, exponents, odd_keys, partials, counters, odd_rows, end;
   Sections(int heads, int m, const Shape& s) {
     const size_t rows = 2ull * heads * s.np, tiles = 4ull * heads * s.tiles;
     k = 0;
     v = k + round256(rows * s.dk * 2);
     exponents = v + round256(rows * s.dvk * 2);
-    partials = exponents + round256(tiles);
+    odd_keys = exponents + round256(tiles);
+    partials = odd_keys + round256(rows / 16);
     counters = partials + round256(2ull * kNumSMs * 128 * s.dvp * 4);
-    end = counters + round256(16ull * kGroups * heads * ((m + 127) / 128));
+    odd_rows = counters + round256(16ull * kGroups * heads * ((m + 127) / 128));
+    end = odd_rows + round256(16ull * kGroups * heads * ((m + 127) / 128));
   }
 };
 
@@ -869,9 +904,11 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   __half* k_planes = reinterpret_cast<__half*>(ws + at.k);
   __half* v_planes = reinterpret_cast<__half*>(ws + at.v);
   int* exponents = reinterpret_cast<int*>(ws + at.exponents);
+  uint32_t* odd_keys = reinterpret_cast<uint32_t*>(ws + at.odd_keys);
   AttnParams p{};
   p.partials = reinterpret_cast<float4*>(ws + at.partials);
   p.counters = reinterpret_cast<int*>(ws + at.counters);
+  p.odd_rows = reinterpret_cast<uint32_t*>(ws + at.odd_rows);
   p.heads = heads; p.m = m; p.n = n; p.d = d; p.dv = dv;
   p.bands = (m + 127) / 128;
   p.tiles = s.tiles;
@@ -884,6 +921,7 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   p.row_offsets = row_offsets;
   p.cols = column_indices;
   p.exponents = exponents;
+  p.odd_keys = odd_keys;
   p.status = status_word();
   const int sms = std::min(sm_count(), kNumSMs), ctas = cta_count(heads * p.bands, p.tiles, sms);
   CUtensorMap mq, mk, mv;
@@ -898,9 +936,9 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   const dim3 prep_grid(p.tiles, heads + 1);
   auto prepare = s.kt == 128 ? attention_prepare_kernel<1, 128> : attention_prepare_kernel<2, 64>;
   if (3 * ctas <= 2 * sms) {
-    st = launch_overlapped(prepare, prep_grid, dim3(kPrepThreads), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, exponents);
+    st = launch_overlapped(prepare, prep_grid, dim3(kPrepThreads), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, exponents, odd_keys);
   } else {
-    prepare<<<prep_grid, kPrepThreads, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, exponents);
+    prepare<<<prep_grid, kPrepThreads, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, exponents, odd_keys);
     st = launch_status();
   }
   if (st != 0) return st;

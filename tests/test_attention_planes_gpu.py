@@ -75,6 +75,22 @@ def test_tiles_that_do_not_suit_the_planes(d, what):
         assert torch.equal(out[0], _run(chain, q, k, v)[0])
 
 
+@pytest.mark.parametrize("d", [64, 96])
+@pytest.mark.parametrize("what", ["elements", "keys"])
+@pytest.mark.parametrize("exponent", [8, 14, 20, 26, 27, 30, 34, 40, 60])
+def test_small_elements_of_a_tile_of_v(d, what, exponent):
+    """Every other element, or key, of v 2^-exponent times as large, under rows that store one key: nothing else in the sum
+    hides what it loses."""
+    _mask, _chain, q, k, v, _g = _case(2, 300, 200, d, d, 11)
+    rows, keys, columns = (torch.arange(n, device=DEV) for n in (300, 200, d))
+    mask = keys[None, :] == (7 * rows % 200)[:, None]
+    _values, _ri, ro, ci = dense_to_sparse_cuda(mask.to(torch.float16))
+    chain = SparseAttentionChain(ro, ci, 300, 200)
+    small = (keys[:, None] + (columns[None, :] if what == "elements" else 0)) % 2 == 1
+    v = torch.where(small, v * 2.0 ** -exponent, v)
+    _check(_run(chain, q, k, v), mask, q, k, v)
+
+
 def test_band_cut_between_blocks_that_does_not_suit():
     mask, chain, q, k, v, _g = _case(1, 130, 3000, 64, 64, 8, density=0.05)
     v[0, 2900] = 0
