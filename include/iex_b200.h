@@ -189,7 +189,8 @@ IEX_API int iex_linear_f16_few_supported(int tokens, int in_features);
  * aligned; d and dv multiples of 4 up to 128; heads * m below 2^31 - 128.  The plan (256-byte aligned, iex_attention_plan_bytes) depends
  * on the pattern only; its first word is nonzero if the pattern stores a position twice, and the plan must
  * then not be used.  The workspace holds k and v as fp16 head and tail planes
- * (22 bits; rows and tiles scaled by powers of two). */
+ * (22 bits of elements that are not much smaller than the largest of their row of q or k or their tile of v; rows of the mask in
+ * which others could show are summed position by position in fp32, some ten times as slowly). */
 IEX_API int iex_attention_f32_supported(int heads, int m, int n, int d, int dv);
 /* Whether this call is expected to beat SDDMM and SpMM head by head: its time follows m * n, theirs the nnz
  * stored positions, so it is not the way for large, very sparse masks (whose plan of m * n / 8 bytes need not

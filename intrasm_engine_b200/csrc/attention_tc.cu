@@ -12,16 +12,21 @@
 // range, so everything is scaled by powers of two, exactly: a row of q or k to a largest magnitude in [8, 16) (then |S| <
 // 2^15 for up to 128 columns), v by the factor its key's row of k lost and by one of its tile (64 or 128 keys), both given
 // back when a tile of O is added up.  Tails are stored 2^11 times as large, so that they run out of exponents no sooner than
-// the heads; the first head * head instruction scales what the tails' products have summed up back (scale-input-d).  The
-// error of a score is about 2^-22 sum |q_i k_i| + 2^-39 (max |q| sum |k_i| + max |k| sum |q_i|); in normally distributed data the result is 2.0e-7
-// off (2-norm), the TF32 planes gave 2.6e-7.  A key with values of v that are not finite, or that would leave fp16's normal range
-// and lose more than 2^-20 of themselves, does not suit the planes: rows of the mask that store it are summed position by
-// position (normally distributed data: for one element of v in 170 million).
+// the heads; the first head * head instruction scales what the tails' products have summed up back (scale-input-d).  In
+// normally distributed data the result is 2.0e-7 off (2-norm), the TF32 planes gave 2.6e-7.
+// What leaves fp16's normal range all the same, 2^-14, is held to 2^-36 instead of 2^-22 of itself.  Rows of the mask that this
+// could show in are summed position by position at the end (sum_again):
+//   v        rows that store a key with such elements (2^-15: 2^-20 of them), or with values that are not finite; in normally
+//            distributed data one element in 170 million
+//   q and k  rows with a score whose terms' magnitudes sum up to next to nothing: a feature that is large in q and small or zero in
+//            k hides what the others give.  That a row of q or k has small elements says too little (normally distributed:
+//            one row in 1500), so 32 rows and a tile of keys are compared as a whole first: columns that are large in all of
+//            them bound the terms from below (unsafe).  Normally distributed data passes that.
 // The tensor core truncates when it adds to an accumulator, which would bias a sum over thousands of positions (2e-6 of the
 // result, measured); a tile's keys are therefore added to fp32 registers with ordinary rounding before the next tile.
 //
 //   prepare kernel   k and v as hi / lo planes that TMA can load; marks the keys that do not suit and clears the counters
-//                    of the bands' pieces (24 heads x 4096 x 64: 100 MB, 20 us cold)
+//                    of the bands' pieces (24 heads x 4096 x 64: 100 MB, 23 us cold)
 //   main kernel      one persistent CTA per SM over a contiguous run of (head, 128-row band, key tile)
 //     warp 0         TMA producer: k and v planes of the next key tiles, q's rows of the next band
 //     warp 1         issues S(t) = Q K(t)^T, warp 2 O(t) = P(t) V(t); A operands (Q, P) in tensor memory.  A thread that
@@ -29,6 +34,7 @@
 //                    70 for a commit.  So there are two of them, each waits once a tile (the barrier of K(t) also counts
 //                    the PV that used up the score tile, that of V(t) the warps that wrote P), and a tile has 128 keys where
 //                    they fit (1536 cycles of the pipe; with 64 and separate barriers: 313 us instead of 288)
+//     warp 3         finds the quarters of a band that may have rows to be summed by position
 //     warps 4-11     read S, keep the mask's positions, write P hi / lo over it; add the O of the tile before to
 //                    registers.  Two warps per tensor-memory quarter share a tile's columns: the tensor pipe has little else
 //                    to do until P(t) is there.  Four per quarter: 294 us, short sequences 25.1 instead of 23.2 us.
@@ -37,9 +43,10 @@
 // The runs are equal shares of all tiles; with fewer bands than SMs, every band is cut into the same number of equal pieces
 // instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
 //
-// 24 heads x 4096 x 4096 at 5 %, d 64: 278 us back to back at the power limit (1590 MHz), about 250 on a cool chip (1965 MHz); with
+// 24 heads x 4096 x 4096 at 5 %, d 64: 281 us back to back at the power limit (1590 MHz), about 245 on a cool chip (1965 MHz); with
 // TF32 planes 532 to 554 and 499; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys, of which the
-// pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.5 us, with TF32 planes 30.7.
+// pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.6 to 23.3 us, with TF32 planes
+// 30.7.  Without a look at the columns of q and k 280 and 22.5.
 // Which masks are faster one way or the other: iex_attention_f32_prefers below.
 //
 // Every mbarrier wait is bounded, as in tc_fused.cu.
@@ -64,10 +71,10 @@ namespace {
 constexpr int kGroups = 2;         // warps that share a quarter of tensor memory: keys and output columns are split between them
 constexpr int kThreads = 128 + 128 * kGroups;
 constexpr int kMaxTiles = 4;       // tiles at a time: in shared memory and, as scores, in tensor memory
-constexpr int kBars = 4 * kMaxTiles + 5;
+constexpr int kBars = 4 * kMaxTiles + 6;
 constexpr int kBarBytes = 8 * kBars + 8;
 constexpr int kExpBytes = kGroups * 128;  // exponents of the parts of a band's rows of q
-constexpr int kShareBytes = kExpBytes + 2 * kGroups * 4 * 4;  // and, for two bands, which rows are to be summed by position
+constexpr int kShareBytes = kExpBytes + 4 * 4 * 4 + 3 * 4;  // what quarters of a band have in common; quarters to be looked at
 constexpr int kBudget = (227 * 1024 - 1024 - kBarBytes) & ~1023;
 constexpr int kRing = kBudget - ((kShareBytes + 1023) & ~1023);  // for the rings and q
 
@@ -77,7 +84,10 @@ constexpr int kTileExp = 14;   // a tile of v to [2^14, 2^15)
 // Scaled elements of v from here on keep all but 2^-20 of themselves: a tail is 2^-36 off at most where it has no more
 // exponents, and as much is lost with the product of the tails.
 constexpr float kSmallV = 1.f / (1 << 15);
-constexpr int kOdd = 1 << 20;  // added to the exponent of a tile with keys that do not suit the planes
+// Elements of q and k, scaled: a large one; a big one, where one in both rows is enough; and from where on fp16 holds them with
+// all their bits.
+constexpr float kLarge = 1.f / 32, kBig = 1.f, kSmall = 1.f / (1 << 14);
+constexpr int kExpBias = 4096;
 
 struct AttnParams {
   int heads, m, n, d, dv;
@@ -93,8 +103,10 @@ struct AttnParams {
   const int* cols;
   float4* partials;              // [2 * CTAs][dvp / 4][128]: sums of a CTA's first and last band where they are cut
   int* counters;                 // [bands of all heads][4 * kGroups]: pieces of a band that are there, per warp ...
-  uint32_t* odd_rows;            // ... and the warps' rows that have to be summed by position
-  const int* exponents;          // [heads][tiles]: v's rows times k's scales are stored times 2^-this (+ kOdd)
+  uint32_t* quarters;            // [bands of all heads], 4 bits each: quarters that may have rows to be summed by position; those of a
+                                 // band that is cut of which half of the columns is complete; those with pairs that have to be looked at
+  uint32_t* odd_rows;            // [bands of all heads][4]: rows of a quarter that have to be summed by position
+  const uint4* tile_info;        // [heads][tiles]: Tile
   const uint32_t* odd_keys;      // [heads][np / 32]: keys that do not suit the planes
   int* status;
 };
@@ -147,6 +159,32 @@ __device__ __forceinline__ void split2(float2 x, uint32_t& hi, uint32_t& lo) {
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
+// A key tile as its prepare block describes it: v's rows times k's scales are stored times 2^-exponent; whether keys of it do not
+// suit the planes; the most small elements that a key's row of k has; the columns that are large in all of them.  Of the first 64
+// columns c is bit (c % 32) / 2 of word c / 32, odd ones 16 further.  A key whose row is zero counts for neither.
+struct Tile {
+  uint32_t word, large0, large1;
+  __device__ __forceinline__ explicit Tile(const uint4* at) {
+    const uint4 x = __ldcg(at);
+    word = x.x;
+    large0 = x.y;
+    large1 = x.z;
+  }
+  static __device__ __forceinline__ uint4 pack(int exponent, bool odd, int small, uint32_t large0, uint32_t large1) {
+    return make_uint4(static_cast<uint32_t>(exponent + kExpBias) | (odd ? 1u << 13 : 0u) | static_cast<uint32_t>(small) << 14, large0,
+                      large1, 0u);
+  }
+  static __device__ __forceinline__ int exponent(uint32_t word) { return static_cast<int>(word & 0x1fffu) - kExpBias; }
+  __device__ __forceinline__ bool odd() const { return (word & (1u << 13)) != 0; }
+  __device__ __forceinline__ int small() const { return static_cast<int>(word >> 14); }
+};
+// Whether scores of some rows of q and a tile's keys can be off by more than 2^-21 of their terms, or P, which follows from them.
+// Of the first 64 columns `large` are large in all these rows but the zero ones, and a row of q and a key together have at most
+// `small` small elements (zeros too, which is on the safe side).  A small element is 2^-36 off and as much is lost with the product
+// of the tails, times at most 16 from the other side: 2^-31.  A large column adds 2^-10 or more to the terms, so that with a small
+// element for each of them 2^-21 of the terms is lost; and P, 2^-35 off at most, wants the terms to be 2^-14.
+__device__ __forceinline__ bool unsafe(int large, int small) { return large == 0 || small > large; }
+
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
@@ -187,45 +225,239 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Of rows [row0, row0 + 32) of one head those set in `rows` position by position, every kGroups-th by this warp: 32 positions'
-// scores at a time, a lane each, then their rows of v one after the other, 4 columns a lane.
-__device__ __noinline__ void rows_by_position(const AttnParams& p, int head, int row0, uint32_t rows, int share, int lane) {
+// Words of a row of q or k, scaled, for pairs of rows: columns of the first 64 that are big, and those that are not zero, c beside
+// c + 64 (a row's 16 threads have 4 columns each, or twice 4; two rows a warp).
+__device__ __forceinline__ uint4 big_and_there(const float4& a, const float4& b) {
+  const int shift = threadIdx.x & 16;
+  auto word = [&](bool even, bool odd) -> uint32_t {
+    return (__ballot_sync(0xffffffffu, even) >> shift & 0xffffu) | __ballot_sync(0xffffffffu, odd) >> shift << 16;
+  };
+  const uint32_t big0 = word(fabsf(a.x) >= kBig, fabsf(a.y) >= kBig), big1 = word(fabsf(a.z) >= kBig, fabsf(a.w) >= kBig);
+  return make_uint4(big0, big1, word(a.x != 0.f || b.x != 0.f, a.y != 0.f || b.y != 0.f),
+                    word(a.z != 0.f || b.z != 0.f, a.w != 0.f || b.w != 0.f));
+}
+__device__ __forceinline__ float4 scaled4(const Scale& s, const float4& x) { return make_float4(s(x.x), s(x.y), s(x.z), s(x.w)); }
+
+// big_and_there of rows [0, rows) of q or k at `x` into `to`, by all threads of the block, 8 rows on their way for each; no exponent
+// below `lowest`.
+__device__ __forceinline__ void row_words(const float* x, int rows, int d, int lowest, uint4* to) {
+  constexpr int kRows = 8, kSide = kThreads / 16;
+  const int lane16 = threadIdx.x & 15;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int row0 = 0; row0 < rows; row0 += kRows * kSide) {
+    float4 a[kRows], b[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int row = row0 + i * kSide + static_cast<int>(threadIdx.x >> 4);
+      const float4* from = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * d);
+      a[i] = row < rows && 4 * lane16 < d ? __ldg(from + lane16) : zero;
+      b[i] = row < rows && 64 + 4 * lane16 < d ? __ldg(from + 16 + lane16) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int row = row0 + i * kSide + static_cast<int>(threadIdx.x >> 4);
+      uint32_t top = finite_max(finite_max(finite_max(finite_max(0u, a[i].x), a[i].y), a[i].z), a[i].w);
+      top = finite_max(finite_max(finite_max(finite_max(top, b[i].x), b[i].y), b[i].z), b[i].w);
+#pragma unroll
+      for (int s = 8; s >= 1; s >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, s));
+      const Scale scale(top != 0u ? kRowExp - max(exponent_of(top), lowest) : 0);
+      const uint4 words = big_and_there(scaled4(scale, a[i]), scaled4(scale, b[i]));
+      if (lane16 == 0 && row < rows) to[row] = words;
+    }
+  }
+}
+
+// Whether a row of q and a key have terms in common and these are next to nothing: below 2^-14 or, with small elements, below
+// what makes 2^-31 for each of them 2^-21.
+__device__ __noinline__ bool next_to_nothing(const float4* q, const float4* k, int quads) {
+  uint32_t top_q = 0, top_k = 0;
+#pragma unroll 8
+  for (int c = 0; c < quads; ++c) {
+    const float4 a = __ldg(q + c), b = __ldg(k + c);
+    top_q = finite_max(finite_max(finite_max(finite_max(top_q, a.x), a.y), a.z), a.w);
+    top_k = finite_max(finite_max(finite_max(finite_max(top_k, b.x), b.y), b.z), b.w);
+  }
+  if (top_q == 0u || top_k == 0u) return false;
+  const Scale scale_q(kRowExp - max(exponent_of(top_q), -126)), scale_k(kRowExp - exponent_of(top_k));
+  float terms = 0.f;
+  int small = 0;
+  bool any = false;
+  auto add = [&](float a, float b) {
+    const float x = fabsf(scale_q(a)), y = fabsf(scale_k(b));
+    any = any || (a != 0.f && b != 0.f);
+    small += (a != 0.f && x < kSmall ? 1 : 0) + (b != 0.f && y < kSmall ? 1 : 0);
+    terms = fmaf(x, y, terms);
+  };
+#pragma unroll 8
+  for (int c = 0; c < quads; ++c) {
+    const float4 a = __ldg(q + c), b = __ldg(k + c);
+    add(a.x, b.x);
+    add(a.y, b.y);
+    add(a.z, b.z);
+    add(a.w, b.w);
+  }
+  return any && terms < fmaxf(kSmall, small * (1.f / 1024));
+}
+
+// Row r of a head position by position (a warp), 32 at a time: 8 lanes share a score, and a row of v takes a lane for 4 columns, two
+// rows at a time up to 64 columns.
+__device__ __forceinline__ void row_by_position(const AttnParams& p, int head, int r, int lane) {
   const float* k = p.k + static_cast<size_t>(head) * p.n * p.d;
   const float* v = p.v + static_cast<size_t>(head) * p.n * p.dv;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i = 0; rows != 0; ++i, rows &= rows - 1) {
-    if (i % kGroups != share) continue;
-    const int r = row0 + __ffs(rows) - 1, end = __ldg(p.row_offsets + r + 1);
-    const float4* q = reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(head) * p.m + r) * p.d);
-    float4 acc = zero;
-    for (int e0 = __ldg(p.row_offsets + r); e0 < end; e0 += 32) {
-      const int j = e0 + lane < end ? __ldg(p.cols + e0 + lane) : 0;
-      float4 s = zero;
-      if (e0 + lane < end) {
-        const float4* kj = reinterpret_cast<const float4*>(k + static_cast<size_t>(j) * p.d);
-#pragma unroll 8
-        for (int c = 0; c < p.d / 4; ++c) {
-          const float4 a = __ldg(q + c), b = __ldg(kj + c);
-          s.x = fmaf(a.x, b.x, s.x);
-          s.y = fmaf(a.y, b.y, s.y);
-          s.z = fmaf(a.z, b.z, s.z);
-          s.w = fmaf(a.w, b.w, s.w);
-        }
+  const int lane8 = lane & 7, split = p.dv <= 64 ? 2 : 1, half = split == 2 ? lane >> 4 : 0;
+  const int vc = split == 2 ? lane & 15 : lane;  // this lane's 4 columns of v
+  auto add = [](float4& to, const float4& a, const float4& b) {
+    to.x = fmaf(a.x, b.x, to.x);
+    to.y = fmaf(a.y, b.y, to.y);
+    to.z = fmaf(a.z, b.z, to.z);
+    to.w = fmaf(a.w, b.w, to.w);
+  };
+  const int begin = __ldg(p.row_offsets + r), end = __ldg(p.row_offsets + r + 1);
+  const float4* q = reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(head) * p.m + r) * p.d);
+  float4 q4[4], acc = zero;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) q4[c] = lane8 + 8 * c < p.d / 4 ? __ldg(q + lane8 + 8 * c) : zero;
+  int coming = begin + lane < end ? __ldg(p.cols + begin + lane) : 0;
+  for (int e = begin; e < end; e += 32) {
+    const int j = coming, here = min(32, end - e);
+    coming = e + 32 + lane < end ? __ldg(p.cols + e + 32 + lane) : 0;
+    float score = 0.f;  // of position e + lane
+#pragma unroll
+    for (int u0 = 0; u0 < 8; u0 += 4) {
+      float4 x[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int key = __shfl_sync(0xffffffffu, j, 4 * (u0 + u) + (lane >> 3));  // key 0 past the end
+        const float4* kj = reinterpret_cast<const float4*>(k + static_cast<size_t>(key) * p.d);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) x[u][c] = lane8 + 8 * c < p.d / 4 ? __ldg(kj + lane8 + 8 * c) : zero;
       }
-      const float score = (s.x + s.y) + (s.z + s.w);
-      const int here = min(32, end - e0);
-#pragma unroll 8
-      for (int u = 0; u < here; ++u) {
-        const float f = __shfl_sync(0xffffffffu, score, u);
-        const int key = __shfl_sync(0xffffffffu, j, u);
-        const float4 x = 4 * lane < p.dv ? __ldg(reinterpret_cast<const float4*>(v + static_cast<size_t>(key) * p.dv) + lane) : zero;
-        acc.x = fmaf(f, x.x, acc.x);
-        acc.y = fmaf(f, x.y, acc.y);
-        acc.z = fmaf(f, x.z, acc.z);
-        acc.w = fmaf(f, x.w, acc.w);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float4 part = zero;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (lane8 + 8 * c < p.d / 4) add(part, q4[c], x[u][c]);
+        float s = (part.x + part.y) + (part.z + part.w);
+#pragma unroll
+        for (int w = 4; w >= 1; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
+        // position 4 (u0 + u) + i is in lanes 8 i to 8 i + 7
+        const float mine = __shfl_sync(0xffffffffu, s, 8 * (lane & 3));
+        if (lane >> 2 == u0 + u) score = mine;
       }
     }
-    if (4 * lane < p.dv) reinterpret_cast<float4*>(p.out + (static_cast<size_t>(head) * p.m + r) * p.dv)[lane] = acc;
+#pragma unroll 1
+    for (int u0 = 0; u0 < here; u0 += 16 * split) {
+      float4 x[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int key = __shfl_sync(0xffffffffu, j, (u0 + split * u + half) & 31);
+        x[u] = 4 * vc < p.dv ? __ldg(reinterpret_cast<const float4*>(v + static_cast<size_t>(key) * p.dv) + vc) : zero;
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int at = u0 + split * u + half;
+        const float f = __shfl_sync(0xffffffffu, score, at & 31);
+        if (at < here) add(acc, make_float4(f, f, f, f), x[u]);
+      }
+    }
+  }
+  if (split == 2) {
+    acc.x += __shfl_down_sync(0xffffffffu, acc.x, 16);
+    acc.y += __shfl_down_sync(0xffffffffu, acc.y, 16);
+    acc.z += __shfl_down_sync(0xffffffffu, acc.z, 16);
+    acc.w += __shfl_down_sync(0xffffffffu, acc.w, 16);
+  }
+  if (half == 0 && 4 * vc < p.dv) reinterpret_cast<float4*>(p.out + (static_cast<size_t>(head) * p.m + r) * p.dv)[vc] = acc;
+}
+
+// After everything else, by all threads: rows of this block's bands, tiles [r0, r1), that have to be summed by position.  `cut`:
+// the quarters (4 bits each) of its first and its last band that it has to see to where these are cut between blocks; all others,
+// and whether there may be such rows in them, are in p.quarters.  Which rows that are is found from the words of q's and k's rows: a
+// column that is big on both sides makes a pair's terms 1 or more, and nothing in common makes them zero; other pairs are looked
+// at.  `words`: shared memory for kAgainWords of them.
+// 24 heads x 4096, d 64 on a cool chip (245 us otherwise): one key in every head 389 us, q and k after a ReLU, where all pairs are
+// looked at, 519, one column of q and k 2^8 times the others 1080, and one of q 2^24, one of k 2^-24 times the others, where
+// every row is summed, 2970.  At the end and not in the loop over the tiles: any code there that looks at the scores, even if it is
+// passed over, makes the loop 3 to 12 % longer, and so does one that keeps such a row's number.
+constexpr int kAgainKeys = 8192, kAgainWords = kAgainKeys + 128;
+__device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint32_t cut, uint4* words) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = warp & 3;
+  struct Band {
+    int item, head, row0, rows;
+    uint32_t quarters, pairs;  // to look at; with pairs to be looked at
+  };
+  auto band_of = [&](int r) -> Band {
+    const int item = r / p.tiles, head = item / p.bands, row0 = (item - head * p.bands) * 128, first = item * p.tiles;
+    const uint32_t marks = __ldcg(p.quarters + item);
+    const uint32_t mine = r == first && r1 - first >= p.tiles ? 15u : (r == r0 ? cut : cut >> 4) & 15u;
+    return {item, head, row0, min(128, p.m - row0), marks & mine, marks >> 8 & mine};
+  };
+  auto next_band = [&](int r) { return (r / p.tiles + 1) * p.tiles; };
+  uint4* q_words = words + kAgainKeys;
+  int held = -1;  // head whose keys' words are there
+  for (int r = r0; r < r1; r = next_band(r)) {
+    const Band at = band_of(r);
+    if (at.quarters == 0) continue;
+    __syncthreads();
+    if (at.pairs != 0) row_words(p.q + (static_cast<size_t>(at.head) * p.m + at.row0) * p.d, at.rows, p.d, -126, q_words);
+    for (int key0 = 0; key0 < p.n; key0 += kAgainKeys) {
+      const int keys = min(kAgainKeys, p.n - key0);
+      __syncthreads();
+      if (at.pairs != 0 && (held != at.head || keys != p.n)) {
+        row_words(p.k + (static_cast<size_t>(at.head) * p.n + key0) * p.d, keys, p.d, -149, words);
+        held = at.head;
+      }
+      __syncthreads();
+      if (!(at.quarters >> part & 1u)) continue;
+      // a warp takes every third run of 32 words of mask of a quarter
+      const bool pairs = at.pairs >> part & 1u;
+      const int row = part * 32 + lane;
+      const float4* q = reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(at.head) * p.m + min(at.row0 + row, p.m - 1)) * p.d);
+      const uint4 mine = row < at.rows && pairs ? q_words[row] : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t* mask = p.bits + static_cast<size_t>(key0 / 32) * p.mp + at.row0 + row;
+      const uint32_t* odd_keys = p.odd_keys + (static_cast<size_t>(at.head) * p.np + key0) / 32;
+      const int count = (keys + 31) / 32;
+      bool found = row >= at.rows;
+      for (int w0 = warp >> 2; w0 < count; w0 += 32 * (kThreads / 128)) {
+        const int mine_at = w0 + lane * (kThreads / 128);
+        const uint32_t odd_here = mine_at < count ? __ldcg(odd_keys + mine_at) : 0u;
+        const uint32_t visit = pairs ? 0xffffffffu : __ballot_sync(0xffffffffu, odd_here != 0);
+        auto bits_of = [&](int i) -> uint32_t {
+          const int w = w0 + i * (kThreads / 128);
+          return i < 32 && w < count && !found && visit >> i & 1u ? __ldg(mask + static_cast<size_t>(w) * p.mp) : 0u;
+        };
+        uint32_t coming = bits_of(0);
+        for (int i = 0; i < 32 && w0 + i * (kThreads / 128) < count; ++i) {
+          uint32_t bits = coming;
+          coming = bits_of(i + 1);
+          const uint32_t odd = __shfl_sync(0xffffffffu, odd_here, i);  // by all lanes, found or not
+          found = found || (bits & odd) != 0;
+          if (!pairs) continue;
+          for (; bits != 0 && !found; bits &= bits - 1) {
+            const int key = 32 * (w0 + i * (kThreads / 128)) + __ffs(bits) - 1;
+            const uint4 theirs = words[key];
+            if (((mine.x & theirs.x) | (mine.y & theirs.y)) == 0 && ((mine.z & theirs.z) | (mine.w & theirs.w)) != 0)
+              found = next_to_nothing(q, reinterpret_cast<const float4*>(p.k + (static_cast<size_t>(at.head) * p.n + key0 + key) * p.d), p.d / 4);
+          }
+          __syncwarp();
+        }
+      }
+      const uint32_t odd = __ballot_sync(0xffffffffu, found && row < at.rows);
+      if (lane == 0 && odd != 0) atomicOr(p.odd_rows + 4 * at.item + part, odd);
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  int turn = 0;  // the warps take the rows in turn
+  for (int r = r0; r < r1; r = next_band(r)) {
+    const Band at = band_of(r);
+    for (int i = 0; i < 4; ++i)
+      for (uint32_t odd = at.quarters >> i & 1u ? __ldcg(p.odd_rows + 4 * at.item + i) : 0u; odd != 0; odd &= odd - 1) {
+        if (turn == warp) row_by_position(p, at.head, at.row0 + i * 32 + __ffs(odd) - 1, lane);
+        if (++turn == kThreads / 32) turn = 0;
+      }
   }
 }
 
@@ -260,9 +492,15 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const uint32_t v_base = base + kTiles * 2u * kKPlane, q_base = v_base + kTiles * 2u * kVPlane;
   constexpr uint32_t kB1 = 32u * kMaxTiles;
   const uint32_t q_full = bar + kB1, raw_full = bar + kB1 + 8u, raw_empty = bar + kB1 + 16u, exps_there = bar + kB1 + 24u,
-                 odd_there = bar + kB1 + 32u;
+                 looked_at = bar + kB1 + 32u;  // the first band, and 8 further the last one, by warp 3
   volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kBudget + 8 * kBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+  // Of each quarter of a band: columns of the first 64 that are large in all its rows (as in Tile), the most small elements of a
+  // row in each of its warps' columns
+  volatile uint32_t* common = reinterpret_cast<volatile uint32_t*>(base_ptr + kRing + kExpBytes);
+  // quarters that this block has to see to at the end, if there is anything: of its first band, of its last; 256: of others
+  uint32_t* again = reinterpret_cast<uint32_t*>(base_ptr + kRing + kExpBytes + 64);
+  volatile uint32_t* piece = again + 1;  // quarters of the first band, and of the last, as far as this block's tiles tell
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -274,10 +512,12 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     }
     mbar_init(q_full, 4 * kGroups);
     mbar_init(raw_full, 1);
-    mbar_init(raw_empty, 4 * kGroups);
+    mbar_init(raw_empty, 4 * kGroups + 1);
     mbar_init(exps_there, 4 * kGroups);
-    mbar_init(odd_there, 4 * kGroups);
+    mbar_init(looked_at, 1);
+    mbar_init(looked_at + 8u, 1);
     *abort_flag = 0;
+    *again = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     for (int b = 0; b < kTiles; ++b) mbar_arrive(k_full(b));  // nothing to use up before the first tiles
@@ -398,7 +638,44 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       }
     }
     __syncwarp();
-  } else if (warp >= 4) {
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ quarters that may have rows to be summed by position
+    uint32_t seg = 0;
+    for (int r = r0; r < r1; ++seg) {
+      const int item = r / p.tiles, first = item * p.tiles, seg_end = min(r1, first + p.tiles);
+      const uint4* info = p.tile_info + item / p.bands * p.tiles;
+      if (!mbar_wait(q_full, seg & 1u, abort_flag, p.status, 200)) break;
+      __syncwarp();
+      const uint32_t mine = common[lane & 15];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(raw_empty);  // the next band's may be written
+      uint32_t quarters = 0;
+      for (int t = r - first; t < seg_end - first; t += 32) {
+        const Tile tile(info + min(t + lane, seg_end - first - 1));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t large0 = __shfl_sync(0xffffffffu, mine, 4 * i) & tile.large0;
+          const uint32_t large1 = __shfl_sync(0xffffffffu, mine, 4 * i + 1) & tile.large1;
+          const int small = static_cast<int>(__shfl_sync(0xffffffffu, mine, 4 * i + 2) + __shfl_sync(0xffffffffu, mine, 4 * i + 3));
+          if (tile.odd()) quarters |= 1u << i;
+          if (unsafe(__popc(large0) + __popc(large1), small + tile.small())) quarters |= 0x101u << i;
+        }
+      }
+      quarters = __reduce_or_sync(0xffffffffu, quarters);
+      if (lane == 0) {
+        if (quarters != 0) {
+          atomicOr(p.quarters + item, quarters);
+          if (seg_end - r == p.tiles) atomicOr(again, 256u);
+        }
+        if (r == r0 || seg_end == r1) {
+          const int which = r == r0 ? 0 : 1;
+          piece[which] = quarters;
+          mbar_arrive(looked_at + 8u * which);
+        }
+      }
+      r = seg_end;
+    }
+  } else {
     // ------------------------------------------------------------------ mask and sums
     const int wg = (warp >> 2) - 1, q4 = warp & 3;
     const uint32_t lanes = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
@@ -407,43 +684,65 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     // tile's exponent.
     const uint8_t* q_ptr = base_ptr + (q_base - base);
     volatile uint8_t* exp_ptr = base_ptr + kRing;
-    volatile uint32_t* odd_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kRing + kExpBytes);
-    auto put_q = [&](uint32_t seg, int& row_exp) -> bool {
+    auto put_q = [&](uint32_t seg, int band, int& row_exp) -> bool {
       constexpr int kShare = kQ / kGroups;
       if (!mbar_wait(raw_full, seg & 1u, abort_flag, p.status, 20)) return false;
-      float4 x[kShare / 4];
+      // four columns; 128-byte swizzle; whole 32-column atoms are there
+      auto quad = [&](int c) -> float4 {
+        const float4 x = *reinterpret_cast<const float4*>(q_ptr + (c >> 5) * 16384 + row_local * 128 + ((((c >> 2) & 7) ^ (row_local & 7)) << 4));
+        return c < p.d ? x : make_float4(0.f, 0.f, 0.f, 0.f);
+      };
       uint32_t top = 0;
 #pragma unroll
-      for (int j = 0; j < kShare / 4; ++j) {
-        const int c = wg * kShare + 4 * j;  // 128-byte swizzle; whole 32-column atoms are there
-        x[j] = *reinterpret_cast<const float4*>(q_ptr + (c >> 5) * 16384 + row_local * 128 + ((((c >> 2) & 7) ^ (row_local & 7)) << 4));
-        if (c >= p.d) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        top = finite_max(finite_max(finite_max(finite_max(top, x[j].x), x[j].y), x[j].z), x[j].w);
-      }
-      exp_ptr[wg * 128 + row_local] = static_cast<uint8_t>(top >> 23);
+      for (int h = 0; h < kShare / 16; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 x = quad(wg * kShare + 16 * h + 4 * j);
+          top = finite_max(finite_max(finite_max(finite_max(top, x.x), x.y), x.z), x.w);
+        }
+      exp_ptr[wg * 128 + row_local] = static_cast<uint8_t>(top != 0u ? max(top >> 23, 1u) : 0u);
       __syncwarp();
       if (lane == 0) mbar_arrive(exps_there);
       if (!mbar_wait(exps_there, seg & 1u, abort_flag, p.status, 20)) return false;
       int e = 0;
 #pragma unroll
       for (int i = 0; i < kGroups; ++i) e = max(e, static_cast<int>(exp_ptr[i * 128 + row_local]));
+      const bool counts = e != 0 && band * 128 + row_local < p.m;
       e = max(e, 1) - 127;  // of the whole row; of subnormal ones as of 2^-126
       const Scale scale(kRowExp - e);
       row_exp = e - 2 * kRowExp;
+      uint32_t large = 0, smalls = 0;
 #pragma unroll
       for (int h = 0; h < kShare / 16; ++h) {
-        uint32_t hi[8], lo[8];
+        uint32_t hi[8], lo[8], large_here = 0, small_here = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float4 f = x[4 * h + j];
+          const float4 f = quad(wg * kShare + 16 * h + 4 * j);
           split2(make_float2(scale(f.x), scale(f.y)), hi[2 * j], lo[2 * j]);
           split2(make_float2(scale(f.z), scale(f.w)), hi[2 * j + 1], lo[2 * j + 1]);
         }
         tmem_st8(lanes + kQHi + wg * (kShare / 2) + h * 8, hi);
         tmem_st8(lanes + kQLo + wg * (kShare / 2) + h * 8, lo);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {  // a bit for even columns, 16 further one for odd ones
+          const __half2 x = __habs2(*reinterpret_cast<const __half2*>(&hi[j]));
+          large_here |= (0x00010001u << j) & __hge2_mask(x, __float2half2_rn(kLarge));
+          small_here |= (0x00010001u << j) & __hlt2_mask(x, __float2half2_rn(kSmall));
+        }
+        const int here = min(max(p.d - (wg * kShare + 16 * h), 0), 16);  // columns that there are
+        smalls += __popc(small_here & ((1u << here / 2) - 1u) * 0x00010001u);
+        large |= large_here << (h % 2 * 8);
+        if (h % 2 == 1) {
+          const int word = (wg * kShare + 16 * h) / 32;
+          const uint32_t all = __reduce_and_sync(0xffffffffu, counts ? large : 0xffffffffu);
+          if (word < 2 && lane == 0) common[4 * q4 + word] = all;
+          large = 0;
+        }
       }
       tmem_wait_st();
       tcgen05_fence_before();
+      smalls = __reduce_max_sync(0xffffffffu, counts ? smalls : 0u);
+      if (lane == 0) common[4 * q4 + 2 + wg] = smalls;
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(q_full);
@@ -452,7 +751,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       return true;
     };
     int row_exp = 0, row_exp_next = 0;
-    bool ok = r0 >= r1 || put_q(0, row_exp_next);
+    bool ok = r0 >= r1 || put_q(0, r0 / p.tiles % p.bands, row_exp_next);
     uint32_t seg = 0, ph_b = 0, ph_add = 0;  // of the score tile that is next, and of the one whose O is
     int b = 0, b_add = 0;
     for (int r = r0; r < r1 && ok; ++seg) {
@@ -489,18 +788,17 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const int key = (t_begin + t) * KT + wg * kKeys + 32 * i, word = key >> 5;
         return t < tiles_here && word < p.words ? __ldg(bits + static_cast<size_t>(word) * p.mp) >> (key & 31) : 0u;
       };
-      const int* exponents = p.exponents + head * p.tiles + t_begin;
+      const uint4* tile_info = p.tile_info + head * p.tiles + t_begin;
       uint32_t w[kWords];
 #pragma unroll
       for (int i = 0; i < kWords; ++i) w[i] = mask_of(0, i);
-      int e_before = 0, e_now = __ldcg(exponents);
-      bool odd_row = false;
+      int e_before = 0, e_now = Tile::exponent(__ldcg(&tile_info->x));
       for (int t = 0; t < tiles_here; ++t) {
         const int g = g0 + t;
         uint32_t next[kWords];
 #pragma unroll
         for (int i = 0; i < kWords; ++i) next[i] = mask_of(t + 1, i);
-        const int e_next = __ldcg(exponents + min(t + 1, tiles_here - 1));
+        const int e_next = Tile::exponent(__ldcg(&tile_info[min(t + 1, tiles_here - 1)].x));
         if (!mbar_wait(s_full(b), ph_b, abort_flag, p.status, 20)) { ok = false; break; }
         __syncwarp();
         tcgen05_fence_after();
@@ -533,36 +831,22 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         if (lane == 0) mbar_arrive(p_full(b));
         if (++b == kTiles) { b = 0; ph_b ^= 1u; }
         // q has been read when the band's last S is there: the next band's goes in under the last PV
-        if (t + 1 == tiles_here && seg_end < r1 && !put_q(seg + 1, row_exp_next)) { ok = false; break; }
+        if (t + 1 == tiles_here && seg_end < r1 && !put_q(seg + 1, band + 1 == p.bands ? 0 : band + 1, row_exp_next)) { ok = false; break; }
         if (t > 0 && !add_tile(g - 1, e_before)) { ok = false; break; }
-        if (e_now >= kOdd / 2) {
-          const uint32_t* keys = p.odd_keys + ((head * p.tiles + t_begin + t) * KT + wg * kKeys) / 32;
-#pragma unroll
-          for (int i = 0; i < kWords; ++i) odd_row = odd_row || (w[i] & __ldcg(keys + i)) != 0;
-          e_now -= kOdd;
-        }
 #pragma unroll
         for (int i = 0; i < kWords; ++i) w[i] = next[i];
         e_before = e_now;
         e_now = e_next;
       }
       if (!ok) break;
-      uint32_t odd = __ballot_sync(0xffffffffu, odd_row);
-      if (lane == 0) {  // the warps of a quarter have seen different keys
-        odd_ptr[((seg & 1u) * kGroups + wg) * 4 + q4] = odd;
-        mbar_arrive(odd_there);
-      }
       if (!add_tile(g0 + tiles_here - 1, e_before)) { ok = false; break; }
-      if (!mbar_wait(odd_there, seg & 1u, abort_flag, p.status, 20)) { ok = false; break; }
-#pragma unroll
-      for (int i = 0; i < kGroups; ++i) odd |= odd_ptr[((seg & 1u) * kGroups + i) * 4 + q4];
       float acc[kCols];
 #pragma unroll
       for (int j = 0; j < kCols / 2; ++j) {
         acc[2 * j] = acc2[j].x;
         acc[2 * j + 1] = acc2[j].y;
       }
-      bool write = true;
+      bool write = true, look = false;
       if (tiles_here != p.tiles) {
         // A band cut between CTAs: this piece goes to the workspace, and the warp that finds all the others there adds them
         // up in the order of the keys.
@@ -574,17 +858,21 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
         for (int j = 0; j < kQuads; ++j)
           __stcg(to + j * 128, make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]));
-        const int counter = item * 4 * kGroups + wg * 4 + q4;
-        if (lane == 0 && odd != 0) atomicOr(p.odd_rows + counter, odd);
         __threadfence();
         __syncwarp();
+        // what warp 3 has found out about this piece is counted with it, in the upper half
+        const int which = r == r0 ? 0 : 1;
+        if (!mbar_wait(looked_at + 8u * which, 0, abort_flag, p.status, 20)) { ok = false; break; }
         int there = 0;
-        if (lane == 0) there = atomicAdd(p.counters + counter, 1);
+        if (lane == 0) {
+          const int mine = piece[which] >> q4 & 1u ? 0x10001 : 1;
+          there = atomicAdd(p.counters + item * 4 * kGroups + wg * 4 + q4, mine) + (mine & 0x10000);
+        }
         there = __shfl_sync(0xffffffffu, there, 0);
-        write = there == last - first;
+        write = (there & 0xffff) == last - first;
+        look = write && there > 0xffff;
         if (write) {
           __threadfence();
-          odd = __ldcg(p.odd_rows + counter);
 #pragma unroll
           for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
           for (int c = first; c <= last; ++c) {
@@ -603,14 +891,18 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           }
         }
       }
-      if (write && row < p.m && !(odd >> lane & 1u)) {
+      if (write && row < p.m) {
         float* dst = p.out + (static_cast<size_t>(head) * p.m + row) * p.dv + wg * kCols;
 #pragma unroll
         for (int j = 0; j < kCols / 4; ++j)
           if (wg * kCols + 4 * j < p.dv)
             reinterpret_cast<float4*>(dst)[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
       }
-      if (write && odd != 0) rows_by_position(p, head, band * 128 + q4 * 32, odd, wg, lane);
+      if (look) {  // the other warp of the quarter may be another block's; the later one sees to the rows
+        __threadfence();
+        __syncwarp();
+        if (lane == 0 && (atomicXor(p.quarters + item, 16u << q4) >> (4 + q4) & 1u)) atomicOr(again, (r == r0 ? 1u : 16u) << q4);
+      }
       r = seg_end;
     }
   }
@@ -619,6 +911,11 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   if (warp == 1) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+  const uint32_t cut = *again;
+  if (cut != 0 && *abort_flag == 0) {
+    static_assert(kAgainWords * 16 <= kRing, "the rings and q are free by now");
+    sum_again(p, r0, r1, cut, reinterpret_cast<uint4*>(base_ptr));
   }
 }
 
@@ -629,26 +926,29 @@ constexpr int kPrepThreads = 512;
 
 // Block (x, h): key tile x of head h as head / tail planes, [2][heads * np][dk] and [2][heads * np][dvk], zeros past n, d and
 // dv.  16 threads a row, everything read once and kept in registers.  A row of k is scaled to a largest magnitude in
-// [2^kRowExp, 2^(kRowExp + 1)); v takes the factor that k's row lost, and the tile's rows of v together another (exponents).
+// [2^kRowExp, 2^(kRowExp + 1)); v takes the factor that k's row lost, and the tile's rows of v together another (exponent).
 // Keys where that leaves an element of v too few bits, or that have values of v that are not finite, which are stored as zeros, are
-// marked.  The blocks of the last y zero the main kernel's counters.
+// marked.  And the columns of k are described (Tile).  The blocks of the
+// last y zero the main kernel's counters.
 template <int kVecs, int KT>
 __global__ void __launch_bounds__(kPrepThreads)
 attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict__ k_planes, __half* __restrict__ v_planes,
-                         int* __restrict__ exponents, uint32_t* __restrict__ odd_keys) {
+                         uint4* __restrict__ tile_info, uint32_t* __restrict__ odd_keys) {
   constexpr int kSide = kPrepThreads / 16, kRows = KT / kSide, kNone = -100000;
   static_assert(kSide == 32, "the keys of a block's i-th rows are a word of odd_keys");
-  __shared__ int top_exp;
-  __shared__ uint32_t odd_words[kRows];
-  if (threadIdx.x == 0) top_exp = kNone;
+  __shared__ int top_exp, most_small;
+  __shared__ uint32_t odd_words[kRows], all_large[2];
+  if (threadIdx.x == 0) { top_exp = kNone; most_small = 0; }
+  if (threadIdx.x < 2) all_large[threadIdx.x] = 0xffffffffu;
   if (threadIdx.x < kRows) odd_words[threadIdx.x] = 0;
   grid_dependency_wait();
   grid_launch_dependents();
   if (static_cast<int>(blockIdx.y) == p.heads) {
-    const int counters = p.heads * p.bands * 4 * kGroups;
-    for (int i = blockIdx.x * kPrepThreads + threadIdx.x; i < counters; i += gridDim.x * kPrepThreads) {
+    const int items = p.heads * p.bands;
+    for (int i = blockIdx.x * kPrepThreads + threadIdx.x; i < items * 4 * kGroups; i += gridDim.x * kPrepThreads) {
       p.counters[i] = 0;
-      p.odd_rows[i] = 0;
+      if (i < 4 * items) p.odd_rows[i] = 0;
+      if (i < items) p.quarters[i] = 0;
     }
     return;
   }
@@ -690,15 +990,17 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
   __syncthreads();
   const int exponent = top_exp == kNone ? 0 : top_exp - kTileExp;
   const size_t row0 = static_cast<size_t>(head) * p.np + key0, rows = static_cast<size_t>(p.heads) * p.np;
-  auto put = [&](__half* planes, int width, int row, int c, const float4& x) {
-    if (c >= width) return;
-    uint2 hi, lo;
+  auto put = [&](__half* planes, int width, int row, int c, const float4& x, uint2& hi) {
+    uint2 lo;
     split2(make_float2(x.x, x.y), hi.x, lo.x);
     split2(make_float2(x.z, x.w), hi.y, lo.y);
+    if (c >= width) return;
     __half* dst = planes + (row0 + row) * width + c;
     *reinterpret_cast<uint2*>(dst) = hi;
     *reinterpret_cast<uint2*>(dst + rows * width) = lo;
   };
+  uint2 large = make_uint2(0xffffffffu, 0xffffffffu);  // whether this thread's first four columns of k are, in all its rows
+  __half2 least = __float2half2_rn(1.f);               // least magnitudes in them
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
     const Scale scale_k(kRowExp - ek[i]), scale_v(ek[i] - exponent);
@@ -712,15 +1014,46 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
     };
 #pragma unroll
     for (int j = 0; j < kVecs; ++j) {
-      const int c = (lane16 + 16 * j) * 4, row = group + kSide * i;
-      const float4 a = xk[i][j], b = xv[i][j];
-      put(k_planes, dk, row, c, make_float4(scale_k(a.x), scale_k(a.y), scale_k(a.z), scale_k(a.w)));
-      put(v_planes, dvk, row, c, make_float4(scaled(b.x), scaled(b.y), scaled(b.z), scaled(b.w)));
+      const int c = (lane16 + 16 * j) * 4, row_in_tile = group + kSide * i;
+      const float4 b = xv[i][j];
+      uint2 hi;
+      put(k_planes, dk, row_in_tile, c, scaled4(scale_k, xk[i][j]), hi);
+      const __half2 x = __habs2(*reinterpret_cast<const __half2*>(&hi.x)), y = __habs2(*reinterpret_cast<const __half2*>(&hi.y));
+      if (!none) {
+        if (j == 0) {
+          large.x &= __hge2_mask(x, __float2half2_rn(kLarge));
+          large.y &= __hge2_mask(y, __float2half2_rn(kLarge));
+        }
+        if (c < p.d) least = __hmin2(least, __hmin2(x, y));
+      }
+      put(v_planes, dvk, row_in_tile, c, make_float4(scaled(b.x), scaled(b.y), scaled(b.z), scaled(b.w)), hi);
     }
     const uint32_t both = __ballot_sync(0xffffffffu, odd);  // two keys a warp
     if (both != 0 && (threadIdx.x & 31) == 0)
       atomicOr(&odd_words[i], (both & 0xffffu ? 1u << group : 0u) | (both >> 16 ? 2u << group : 0u));
   }
+  if (__any_sync(0xffffffffu, __low2float(least) < kSmall || __high2float(least) < kSmall)) {  // rare
+    int most = 0;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const Scale scale_k(kRowExp - ek[i]);
+      int small = 0;
+#pragma unroll
+      for (int j = 0; j < kVecs; ++j) {
+        const float4 a = scaled4(scale_k, xk[i][j]);
+        if ((lane16 + 16 * j) * 4 < p.d && ek[i] != kNone)
+          small += (fabsf(a.x) < kSmall ? 1 : 0) + (fabsf(a.y) < kSmall ? 1 : 0) + (fabsf(a.z) < kSmall ? 1 : 0) + (fabsf(a.w) < kSmall ? 1 : 0);
+      }
+#pragma unroll
+      for (int s = 8; s >= 1; s >>= 1) small += __shfl_xor_sync(0xffffffffu, small, s);
+      most = max(most, small);
+    }
+    if (lane16 == 0) atomicMax(&most_small, most);
+  }
+  uint32_t word = ((large.x & 0x00010001u) | (large.y & 0x00010001u) << 1) << (2 * (lane16 & 7));
+#pragma unroll
+  for (int s = 4; s >= 1; s >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, s);
+  if ((lane16 & 7) == 0) atomicAnd(&all_large[lane16 >> 3], word);
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t any = 0;
@@ -729,7 +1062,7 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
       odd_keys[(head * p.np + key0) / 32 + i] = odd_words[i];
       any |= odd_words[i];
     }
-    exponents[head * p.tiles + blockIdx.x] = exponent + (any != 0 ? kOdd : 0);
+    tile_info[head * p.tiles + blockIdx.x] = Tile::pack(exponent, any != 0, most_small, all_large[0], all_large[1]);
   }
 }
 
@@ -866,17 +1199,18 @@ namespace {
 
 // Sections of the workspace, each on 256 bytes.
 struct Sections {
-  size_t k, v, exponents, odd_keys, partials, counters, odd_rows, end;
+  size_t k, v, tile_info, odd_keys, partials, counters, quarters, odd_rows, end;
   Sections(int heads, int m, const Shape& s) {
-    const size_t rows = 2ull * heads * s.np, tiles = 4ull * heads * s.tiles;
+    const size_t rows = 2ull * heads * s.np, tiles = 16ull * heads * s.tiles, items = static_cast<size_t>(heads) * ((m + 127) / 128);
     k = 0;
     v = k + round256(rows * s.dk * 2);
-    exponents = v + round256(rows * s.dvk * 2);
-    odd_keys = exponents + round256(tiles);
+    tile_info = v + round256(rows * s.dvk * 2);
+    odd_keys = tile_info + round256(tiles);
     partials = odd_keys + round256(rows / 16);
     counters = partials + round256(2ull * kNumSMs * 128 * s.dvp * 4);
-    odd_rows = counters + round256(16ull * kGroups * heads * ((m + 127) / 128));
-    end = odd_rows + round256(16ull * kGroups * heads * ((m + 127) / 128));
+    quarters = counters + round256(16 * kGroups * items);
+    odd_rows = quarters + round256(4 * items);
+    end = odd_rows + round256(16 * items);
   }
 };
 
@@ -903,12 +1237,13 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   __half* k_planes = reinterpret_cast<__half*>(ws + at.k);
   __half* v_planes = reinterpret_cast<__half*>(ws + at.v);
-  int* exponents = reinterpret_cast<int*>(ws + at.exponents);
+  uint4* tile_info = reinterpret_cast<uint4*>(ws + at.tile_info);
   uint32_t* odd_keys = reinterpret_cast<uint32_t*>(ws + at.odd_keys);
   AttnParams p{};
   p.partials = reinterpret_cast<float4*>(ws + at.partials);
   p.counters = reinterpret_cast<int*>(ws + at.counters);
   p.odd_rows = reinterpret_cast<uint32_t*>(ws + at.odd_rows);
+  p.quarters = reinterpret_cast<uint32_t*>(ws + at.quarters);
   p.heads = heads; p.m = m; p.n = n; p.d = d; p.dv = dv;
   p.bands = (m + 127) / 128;
   p.tiles = s.tiles;
@@ -920,7 +1255,7 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   p.q = q; p.k = k; p.v = v; p.out = out;
   p.row_offsets = row_offsets;
   p.cols = column_indices;
-  p.exponents = exponents;
+  p.tile_info = tile_info;
   p.odd_keys = odd_keys;
   p.status = status_word();
   const int sms = std::min(sm_count(), kNumSMs), ctas = cta_count(heads * p.bands, p.tiles, sms);
@@ -936,9 +1271,9 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   const dim3 prep_grid(p.tiles, heads + 1);
   auto prepare = s.kt == 128 ? attention_prepare_kernel<1, 128> : attention_prepare_kernel<2, 64>;
   if (3 * ctas <= 2 * sms) {
-    st = launch_overlapped(prepare, prep_grid, dim3(kPrepThreads), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, exponents, odd_keys);
+    st = launch_overlapped(prepare, prep_grid, dim3(kPrepThreads), 0, cs, p, s.dk, s.dvk, k_planes, v_planes, tile_info, odd_keys);
   } else {
-    prepare<<<prep_grid, kPrepThreads, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, exponents, odd_keys);
+    prepare<<<prep_grid, kPrepThreads, 0, cs>>>(p, s.dk, s.dvk, k_planes, v_planes, tile_info, odd_keys);
     st = launch_status();
   }
   if (st != 0) return st;

@@ -91,6 +91,68 @@ def test_small_elements_of_a_tile_of_v(d, what, exponent):
     _check(_run(chain, q, k, v), mask, q, k, v)
 
 
+def _unlike(q, k, what, c, column):
+    """Features that are large on one side and small on the other, in all rows or some."""
+    q, k = q.clone(), k.clone()
+    if what == "feature of q":
+        q[..., column] *= 2.0 ** c
+        k[..., column] *= 2.0 ** -c
+    elif what == "feature of k":
+        q[..., column] *= 2.0 ** -c
+        k[..., column] *= 2.0 ** c
+    elif what == "feature off":
+        q[..., column] *= 2.0 ** c
+        k[..., column] = 0
+    elif what == "one row":
+        q[1, 77, column] *= 2.0 ** c
+        k[..., column] *= 2.0 ** -c
+    elif what == "one key":
+        q[..., column] *= 2.0 ** -c
+        k[0, 33, column] *= 2.0 ** c
+    elif what == "every element":  # also disjoint features whose common ones are small on both sides
+        g = torch.Generator(device=DEV)
+        g.manual_seed(c)
+        for x in (q, k):
+            x *= torch.exp2(-torch.randint(0, c + 1, x.shape, generator=g, device=DEV).float())
+            x *= torch.rand(x.shape, generator=g, device=DEV) < 0.3
+    return q, k
+
+
+@pytest.mark.parametrize("d,column", [(64, 0), (64, 37), (96, 80), (32, 3)])
+@pytest.mark.parametrize("what", ["feature of q", "feature of k", "feature off", "one row", "one key", "every element"])
+@pytest.mark.parametrize("c", [8, 12, 16, 20, 24, 28, 32, 40, 60])
+def test_small_elements_of_a_row_of_q_or_k(d, column, what, c):
+    """Rows that are summed by position add up to d / 4 products and 2 sums a score and 45 or so positions of the row:
+    2^-24 each, 4e-6 of the terms."""
+    mask, chain, q, k, v, _g = _case(2, 300, 200, d, d, 13)
+    q, k = _unlike(q, k, what, c, column)
+    _check(_run(chain, q, k, v), mask, q, k, v, 4e-6)
+
+
+@pytest.mark.parametrize("d", [64, 96])
+def test_small_elements_with_more_keys_than_are_held_at_a_time(d):
+    mask, chain, q, k, v, _g = _case(2, 140, 17000, d, d, 15, density=0.002)
+    q[0, :, 9] *= 2.0 ** 30
+    k[0, 8000:8400, 9] *= 2.0 ** -30
+    k[0, 16990:, 9] = 0
+    v[1, 16500, 3] = float("inf")
+    out = _run(chain, q, k, v)
+    rows = ~mask[:, 16500]
+    v[1, 16500] = 0
+    _check(out[:1], mask, q[:1], k[:1], v[:1], 4e-6)
+    _check(out[1:, rows], mask[rows], q[1:, rows], k[1:], v[1:], 4e-6)
+    assert bool(torch.isinf(out[1, ~rows, 3]).all())
+
+
+def test_small_elements_in_a_band_cut_between_blocks():
+    mask, chain, q, k, v, _g = _case(1, 130, 3000, 64, 64, 14, density=0.01)
+    q[0, 40, 9] *= 2.0 ** 40
+    k[0, 2000:, 9] = 0
+    k[0, 2100] = 0
+    _check(_run(chain, q, k, v), mask, q, k, v, 4e-6)
+    assert torch.equal(_run(chain, q, k, v), _run(chain, q, k, v))
+
+
 def test_band_cut_between_blocks_that_does_not_suit():
     mask, chain, q, k, v, _g = _case(1, 130, 3000, 64, 64, 8, density=0.05)
     v[0, 2900] = 0
