@@ -22,6 +22,10 @@
 //            k hides what the others give.  That a row of q or k has small elements says too little (normally distributed:
 //            one row in 1500), so 32 rows and a tile of keys are compared as a whole first: columns that are large in all of
 //            them bound the terms from below (unsafe).  Normally distributed data passes that.
+//   factors  rows with a tile whose factor is out of fp32's range (q, k and v of 2^-45 all together, say, or v of 2^110 at one key):
+//            its product with the tile's sums need not be.  Tiles say whether some row of q can have one; only then the rows' exponents
+//            are looked at (24 heads x 4096, d 64 the same; 6 x 1003, d 80 22.9 -> 24.1 to 24.5 us, as with a branch where a
+//            tile is added up; 6 x 1003, d 64 and 128 the same: launches back to back start 1 us apart or a multiple of it).
 // The tensor core truncates when it adds to an accumulator, which would bias a sum over thousands of positions (2e-6 of the
 // result, measured); a tile's keys are therefore added to fp32 registers with ordinary rounding before the next tile.
 //
@@ -104,7 +108,8 @@ struct AttnParams {
   float4* partials;              // [2 * CTAs][dvp / 4][128]: sums of a CTA's first and last band where they are cut
   int* counters;                 // [bands of all heads][4 * kGroups]: pieces of a band that are there, per warp ...
   uint32_t* quarters;            // [bands of all heads], 4 bits each: quarters that may have rows to be summed by position; those of a
-                                 // band that is cut of which half of the columns is complete; those with pairs that have to be looked at
+                                 // band that is cut of which half of the columns is complete; those with pairs that have to be looked
+                                 // at; those with rows and tiles whose factor is out of range
   uint32_t* odd_rows;            // [bands of all heads][4]: rows of a quarter that have to be summed by position
   const uint4* tile_info;        // [heads][tiles]: Tile
   const uint32_t* odd_keys;      // [heads][np / 32]: keys that do not suit the planes
@@ -184,6 +189,12 @@ struct Tile {
 // of the tails, times at most 16 from the other side: 2^-31.  A large column adds 2^-10 or more to the terms, so that with a small
 // element for each of them 2^-21 of the terms is lost; and P, 2^-35 off at most, wants the terms to be 2^-14.
 __device__ __forceinline__ bool unsafe(int large, int small) { return large == 0 || small > large; }
+// Whether 2^exponent, the factor of a tile's sums O, is no fp32 number.  O is up to 2^37 and may be small, so O * 2^exponent can be one.
+__device__ __forceinline__ bool out_of_range(int exponent) { return exponent < -149 || exponent > 127; }
+// The same for some row of q, whose share is in [-126, 127] - 2 kRowExp.
+__device__ __forceinline__ bool may_be_out_of_range(int tile_exponent) {
+  return out_of_range(tile_exponent - 126 - 2 * kRowExp) || out_of_range(tile_exponent + 127 - 2 * kRowExp);
+}
 
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
@@ -299,6 +310,49 @@ __device__ __noinline__ bool next_to_nothing(const float4* q, const float4* k, i
   return any && terms < fmaxf(kSmall, small * (1.f / 1024));
 }
 
+// Quarters of a band that have rows and tiles [0, tiles) whose factor is out of range, from the exponent bytes of the rows (a warp).
+__device__ __noinline__ uint32_t far_quarters(const volatile uint8_t* exps, int rows, const uint4* info, int tiles) {
+  const int lane = threadIdx.x & 31;
+  int lowest = 10000, highest = -10000;
+  for (int t = lane; t < tiles; t += 32) {
+    const int e = Tile::exponent(__ldcg(&info[t].x));
+    lowest = min(lowest, e);
+    highest = max(highest, e);
+  }
+  lowest = __reduce_min_sync(0xffffffffu, lowest);
+  highest = __reduce_max_sync(0xffffffffu, highest);
+  uint32_t far = 0;
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    const int row = 32 * i + lane;
+    int e = 0;
+    for (int w = 0; w < kGroups; ++w) e = max(e, static_cast<int>(exps[w * 128 + row]));
+    e -= 127 + 2 * kRowExp;
+    if (__any_sync(0xffffffffu, e != -127 - 2 * kRowExp && row < rows && (out_of_range(e + lowest) || out_of_range(e + highest))))
+      far |= 1u << i;
+  }
+  return far;
+}
+
+// Marks the rows of a quarter of a band (a warp) that have a tile whose factor is out of range.
+__device__ __noinline__ void mark_far(const AttnParams& p, int item, int part) {
+  const int head = item / p.bands, lane = threadIdx.x & 31, row = (item - head * p.bands) * 128 + part * 32 + lane;
+  const float4* q = reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(head) * p.m + min(row, p.m - 1)) * p.d);
+  const uint4* info = p.tile_info + head * p.tiles;
+  uint32_t top = 0;
+#pragma unroll 1
+  for (int c = 0; c < p.d / 4; ++c) {
+    const float4 a = __ldg(q + c);
+    top = finite_max(finite_max(finite_max(finite_max(top, a.x), a.y), a.z), a.w);
+  }
+  bool far = false;
+  const int e = max(exponent_of(max(top, 1u)), -126) - 2 * kRowExp;
+#pragma unroll 1
+  for (int t = 0; t < p.tiles; ++t) far = far || out_of_range(e + Tile::exponent(__ldcg(&info[t].x)));
+  const uint32_t rows = __ballot_sync(0xffffffffu, far && top != 0u && row < p.m);
+  if (lane == 0 && rows != 0) atomicOr(p.odd_rows + 4 * item + part, rows);
+}
+
 // Row r of a head position by position (a warp), 32 at a time: 8 lanes share a score, and a row of v takes a lane for 4 columns, two
 // rows at a time up to 64 columns.
 __device__ __forceinline__ void row_by_position(const AttnParams& p, int head, int r, int lane) {
@@ -386,13 +440,13 @@ __device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = warp & 3;
   struct Band {
     int item, head, row0, rows;
-    uint32_t quarters, pairs;  // to look at; with pairs to be looked at
+    uint32_t quarters, pairs, far;  // to look at; with pairs to be looked at; with rows that may have factors out of range
   };
   auto band_of = [&](int r) -> Band {
     const int item = r / p.tiles, head = item / p.bands, row0 = (item - head * p.bands) * 128, first = item * p.tiles;
     const uint32_t marks = __ldcg(p.quarters + item);
     const uint32_t mine = r == first && r1 - first >= p.tiles ? 15u : (r == r0 ? cut : cut >> 4) & 15u;
-    return {item, head, row0, min(128, p.m - row0), marks & mine, marks >> 8 & mine};
+    return {item, head, row0, min(128, p.m - row0), marks & mine, marks >> 8 & mine, marks >> 12 & mine};
   };
   auto next_band = [&](int r) { return (r / p.tiles + 1) * p.tiles; };
   uint4* q_words = words + kAgainKeys;
@@ -400,6 +454,7 @@ __device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint
   for (int r = r0; r < r1; r = next_band(r)) {
     const Band at = band_of(r);
     if (at.quarters == 0) continue;
+    if (warp < 4 && at.far >> part & 1u) mark_far(p, at.item, part);
     __syncthreads();
     if (at.pairs != 0) row_words(p.q + (static_cast<size_t>(at.head) * p.m + at.row0) * p.d, at.rows, p.d, -126, q_words);
     for (int key0 = 0; key0 < p.n; key0 += kAgainKeys) {
@@ -647,11 +702,11 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (!mbar_wait(q_full, seg & 1u, abort_flag, p.status, 200)) break;
       __syncwarp();
       const uint32_t mine = common[lane & 15];
-      __syncwarp();
-      if (lane == 0) mbar_arrive(raw_empty);  // the next band's may be written
       uint32_t quarters = 0;
+      bool far = false;
       for (int t = r - first; t < seg_end - first; t += 32) {
         const Tile tile(info + min(t + lane, seg_end - first - 1));
+        far = far || may_be_out_of_range(Tile::exponent(tile.word));
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const uint32_t large0 = __shfl_sync(0xffffffffu, mine, 4 * i) & tile.large0;
@@ -662,6 +717,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         }
       }
       quarters = __reduce_or_sync(0xffffffffu, quarters);
+      if (__any_sync(0xffffffffu, far))
+        quarters |= 0x1001u * far_quarters(base_ptr + kRing, p.m - item % p.bands * 128, info + (r - first), seg_end - r);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(raw_empty);  // the next band's may be written
       if (lane == 0) {
         if (quarters != 0) {
           atomicOr(p.quarters + item, quarters);
@@ -714,6 +773,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       uint32_t large = 0, smalls = 0;
 #pragma unroll
       for (int h = 0; h < kShare / 16; ++h) {
+        if (kQ == 128 && h % 2 == 0 && wg * kShare + 16 * h >= p.d) break;  // nothing multiplies these columns
         uint32_t hi[8], lo[8], large_here = 0, small_here = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

@@ -58,6 +58,35 @@ def test_scales_far_from_one(d, scale):
     _check(_run(chain, q2, k2, v2), mask, q2, k2, v2)
 
 
+@pytest.mark.parametrize("d", [4, 64, 96])
+@pytest.mark.parametrize("exponent", [-36, -42, -45, -48])
+def test_all_operands_small(d, exponent):
+    """The factor of a tile's sums is below fp32's range, the sums are not."""
+    mask, chain, q, k, v, _g = _case(2, 200, 300, d, d, 5)
+    q, k, v = q * 2.0 ** exponent, k * 2.0 ** exponent, v * 2.0 ** exponent
+    out = _run(chain, q, k, v)
+    assert bool(out.any())
+    _check(out, mask, q, k, v)
+
+
+@pytest.mark.parametrize("d", [4, 64, 96])
+@pytest.mark.parametrize("exponent", [16, 20])
+def test_large_sums_beside_a_larger_key(d, exponent):
+    """The factor is above fp32's range because of a key that no row stores: rows store one of the others, four features."""
+    _mask, _chain, q, k, v, _g = _case(2, 300, 200, d, d, 11)
+    rows, keys = (torch.arange(n, device=DEV) for n in (300, 200))
+    mask = (keys[None, :] == (7 * rows % 200)[:, None]) & (keys[None, :] != 70)
+    _values, _ri, ro, ci = dense_to_sparse_cuda(mask.to(torch.float16))
+    chain = SparseAttentionChain(ro, ci, 300, 200)
+    q, k, v = (torch.sign(x) * (1 + torch.frac(x.abs())) for x in (q, k, v))
+    q[..., 4:], k[..., 4:] = 0, 0
+    q, k, v = q * 2.0 ** exponent, k * 2.0 ** exponent, v * 2.0 ** (82 + 40 - 2 * exponent)
+    v[:, 70] *= 2.0 ** 28
+    out = _run(chain, q, k, v)
+    assert bool(torch.isfinite(out).all())
+    _check(out, mask, q, k, v)
+
+
 @pytest.mark.parametrize("d", [64, 96])
 @pytest.mark.parametrize("what", ["key of k", "key of v", "column of v"])
 def test_tiles_that_do_not_suit_the_planes(d, what):
