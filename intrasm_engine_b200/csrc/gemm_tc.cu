@@ -680,7 +680,8 @@ extern "C" int iex_linear_f16_any(int tokens, int in_features, int out_features,
   using namespace iex::tc;
   const int t = tokens, i = in_features, o = out_features;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (t > 0 && o > 0 && linear_few_us(t, i, o, false) < 1e30 && iex::aligned16(input) && iex::aligned16(weight)) {  // a handful of tokens
+  if (t > 0 && o > 0 && input && weight && out && linear_few_us(t, i, o, false) < 1e30 && iex::aligned16(input) &&
+      iex::aligned16(weight)) {  // a handful of tokens
     GemmPlan plan{};
     const double gemm = std::min(plan_gemm(o, t, i, false, true, sm_count(), &plan), plan_gemm(t, o, i, false, false, sm_count(), &plan));
     if (1.15 * linear_few_us(t, i, o, false) <= gemm) return linear_few(t, i, o, input, i, weight, i, out, o, false, nullptr, s);
