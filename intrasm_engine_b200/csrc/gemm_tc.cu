@@ -553,7 +553,7 @@ int gemm_f16(int m, int n, int k, const void* a, bool a_mn, long long lda, const
   if (out_t && !tma_out) return IEX_ERR_UNSUPPORTED;
   const int sms = sm_count();
   GemmPlan plan{};
-  plan_gemm(m, n, k, b_mn, out_t, sms, &plan);
+  if (force_bn <= 0 || force_parts <= 0) plan_gemm(m, n, k, b_mn, out_t, sms, &plan);
   if (force_bn > 0) plan.bn = force_bn;
   if (force_parts > 0) plan.parts = force_parts;
   if (plan.bn % (b_mn || !out_t ? 64 : 32) != 0 || plan.bn > 256 || plan.bn <= 0) return IEX_ERR_BAD_ARG;
@@ -680,15 +680,17 @@ extern "C" int iex_linear_f16_any(int tokens, int in_features, int out_features,
   using namespace iex::tc;
   const int t = tokens, i = in_features, o = out_features;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (t > 0 && o > 0 && input && weight && out && linear_few_us(t, i, o, false) < 1e30 && iex::aligned16(input) &&
-      iex::aligned16(weight)) {  // a handful of tokens
-    GemmPlan plan{};
-    const double gemm = std::min(plan_gemm(o, t, i, false, true, sm_count(), &plan), plan_gemm(t, o, i, false, false, sm_count(), &plan));
-    if (1.15 * linear_few_us(t, i, o, false) <= gemm) return linear_few(t, i, o, input, i, weight, i, out, o, false, nullptr, s);
-  }
-  if (o % 8 == 0 && iex::aligned16(out) && weight_as_a(t, o, i, false))
-    return gemm_f16(o, t, i, weight, false, i, input, false, i, out, true, o, 0, 0, s);
-  return gemm_f16(t, o, i, input, false, i, weight, false, i, out, false, o, 0, 0, s);
+  GemmPlan plan{}, rows_plan{};
+  // the weight as A writes the result transposed, by TMA
+  double gemm_us = o % 8 == 0 && iex::aligned16(out) ? plan_gemm(o, t, i, false, true, sm_count(), &plan) : 1e30;
+  const double rows_us = plan_gemm(t, o, i, false, false, sm_count(), &rows_plan);
+  const bool as_a = gemm_us <= rows_us;
+  if (!as_a) gemm_us = rows_us;
+  if (t > 0 && o > 0 && 1.15 * linear_few_us(t, i, o, false) <= gemm_us && input && weight && out && iex::aligned16(input) &&
+      iex::aligned16(weight))
+    return linear_few(t, i, o, input, i, weight, i, out, o, false, nullptr, s);  // a handful of tokens
+  if (as_a) return gemm_f16(o, t, i, weight, false, i, input, false, i, out, true, o, plan.bn, plan.parts, s);
+  return gemm_f16(t, o, i, input, false, i, weight, false, i, out, false, o, rows_plan.bn, rows_plan.parts, s);
 }
 
 extern "C" int iex_linear_f16_dgrad(int tokens, int in_features, int out_features, const void* grad,

@@ -103,3 +103,18 @@ def test_layers_with_a_handful_of_tokens(tokens):
     stored = kept[:, 4] != 0
     y = layer(x)
     assert bool(torch.isnan(y[0, stored]).all()) and bool(torch.isfinite(y[0, ~stored]).all()) and torch.equal(y[1:], clean[1:])
+
+
+@pytest.mark.parametrize("tokens,in_features,out_features,shift", [(9, 2048, 5001, 0), (16, 4096, 5001, 0), (12, 8192, 2001, 0), (9, 4096, 4096, 1)])
+def test_compared_with_the_gemm_that_can_run(tokens, in_features, out_features, shift):
+    """Odd numbers of features, and results at odd addresses, rule the weight-as-A product out: its estimate, the lower one, does not count."""
+    few = 1.15 * _lib.lib.iex_linear_f16_few_estimate_us(tokens, in_features, out_features, 0)
+    assert _lib.lib.iex_gemm_f16_estimate_us(out_features, tokens, in_features, 0, 1) < few
+    assert few <= _lib.lib.iex_gemm_f16_estimate_us(tokens, out_features, in_features, 0, 0)
+    x, w = _rand((tokens, in_features), 6), _rand((out_features, in_features), 7)
+    y, own = (torch.zeros(tokens * out_features + 8, dtype=torch.float16, device=DEV)[shift:tokens * out_features + shift] for _ in range(2))
+    stream = torch.cuda.current_stream().cuda_stream
+    assert _lib.lib.iex_linear_f16_any(tokens, in_features, out_features, x.data_ptr(), w.data_ptr(), y.data_ptr(), stream) == 0
+    assert _lib.lib.iex_linear_f16_few(tokens, in_features, out_features, x.data_ptr(), w.data_ptr(), own.data_ptr(), 0, 0, 0, 0, 0,
+                                       stream) == 0
+    assert _close(y.view(tokens, out_features), x, w) and torch.equal(y, own)  # its order of summation
