@@ -1169,16 +1169,18 @@ int cta_count(int items, int tiles, int sms) {
   return items >= sms ? sms : items * std::min(pieces, sms / items);
 }
 
-// Times in microseconds, fitted on B200 to 70 measurements: 1 to 32 heads, 256 to 16384 rows and keys, 32 to 128 columns;
-// within 18 %, launches of more than 100 us within 8 %.
+// Times in microseconds, fitted on B200 to 50 measurements: 1 to 32 heads, 256 to 16384 rows and keys, 32 to 128 columns;
+// 8 % off (root mean square), 27 % at most.
 //
-// This kernel multiplies every tile, empty or not: m * n counts, not the positions.
+// This kernel multiplies every tile, empty or not: m * n counts, not the positions.  What takes long runs at a lower clock (at
+// the power limit) and shares L2: up to 1.7 times as long for the same tiles.
 double one_launch_us(int heads, int m, int n, const Shape& s, int sms) {
   const int bands = (m + 127) / 128, items = heads * bands;
   const int ctas = cta_count(items, s.tiles, sms);
-  const double tile = 0.58 + 2.87e-5 * (s.dk + s.dvk) * s.kt + (s.q == 128 ? 0.13 : 0.0);
+  const double tile = 0.57 + 2.5e-5 * (s.dk + s.dvk) * s.kt;
   const double planes = 1.8e-6 * heads * n * (s.dk + s.dvk);
-  return 14.0 + planes + (static_cast<long long>(items) * s.tiles + ctas - 1) / ctas * tile;
+  const double cool = planes + (static_cast<long long>(items) * s.tiles + ctas - 1) / ctas * tile;
+  return 18.0 + cool * (1.0 + 0.7 * cool / (cool + 240.0));
 }
 
 // SDDMM and SpMM head by head over two streams (pytorch/attention.py), fitted to 578 measurements with masks of 0.05 to
@@ -1225,15 +1227,14 @@ extern "C" int iex_attention_f32_supported(int heads, int m, int n, int d, int d
   return attention_shape(heads, m, n, d, dv, &s) ? 1 : 0;
 }
 
-// One launch where it is estimated 1.4 times as fast as the operators.  Below that the two are within their estimates' errors
-// of one another, and the operators, which give the same bits as a call that returns the scores, keep the masks they were
-// measured faster for when the launch took TF32 planes.  Measured (us, one launch / head by head): 4096 x 4096, 12 heads,
-// d 64: 129 / 265 from 0.05 to 2 %, / 375 at 5 %; 32 heads, d 128: about 600 / 1075 at 2 % (estimated 1.2 times: operators), /
-// 4330 at 10 %; 16384 x 16384, 1 head, d 64: 156 / 49 for a band of 32; 32 heads x 8192, d 64: 1000 / 640 at 0.2 %.
+// One launch where it is estimated faster than the operators: of the 50 measurements 49 are, a tie goes the other way.  Measured (us,
+// one launch / head by head): 4096 x 4096, 12 heads, d 64: 139 / 269 at 2 %; d 80: 213 / 258 at 0.2 %, 222 / 698 at 5 %; 32 heads,
+// d 128: 785 / 780 at 2 %, 772 / 3514 at 10 %; 16384 x 16384, 1 head, d 64: 162 / 50 for a band of 32; 32 heads x 8192, d 64:
+// 1517 / 635 at 0.2 %; 6314 x 6314, 1 head, d 32: 41 / 50 at 1 %.
 extern "C" int iex_attention_f32_prefers(int heads, int m, int n, int d, int dv, int nnz) {
   Shape s;
   if (!attention_shape(heads, m, n, d, dv, &s)) return 0;
-  return 1.4 * one_launch_us(heads, m, n, s, std::min(sm_count(), kNumSMs)) <= head_by_head_us(heads, m, n, d, dv, nnz);
+  return one_launch_us(heads, m, n, s, std::min(sm_count(), kNumSMs)) <= head_by_head_us(heads, m, n, d, dv, nnz);
 }
 
 // Plan: one word (nonzero if a position is stored twice), then, 256 bytes on, the mask's bits.
