@@ -196,6 +196,8 @@ IEX_API int iex_attention_f32_supported(int heads, int m, int n, int d, int dv);
  * stored positions, so it is not the way for large, very sparse masks (whose plan of m * n / 8 bytes need not
  * be built then either). */
 IEX_API int iex_attention_f32_prefers(int heads, int m, int n, int d, int dv, int nnz);
+/* Whether that is so for some widths and some number of heads up to 64, so that a plan is worth building. */
+IEX_API int iex_attention_f32_may_prefer(int m, int n, int nnz);
 IEX_API size_t iex_attention_plan_bytes(int m, int n);
 IEX_API int iex_attention_plan_build(int m, int n, const int32_t* row_offsets, const int32_t* column_indices,
                                      void* plan, size_t bytes, void* stream);

@@ -64,6 +64,7 @@ SIGNATURES = {
     # heads m n d dv
     "iex_attention_f32_supported": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "iex_attention_f32_prefers": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int]),
+    "iex_attention_f32_may_prefer": (c_int, [c_int, c_int, c_int]),
     "iex_attention_plan_bytes": (c_size, [c_int, c_int]),
     # m n row_offsets cols plan bytes stream
     "iex_attention_plan_build": (c_int, [c_int, c_int, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),

@@ -1237,6 +1237,17 @@ extern "C" int iex_attention_f32_prefers(int heads, int m, int n, int d, int dv,
   return one_launch_us(heads, m, n, s, std::min(sm_count(), kNumSMs)) <= head_by_head_us(heads, m, n, d, dv, nnz);
 }
 
+// Whether a mask of this size and number of stored positions has up to 64 heads of some widths that prefer one launch.  The widths
+// are the least of every class that the operators' time has, where the launch is cheapest; a tensor-core SDDMM takes 32 and 64
+// alone.  25 us on the host where nothing does.
+extern "C" int iex_attention_f32_may_prefer(int m, int n, int nnz) {
+  for (int d : {4, 36, 68, 32, 64})
+    for (int dv : {4, 36, 68})
+      for (int heads = 1; heads <= 64; ++heads)
+        if (iex_attention_f32_prefers(heads, m, n, d, dv, nnz)) return 1;
+  return 0;
+}
+
 // Plan: one word (nonzero if a position is stored twice), then, 256 bytes on, the mask's bits.
 extern "C" size_t iex_attention_plan_bytes(int m, int n) {
   if (m <= 0 || n <= 0) return 256;

@@ -37,10 +37,10 @@ class SparseAttentionChain:
         self.row_indices = swizzle_rows(self.row_offsets)
         self.nnz = int(column_indices.numel())
         self.plan = None  # tile plan of the tensor-core SDDMM, built on first use for a given k
-        # the mask's bits (m * n / 8 bytes) for the one-launch kernel, if any width and number of heads would
+        # the mask's bits (m * n / 8 bytes) for the one-launch kernel, if some width and number of heads would
         # prefer it; it takes every position once, which is read back here (not while a stream is recorded)
         self.bits = None
-        if (self.nnz > 0 and any(_lib.lib.iex_attention_f32_prefers(h, self.m, self.n, 4, 4, self.nnz) for h in (1, 64))
+        if (self.nnz > 0 and _lib.lib.iex_attention_f32_may_prefer(self.m, self.n, self.nnz)
                 and not ops.native.stream_capturing(self.row_offsets)):
             bits = ops.native.attention_plan(self.row_offsets, self.column_indices, self.m, self.n)
             if int(bits[:4].view(torch.int32).item()) == 0:

@@ -1,5 +1,7 @@
 """CPU: the choice between one launch over all heads and SDDMM -> SpMM head by head, at masks where both
 were measured on B200 (us: one launch, head by head)."""
+import random
+
 import pytest
 
 from intrasm_engine_b200 import _lib
@@ -30,6 +32,22 @@ def test_measured_masks(heads, m, n, d, stored, one_launch, head_by_head):
     nnz = int(m * n * stored) if stored < 1 else m * (stored + 1)
     one = bool(_lib.lib.iex_attention_f32_prefers(heads, m, n, d, d, nnz))
     assert one == (one_launch < head_by_head) or max(one_launch, head_by_head) <= 1.03 * min(one_launch, head_by_head)
+
+
+def test_bits_are_built_for_every_mask_that_some_call_prefers():
+    assert _lib.lib.iex_attention_f32_prefers(7, 7176, 7176, 64, 64, int(7176 * 7176 * 0.0203))
+    assert _lib.lib.iex_attention_f32_may_prefer(7176, 7176, int(7176 * 7176 * 0.0203))
+    rng, missed, preferred, refused = random.Random(5), [], 0, 0
+    for _ in range(20000):
+        m, n = (int(2 ** rng.uniform(7, 15)) for _ in range(2))
+        d, dv = (rng.choice([4, 20, 32, 36, 48, 64, 68, 80, 96, 128]) for _ in range(2))
+        heads, nnz = rng.randint(1, 64), int(m * n * 2 ** rng.uniform(-14, -1)) + 1
+        one, may = (bool(f) for f in (_lib.lib.iex_attention_f32_prefers(heads, m, n, d, dv, nnz),
+                                      _lib.lib.iex_attention_f32_may_prefer(m, n, nnz)))
+        preferred, refused = preferred + one, refused + (not may)
+        if one and not may:
+            missed.append((heads, m, n, d, dv, nnz))
+    assert not missed and preferred > 1000 and refused > 1000
 
 
 def test_shapes_the_kernel_does_not_take():
