@@ -467,8 +467,18 @@ std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Te
   return {out0, out1};
 }
 
+// Whether 1 or 2 tokens take the CSR arrays (spmm_skinny.cu) although there is a dense copy, whose product is estimated at
+// `copy_us`.  A call has 7.8 us of host time either way and 0.4 more with the copy (its checks), so that a kernel below that is as
+// good as any.  The kernel takes 2.5 us and 1.05 ns a nonzero for one token, for two up to 4 us and 2.2 ns.  Measured (us a call with
+// the CSR arrays, with the copy): 1024 x 1024, half stored, 1 token 7.8, 8.2; 4096 x 2048 30 % 7.7, 8.1; 4096 x 4096 30 % 2 tokens
+// 19 (the kernel 15.8), 8.2.
+bool skinny_first(int64_t tokens, int64_t nnz, double copy_us) {
+  const double skinny_us = tokens == 1 ? 2.5 + 1.05e-6 * nnz : 4.0 + 2.2e-6 * nnz;
+  return skinny_us <= std::max(7.8, copy_us);
+}
+
 // SparseLinear without gradients: x [tokens, k] @ W_csr^T -> [tokens, m], W_csr [m, k].
-//   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu), where they are smaller than a dense copy
+//   1 or 2 tokens    CUDA cores, the CSR arrays read once (spmm_skinny.cu), without a dense copy or where it is no slower
 //   with `dense`     the layer's dense copy of W: for a handful of tokens linear_few.cu, else the dense GEMM
 //   up to 256        block decoder on tensor cores (spmm_tile.cu), unless ...
 //   otherwise        ... expanding W for the dense GEMM is estimated faster (many tokens)
@@ -494,11 +504,9 @@ std::optional<at::Tensor> sparse_linear(const at::Tensor& x, const at::Tensor& v
   const int64_t nnz = values.numel();
   const double gemm_us = std::min(m % 8 == 0 ? iex_gemm_f16_estimate_us(m, tokens, k, 0, 1) : 1e30,
                                   iex_gemm_f16_estimate_us(tokens, m, k, 0, 0));
-  // 2.5 us + 1.05 ns per nonzero for one token, 9 + 1.15 for two (a gather more for each); at three the
-  // decoder is as fast
   const double few_us = dense_weight.has_value() ? iex_linear_f16_few_estimate_us(tokens, k, m, settled) : 1e30;
-  const double skinny_us = tokens == 1 ? 2.5 + 1.05e-6 * nnz : 3.5 + 6e-6 * m / 11 + 1.15e-6 * nnz;
-  if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) && (!dense_weight.has_value() || skinny_us <= std::min(gemm_us, few_us))) {
+  if (tokens <= 2 && iex_spmm_f16_skinny_supported(k, tokens) &&
+      (!dense_weight.has_value() || skinny_first(tokens, nnz, std::min(gemm_us, few_us)))) {
     const int st = iex_spmm_f16_skinny(m, k, tokens, nnz, ro.data_ptr<int>(), ci.data_ptr(), index_bits(ci),
                                        values.data_ptr(), x.data_ptr(), 1, k, out.data_ptr(), 1, m, stream_of(x));
     if (st == 0) return out;
@@ -614,6 +622,7 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
   mod.def("spmm_half_way", [](int64_t m, int64_t k, int64_t n, int64_t nnz, int bits, bool eager) {
     return static_cast<int>(iex_torch::spmm_half_way(m, k, n, nnz, bits, iex_torch::kAuto, true, eager));
   });
+  mod.def("skinny_first", &iex_torch::skinny_first);
   mod.def("mylinear", &iex_torch::mylinear);
   mod.def("sparse_linear", &iex_torch::sparse_linear, pybind11::arg("x"), pybind11::arg("values"), pybind11::arg("row_offsets"),
           pybind11::arg("column_indices"), pybind11::arg("out_features"), pybind11::arg("in_features"),
