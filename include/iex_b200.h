@@ -279,6 +279,12 @@ IEX_API int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n, in
 IEX_API int iex_linear_pair_f16(int m0, int m1, int k, int n, const void* weight0, const void* weight1,
                                 const void* x, int x_tokens_major, void* out0, int tokens_major0, void* out1,
                                 int tokens_major1, void* stream);
+/* The same where weight0 is the dense copy of a CSR matrix: outputs of it that come out NaN are summed again from the
+ * stored positions alone. */
+IEX_API int iex_linear_pair_f16_csr(int m0, int m1, int k, int n, const void* weight0, const int32_t* row_offsets,
+                                    const void* column_indices, int index_bits, const void* values, const void* weight1,
+                                    const void* x, int x_tokens_major, void* out0, int tokens_major0, void* out1,
+                                    int tokens_major1, void* stream);
 
 /* CSR SpMM with 1 to 16 dense columns (decoding steps; one launch up to 8, else two), fp16, fp32 accumulation, CUDA cores:
  * out(r, t) = sum_p values[p] * x(col[p], t).  The strides are in elements, so x and out may be

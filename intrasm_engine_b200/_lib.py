@@ -92,6 +92,9 @@ SIGNATURES = {
     # out_sparse sparse_tokens_major out_dense dense_tokens_major stream
     "iex_spmm_linear_f16_tile": (c_int, [c_int, c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr,
                                          c_int, c_ptr, c_ptr, c_int, c_ptr, c_int, c_ptr]),
+    # m0 m1 k n weight0 row_offsets cols index_bits values weight1 x x_tokens_major out0 tokens_major0 out1 tokens_major1 stream
+    "iex_linear_pair_f16_csr": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_int,
+                                        c_ptr, c_int, c_ptr]),
     # m0 m1 k n weight0 weight1 x x_tokens_major out0 tokens_major0 out1 tokens_major1 stream
     "iex_linear_pair_f16": (c_int, [c_int, c_int, c_int, c_int, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_int, c_ptr, c_int,
                                     c_ptr]),

@@ -77,7 +77,7 @@ struct TileParams {
   int x_slots, stages;
   int acc_cols, tmem_cols;
   int ahead;           // nonzeros of L2 prefetch distance
-  CsrTerms terms;      // of the sparse units
+  CsrTerms terms;      // of the sparse units, or of the first dense matrix where that is a CSR matrix's dense copy
   int* status;
 };
 
@@ -90,7 +90,7 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
       : "memory");
 }
 
-// This thread's outputs of a sparse unit, for token t_local and, if the bits say so, the one inst_m further: summed again
+// This thread's outputs of a unit whose matrix is a CSR one, for token t_local and, if the bits say so, the one inst_m further: summed again
 // (csr_terms.cuh) and stored over what is there.  Called with next to nothing live: the decoders have no registers to spare.
 __device__ __noinline__ void store_again(const TileParams& p, int row0, int rows, int first, int t_local, uint32_t blocks) {
   for (int mb = 0; mb < p.m_blocks; ++mb) {
@@ -479,6 +479,7 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __half* out = sparse ? p.s_out : p.d_out[which];
         const long long st_row = sparse ? p.s_row : p.d_row[which], st_tok = sparse ? p.s_tok : p.d_tok[which];
         const bool vec = st_row == 1 && (st_tok & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+        const bool stored = kSparse ? sparse : which == 0 && p.terms.row_offsets != nullptr;
         uint32_t again = 0;
         for (int mb = 0; mb < p.m_blocks; ++mb) {
           const int t = mb * p.inst_m + t_local;
@@ -487,7 +488,7 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             tmem_ld32(tmem + (static_cast<uint32_t>(q * 32) << 16) + mb * p.acc_cols + c, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             const int left = min(min(rows - c, 32), m_rows - row0 - c);  // what the unit has of these rows
-            if (sparse && lane_ok && t < p.n && any_nan(r, left)) again |= 1u << mb;
+            if (stored && lane_ok && t < p.n && any_nan(r, left)) again |= 1u << mb;
             if (sparse && p.bias != nullptr) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
@@ -655,10 +656,12 @@ struct DenseArg {
 int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets, const void* cols, int index_bits,
                 const void* values, const float* bias, void* out_sparse, int sparse_tokens_major,
                 const DenseArg (&dense)[2], const void* x, int x_tokens_major, void* stream) {
+  const bool copy = m_sparse == 0 && row_offsets != nullptr;  // the CSR arrays are those of dense[0]
   const int m_dense = dense[0].m + dense[1].m;
   if (m_sparse < 0 || dense[0].m < 0 || dense[1].m < 0 || k < 0 || n < 0 || nnz < 0) return IEX_ERR_BAD_ARG;
   if (index_bits != 16 && index_bits != 32) return IEX_ERR_BAD_ARG;
   if ((m_sparse == 0 && m_dense == 0) || n == 0) return IEX_OK;
+  if (copy && dense[0].m > 0 && (!cols || !values)) return IEX_ERR_BAD_ARG;
   if (!x || (m_sparse > 0 && (!row_offsets || !out_sparse || (nnz > 0 && (!cols || !values))))) return IEX_ERR_BAD_ARG;
   for (const auto& d : dense)
     if (d.m > 0 && (!d.weight || !d.out)) return IEX_ERR_BAD_ARG;
@@ -666,8 +669,8 @@ int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets,
   if (index_bits == 16 && k > 65024) return IEX_ERR_UNSUPPORTED;  // 0xffff marks padding in every block
   if (!aligned16(x) || (dense[0].m > 0 && !aligned16(dense[0].weight)) || (dense[1].m > 0 && !aligned16(dense[1].weight)))
     return IEX_ERR_UNSUPPORTED;
-  if ((reinterpret_cast<uintptr_t>(values) & 3u) != 0 ||
-      (reinterpret_cast<uintptr_t>(cols) & static_cast<uintptr_t>(index_bits / 4 - 1)) != 0)
+  if (m_sparse > 0 && ((reinterpret_cast<uintptr_t>(values) & 3u) != 0 ||
+                       (reinterpret_cast<uintptr_t>(cols) & static_cast<uintptr_t>(index_bits / 4 - 1)) != 0))
     return IEX_ERR_UNSUPPORTED;  // pairs of nonzeros are loaded together
   TileParams p{};
   p.inst_m = n <= 64 ? 64 : 128;
@@ -696,6 +699,12 @@ int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets,
     p.d_row[i] = dense[i].tokens_major ? 1 : n;
     p.d_tok[i] = dense[i].tokens_major ? dense[i].m : 1;
   }
+  if (copy) {  // where store_again finds its outputs
+    p.s_m = dense[0].m;
+    p.s_out = p.d_out[0];
+    p.s_row = p.d_row[0];
+    p.s_tok = p.d_tok[0];
+  }
   p.k = k;
   p.n = n;
   p.x_mn = x_tokens_major ? 0 : 1;
@@ -705,7 +714,7 @@ int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets,
   p.terms.dense = static_cast<const __half*>(x);
   p.terms.dense_c = p.x_mn ? n : 1;
   p.terms.dense_t = p.x_mn ? 1 : k;
-  p.terms.rows = m_sparse;
+  p.terms.rows = copy ? dense[0].m : m_sparse;
   p.terms.columns = n;
   p.terms.index_bits = index_bits;
   p.kb = pl.kb;
@@ -757,10 +766,18 @@ extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n,
                               sparse_tokens_major, dense, x, x_tokens_major, stream);
 }
 
+extern "C" int iex_linear_pair_f16_csr(int m0, int m1, int k, int n, const void* weight0, const int32_t* row_offsets,
+                                       const void* column_indices, int index_bits, const void* values, const void* weight1,
+                                       const void* x, int x_tokens_major, void* out0, int tokens_major0, void* out1,
+                                       int tokens_major1, void* stream) {
+  const iex::tc::DenseArg dense[2] = {{m0, weight0, out0, tokens_major0}, {m1, weight1, out1, tokens_major1}};
+  return iex::tc::tile_launch(0, k, n, 0, row_offsets, column_indices, index_bits, values, nullptr, nullptr, 0, dense, x,
+                              x_tokens_major, stream);
+}
+
 extern "C" int iex_linear_pair_f16(int m0, int m1, int k, int n, const void* weight0, const void* weight1, const void* x,
                                    int x_tokens_major, void* out0, int tokens_major0, void* out1, int tokens_major1,
                                    void* stream) {
-  const iex::tc::DenseArg dense[2] = {{m0, weight0, out0, tokens_major0}, {m1, weight1, out1, tokens_major1}};
-  return iex::tc::tile_launch(0, k, n, 0, nullptr, nullptr, 16, nullptr, nullptr, nullptr, 0, dense, x, x_tokens_major,
-                              stream);
+  return iex_linear_pair_f16_csr(m0, m1, k, n, weight0, nullptr, nullptr, 16, nullptr, weight1, x, x_tokens_major, out0,
+                                 tokens_major0, out1, tokens_major1, stream);
 }

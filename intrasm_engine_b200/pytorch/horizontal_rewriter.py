@@ -315,7 +315,7 @@ class SparseDenseLayer(ModuleToReplay):
             if ops.native.plain(x, values, weight) and _fused_operands(x, values, self.column_indices, weight):
                 dense = self._dense.current(values, self.row_offsets, self.column_indices)
                 if dense is not None and dense.size(1) == x.size(0):
-                    return ops.native.linear_pair(x, dense, weight)
+                    return ops.native.linear_pair(x, dense, weight, (values, self.row_offsets, self.column_indices))
                 return ops.native.fused_spmm_linear_half(x, self.row_offsets, values, self.column_indices, self.m,
                                                          weight)
         args = (x, self.row_indices, values, self.row_offsets, self.column_indices, self.m,

@@ -453,17 +453,33 @@ class KeptCopy {
 };
 
 // The two branches of a sparse || dense layer with both weights dense: x [k, n] ->
-// (weight0 @ x [m0, n], (weight1 @ x)^T [n, m1]) in one launch.  weight0 is the layer's dense copy.
-std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Tensor& weight0, const at::Tensor& weight1) {
+// (weight0 @ x [m0, n], (weight1 @ x)^T [n, m1]) in one launch.  weight0 is the layer's dense copy of a CSR matrix, `stored`
+// (values, row_offsets, column_indices) or, for two dense matrices, nothing.
+std::tuple<at::Tensor, at::Tensor> linear_pair(const at::Tensor& x, const at::Tensor& weight0, const at::Tensor& weight1,
+                                               const std::vector<at::Tensor>& stored) {
   check_common({{"x", &x}, {"weight0", &weight0}, {"weight1", &weight1}});
+  TORCH_CHECK(stored.empty() || stored.size() == 3, "stored must be (values, row_offsets, column_indices)");
   const int64_t k = x.size(0), n = x.size(1), m0 = weight0.size(0), m1 = weight1.size(0);
   TORCH_CHECK(weight0.size(1) == k && weight1.size(1) == k, "weights must be [rows, k]");
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor out0 = empty(x, {m0, n}), out1 = empty(x, {n, m1});
   mark_stream(weight0);
-  check_status(iex_linear_pair_f16(m0, m1, k, n, weight0.data_ptr(), weight1.data_ptr(), x.data_ptr(), 0, out0.data_ptr(), 0,
-                                   out1.data_ptr(), 1, stream_of(x)),
-               "iex_linear_pair_f16");
+  const int* ro = nullptr;
+  const void *ci = nullptr, *values = nullptr;
+  int bits = 16;
+  if (!stored.empty()) {
+    check_common({{"values", &stored[0]}, {"row_offsets", &stored[1]}, {"column_indices", &stored[2]}});
+    TORCH_CHECK(stored[0].scalar_type() == at::kHalf && stored[0].device() == x.device(), "values must be float16 on x's device");
+    TORCH_CHECK(stored[1].scalar_type() == at::kInt && stored[1].numel() == m0 + 1, "row_offsets must be int32 with m + 1 entries");
+    TORCH_CHECK(stored[2].scalar_type() == at::kShort || stored[2].scalar_type() == at::kInt, "column_indices must be int16 or int32");
+    values = stored[0].data_ptr();
+    ro = stored[1].data_ptr<int>();
+    ci = stored[2].data_ptr();
+    bits = index_bits(stored[2]);
+  }
+  check_status(iex_linear_pair_f16_csr(m0, m1, k, n, weight0.data_ptr(), ro, ci, bits, values, weight1.data_ptr(), x.data_ptr(), 0,
+                                       out0.data_ptr(), 0, out1.data_ptr(), 1, stream_of(x)),
+               "iex_linear_pair_f16_csr");
   return {out0, out1};
 }
 
@@ -637,7 +653,8 @@ PYBIND11_MODULE(iex_torch_ext, mod) {
            pybind11::arg("column_indices"));
   mod.def("stream_capturing", [](const at::Tensor& t) { return iex_stream_is_capturing(iex_torch::stream_of(t)) != 0; });
   mod.def("plain", [](const at::Tensor& a, const at::Tensor& b, const at::Tensor& c) { return iex_torch::plain({&a, &b, &c}); });
-  mod.def("linear_pair", &iex_torch::linear_pair);
+  mod.def("linear_pair", &iex_torch::linear_pair, pybind11::arg("x"), pybind11::arg("weight0"), pybind11::arg("weight1"),
+          pybind11::arg("stored") = std::vector<at::Tensor>());
   mod.def("attention_plan", &iex_torch::attention_plan);
   mod.def("attention", &iex_torch::attention);
   mod.def("ffn_down", &iex_torch::ffn_down);

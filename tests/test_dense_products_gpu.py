@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from intrasm_engine_b200 import _lib, ops
+from intrasm_engine_b200.pytorch.horizontal_rewriter import SparseDenseLayer
 from intrasm_engine_b200.pytorch.utils import DenseCopy, dense_to_sparse_cuda
 
 pytestmark = pytest.mark.gpu
@@ -105,6 +106,39 @@ def test_linear_pair(m0, m1, k, n):
     o0, o1 = ops.native.linear_pair(_dev(x), _dev(w0), _dev(w1))
     np.testing.assert_array_equal(o0.cpu().numpy(), _exact(w0, x))
     np.testing.assert_array_equal(o1.cpu().numpy(), _exact(w1, x).T)
+
+
+@pytest.mark.parametrize("n", [64, 128, 256])
+@pytest.mark.parametrize("m0,m1,k,index", [(8, 40, 64, torch.int16), (203, 1000, 264, torch.int16), (2500, 37, 512, torch.int32)])
+@pytest.mark.parametrize("what", ["a column twice", "descending", "inputs that are not finite"])
+def test_sparse_dense_layer_multiplies_what_is_stored(m0, m1, k, n, index, what):
+    """The dense copy it keeps has marks for columns that a row stores twice, and zeros that the CSR matrix has not."""
+    a, w, x = _ints((m0, k), 1, density=0.6), _ints((m1, k), 2), _ints((k, n), 3, -1, 2)
+    values, ri, ro, ci = dense_to_sparse_cuda(_dev(a), index_dtype=index)
+    rows = np.repeat(np.arange(m0), np.diff(ro.cpu().numpy()))
+    cols = ci.cpu().numpy().astype(np.int64)
+    v = values.cpu().numpy().astype(np.float64)
+    if what == "a column twice":
+        again = np.flatnonzero((np.diff(rows) == 0) & (rows[1:] % 3 == 1))[::5] + 1
+        cols[again] = cols[again - 1]
+    elif what == "descending":
+        order = np.lexsort((-cols, rows))
+        cols, v = cols[order], v[order]
+    xs = x.astype(np.float64)
+    if what == "inputs that are not finite":
+        xs[3, 5], xs[k - 1, n - 1], xs[7, 0] = np.inf, np.nan, -np.inf
+    ref = np.zeros((m0, n))
+    with np.errstate(invalid="ignore"):
+        np.add.at(ref, rows, v[:, None] * xs[cols])
+        ref_d = (w.astype(np.float64) @ xs).T
+    values.copy_(torch.as_tensor(v).half())
+    ci.copy_(torch.as_tensor(cols).to(index))
+    layer = SparseDenseLayer(values, ri, ro, ci, m0, _dev(w))
+    assert layer._dense.current(layer.values, layer.row_offsets, layer.column_indices) is not None
+    out, dense = layer(torch.as_tensor(xs).half().to(DEV))
+    np.testing.assert_array_equal(out.cpu().numpy().astype(np.float64), ref)  # whole numbers below 2048
+    np.testing.assert_array_equal(dense.cpu().numpy().astype(np.float64), ref_d)
+    assert _lib.lib.iex_last_device_status(1) == 0
 
 
 @pytest.mark.parametrize("n", [1, 2, 3, 8, 16])
