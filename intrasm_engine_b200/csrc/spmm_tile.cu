@@ -479,7 +479,7 @@ spmm_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __half* out = sparse ? p.s_out : p.d_out[which];
         const long long st_row = sparse ? p.s_row : p.d_row[which], st_tok = sparse ? p.s_tok : p.d_tok[which];
         const bool vec = st_row == 1 && (st_tok & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-        const bool stored = kSparse ? sparse : which == 0 && p.terms.row_offsets != nullptr;
+        const bool stored = kSparse ? sparse : which == 0 && p.s_m > 0;
         uint32_t again = 0;
         for (int mb = 0; mb < p.m_blocks; ++mb) {
           const int t = mb * p.inst_m + t_local;
@@ -653,15 +653,15 @@ struct DenseArg {
   int tokens_major;
 };
 
-int tile_launch(int m_sparse, int k, int n, int nnz, const int32_t* row_offsets, const void* cols, int index_bits,
+// `copy`: the CSR arrays are those of dense[0], which is their dense copy, and not of a matrix that is decoded.
+int tile_launch(bool copy, int m_sparse, int k, int n, int nnz, const int32_t* row_offsets, const void* cols, int index_bits,
                 const void* values, const float* bias, void* out_sparse, int sparse_tokens_major,
                 const DenseArg (&dense)[2], const void* x, int x_tokens_major, void* stream) {
-  const bool copy = m_sparse == 0 && row_offsets != nullptr;  // the CSR arrays are those of dense[0]
   const int m_dense = dense[0].m + dense[1].m;
   if (m_sparse < 0 || dense[0].m < 0 || dense[1].m < 0 || k < 0 || n < 0 || nnz < 0) return IEX_ERR_BAD_ARG;
   if (index_bits != 16 && index_bits != 32) return IEX_ERR_BAD_ARG;
   if ((m_sparse == 0 && m_dense == 0) || n == 0) return IEX_OK;
-  if (copy && dense[0].m > 0 && (!cols || !values)) return IEX_ERR_BAD_ARG;
+  if (copy && dense[0].m > 0 && (!row_offsets || !cols || !values)) return IEX_ERR_BAD_ARG;
   if (!x || (m_sparse > 0 && (!row_offsets || !out_sparse || (nnz > 0 && (!cols || !values))))) return IEX_ERR_BAD_ARG;
   for (const auto& d : dense)
     if (d.m > 0 && (!d.weight || !d.out)) return IEX_ERR_BAD_ARG;
@@ -762,7 +762,7 @@ extern "C" int iex_spmm_linear_f16_tile(int m_sparse, int m_dense, int k, int n,
                                         void* out_sparse, int sparse_tokens_major, void* out_dense,
                                         int dense_tokens_major, void* stream) {
   const iex::tc::DenseArg dense[2] = {{m_dense, weight, out_dense, dense_tokens_major}, {0, nullptr, nullptr, 0}};
-  return iex::tc::tile_launch(m_sparse, k, n, nnz, row_offsets, column_indices, index_bits, values, bias, out_sparse,
+  return iex::tc::tile_launch(false, m_sparse, k, n, nnz, row_offsets, column_indices, index_bits, values, bias, out_sparse,
                               sparse_tokens_major, dense, x, x_tokens_major, stream);
 }
 
@@ -771,7 +771,7 @@ extern "C" int iex_linear_pair_f16_csr(int m0, int m1, int k, int n, const void*
                                        const void* x, int x_tokens_major, void* out0, int tokens_major0, void* out1,
                                        int tokens_major1, void* stream) {
   const iex::tc::DenseArg dense[2] = {{m0, weight0, out0, tokens_major0}, {m1, weight1, out1, tokens_major1}};
-  return iex::tc::tile_launch(0, k, n, 0, row_offsets, column_indices, index_bits, values, nullptr, nullptr, 0, dense, x,
+  return iex::tc::tile_launch(row_offsets != nullptr, 0, k, n, 0, row_offsets, column_indices, index_bits, values, nullptr, nullptr, 0, dense, x,
                               x_tokens_major, stream);
 }
 
