@@ -48,8 +48,8 @@
 // instead (cta_count).  The pieces of a band meet in a workspace and are added in order by whichever comes last.
 //
 // 24 heads x 4096 x 4096 at 5 %, d 64: 281 us back to back at the power limit (1590 MHz), about 245 on a cool chip (1965 MHz); with
-// TF32 planes 532 to 554 and 499; head by head over two streams 723 us.  About 2100 cycles a tile of 128 keys, of which the
-// pipe needs 1536.  6 heads x 1003 x 1003 at 10 %, d 80: 22.6 to 23.3 us, with TF32 planes
+// TF32 planes 532 to 554 and 499; head by head over two streams 723 us.  About 2260 cycles a tile of 128 keys, of which the
+// pipe needs 1536 (68 % active).  From one clock to the other cycles grow by a tenth: memory and the chain S - P - O count too.  6 heads x 1003 x 1003 at 10 %, d 80: 22.6 to 23.3 us, with TF32 planes
 // 30.7.  Without a look at the columns of q and k 280 and 22.5.
 // Which masks are faster one way or the other: iex_attention_f32_prefers below.
 //

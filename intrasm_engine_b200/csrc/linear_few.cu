@@ -9,7 +9,8 @@
 // a lane's fragment of w is the 16 consecutive bytes it has loaded, of x likewise: nothing goes through shared memory, and x
 // is read once by a block, which holds all its rows' sums.  The warps' sums meet in shared memory, in order, at the end.
 //
-// Measured (us; weight settled, not settled / gemm_tc.cu) for 1, 8 and 16 tokens: 11008 x 4096 16.4 17.9 / 19.7, 16.8 18.2 / 19.8,
+// Measured (us, one layer called again and again; with three layers in turn 15.3 where the first figure is 16.4; weight settled, not
+// settled / gemm_tc.cu) for 1, 8 and 16 tokens: 11008 x 4096 16.4 17.9 / 19.7, 16.8 18.2 / 19.8,
 // 18.8 20.5 / 19.9; 4096 x 4096 8.0 9.3 / 10.0, 8.8 10.0 / 10.0, 9.7 10.7 / 10.0; 8192 x 1024 4.8 5.9 / 6.5, 5.3 6.3 / 6.5,
 // 6.5 7.5 / 6.5; 2048 x 2048 4.3 / 5.7.  32 tokens would need more registers than there are (28.7 / 20.4).  Fused multiply-adds with x
 // in shared memory instead: as fast for one token and long rows, 29.6 for 8 tokens at 11008 x 4096.
