@@ -113,6 +113,7 @@ struct AttnParams {
   uint32_t* odd_rows;            // [bands of all heads][4]: rows of a quarter that have to be summed by position
   const uint4* tile_info;        // [heads][tiles]: Tile
   const uint32_t* odd_keys;      // [heads][np / 32]: keys that do not suit the planes
+  uint4* key_words;              // [heads][np]: big_and_there of the keys of tiles whose info says so
   int* status;
 };
 
@@ -165,7 +166,8 @@ __device__ __forceinline__ void split2(float2 x, uint32_t& hi, uint32_t& lo) {
 }
 
 // A key tile as its prepare block describes it: v's rows times k's scales are stored times 2^-exponent; whether keys of it do not
-// suit the planes; the most small elements that a key's row of k has; the columns that are large in all of them.  Of the first 64
+// suit the planes; the most small elements that a key's row of k has; the columns that are large in all of them; whether its keys'
+// words are in key_words.  Of the first 64
 // columns c is bit (c % 32) / 2 of word c / 32, odd ones 16 further.  A key whose row is zero counts for neither.
 struct Tile {
   uint32_t word, large0, large1;
@@ -175,9 +177,9 @@ struct Tile {
     large0 = x.y;
     large1 = x.z;
   }
-  static __device__ __forceinline__ uint4 pack(int exponent, bool odd, int small, uint32_t large0, uint32_t large1) {
+  static __device__ __forceinline__ uint4 pack(int exponent, bool odd, int small, uint32_t large0, uint32_t large1, bool described) {
     return make_uint4(static_cast<uint32_t>(exponent + kExpBias) | (odd ? 1u << 13 : 0u) | static_cast<uint32_t>(small) << 14, large0,
-                      large1, 0u);
+                      large1, described ? 1u : 0u);
   }
   static __device__ __forceinline__ int exponent(uint32_t word) { return static_cast<int>(word & 0x1fffu) - kExpBias; }
   __device__ __forceinline__ bool odd() const { return (word & (1u << 13)) != 0; }
@@ -461,7 +463,15 @@ __device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint
       const int keys = min(kAgainKeys, p.n - key0);
       __syncthreads();
       if (at.pairs != 0 && (held != at.head || keys != p.n)) {
-        row_words(p.k + (static_cast<size_t>(at.head) * p.n + key0) * p.d, keys, p.d, -149, words);
+        const uint4* info = p.tile_info + at.head * p.tiles;
+        bool described = true;
+        for (int t = threadIdx.x; t < p.tiles; t += kThreads) described = described && __ldcg(&info[t].w) != 0u;
+        if (__syncthreads_and(described)) {
+          const uint4* from = p.key_words + static_cast<size_t>(at.head) * p.np + key0;
+          for (int i = threadIdx.x; i < keys; i += kThreads) words[i] = __ldcg(from + i);
+        } else {
+          row_words(p.k + (static_cast<size_t>(at.head) * p.n + key0) * p.d, keys, p.d, -149, words);
+        }
         held = at.head;
       }
       __syncthreads();
@@ -1115,6 +1125,18 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
   for (int s = 4; s >= 1; s >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, s);
   if ((lane16 & 7) == 0) atomicAnd(&all_large[lane16 >> 3], word);
   __syncthreads();
+  // A tile that no row of q is safe with: whoever looks at pairs finds its keys' words here, since a block that makes a head's own takes
+  // 100 us for it (24 heads x 4096, d 64, q and k after a ReLU: 523 -> 437 us at 5 %, 500 -> 385 at 1 %).
+  const bool described = unsafe(__popc(all_large[0]) + __popc(all_large[1]), most_small);
+  if (described) {
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const Scale scale_k(kRowExp - ek[i]);
+      const uint4 words = big_and_there(scaled4(scale_k, xk[i][0]), kVecs > 1 ? scaled4(scale_k, xk[i][kVecs - 1]) : zero);
+      const int key = key0 + group + kSide * i;
+      if (lane16 == 0 && key < p.n) p.key_words[static_cast<size_t>(head) * p.np + key] = words;
+    }
+  }
   if (threadIdx.x == 0) {
     uint32_t any = 0;
 #pragma unroll
@@ -1122,7 +1144,7 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
       odd_keys[(head * p.np + key0) / 32 + i] = odd_words[i];
       any |= odd_words[i];
     }
-    tile_info[head * p.tiles + blockIdx.x] = Tile::pack(exponent, any != 0, most_small, all_large[0], all_large[1]);
+    tile_info[head * p.tiles + blockIdx.x] = Tile::pack(exponent, any != 0, most_small, all_large[0], all_large[1], described);
   }
 }
 
@@ -1271,14 +1293,15 @@ namespace {
 
 // Sections of the workspace, each on 256 bytes.
 struct Sections {
-  size_t k, v, tile_info, odd_keys, partials, counters, quarters, odd_rows, end;
+  size_t k, v, tile_info, odd_keys, key_words, partials, counters, quarters, odd_rows, end;
   Sections(int heads, int m, const Shape& s) {
     const size_t rows = 2ull * heads * s.np, tiles = 16ull * heads * s.tiles, items = static_cast<size_t>(heads) * ((m + 127) / 128);
     k = 0;
     v = k + round256(rows * s.dk * 2);
     tile_info = v + round256(rows * s.dvk * 2);
     odd_keys = tile_info + round256(tiles);
-    partials = odd_keys + round256(rows / 16);
+    key_words = odd_keys + round256(rows / 16);
+    partials = key_words + round256(rows * 8);
     counters = partials + round256(2ull * kNumSMs * 128 * s.dvp * 4);
     quarters = counters + round256(16 * kGroups * items);
     odd_rows = quarters + round256(4 * items);
@@ -1329,6 +1352,7 @@ extern "C" int iex_attention_f32(int heads, int m, int n, int d, int dv, const v
   p.cols = column_indices;
   p.tile_info = tile_info;
   p.odd_keys = odd_keys;
+  p.key_words = reinterpret_cast<uint4*>(ws + at.key_words);
   p.status = status_word();
   const int sms = std::min(sm_count(), kNumSMs), ctas = cta_count(heads * p.bands, p.tiles, sms);
   CUtensorMap mq, mk, mv;

@@ -173,6 +173,21 @@ def test_small_elements_with_more_keys_than_are_held_at_a_time(d):
     assert bool(torch.isinf(out[1, ~rows, 3]).all())
 
 
+@pytest.mark.parametrize("d", [36, 64, 96])
+@pytest.mark.parametrize("m,n,density", [(140, 17000, 0.002), (300, 200, 0.1), (1300, 450, 0.1)])
+def test_features_that_are_off_in_half_of_the_rows(d, m, n, density):
+    """No tile of keys has a column that is large in all of them: their words come with the planes."""
+    mask, chain, q, k, v, _g = _case(2, m, n, d, d, 17, density=density)
+    q, k = q.relu(), k.relu()
+    _check(_run(chain, q, k, v), mask, q, k, v, 4e-6)
+    k[0, ::7] = 0
+    k[0, 3::7] *= torch.arange(d, device=DEV) % 9 == 0  # little in common
+    q[0, 5::11] *= torch.arange(d, device=DEV) % 9 != 0
+    q[0, 5::11, 9] = 1e-7  # all that they have
+    k[1, n // 2:] = k[1, n // 2:].clamp(min=0.5)  # tiles that are not described beside ones that are
+    _check(_run(chain, q, k, v), mask, q, k, v, 4e-6)
+
+
 def test_small_elements_in_a_band_cut_between_blocks():
     mask, chain, q, k, v, _g = _case(1, 130, 3000, 64, 64, 14, density=0.01)
     q[0, 40, 9] *= 2.0 ** 40
