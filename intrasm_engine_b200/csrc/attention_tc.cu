@@ -88,9 +88,9 @@ constexpr int kTileExp = 14;   // a tile of v to [2^14, 2^15)
 // Scaled elements of v from here on keep all but 2^-20 of themselves: a tail is 2^-36 off at most where it has no more
 // exponents, and as much is lost with the product of the tails.
 constexpr float kSmallV = 1.f / (1 << 15);
-// Elements of q and k, scaled: a large one; a big one, where one in both rows is enough; and from where on fp16 holds them with
+// Elements of q and k, scaled: a large one; a big one, where one in both rows is enough (sum_again); and from where on fp16 holds them with
 // all their bits.
-constexpr float kLarge = 1.f / 32, kBig = 1.f, kSmall = 1.f / (1 << 14);
+constexpr float kLarge = 1.f / 32, kBig = 1.f / 2, kSmall = 1.f / (1 << 14);
 constexpr int kExpBias = 4096;
 
 struct AttnParams {
@@ -280,36 +280,32 @@ __device__ __forceinline__ void row_words(const float* x, int rows, int d, int l
   }
 }
 
-// Whether a row of q and a key have terms in common and these are next to nothing: below 2^-14 or, with small elements, below
+// By a warp: whether a row of q and a key have terms in common and these are next to nothing: below 2^-14 or, with small elements, below
 // what makes 2^-31 for each of them 2^-21.
 __device__ __noinline__ bool next_to_nothing(const float4* q, const float4* k, int quads) {
-  uint32_t top_q = 0, top_k = 0;
-#pragma unroll 8
-  for (int c = 0; c < quads; ++c) {
-    const float4 a = __ldg(q + c), b = __ldg(k + c);
-    top_q = finite_max(finite_max(finite_max(finite_max(top_q, a.x), a.y), a.z), a.w);
-    top_k = finite_max(finite_max(finite_max(finite_max(top_k, b.x), b.y), b.z), b.w);
-  }
+  const int lane = threadIdx.x & 31;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = lane < quads ? __ldg(q + lane) : zero, b = lane < quads ? __ldg(k + lane) : zero;
+  const uint32_t top_q = __reduce_max_sync(0xffffffffu, finite_max(finite_max(finite_max(finite_max(0u, a.x), a.y), a.z), a.w));
+  const uint32_t top_k = __reduce_max_sync(0xffffffffu, finite_max(finite_max(finite_max(finite_max(0u, b.x), b.y), b.z), b.w));
   if (top_q == 0u || top_k == 0u) return false;
   const Scale scale_q(kRowExp - max(exponent_of(top_q), -126)), scale_k(kRowExp - exponent_of(top_k));
   float terms = 0.f;
   int small = 0;
   bool any = false;
-  auto add = [&](float a, float b) {
-    const float x = fabsf(scale_q(a)), y = fabsf(scale_k(b));
-    any = any || (a != 0.f && b != 0.f);
-    small += (a != 0.f && x < kSmall ? 1 : 0) + (b != 0.f && y < kSmall ? 1 : 0);
+  auto add = [&](float u, float v) {
+    const float x = fabsf(scale_q(u)), y = fabsf(scale_k(v));
+    any = any || (u != 0.f && v != 0.f);
+    small += (u != 0.f && x < kSmall ? 1 : 0) + (v != 0.f && y < kSmall ? 1 : 0);
     terms = fmaf(x, y, terms);
   };
-#pragma unroll 8
-  for (int c = 0; c < quads; ++c) {
-    const float4 a = __ldg(q + c), b = __ldg(k + c);
-    add(a.x, b.x);
-    add(a.y, b.y);
-    add(a.z, b.z);
-    add(a.w, b.w);
-  }
-  return any && terms < fmaxf(kSmall, small * (1.f / 1024));
+  add(a.x, b.x);
+  add(a.y, b.y);
+  add(a.z, b.z);
+  add(a.w, b.w);
+#pragma unroll
+  for (int w = 16; w >= 1; w >>= 1) terms += __shfl_xor_sync(0xffffffffu, terms, w);
+  small = __reduce_add_sync(0xffffffffu, small);
+  return __any_sync(0xffffffffu, any) && terms < fmaxf(kSmall, small * (1.f / 1024));
 }
 
 // Quarters of a band that have rows and tiles [0, tiles) whose factor is out of range, from the exponent bytes of the rows (a warp).
@@ -431,11 +427,12 @@ __device__ __forceinline__ void row_by_position(const AttnParams& p, int head, i
 // After everything else, by all threads: rows of this block's bands, tiles [r0, r1), that have to be summed by position.  `cut`:
 // the quarters (4 bits each) of its first and its last band that it has to see to where these are cut between blocks; all others,
 // and whether there may be such rows in them, are in p.quarters.  Which rows that are is found from the words of q's and k's rows: a
-// column that is big on both sides makes a pair's terms 1 or more, and nothing in common makes them zero; other pairs are looked
-// at.  `words`: shared memory for kAgainWords of them.
-// 24 heads x 4096, d 64 on a cool chip (245 us otherwise): one key in every head 389 us, q and k after a ReLU, where all pairs are
-// looked at, 519, one column of q and k 2^8 times the others 1080, and one of q 2^24, one of k 2^-24 times the others, where
-// every row is summed, 2970.  At the end and not in the loop over the tiles: any code there that looks at the scores, even if it is
+// column that is big on both sides makes a pair's terms 1 / 4 or more, enough for 256 small elements, and nothing in common makes them
+// zero; other pairs are looked at.  `words`: shared memory for kAgainWords of them.
+// 24 heads x 4096, d 64 on a cool chip (245 us otherwise): one key in every head 415 us, q and k after a ReLU, where all pairs are
+// looked at, 440, one column of q and k 2^4 times the others 465, 2^8 times 610, and one of q 2^24, one of k 2^-24 times the others,
+// where every row is summed, 2200.  (A lane for a pair and big only from 1 on: 710, 1080 and 2980 for the last three.)  At the end
+// and not in the loop over the tiles: any code there that looks at the scores, even if it is
 // passed over, makes the loop 3 to 12 % longer, and so does one that keeps such a row's number.
 constexpr int kAgainKeys = 8192, kAgainWords = kAgainKeys + 128;
 __device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint32_t cut, uint4* words) {
@@ -479,7 +476,6 @@ __device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint
       // a warp takes every third run of 32 words of mask of a quarter
       const bool pairs = at.pairs >> part & 1u;
       const int row = part * 32 + lane;
-      const float4* q = reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(at.head) * p.m + min(at.row0 + row, p.m - 1)) * p.d);
       const uint4 mine = row < at.rows && pairs ? q_words[row] : make_uint4(0u, 0u, 0u, 0u);
       const uint32_t* mask = p.bits + static_cast<size_t>(key0 / 32) * p.mp + at.row0 + row;
       const uint32_t* odd_keys = p.odd_keys + (static_cast<size_t>(at.head) * p.np + key0) / 32;
@@ -500,13 +496,23 @@ __device__ __noinline__ void sum_again(const AttnParams& p, int r0, int r1, uint
           const uint32_t odd = __shfl_sync(0xffffffffu, odd_here, i);  // by all lanes, found or not
           found = found || (bits & odd) != 0;
           if (!pairs) continue;
-          for (; bits != 0 && !found; bits &= bits - 1) {
-            const int key = 32 * (w0 + i * (kThreads / 128)) + __ffs(bits) - 1;
-            const uint4 theirs = words[key];
-            if (((mine.x & theirs.x) | (mine.y & theirs.y)) == 0 && ((mine.z & theirs.z) | (mine.w & theirs.w)) != 0)
-              found = next_to_nothing(q, reinterpret_cast<const float4*>(p.k + (static_cast<size_t>(at.head) * p.n + key0 + key) * p.d), p.d / 4);
+          for (;;) {  // pairs that the words leave open, one of each row at a time, are looked at by the warp
+            int key = -1;
+            for (; bits != 0 && !found && key < 0; bits &= bits - 1) {
+              const int next = 32 * (w0 + i * (kThreads / 128)) + __ffs(bits) - 1;
+              const uint4 theirs = words[next];
+              if (((mine.x & theirs.x) | (mine.y & theirs.y)) == 0 && ((mine.z & theirs.z) | (mine.w & theirs.w)) != 0) key = next;
+            }
+            uint32_t open = __ballot_sync(0xffffffffu, key >= 0);
+            if (open == 0) break;
+            for (; open != 0; open &= open - 1) {
+              const int whose = __ffs(open) - 1, which = __shfl_sync(0xffffffffu, key, whose);
+              const float* q = p.q + (static_cast<size_t>(at.head) * p.m + at.row0 + part * 32 + whose) * p.d;
+              const float* k = p.k + (static_cast<size_t>(at.head) * p.n + key0 + which) * p.d;
+              const bool next_to = next_to_nothing(reinterpret_cast<const float4*>(q), reinterpret_cast<const float4*>(k), p.d / 4);
+              found = found || (lane == whose && next_to);
+            }
           }
-          __syncwarp();
         }
       }
       const uint32_t odd = __ballot_sync(0xffffffffu, found && row < at.rows);
@@ -1127,7 +1133,8 @@ attention_prepare_kernel(const AttnParams p, int dk, int dvk, __half* __restrict
   __syncthreads();
   // A tile that no row of q is safe with: whoever looks at pairs finds its keys' words here, since a block that makes a head's own takes
   // 100 us for it (24 heads x 4096, d 64, q and k after a ReLU: 523 -> 437 us at 5 %, 500 -> 385 at 1 %).
-  const bool described = unsafe(__popc(all_large[0]) + __popc(all_large[1]), most_small);
+  const int large_columns = __popc(all_large[0]) + __popc(all_large[1]);
+  const bool described = 4 * large_columns < min(p.d, 64) || 8 * most_small > large_columns;
   if (described) {
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
